@@ -630,45 +630,6 @@ __global__ void invert_diag_blocks(const T* __restrict__ A, long long ld, int N,
   }
 }
 
-// One block step of a triangular solve with M = A (trans = 0) or A^T:
-//   x = Dinv * b[r0 : r0+n]  (Dinv^T when dinv_t),  y[r0 : r0+n] = x,
-//   b[row] -= sum_k M(row, r0+k) x_k  for row in [q0, q1).
-// Rows of the block itself are only read, so every CTA sees the same x.
-template <class T>
-__global__ void trsv_step(const T* __restrict__ A, long long ld, double* __restrict__ b, double* __restrict__ y, int r0,
-                          int n, const double* __restrict__ Dinv, int dinv_t, int q0, int q1, int trans) {
-  __shared__ double bb[TB];
-  __shared__ double xx[TB];
-  for (int i = threadIdx.x; i < TB; i += blockDim.x) bb[i] = (i < n) ? b[r0 + i] : 0.0;
-  __syncthreads();
-  for (int i = threadIdx.x; i < n; i += blockDim.x) {
-    double s = 0.0;
-    for (int k = 0; k < n; k++) s += (dinv_t ? Dinv[k * TB + i] : Dinv[i * TB + k]) * bb[k];
-    xx[i] = s;
-  }
-  __syncthreads();
-  if (blockIdx.x == 0)
-    for (int i = threadIdx.x; i < n; i += blockDim.x) y[r0 + i] = xx[i];
-  if (q1 <= q0) return;
-  if (!trans) {
-    int row = q0 + blockIdx.x * blockDim.x + threadIdx.x;
-    if (row >= q1) return;
-    double s = 0.0;
-    for (int k = 0; k < n; k++) s += static_cast<double>(A[static_cast<long long>(r0 + k) * ld + row]) * xx[k];
-    b[row] -= s;
-  } else {
-    int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    int lane = threadIdx.x & 31;
-    int row = q0 + warp;
-    if (row >= q1) return;
-    const T* colp = A + static_cast<long long>(row) * ld + r0;
-    double s = 0.0;
-    for (int k = lane; k < n; k += 32) s += static_cast<double>(colp[k]) * xx[k];
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    if (lane == 0) b[row] -= s;
-  }
-}
-
 // y = alpha A x + beta b (FP64, column-major).  The columns are split into
 // chunks so that the grid covers the GPU: gemv_partial writes one partial
 // sum per (chunk, row), gemv_finish adds them in chunk order (deterministic).
@@ -807,10 +768,6 @@ double now_ms() {
 }  // namespace
 
 DenseLU::DenseLU(Context* ctx) : ctx_(ctx) {
-  if (const char* e = std::getenv("KD_SWEEP")) {
-    const std::string v(e);
-    sweep_kind = v == "barrier" ? 0 : v == "pull" ? 1 : 2;
-  }
   if (cublasCreate(&blas_) != CUBLAS_STATUS_SUCCESS) throw KdError(KD_ERR_CUDA, "cublasCreate failed");
   cublasSetStream(blas_, ctx_->stream());
   cuda_check(cudaMalloc(&d_info_, sizeof(int)), "cudaMalloc(info)");
@@ -1089,50 +1046,6 @@ __device__ void block_argmax(V& v, int& i, int& tag, V* rv, int* ri, int* rt) {
   __syncthreads();
 }
 
-// A whole triangular sweep with the factors in one cooperative launch: per
-// 64-row block k (in order for L, reversed for U), every CTA forms
-// x_k = Dinv_k b[block] (Dinv_k row-major; warp w owns rows 8w..8w+7, lanes
-// along the row, all loads issued before the reductions), CTA 0 stores x_k
-// in y, and the rows below (L) or above (U) get b[row] -= A(row, block) x_k;
-// then one grid barrier.  Rows go by 64-row tiles, tile t to CTA t % grid:
-// within a CTA, warp w takes rows 32 (w >> 2) .. + 31 of the tile and the
-// 16 block columns 16 (w & 3) .. + 15 (16 independent loads per thread), and
-// the four column quarters are added in shared memory.  A row of b is only
-// ever written by its tile's CTA; block rows written by other CTAs are read
-// past L1.
-constexpr int SW_TILE = 64;
-constexpr int SW_MAXT = 24;  // tiles a CTA keeps in shared memory during a sweep
-
-// Geometry of one block step of a sweep.
-struct SweepStep {
-  int k, r0, n, q0, q1, first, t1;
-};
-
-__device__ __forceinline__ SweepStep sweep_step(int step, int nblk, int N, int lower, int ntiles) {
-  SweepStep s;
-  s.k = lower ? step : nblk - 1 - step;
-  s.r0 = s.k * TB;
-  s.n = (N - s.r0 < TB) ? N - s.r0 : TB;
-  s.q0 = lower ? s.r0 + s.n : 0;
-  s.q1 = lower ? N : s.r0;
-  const int t0 = s.q0 / SW_TILE;
-  s.t1 = (s.q1 + SW_TILE - 1) / SW_TILE;
-  if (s.t1 > ntiles) s.t1 = ntiles;
-  s.first = t0 - (t0 % static_cast<int>(gridDim.x)) + static_cast<int>(blockIdx.x);
-  if (s.first < t0) s.first += gridDim.x;
-  return s;
-}
-
-// The values this thread needs from Dinv_k and from the factor's block
-// columns for its first two tiles: loaded one step ahead, before the grid
-// barrier, since they do not depend on b.
-template <class T>
-struct SweepPrefetch {
-  double lo[8], hi[8];  // Dinv_k entries (FP64 factors)
-  float2 dlo[8], dhi[8];  // Dinv_k entries as (hi, lo) FP32 pairs (FP32 factors)
-  T va[16], vb[16];
-};
-
 // Double-float arithmetic (a value is an unevaluated sum hi + lo of two
 // floats): Dekker's product with a fused multiply-add and Knuth's two-sum,
 // about 48 significant bits on the FP32 pipe.
@@ -1165,187 +1078,12 @@ __global__ void split_df_kernel(const double* __restrict__ d, float2* __restrict
   }
 }
 
-template <class T>
-__device__ __forceinline__ void sweep_prefetch(const T* __restrict__ A, long long ld, const double* __restrict__ Dinv,
-                                               const float2* __restrict__ Dinv2, const SweepStep& s,
-                                               SweepPrefetch<T>& pf) {
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int quarter = warp & 3, half = warp >> 2;
-  const size_t dofs = static_cast<size_t>(s.k) * TB * TB + static_cast<size_t>(warp) * 8 * TB;
-  if constexpr (std::is_same<T, float>::value) {
-    const float2* D = Dinv2 + dofs;
-#pragma unroll
-    for (int q = 0; q < 8; q++) {
-      pf.dlo[q] = D[q * TB + lane];
-      pf.dhi[q] = D[q * TB + lane + 32];
-    }
-  } else {
-    const double* D = Dinv + dofs;
-#pragma unroll
-    for (int q = 0; q < 8; q++) {
-      pf.lo[q] = D[q * TB + lane];
-      pf.hi[q] = D[q * TB + lane + 32];
-    }
-  }
-  const int c0 = quarter * 16;
-  {
-    const int t = s.first;
-    const int row = t * SW_TILE + half * 32 + lane;
-    const bool act = t < s.t1 && row >= s.q0 && row < s.q1;
-    const T* a = A + static_cast<long long>(s.r0 + c0) * ld + row;
-#pragma unroll
-    for (int j = 0; j < 16; j++) pf.va[j] = (act && c0 + j < s.n) ? a[static_cast<long long>(j) * ld] : T(0);
-  }
-  {
-    const int t = s.first + gridDim.x;
-    const int row = t * SW_TILE + half * 32 + lane;
-    const bool act = t < s.t1 && row >= s.q0 && row < s.q1;
-    const T* a = A + static_cast<long long>(s.r0 + c0) * ld + row;
-#pragma unroll
-    for (int j = 0; j < 16; j++) pf.vb[j] = (act && c0 + j < s.n) ? a[static_cast<long long>(j) * ld] : T(0);
-  }
-}
-
-// A whole triangular sweep with the factors in one cooperative launch: per
-// 64-row block k (in order for L, reversed for U), every CTA forms
-// x_k = Dinv_k b[block] in FP64 (Dinv_k row-major; warp w owns rows
-// 8w..8w+7, lanes along the row), CTA 0 stores x_k in y, and the rows below
-// (L) or above (U) get b[row] -= A(row, block) x_k; then one grid barrier.
-// Rows go by 64-row tiles, tile t to CTA t % grid: within a CTA, warp w
-// takes rows 32 (w >> 2) .. + 31 of the tile and the 16 block columns
-// 16 (w & 3) .. + 15, and the four column quarters are added in shared
-// memory.  Dinv_k and the block columns of the first two tiles are loaded
-// a step ahead (before the barrier).  A row of b is only ever written by
-// its tile's CTA; block rows written by other CTAs are read past L1.
-template <class T>
-__global__ void __launch_bounds__(256) trsv_sweep(const T* __restrict__ A, long long ld, int N, double* b,
-                                                  double* __restrict__ y, const double* __restrict__ Dinv,
-                                                  const float2* __restrict__ Dinv2, int lower, unsigned* bar,
-                                                  int* err, unsigned long long wait_ns, unsigned stall) {
-  // x_k = Dinv_k b in FP64, or in double-float with FP32 factors (an
-  // explicit inverse amplifies rounding by its condition number, so a plain
-  // FP32 product would cost refinement iterations); the row updates in the
-  // factors' precision T
-  __shared__ double bb[TB];
-  __shared__ float bh[TB], bl[TB];
-  __shared__ double xx[TB];
-  __shared__ T xt[TB];
-  __shared__ T part[4][SW_TILE];
-  // The right-hand side of the rows this CTA updates (its tiles t with
-  // t = blockIdx.x mod gridDim.x), kept in shared memory for the whole
-  // sweep; a tile goes back to global memory when it is the next block.
-  __shared__ double bown[SW_MAXT][SW_TILE];
-  __shared__ int s_ok;
-  const int nblk = (N + TB - 1) / TB;
-  const int ntiles = (N + SW_TILE - 1) / SW_TILE;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int quarter = warp & 3, half = warp >> 2;
-  const bool own = ntiles <= SW_MAXT * static_cast<int>(gridDim.x);
-  if (own && tid < SW_TILE)
-    for (int j = 0, t = blockIdx.x; t < ntiles; j++, t += gridDim.x) {
-      const int r = t * SW_TILE + tid;
-      bown[j][tid] = (r < N) ? b[r] : 0.0;
-    }
-  SweepPrefetch<T> pf;
-  sweep_prefetch(A, ld, Dinv, Dinv2, sweep_step(0, nblk, N, lower, ntiles), pf);
-  for (int step = 0; step < nblk; step++) {
-    const SweepStep s = sweep_step(step, nblk, N, lower, ntiles);
-    if (tid < TB) {
-      const double v = (tid < s.n) ? __ldcg(b + s.r0 + tid) : 0.0;
-      bb[tid] = v;
-      const float h = static_cast<float>(v);
-      bh[tid] = h;
-      bl[tid] = static_cast<float>(v - static_cast<double>(h));
-    }
-    __syncthreads();
-    if constexpr (std::is_same<T, float>::value) {
-      const float b0h = bh[lane], b0l = bl[lane], b1h = bh[lane + 32], b1l = bl[lane + 32];
-#pragma unroll
-      for (int q = 0; q < 8; q++) {
-        DF p = df_add(df_mul(pf.dlo[q].x, pf.dlo[q].y, b0h, b0l), df_mul(pf.dhi[q].x, pf.dhi[q].y, b1h, b1l));
-        for (int o = 16; o > 0; o >>= 1) {
-          DF r;
-          r.h = __shfl_xor_sync(0xffffffffu, p.h, o);
-          r.l = __shfl_xor_sync(0xffffffffu, p.l, o);
-          p = df_add(p, r);
-        }
-        if (lane == 0) {
-          const double x = static_cast<double>(p.h) + static_cast<double>(p.l);
-          xx[warp * 8 + q] = x;
-          xt[warp * 8 + q] = static_cast<T>(x);
-        }
-      }
-    } else {
-      const double b0 = bb[lane], b1 = bb[lane + 32];
-#pragma unroll
-      for (int q = 0; q < 8; q++) {
-        double p = pf.lo[q] * b0 + pf.hi[q] * b1;
-        for (int o = 16; o > 0; o >>= 1) p += __shfl_xor_sync(0xffffffffu, p, o);
-        if (lane == 0) {
-          xx[warp * 8 + q] = p;
-          xt[warp * 8 + q] = static_cast<T>(p);
-        }
-      }
-    }
-    __syncthreads();
-    if (blockIdx.x == 0 && tid < s.n) y[s.r0 + tid] = xx[tid];
-    const int c0 = quarter * 16;
-    int tix = 0;
-    for (int t = s.first; t < s.t1; t += gridDim.x, tix++) {
-      const int row = t * SW_TILE + half * 32 + lane;
-      T acc = T(0);
-      if (tix == 0) {
-#pragma unroll
-        for (int j = 0; j < 16; j++) acc = fma(pf.va[j], xt[c0 + j], acc);
-      } else if (tix == 1) {
-#pragma unroll
-        for (int j = 0; j < 16; j++) acc = fma(pf.vb[j], xt[c0 + j], acc);
-      } else if (row >= s.q0 && row < s.q1) {
-        const T* a = A + static_cast<long long>(s.r0 + c0) * ld + row;
-        T v[16];
-#pragma unroll
-        for (int j = 0; j < 16; j++) v[j] = (c0 + j < s.n) ? a[static_cast<long long>(j) * ld] : T(0);
-#pragma unroll
-        for (int j = 0; j < 16; j++) acc = fma(v[j], xt[c0 + j], acc);
-      }
-      part[quarter][half * 32 + lane] = acc;
-      __syncthreads();
-      if (tid < SW_TILE) {
-        const int r = t * SW_TILE + tid;
-        if (r >= s.q0 && r < s.q1) {
-          const double sub = static_cast<double>((part[0][tid] + part[1][tid]) + (part[2][tid] + part[3][tid]));
-          if (own) {
-            const int j = (t - static_cast<int>(blockIdx.x)) / static_cast<int>(gridDim.x);
-            const double v = bown[j][tid] - sub;
-            bown[j][tid] = v;
-            // the next block in sweep order reads its rows from global memory
-            if (t == (lower ? s.k + 1 : s.k - 1)) b[r] = v;
-          } else {
-            b[r] = __ldcg(b + r) - sub;
-          }
-        }
-      }
-      __syncthreads();
-    }
-    if (step + 1 < nblk) sweep_prefetch(A, ld, Dinv, Dinv2, sweep_step(step + 1, nblk, N, lower, ntiles), pf);
-    if (!grid_barrier(bar, gridDim.x * static_cast<unsigned>(step + 1) + stall, err, &s_ok, wait_ns)) return;
-  }
-}
-
-// ---- triangular sweeps that pull finished blocks (no grid barrier) --------
+// ---- triangular sweeps -----------------------------------------------------
 // Block k of the solution, x_k = Dinv_k (b_k - sum_i T_ki x_i) over the
-// blocks i before k in sweep order (T = L forward, U backward).  CTA c owns
-// the blocks at sweep positions c, c + G, ... (G = gridDim.x, every CTA
-// resident: cooperative launch).  A CTA accumulates the products of its
-// block's rows with every finished x_i as soon as that block is done, so
-// only the last product and the Dinv_k product remain on the critical path
-// once x_{k-1} appears.  Finished blocks are announced through one progress
-// counter (release max by the producer, acquire loads by the consumers),
-// the number of sweep positions whose x is in y.  Thread (warp w, lane):
-// row h*32 + lane of the block (h = w >> 2), columns 16 q .. 16 q + 15
-// (q = w & 3) of each contributing block; products in the factors'
-// precision T, 16 at a time, summed in FP64.  Every wait is bounded by
-// wait_ns: on timeout the CTA sets *err and leaves.
+// 64-row blocks i before k in sweep order.  Finished blocks are announced
+// through one progress counter (release max by the producer, acquire loads
+// by the consumers), the number of sweep positions whose x is in y.  Every
+// wait is bounded by wait_ns: on timeout the CTA sets *err and leaves.
 __device__ __forceinline__ unsigned ld_acquire_u32(const unsigned* p) {
   unsigned v;
   asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
@@ -1366,136 +1104,37 @@ __device__ __forceinline__ unsigned wait_progress(const unsigned* progress, unsi
   }
 }
 
-template <class T>
-__global__ void __launch_bounds__(256) trsv_pull(const T* __restrict__ A, long long ld, int N,
-                                                 const double* __restrict__ b, double* __restrict__ y,
-                                                 const double* __restrict__ Dinv, const float2* __restrict__ Dinv2,
-                                                 int lower, unsigned* progress, int* err,
-                                                 unsigned long long wait_ns, unsigned stall) {
-  __shared__ double part[4][TB];
-  __shared__ float vh[TB], vl[TB];
-  __shared__ double vd[TB];
-  __shared__ int s_abort;
-  const int nblk = (N + TB - 1) / TB;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int q = warp & 3, h = warp >> 2;
-  const int rr = h * 32 + lane;  // row within the block
-  const int c0 = q * 16;
-  if (tid == 0) s_abort = 0;
-  __syncthreads();
-  unsigned avail = 0;  // sweep positions known finished
-  for (int p = blockIdx.x; p < nblk; p += gridDim.x) {
-    const int k = lower ? p : nblk - 1 - p;
-    const int r0 = k * TB;
-    const int n = (N - r0 < TB) ? N - r0 : TB;
-    const int row = r0 + rr;
-    // this warp's 8 rows of Dinv_k, loaded before any wait
-    float2 dlo[8], dhi[8];
-    double lo[8], hi[8];
-    const size_t dofs = static_cast<size_t>(k) * TB * TB + static_cast<size_t>(warp) * 8 * TB;
-    if constexpr (std::is_same<T, float>::value) {
-#pragma unroll
-      for (int j = 0; j < 8; j++) {
-        dlo[j] = Dinv2[dofs + j * TB + lane];
-        dhi[j] = Dinv2[dofs + j * TB + lane + 32];
-      }
-    } else {
-#pragma unroll
-      for (int j = 0; j < 8; j++) {
-        lo[j] = Dinv[dofs + j * TB + lane];
-        hi[j] = Dinv[dofs + j * TB + lane + 32];
-      }
-    }
-    double acc = 0.0;
-    bool ok = true;
-    for (int pi = 0; pi < p; pi++) {
-      const int i = lower ? pi : nblk - 1 - pi;
-      const int cb = i * TB + c0;  // first column of this thread's quarter
-      T a[16];
-#pragma unroll
-      for (int j = 0; j < 16; j++)
-        a[j] = (row < N && cb + j < N) ? A[static_cast<long long>(cb + j) * ld + row] : T(0);
-      if (static_cast<unsigned>(pi) >= avail) {
-        const unsigned v = wait_progress(progress, static_cast<unsigned>(pi) + 1 + stall, wait_ns);
-        if (v == 0) {
-          ok = false;
-          break;
-        }
-        avail = v - stall;  // positions known finished
-      }
-      T sum = T(0);
-#pragma unroll
-      for (int j = 0; j < 16; j++) {
-        const double xj = (cb + j < N) ? __ldcg(y + cb + j) : 0.0;
-        sum = fma(a[j], static_cast<T>(xj), sum);
-      }
-      acc += static_cast<double>(sum);
-    }
-    if (!ok) s_abort = 1;
-    part[q][rr] = acc;
-    __syncthreads();
-    if (s_abort) {
-      if (tid == 0) atomicExch(err, 1);
-      return;
-    }
-    if (tid < TB) {
-      const double v = (tid < n) ? b[r0 + tid] - ((part[0][tid] + part[1][tid]) + (part[2][tid] + part[3][tid]))
-                                 : 0.0;
-      vd[tid] = v;
-      const float hv = static_cast<float>(v);
-      vh[tid] = hv;
-      vl[tid] = static_cast<float>(v - static_cast<double>(hv));
-    }
-    __syncthreads();
-    // x_k = Dinv_k v: warp w computes rows 8 w .. 8 w + 7
-    if constexpr (std::is_same<T, float>::value) {
-      const float b0h = vh[lane], b0l = vl[lane], b1h = vh[lane + 32], b1l = vl[lane + 32];
-#pragma unroll
-      for (int j = 0; j < 8; j++) {
-        DF pr = df_add(df_mul(dlo[j].x, dlo[j].y, b0h, b0l), df_mul(dhi[j].x, dhi[j].y, b1h, b1l));
-        for (int o = 16; o > 0; o >>= 1) {
-          DF r;
-          r.h = __shfl_xor_sync(0xffffffffu, pr.h, o);
-          r.l = __shfl_xor_sync(0xffffffffu, pr.l, o);
-          pr = df_add(pr, r);
-        }
-        const int xr = warp * 8 + j;
-        if (lane == 0 && xr < n) y[r0 + xr] = static_cast<double>(pr.h) + static_cast<double>(pr.l);
-      }
-    } else {
-      const double b0 = vd[lane], b1 = vd[lane + 32];
-#pragma unroll
-      for (int j = 0; j < 8; j++) {
-        double pr = lo[j] * b0 + hi[j] * b1;
-        for (int o = 16; o > 0; o >>= 1) pr += __shfl_xor_sync(0xffffffffu, pr, o);
-        const int xr = warp * 8 + j;
-        if (lane == 0 && xr < n) y[r0 + xr] = pr;
-      }
-    }
-    __syncthreads();
-    if (tid == 0) {
-      __threadfence();
-      asm volatile("red.release.gpu.global.max.u32 [%0], %1;" ::"l"(progress), "r"(static_cast<unsigned>(p) + 1)
-                   : "memory");
-    }
-  }
-}
-
-// The same sweep with CH_R consecutive blocks per CTA: CTA c owns sweep
-// positions c R .. c R + R - 1.  While earlier CTAs work it accumulates, for
-// all its blocks at once, the products with every finished x (phase A, one
-// progress wait per finished block).  Its own blocks then chain inside the
-// CTA (phase B): x_p from the accumulated rows and Dinv, published, and its
-// products with the CTA's later blocks from the internal L blocks, which
-// were staged in shared memory before phase A.  Only ceil(nblk / R)
-// hand-offs between CTAs remain on the critical path.
+// A whole sweep in one cooperative launch, CH_R consecutive blocks per group
+// and one group at a time per CTA: CTA c owns the groups c, c + grid, ..., group g the sweep
+// positions g R .. g R + R - 1.  While earlier groups are worked on it
+// accumulates, for all the group's blocks at once, the products with every
+// finished x (phase A, one progress wait per finished block).  The group's
+// own blocks then chain inside the CTA (phase B): x_p from the accumulated
+// rows and Dinv, published, and its products with the group's later blocks
+// from the internal L blocks, which were staged in shared memory before
+// phase A.  Thread (warp w, lane) works on row h*32 + lane of each block
+// (h = w >> 2) and columns 16 q .. 16 q + 15 (q = w & 3).  Only
+// ceil(nblk / R) hand-offs between CTAs remain on the
+// critical path.  A group waits for lower groups only, and every CTA is
+// resident, so the lowest unfinished group can always go on.
+//
+// Bound: the chain of dependent blocks (about 1.8 us each), not the factor's
+// bytes.  Matrices of more than R * 64 rows per SM (29,184 on 152 SMs) give
+// a CTA several groups: while the other CTAs' groups chain (456 blocks,
+// about 0.8 ms) it reads its next group's factor rows (22 MB in all SMs per
+// block column), so the chain stays the bound there too.
+// TRANS sweeps solve with the transposed factor: the tile of output block p
+// and finished block pi is the stored block (pi, p), whose columns are the
+// output rows, so a thread reads 16 consecutive entries of one column
+// (64 contiguous bytes with FP32 factors).
 constexpr int CH_R = 3;
 constexpr int CH_DST = TB + 1;  // row stride of the staged Dinv blocks (8-byte entries: conflict-free row reads)
+constexpr int CH_LST = TB + 1;  // column stride of the staged internal blocks (transposed staging without conflicts)
 // dynamic shared memory: the internal L blocks, then Dinv of the own blocks
 // (8 bytes an entry: a (hi, lo) float pair or a double)
 template <class T>
 constexpr size_t chain_smem() {
-  return static_cast<size_t>(CH_R * (CH_R - 1) / 2) * TB * TB * sizeof(T) +
+  return static_cast<size_t>(CH_R * (CH_R - 1) / 2) * TB * CH_LST * sizeof(T) +
          static_cast<size_t>(CH_R) * TB * CH_DST * 8;
 }
 
@@ -1505,7 +1144,7 @@ constexpr size_t chain_smem() {
 // GPU FP64 adds and FP64 <-> FP32 conversions run at the FP64 rate, a few
 // per clock per SM: one conversion per product would cost more than the
 // products.)
-template <class T>
+template <class T, bool TRANS>
 __global__ void __launch_bounds__(256) trsv_chain(const T* __restrict__ A, long long ld, int N,
                                                   const double* __restrict__ b, double* __restrict__ y,
                                                   float* __restrict__ yf, const double* __restrict__ Dinv,
@@ -1513,9 +1152,9 @@ __global__ void __launch_bounds__(256) trsv_chain(const T* __restrict__ A, long 
                                                   int* err, unsigned long long wait_ns, unsigned stall) {
   constexpr bool kF = std::is_same<T, float>::value;
   extern __shared__ __align__(16) unsigned char ch_raw[];
-  T* Lin = reinterpret_cast<T*>(ch_raw);  // internal blocks (r2, r1), r1 < r2: column-major 64 x 64
+  T* Lin = reinterpret_cast<T*>(ch_raw);  // internal blocks (r2, r1), r1 < r2: column-major, stride CH_LST
   // Dinv of the own blocks, row-major 64 x 64 each with row stride CH_DST
-  unsigned char* dsm = ch_raw + static_cast<size_t>(CH_R * (CH_R - 1) / 2) * TB * TB * sizeof(T);
+  unsigned char* dsm = ch_raw + static_cast<size_t>(CH_R * (CH_R - 1) / 2) * TB * CH_LST * sizeof(T);
   float2* D2s = reinterpret_cast<float2*>(dsm);
   double* Dds = reinterpret_cast<double*>(dsm);
   __shared__ double bsm[CH_R][TB];
@@ -1531,11 +1170,16 @@ __global__ void __launch_bounds__(256) trsv_chain(const T* __restrict__ A, long 
   const int q = warp & 3, h = warp >> 2;
   const int rr = h * 32 + lane;
   const int c0 = q * 16;
-  const int p0 = blockIdx.x * CH_R;
-  const int np = (nblk - p0 < CH_R) ? nblk - p0 : CH_R;
   auto blk = [&](int pos) { return lower ? pos : nblk - 1 - pos; };
   auto tri = [](int r2, int r1) { return r2 * (r2 - 1) / 2 + r1; };  // index of block (r2, r1), r1 < r2
   if (tid == 0) s_abort = 0;
+  unsigned avail = 0;
+  // 16-byte vector loads of x only from an aligned y (callers pass offset
+  // vectors, e.g. a work vector at an odd offset N)
+  const bool y_aligned = (reinterpret_cast<unsigned long long>(y) & 15ull) == 0;
+  const bool yf_aligned = kF && (reinterpret_cast<unsigned long long>(yf) & 15ull) == 0;
+  for (int p0 = blockIdx.x * CH_R; p0 < nblk; p0 += gridDim.x * CH_R) {
+  const int np = (nblk - p0 < CH_R) ? nblk - p0 : CH_R;
   // Stage what the own blocks need besides the x of earlier blocks: the
   // internal L blocks (rows of position p0 + r2, columns of p0 + r1), the
   // Dinv blocks and the right-hand side, 16 independent loads in flight
@@ -1543,23 +1187,27 @@ __global__ void __launch_bounds__(256) trsv_chain(const T* __restrict__ A, long 
   for (int r2 = 1; r2 < np; r2++)
     for (int r1 = 0; r1 < r2; r1++) {
       const int kr = blk(p0 + r2), kc = blk(p0 + r1);
-      T* dst = Lin + static_cast<size_t>(tri(r2, r1)) * TB * TB;
+      T* dst = Lin + static_cast<size_t>(tri(r2, r1)) * TB * CH_LST;
       for (int e0 = 0; e0 < TB * TB; e0 += 16 * 256) {
         T v[16];
 #pragma unroll
         for (int u = 0; u < 16; u++) {
           const int e = e0 + u * 256 + tid;
-          const int row = kr * TB + e % TB, col = kc * TB + e / TB;
+          const int row = (TRANS ? kc : kr) * TB + e % TB, col = (TRANS ? kr : kc) * TB + e / TB;
           v[u] = (row < N && col < N) ? A[static_cast<long long>(col) * ld + row] : T(0);
         }
 #pragma unroll
-        for (int u = 0; u < 16; u++) dst[e0 + u * 256 + tid] = v[u];  // dst[j * TB + i], e = j * TB + i
+        for (int u = 0; u < 16; u++) {  // entry (i, j) of the block at dst[j * CH_LST + i]
+          const int e = e0 + u * 256 + tid;
+          dst[TRANS ? (e % TB) * CH_LST + e / TB : (e / TB) * CH_LST + e % TB] = v[u];
+        }
       }
     }
   for (int r = 0; r < np; r++) {
     const size_t src = static_cast<size_t>(blk(p0 + r)) * TB * TB;
     for (int e0 = 0; e0 < TB * TB; e0 += 16 * 256) {
       // entry e = row * TB + col of the block goes to row * CH_DST + col
+      // (TRANS: the transposed inverse, to col * CH_DST + row)
       if constexpr (std::is_same<T, float>::value) {
         float2 v[16];
 #pragma unroll
@@ -1567,7 +1215,8 @@ __global__ void __launch_bounds__(256) trsv_chain(const T* __restrict__ A, long 
 #pragma unroll
         for (int u = 0; u < 16; u++) {
           const int e = e0 + u * 256 + tid;
-          D2s[static_cast<size_t>(r) * TB * CH_DST + (e / TB) * CH_DST + e % TB] = v[u];
+          D2s[static_cast<size_t>(r) * TB * CH_DST + (TRANS ? (e % TB) * CH_DST + e / TB : (e / TB) * CH_DST + e % TB)] =
+              v[u];
         }
       } else {
         double v[16];
@@ -1576,7 +1225,8 @@ __global__ void __launch_bounds__(256) trsv_chain(const T* __restrict__ A, long 
 #pragma unroll
         for (int u = 0; u < 16; u++) {
           const int e = e0 + u * 256 + tid;
-          Dds[static_cast<size_t>(r) * TB * CH_DST + (e / TB) * CH_DST + e % TB] = v[u];
+          Dds[static_cast<size_t>(r) * TB * CH_DST + (TRANS ? (e % TB) * CH_DST + e / TB : (e / TB) * CH_DST + e % TB)] =
+              v[u];
         }
       }
     }
@@ -1597,14 +1247,9 @@ __global__ void __launch_bounds__(256) trsv_chain(const T* __restrict__ A, long 
   // tile of the next block is loaded while the current one is used (it
   // does not depend on x), so the factor's HBM latency overlaps the
   // progress waits and the x loads.
-  unsigned avail = 0;
   bool ok = true;
   constexpr bool kAhead = sizeof(T) == 4;  // FP64 tiles would not fit twice in registers
   T a[CH_R][16], an[kAhead ? CH_R : 1][16];
-  // 16-byte vector loads of x only from an aligned y (callers pass offset
-  // vectors, e.g. a work vector at an odd offset N)
-  const bool y_aligned = (reinterpret_cast<unsigned long long>(y) & 15ull) == 0;
-  const bool yf_aligned = kF && (reinterpret_cast<unsigned long long>(yf) & 15ull) == 0;
   // rows of this thread in its CTA's blocks (N when past the matrix)
   int rowof[CH_R];
 #pragma unroll
@@ -1614,6 +1259,31 @@ __global__ void __launch_bounds__(256) trsv_chain(const T* __restrict__ A, long 
   }
   auto load_tile = [&](int pi, T(&dst)[CH_R][16]) {
     const int cb = blk(pi) * TB + c0;
+    if constexpr (TRANS) {
+      // entries cb .. cb + 15 of column rowof[r]; the FP32 copy's columns
+      // are 128-byte aligned and cb is a multiple of 16
+      const bool vec = kF && cb + 16 <= N && (ld & 3) == 0 && (reinterpret_cast<unsigned long long>(A) & 15ull) == 0;
+#pragma unroll
+      for (int r = 0; r < CH_R; r++) {
+        const T* q = A + static_cast<long long>(rowof[r] < N ? rowof[r] : 0) * ld + cb;
+        if (rowof[r] < N && vec) {
+          if constexpr (kF) {
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+              const float4 v = __ldg(reinterpret_cast<const float4*>(q) + j);
+              dst[r][4 * j] = v.x;
+              dst[r][4 * j + 1] = v.y;
+              dst[r][4 * j + 2] = v.z;
+              dst[r][4 * j + 3] = v.w;
+            }
+          }
+        } else {
+#pragma unroll
+          for (int j = 0; j < 16; j++) dst[r][j] = (rowof[r] < N && cb + j < N) ? q[j] : T(0);
+        }
+      }
+      return;
+    }
     const T* colp = A + static_cast<long long>(cb) * ld;
     if (cb + 16 <= N) {  // whole column quarter inside the matrix: no column predicates
 #pragma unroll
@@ -1790,18 +1460,20 @@ __global__ void __launch_bounds__(256) trsv_chain(const T* __restrict__ A, long 
 #pragma unroll
     for (int r2 = r + 1; r2 < CH_R; r2++) {
       if (r2 >= np) break;
-      const T* L = Lin + static_cast<size_t>(tri(r2, r)) * TB * TB;
+      const T* L = Lin + static_cast<size_t>(tri(r2, r)) * TB * CH_LST;
       T sum = T(0);
       if constexpr (kF) {
 #pragma unroll
-        for (int j = 0; j < 16; j++) sum = fmaf(L[(c0 + j) * TB + rr], xsf[c0 + j], sum);
+        for (int j = 0; j < 16; j++) sum = fmaf(L[(c0 + j) * CH_LST + rr], xsf[c0 + j], sum);
         accf[r2] = df_add(accf[r2], {sum, 0.f});
       } else {
 #pragma unroll
-        for (int j = 0; j < 16; j++) sum = fma(L[(c0 + j) * TB + rr], static_cast<T>(xs[c0 + j]), sum);
+        for (int j = 0; j < 16; j++) sum = fma(L[(c0 + j) * CH_LST + rr], static_cast<T>(xs[c0 + j]), sum);
         acc[r2] += static_cast<double>(sum);
       }
     }
+  }
+  __syncthreads();  // the staged blocks are read no more: the next group's may overwrite them
   }
 }
 
@@ -1822,7 +1494,7 @@ __global__ void __launch_bounds__(GP_THREADS) panel_grid_kernel(T* __restrict__ 
   for (int e = tid; e < jb * nr; e += bd) {
     int k = e / nr, r = e % nr;
     tile[k * per + r] = A[static_cast<long long>(j0 + k) * ld + r0 + r];
-  }
+    }
   __syncthreads();
   for (int jj = 0; jj < jb; jj++) {
     const int j = j0 + jj;
@@ -2912,102 +2584,57 @@ void DenseLU::tri_solve(const T* LU, long long ld, int N, double* b, int trans) 
   const size_t rnd = ((static_cast<size_t>(N) + 31) / 32) * 32;
   double* w1 = tri_work_;
   double* w2 = tri_work_ + rnd;  // 256-byte aligned second vector
-  const size_t bs = static_cast<size_t>(TB) * TB;
+  static std::once_flag ch_attr;
+  std::call_once(ch_attr, [] {
+    auto smem = [](auto* kernel, size_t bytes) {
+      cuda_check(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes)),
+                 "cudaFuncSetAttribute(chain sweep)");
+    };
+    smem(trsv_chain<float, false>, chain_smem<float>());
+    smem(trsv_chain<float, true>, chain_smem<float>());
+    smem(trsv_chain<double, false>, chain_smem<double>());
+    smem(trsv_chain<double, true>, chain_smem<double>());
+  });
+  // one group of CH_R blocks per CTA while the device holds that many CTAs;
+  // more groups go round the context's SMs.  The sums' order does not depend
+  // on the grid, so concurrent and serial solves agree bit for bit.
+  const int gch = (nblk + CH_R - 1) / CH_R;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(gch <= nsm_ ? gch : ctx_->sms(), 1, 1);
+  cfg.blockDim = dim3(256, 1, 1);
+  cfg.dynamicSmemBytes = chain_smem<T>();
+  cfg.stream = s;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeCooperative;
+  at[0].val.cooperative = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  cuda_check(cudaMemsetAsync(tri_bar_, 0, 2 * sizeof(unsigned), s), "memset sweep progress");
+  const float2* dl2 = std::is_same<T, float>::value ? dinv2_l_ : nullptr;
+  const float2* du2 = std::is_same<T, float>::value ? dinv2_u_ : nullptr;
+  // FP32 copies of the two sweeps' outputs (FP32 factors only)
+  float* yf1 = std::is_same<T, float>::value ? reinterpret_cast<float*>(tri_work_ + 2 * rnd) : nullptr;
+  float* yf2 = std::is_same<T, float>::value ? yf1 + rnd : nullptr;
+  const unsigned stall = ctx_->stall_waits ? 1u : 0u;
+  auto sweep = [&](auto* kernel, const double* in, double* out, float* outf, const double* dinv, const float2* dinv2,
+                   int lower, unsigned* progress, const char* what) {
+    ProfScope ps(ctx_, Context::PROF_LU_SOLVE, sweep_bytes);
+    cuda_check(cudaLaunchKernelEx(&cfg, kernel, LU, ld, N, in, out, outf, dinv, dinv2, lower, progress, panel_err_,
+                                  ctx_->grid_wait_ns, stall),
+               what);
+  };
   if (!trans) {
+    // L y = P b, then U x = y
     gather_perm<<<blocks(N, 256), 256, 0, s>>>(b, perm_, N, w1);
-    // L y = P b, then U x = y: one cooperative launch per sweep
-    int g = blocks(N, SW_TILE);
-    if (g > ctx_->sms()) g = ctx_->sms();
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(g, 1, 1);
-    cfg.blockDim = dim3(256, 1, 1);
-    cfg.stream = s;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeCooperative;
-    at[0].val.cooperative = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    cuda_check(cudaMemsetAsync(tri_bar_, 0, 2 * sizeof(unsigned), s), "memset sweep barriers");
-    const double* dl = dinv_l_;
-    const double* du = dinv_u_;
-    const float2* dl2 = std::is_same<T, float>::value ? dinv2_l_ : nullptr;
-    const float2* du2 = std::is_same<T, float>::value ? dinv2_u_ : nullptr;
-    const unsigned long long wait = ctx_->grid_wait_ns;
-    const unsigned stall = ctx_->stall_waits ? 1u : 0u;
-    const int gch = (nblk + CH_R - 1) / CH_R;
-    // the choice depends on the device only (not on a context's SM budget),
-    // so that concurrent and serial solves sum in the same order
-    if (sweep_kind == 2 && gch <= nsm_) {
-      static std::once_flag ch_attr;
-      std::call_once(ch_attr, [] {
-        cuda_check(cudaFuncSetAttribute(trsv_chain<float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        static_cast<int>(chain_smem<float>())),
-                   "cudaFuncSetAttribute(chain sweep)");
-        cuda_check(cudaFuncSetAttribute(trsv_chain<double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        static_cast<int>(chain_smem<double>())),
-                   "cudaFuncSetAttribute(chain sweep)");
-      });
-      cfg.gridDim = dim3(gch, 1, 1);
-      cfg.dynamicSmemBytes = chain_smem<T>();
-      const double* w1c = w1;
-      const double* w2c = w2;
-      // FP32 copies of the two sweeps' outputs (FP32 factors only)
-      float* yf1 = std::is_same<T, float>::value ? reinterpret_cast<float*>(tri_work_ + 2 * rnd) : nullptr;
-      float* yf2 = std::is_same<T, float>::value ? yf1 + rnd : nullptr;
-      {
-        ProfScope ps(ctx_, Context::PROF_LU_SOLVE, sweep_bytes);
-        cuda_check(cudaLaunchKernelEx(&cfg, trsv_chain<T>, LU, ld, N, w1c, w2, yf1, dl, dl2, 1, tri_bar_, panel_err_,
-                                      wait, stall),
-                   "forward sweep");
-      }
-      {
-        ProfScope ps(ctx_, Context::PROF_LU_SOLVE, sweep_bytes);
-        cuda_check(cudaLaunchKernelEx(&cfg, trsv_chain<T>, LU, ld, N, w2c, b, yf2, du, du2, 0, tri_bar_ + 1,
-                                      panel_err_, wait, stall),
-                   "backward sweep");
-      }
-    } else if (sweep_kind == 1) {
-      int gp = nblk < ctx_->sms() ? nblk : ctx_->sms();
-      cfg.gridDim = dim3(gp, 1, 1);
-      const double* w1c = w1;
-      const double* w2c = w2;
-      ProfScope ps(ctx_, Context::PROF_LU_SOLVE, 2 * sweep_bytes);
-      cuda_check(cudaLaunchKernelEx(&cfg, trsv_pull<T>, LU, ld, N, w1c, w2, dl, dl2, 1, tri_bar_, panel_err_, wait,
-                                    stall),
-                 "forward sweep");
-      cuda_check(cudaLaunchKernelEx(&cfg, trsv_pull<T>, LU, ld, N, w2c, b, du, du2, 0, tri_bar_ + 1, panel_err_,
-                                    wait, stall),
-                 "backward sweep");
-    } else {
-      ProfScope ps(ctx_, Context::PROF_LU_SOLVE, 2 * sweep_bytes);
-      cuda_check(cudaLaunchKernelEx(&cfg, trsv_sweep<T>, LU, ld, N, w1, w2, dl, dl2, 1, tri_bar_, panel_err_, wait,
-                                    stall),
-                 "forward sweep");
-      cuda_check(cudaLaunchKernelEx(&cfg, trsv_sweep<T>, LU, ld, N, w2, b, du, du2, 0, tri_bar_ + 1, panel_err_,
-                                    wait, stall),
-                 "backward sweep");
-    }
-    ctx_->launches += 3;
-    cuda_check(cudaGetLastError(), "triangular solve");
-    return;
+    sweep(trsv_chain<T, false>, w1, w2, yf1, dinv_l_, dl2, 1, tri_bar_, "forward sweep");
+    sweep(trsv_chain<T, false>, w2, b, yf2, dinv_u_, du2, 0, tri_bar_ + 1, "backward sweep");
   } else {
-    // A^T = U^T L^T P: U^T y = b (forward, lower), L^T z = y (backward), x = P^T z
-    ProfScope ps(ctx_, Context::PROF_LU_SOLVE, 2 * sweep_bytes);
-    for (int k = 0; k < nblk; k++) {
-      int r0 = k * TB, n = (N - r0 < TB) ? N - r0 : TB;
-      int q0 = r0 + n, q1 = N;
-      int g = q1 > q0 ? blocks(static_cast<long long>(q1 - q0) * 32, 256) : 1;
-      trsv_step<T><<<g, 256, 0, s>>>(LU, ld, b, w2, r0, n, dinv_u_ + k * bs, 1, q0, q1, 1);
-    }
-    for (int k = nblk - 1; k >= 0; k--) {
-      int r0 = k * TB, n = (N - r0 < TB) ? N - r0 : TB;
-      int q0 = 0, q1 = r0;
-      int g = q1 > q0 ? blocks(static_cast<long long>(q1 - q0) * 32, 256) : 1;
-      trsv_step<T><<<g, 256, 0, s>>>(LU, ld, w2, w1, r0, n, dinv_l_ + k * bs, 1, q0, q1, 1);
-    }
+    // A^T = U^T L^T P: U^T y = b (forward), L^T z = y (backward), x = P^T z
+    sweep(trsv_chain<T, true>, b, w2, yf1, dinv_u_, du2, 1, tri_bar_, "forward transposed sweep");
+    sweep(trsv_chain<T, true>, w2, w1, yf2, dinv_l_, dl2, 0, tri_bar_ + 1, "backward transposed sweep");
     scatter_perm<<<blocks(N, 256), 256, 0, s>>>(w1, perm_, N, b);
   }
-  ctx_->launches += 2 * nblk + 1;
+  ctx_->launches += 3;
   cuda_check(cudaGetLastError(), "triangular solve");
 }
 
