@@ -6,6 +6,7 @@
 // lines that do not have the symmetry the basis assumes.
 #include "kd_bases.hpp"
 
+#include <algorithm>
 #include <cmath>
 #include <stdexcept>
 
@@ -1103,6 +1104,52 @@ bool build_matrix(int op, int basis, int n_in, int n_out, Mat1d& out) {
   return true;
 }
 
+namespace {
+// Builds the folded form of a transform's matrix.  Mirrored entries agree to
+// rounding; their mean is kept.
+void fold_matrix(Mat1d& mat) {
+  const int op = mat.op, n_in = mat.n_in, n_out = mat.n_out;
+  const std::vector<double>& m = mat.m;
+  if (op != OP_COEF && op != OP_COEF_I) return;
+  const bool forward = op == OP_COEF;  // mirrored entries along a row, else along a column
+  const int n = forward ? n_in : n_out, nf = forward ? n_out : n_in;  // points, functions
+  if (n < 4) return;
+  double scale = 0.0;
+  for (double v : m) scale = std::max(scale, std::fabs(v));
+  auto at = [&](int i, int j) -> size_t {  // function i, point j
+    return forward ? static_cast<size_t>(i) * n_in + j : static_cast<size_t>(j) * n_in + i;
+  };
+  for (int periodic = 0; periodic < 2; periodic++) {
+    const int first = periodic, last = n - 1 + first, pairs = (n - first) / 2;
+    std::vector<double> f(m.size(), 0.0);
+    bool ok = true;
+    for (int i = 0; i < nf && ok; i++) {
+      bool even = true, odd = true;
+      for (int j = first; j <= last - first; j++) {
+        const double a = m[at(i, j)], b = m[at(i, last - j)];
+        even = even && std::fabs(a - b) <= 1e-13 * scale;
+        odd = odd && std::fabs(a + b) <= 1e-13 * scale;
+      }
+      for (int j = 0; j < first; j++) odd = odd && std::fabs(m[at(i, j)]) <= 1e-13 * scale;
+      ok = even || odd;
+      for (int q = 0; q < pairs && ok; q++) {
+        const int j = first + q;
+        const double a = m[at(i, j)], b = m[at(i, last - j)];
+        f[at(i, even ? j : last - j)] = 0.5 * (even ? a + b : a - b);  // slot of the sum or the difference
+      }
+      if (!even) continue;
+      // points that are their own mirror
+      for (int j = 0; j < first; j++) f[at(i, j)] = m[at(i, j)];
+      if ((n - first) % 2) f[at(i, first + pairs)] = m[at(i, first + pairs)];
+    }
+    if (!ok) continue;
+    mat.folded.swap(f);
+    mat.periodic = periodic != 0;
+    return;
+  }
+}
+}  // namespace
+
 int MatrixBank::get(int op, int basis, int n_in, int n_out) {
   auto key = std::make_tuple(op, basis, n_in, n_out);
   auto it = index_.find(key);
@@ -1113,7 +1160,9 @@ int MatrixBank::get(int op, int basis, int n_in, int n_out) {
   while (pool_.size() % 4) pool_.push_back(0.0);
   m.pool_offset = pool_.size();
   pool_.insert(pool_.end(), m.m.begin(), m.m.end());
+  fold_matrix(m);
   int idx = static_cast<int>(mats_.size());
+  by_offset_[static_cast<int>(m.pool_offset)] = idx;
   mats_.push_back(std::move(m));
   index_[key] = idx;
   version_++;

@@ -73,6 +73,23 @@ struct Mat1d {
   int op = 0, basis = 0, n_in = 0, n_out = 0, out_basis = -1;
   std::vector<double> m;  // row-major n_out x n_in
   size_t pool_offset = 0; // offset (in doubles) inside the device matrix pool
+  // The matrix between sums and differences of mirrored entries, for a
+  // transform whose basis functions are even or odd under a reflection of the
+  // collocation points: of the inputs of a forward, the outputs of an inverse
+  // transform; point j pairs with n-1-j, or with n-j on the periodic phi grid.
+  // Empty when the symmetry is not there.
+  std::vector<double> folded;
+  bool periodic = false;
+  bool column_zero(int c) const {
+    for (int r = 0; r < n_out; r++)
+      if (m[static_cast<size_t>(r) * n_in + c] != 0.0) return false;
+    return true;
+  }
+  bool row_zero(int r) const {
+    for (int c = 0; c < n_in; c++)
+      if (m[static_cast<size_t>(r) * n_in + c] != 0.0) return false;
+    return true;
+  }
 };
 
 // Builds the matrix of (op, basis) for a line of n_in inputs and n_out outputs.
@@ -90,12 +107,14 @@ class MatrixBank {
   // Returns the index of the matrix in the bank (creating it if needed), or -1.
   int get(int op, int basis, int n_in, int n_out);
   const Mat1d& at(int idx) const { return mats_[idx]; }
+  const Mat1d& at_offset(int off) const { return mats_[by_offset_.at(off)]; }  // by its place in the pool
   size_t pool_size() const { return pool_.size(); }
   const std::vector<double>& pool() const { return pool_; }
   size_t version() const { return version_; }
 
  private:
   std::map<std::tuple<int, int, int, int>, int> index_;
+  std::map<int, int> by_offset_;
   std::vector<Mat1d> mats_;
   std::vector<double> pool_;
   size_t version_ = 0;

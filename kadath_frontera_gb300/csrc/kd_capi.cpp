@@ -69,16 +69,19 @@ void transform_many(kd_ctx* ctx, int n, const kd_transform_desc* descs, bool inv
   kd::Context& c = *ctx->c;
   std::vector<kd::KdItem> items;
   std::vector<int> batches;
+  long long fields = 0;
+  for (int i = 0; i < n; i++) {
+    check_desc(descs[i]);
+    fields += descs[i].batch;
+  }
   for (int i = 0; i < n; i++) {
     const kd_transform_desc& d = descs[i];
-    check_desc(d);
     if (d.batch == 0) continue;
     kd::Base b = base_from_desc(d);
-    auto specs = inverse ? kd::coef_i_specs(c, b, d.nbr_points, d.nbr_coefs)
-                         : kd::coef_specs(c, b, d.nbr_points, d.nbr_coefs);
+    const kd::LinePlan& plan = kd::coef_plan(c, b, d.nbr_points, d.nbr_coefs, inverse, fields);
     const int* din = inverse ? d.nbr_coefs : d.nbr_points;
     const int* dout = inverse ? d.nbr_points : d.nbr_coefs;
-    items.push_back(kd::make_item(c, specs, d.in, d.out, din, prod3(din), prod3(dout), 1.0));
+    items.push_back(kd::make_item(plan, d.in, d.out, din, prod3(din), prod3(dout), 1.0));
     batches.push_back(d.batch);
   }
   c.run_items(items, batches);
@@ -214,9 +217,9 @@ int kd_ope_1d(kd_ctx* ctx, int op, int dim, const kd_transform_desc* desc, int* 
     kd::Context& c = *ctx->c;
     kd::Base b = base_from_desc(*desc);
     kd::Base bo = b;
-    auto spec = kd::ope_1d_spec(c, op, dim, b, desc->nbr_coefs, bo);
+    const kd::LinePlan& plan = kd::ope_1d_plan(c, op, dim, b, desc->nbr_coefs, bo);
     if (desc->batch > 0) {
-      auto it = kd::make_item(c, {spec}, desc->in, desc->out, desc->nbr_coefs, prod3(desc->nbr_coefs),
+      auto it = kd::make_item(plan, desc->in, desc->out, desc->nbr_coefs, prod3(desc->nbr_coefs),
                               prod3(desc->nbr_coefs), 1.0);
       c.run_items({it}, {desc->batch});
     }

@@ -1,5 +1,6 @@
 #include "kd_context.hpp"
 
+#include <algorithm>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -225,7 +226,7 @@ void Context::run_items(const std::vector<KdItem>& items, const std::vector<int>
     }
     const LpShape sh = line_shape(list, smem, dp);
     ProfScope ps(this, PROF_LINE_PASS, flops);
-    cuda_check(launch_line_passes(list, smem, dp, stream(), sh), "line_passes kernel");
+    cuda_check(launch_line_passes(list, dp, stream(), sh), "line_passes kernel");
     launches++;
   }
 }
@@ -398,14 +399,16 @@ void Context::set_autotune(const std::string& path, int mode) {
 
 LpShape Context::line_shape(const KdItemList& list, int smem_doubles, const double* pool) {
   const int nf = list.prefix[list.nitems];
-  if (tuner.mode == 0 || nf <= 0) return lp_default_shape(nf);
+  int stage = 0;
+  for (int i = 0; i < list.nitems; i++) stage = std::max(stage, list.items[i].stage);
+  if (tuner.mode == 0 || nf <= 0) return lp_default_shape(nf, stage);
   const std::string k = LineTuner::key(list, smem_doubles);
   auto it = tuner.table.find(k);
   if (it != tuner.table.end()) {
     tuner.hits++;
     return it->second.shape;
   }
-  if (tuner.mode < 2 || capturing || prof_on_) return lp_default_shape(nf);
+  if (tuner.mode < 2 || capturing || prof_on_) return lp_default_shape(nf, stage);
   // Time every candidate shape on copies of the launch whose outputs go to
   // a scratch buffer (the real outputs may alias the inputs).
   KdItemList probe = list;
@@ -438,13 +441,13 @@ LpShape Context::line_shape(const KdItemList& list, int smem_doubles, const doub
   cudaEvent_t e0, e1;
   cuda_check(cudaEventCreate(&e0), "cudaEventCreate");
   cuda_check(cudaEventCreate(&e1), "cudaEventCreate");
-  LpShape best = lp_default_shape(nf);
+  LpShape best = lp_default_shape(nf, stage);
   double best_us = 1e30;
   constexpr int reps = 5;
   for (const LpShape& c : cands) {
-    cuda_check(launch_line_passes(probe, smem_doubles, pool, s, c), "autotune warm-up");
+    cuda_check(launch_line_passes(probe, pool, s, c), "autotune warm-up");
     cuda_check(cudaEventRecord(e0, s), "cudaEventRecord");
-    for (int r = 0; r < reps; r++) cuda_check(launch_line_passes(probe, smem_doubles, pool, s, c), "autotune run");
+    for (int r = 0; r < reps; r++) cuda_check(launch_line_passes(probe, pool, s, c), "autotune run");
     cuda_check(cudaEventRecord(e1, s), "cudaEventRecord");
     cuda_check(cudaEventSynchronize(e1), "autotune sync");
     float ms = 0;

@@ -7,6 +7,7 @@
 #include <map>
 #include <stdexcept>
 #include <string>
+#include <unordered_map>
 #include <vector>
 
 #include "kadath_gb300.h"  // status codes
@@ -63,6 +64,16 @@ class LineTuner {
   static std::string key(const KdItemList& list, int smem_doubles);
 };
 
+// A compiled pass list: the passes with their device tables, and the output
+// basis table of a coefficient-space operator's dim.
+struct LinePlan {
+  int npass = 0;
+  int stage = 0, pitch = 0, nmats = 0;  // as in KdItem
+  const double* mats = nullptr;
+  KdPass pass[3] = {};
+  std::vector<int> out_base;
+};
+
 class Context {
  public:
   explicit Context(int device);
@@ -102,6 +113,16 @@ class Context {
   const int* table(const std::vector<int>& content);
   // Device copy of a double table, cached by content.
   const double* dtable(const std::vector<double>& content);
+
+  // Plans of the line passes by content (kd_spectral.cpp): a plan's tables
+  // live as long as the context.
+  const LinePlan* find_plan(const std::vector<int>& key) const {
+    auto it = plans_.find(key);
+    return it == plans_.end() ? nullptr : &it->second;
+  }
+  const LinePlan& add_plan(std::vector<int>&& key, LinePlan&& p) {
+    return plans_.emplace(std::move(key), std::move(p)).first->second;
+  }
 
   // Arena every DVal operation allocates from.  Normally the per-pass
   // scratch arena; redirect_scratch() points it at another arena (the
@@ -192,6 +213,14 @@ class Context {
   double* d_pool_ = nullptr;
   size_t pool_cap_ = 0, pool_uploaded_ = 0;
   std::map<std::vector<int>, int*> itables_;
+  struct KeyHash {  // FNV-1a over the ints
+    size_t operator()(const std::vector<int>& k) const {
+      unsigned long long h = 0xcbf29ce484222325ull;
+      for (int v : k) h = (h ^ static_cast<unsigned>(v)) * 0x100000001b3ull;
+      return static_cast<size_t>(h);
+    }
+  };
+  std::unordered_map<std::vector<int>, LinePlan, KeyHash> plans_;
   std::map<std::vector<double>, double*> dtables_;
   DeviceArena scratch_;
   DeviceArena* active_scratch_ = &scratch_;

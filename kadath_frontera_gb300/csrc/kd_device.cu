@@ -5,190 +5,240 @@
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
+#include <utility>
+
 #include "kd_device.hpp"
 
 namespace kd {
 
 namespace {
 
-__device__ __forceinline__ int line_matrix(const KdPass& p, int c1, int c2) {
-  if (p.dim == 0) return p.mat[c1 * p.mat_ld + c2];
-  if (p.dim == 1) return p.mat[c2];
-  return p.mat[0];
+// Line passes.  Bound: the FP64 pipe (measured 1.10 TFLOP/s on the whole GPU:
+// an SM starts one FP64 warp instruction in 16 cycles, so index arithmetic and
+// shared-memory loads hide behind it).  Hence every pass runs as few FP64 warp
+// instructions as it can: zero entries of a matrix row are skipped (derivatives
+// are triangular with a parity, multiplications and divisions by sin and x are
+// banded or triangular, two phi rows are zero), lines whose output is zero are
+// stored without products, and with many fields the transforms whose basis
+// functions are even or odd under reflection of the line work on sums and
+// differences of mirrored entries, half the products.
+//
+// A few fields are bound by latency instead (a field's three passes are a
+// chain of a few thousand cycles), so everything a thread needs is listed per
+// output by the host (KdOut: one 16-byte load instead of some 1,300 cycles of
+// dependent index arithmetic), the field and the matrices are staged by one
+// round of asynchronous copies, and mirrored entries are not combined there
+// (a fold and its barrier took 1,400 cycles, the products it saves 400).
+
+__device__ __forceinline__ void copy_async16(void* dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(static_cast<unsigned>(__cvta_generic_to_shared(dst))),
+               "l"(src)
+               : "memory");
+}
+__device__ __forceinline__ void copy_async8(void* dst, const void* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(static_cast<unsigned>(__cvta_generic_to_shared(dst))),
+               "l"(src)
+               : "memory");
+}
+__device__ __forceinline__ void copy_async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
+// The field into shared memory, rows (phi) at the item's pitch: an odd pitch
+// keeps the lines of a pass, whose lanes step over theta and r, off each
+// other's banks.
+__device__ __forceinline__ void load_field(const KdItem& it, const double* __restrict__ src, double* X) {
+  const int n = it.n0 * it.n1 * it.n2, skip = it.pitch - it.n2;
+  const float inv = __fdividef(1.0f, static_cast<float>(it.n2));
+  for (int e = threadIdx.x; e < n; e += blockDim.x)  // e / n2 is exact: e < 2^16, half a unit off any integer
+    copy_async8(X + e + skip * static_cast<int>((static_cast<float>(e) + 0.5f) * inv), src + e);
 }
 
-// One pass: X has dims (d0,d1,d2); Y has the pass dim replaced by n_out.
-// Outputs e = e0 + threadIdx.x + k * estride; store(e, value) writes them.
-template <class Store>
-__device__ void run_pass_part(const KdPass& p, const double* __restrict__ X, int d0, int d1, int d2,
-                              const double* __restrict__ pool, double scale, int e0, int estride, Store store) {
-  int o0 = d0, o1 = d1, o2 = d2;
-  if (p.dim == 0) o0 = p.n_out;
-  if (p.dim == 1) o1 = p.n_out;
-  if (p.dim == 2) o2 = p.n_out;
-  const int total = o0 * o1 * o2;
-  const int nin = p.n_in;
-  for (int e = e0 + threadIdx.x; e < total; e += estride) {
-    int c2 = e % o2;
-    int t = e / o2;
-    int c1 = t % o1;
-    int c0 = t / o1;
-    int row, off, base, stride;
-    if (p.dim == 0) {
-      row = c0;
-      off = line_matrix(p, c1, c2);
-      base = c1 * d2 + c2;
-      stride = d1 * d2;
-    } else if (p.dim == 1) {
-      row = c1;
-      off = line_matrix(p, c0, c2);
-      base = c0 * d1 * d2 + c2;
-      stride = d2;
-    } else {
-      row = c2;
-      off = line_matrix(p, c0, c1);
-      base = (c0 * d1 + c1) * d2;
-      stride = 1;
-    }
-    double acc = 0.0;
-    if (off >= 0) {
-      const double* M = pool + off + static_cast<long long>(row) * nin;
+__device__ __forceinline__ void load_mats(const KdItem& it, double* at) {
+  for (int e = 2 * threadIdx.x; e < it.nmats; e += 2 * blockDim.x) copy_async16(at + e, it.mats + e);
+}
+
+__device__ __forceinline__ KdOut load_out(const KdOut* o) {
+  const int4 v = __ldg(reinterpret_cast<const int4*>(o));
+  return {v.x, v.y, v.z, static_cast<unsigned>(v.w)};
+}
+
+__device__ __forceinline__ double line_dot(const KdOut& o, const double* __restrict__ mats,
+                                           const double* __restrict__ X) {
+  const int cnt = static_cast<int>(o.steps & 4095u), mstep = static_cast<int>((o.steps >> 12) & 3u),
+            xstep = static_cast<int>(o.steps >> 14);
+  const double* m = mats + o.m0;
+  const double* x = X + o.x0;
+  double acc = 0.0;
 #pragma unroll 4
-      for (int q = 0; q < nin; q++) acc = fma(__ldg(M + q), X[base + q * stride], acc);
-    }
-    store(e, acc * scale);
+  for (int q = 0; q < cnt; q++) {
+    acc = fma(*m, *x, acc);
+    m += mstep;
+    x += xstep;
+  }
+  return acc;
+}
+
+// (a, b) -> (a + b, a - b) on n pairs of elements of V.
+__device__ __forceinline__ void fold_pairs(const int* __restrict__ pairs, int n, double* V) {
+  for (int t = threadIdx.x; t < n; t += blockDim.x) {
+    const unsigned p = static_cast<unsigned>(__ldg(pairs + t));
+    double* pa = V + (p & 0xffffu);
+    double* pb = V + (p >> 16);
+    const double a = *pa, b = *pb;
+    *pa = a + b;
+    *pb = a - b;
   }
 }
 
-__device__ void run_pass(const KdPass& p, const double* __restrict__ X, double* __restrict__ Y, int d0, int d1,
-                         int d2, const double* __restrict__ pool, double scale) {
-  run_pass_part(p, X, d0, d1, d2, pool, scale, 0, blockDim.x, [Y](int e, double v) { Y[e] = v; });
+__device__ __forceinline__ int output_size(const KdItem& it) {
+  int e0 = it.n0, e1 = it.n1, e2 = it.n2;
+  for (int q = 0; q < it.npass; q++) {
+    if (it.pass[q].dim == 0) e0 = it.pass[q].n_out;
+    if (it.pass[q].dim == 1) e1 = it.pass[q].n_out;
+    if (it.pass[q].dim == 2) e2 = it.pass[q].n_out;
+  }
+  return e0 * e1 * e2;
 }
 
-__global__ void line_passes_kernel(const __grid_constant__ KdItemList list, const double* __restrict__ pool) {
-  extern __shared__ double smem[];
-  const int total_fields = list.prefix[list.nitems];
-  // Grid-stride over fields so that any grid size covers the work.
-  for (int f = blockIdx.x; f < total_fields; f += gridDim.x) {
-    int item = 0;
-    while (item + 1 < list.nitems && list.prefix[item + 1] <= f) item++;
-    const KdItem& it = list.items[item];
-    const int field_in_item = f - list.prefix[item];
-    const int n_in_elems = it.n0 * it.n1 * it.n2;
-    // Buffer sizes: every stage fits in half of the dynamic shared memory.
-    int d0 = it.n0, d1 = it.n1, d2 = it.n2;
-    int maxe = n_in_elems;
-    {
-      int e0 = d0, e1 = d1, e2 = d2;
-      for (int q = 0; q < it.npass; q++) {
-        if (it.pass[q].dim == 0) e0 = it.pass[q].n_out;
-        if (it.pass[q].dim == 1) e1 = it.pass[q].n_out;
-        if (it.pass[q].dim == 2) e2 = it.pass[q].n_out;
-        int e = e0 * e1 * e2;
-        if (e > maxe) maxe = e;
-      }
-    }
-    double* bufA = smem;
-    double* bufB = smem + maxe;
-    const double* src = it.in + static_cast<long long>(field_in_item) * it.in_stride;
-    double* dst = it.out + static_cast<long long>(field_in_item) * it.out_stride;
-    for (int e = threadIdx.x; e < n_in_elems; e += blockDim.x) bufA[e] = src[e];
-    __syncthreads();
-    double* X = bufA;
-    double* Y = bufB;
-    for (int q = 0; q < it.npass; q++) {
-      const KdPass& p = it.pass[q];
-      bool last = (q == it.npass - 1);
-      int o0 = d0, o1 = d1, o2 = d2;
-      if (p.dim == 0) o0 = p.n_out;
-      if (p.dim == 1) o1 = p.n_out;
-      if (p.dim == 2) o2 = p.n_out;
-      // The last pass writes straight to global memory.
-      run_pass(p, X, last ? dst : Y, d0, d1, d2, pool, last ? it.scale : 1.0);
-      __syncthreads();
-      d0 = o0;
-      d1 = o1;
-      d2 = o2;
-      double* tmp = X;
-      X = Y;
-      Y = tmp;
-    }
-    if (it.npass == 0) {
-      for (int e = threadIdx.x; e < n_in_elems; e += blockDim.x) dst[e] = bufA[e] * it.scale;
-    }
-    __syncthreads();
-  }
-}
-
-// Small batches: one LP_CL-CTA cluster per field.  Each CTA computes every
-// LP_CL-th block of a pass's outputs and stores them into all the cluster's
-// shared buffers (distributed shared memory), then one cluster barrier; the
-// last pass writes straight to global memory.  A field's FP64 work is spread
-// over LP_CL SMs instead of one.
-constexpr int LP_CLUSTER_MAX_FIELDS = 32;
-template <int LP_CL>
-__global__ void line_passes_cluster_kernel(const __grid_constant__ KdItemList list, const double* __restrict__ pool) {
-  namespace cg = cooperative_groups;
-  cg::cluster_group cluster = cg::this_cluster();
-  extern __shared__ double smem[];
-  const int rank = static_cast<int>(cluster.block_rank());
-  const int f = blockIdx.x / LP_CL;
-  int item = 0;
-  while (item + 1 < list.nitems && list.prefix[item + 1] <= f) item++;
-  const KdItem& it = list.items[item];
-  const int field_in_item = f - list.prefix[item];
-  const int n_in_elems = it.n0 * it.n1 * it.n2;
-  int d0 = it.n0, d1 = it.n1, d2 = it.n2;
-  int maxe = n_in_elems;
-  {
-    int e0 = d0, e1 = d1, e2 = d2;
-    for (int q = 0; q < it.npass; q++) {
-      if (it.pass[q].dim == 0) e0 = it.pass[q].n_out;
-      if (it.pass[q].dim == 1) e1 = it.pass[q].n_out;
-      if (it.pass[q].dim == 2) e2 = it.pass[q].n_out;
-      int e = e0 * e1 * e2;
-      if (e > maxe) maxe = e;
-    }
-  }
-  double* bufA = smem;
-  double* bufB = smem + maxe;
-  const double* src = it.in + static_cast<long long>(field_in_item) * it.in_stride;
-  double* dst = it.out + static_cast<long long>(field_in_item) * it.out_stride;
-  for (int e = threadIdx.x; e < n_in_elems; e += blockDim.x) bufA[e] = src[e];
-  __syncthreads();
-  double* X = bufA;
-  double* Y = bufB;
-  const int e0 = rank * blockDim.x, estride = LP_CL * blockDim.x;
+// All passes of one field, staged in X, by one CTA; X and Y hold one stage each.
+__device__ __forceinline__ void run_item(const KdItem& it, const double* mats, double* __restrict__ dst, double* X,
+                                         double* Y) {
   for (int q = 0; q < it.npass; q++) {
     const KdPass& p = it.pass[q];
     const bool last = (q == it.npass - 1);
-    int o0 = d0, o1 = d1, o2 = d2;
-    if (p.dim == 0) o0 = p.n_out;
-    if (p.dim == 1) o1 = p.n_out;
-    if (p.dim == 2) o2 = p.n_out;
-    if (last) {
-      const double sc = it.scale;
-      run_pass_part(p, X, d0, d1, d2, pool, sc, e0, estride, [dst](int e, double v) { dst[e] = v; });
-    } else {
-      double* Yr[LP_CL];
-      for (int r = 0; r < LP_CL; r++) Yr[r] = cluster.map_shared_rank(Y, r);
-      run_pass_part(p, X, d0, d1, d2, pool, 1.0, e0, estride, [&Yr](int e, double v) {
-#pragma unroll
-        for (int r = 0; r < LP_CL; r++) Yr[r][e] = v;
-      });
-      cluster.sync();  // every CTA's Y is complete and nobody reads X any more
+    if (p.nbefore) {
+      fold_pairs(p.pairs, p.nbefore, X);
+      __syncthreads();
     }
-    d0 = o0;
-    d1 = o1;
-    d2 = o2;
+    const bool straight = last && !p.nafter;  // the last pass writes straight to global memory
+    double* to = straight ? dst : Y;
+    const double scale = last ? it.scale : 1.0;
+    for (int e = threadIdx.x; e < p.nout; e += blockDim.x) {
+      const KdOut o = load_out(p.out + e);
+      const double v = line_dot(o, mats, X);
+      to[o.y0] = scale == 1.0 ? v : v * scale;
+    }
+    if (straight) return;
+    __syncthreads();
+    if (p.nafter) {
+      fold_pairs(p.pairs + p.nbefore, p.nafter, Y);
+      __syncthreads();
+    }
+    double* t = X;
+    X = Y;
+    Y = t;
+  }
+  const int n_out_elems = output_size(it);  // the last stage has no padding
+  for (int e = threadIdx.x; e < n_out_elems; e += blockDim.x) dst[e] = X[e];
+}
+
+// The item of field f of a launch.
+__device__ __forceinline__ int item_of(const KdItemList1&, int) { return 0; }
+__device__ __forceinline__ int item_of(const KdItemList& list, int f) {
+  int item = 0;
+  while (item + 1 < list.nitems && list.prefix[item + 1] <= f) item++;
+  return item;
+}
+
+template <class List>
+__global__ void line_passes_kernel(const __grid_constant__ List list, const double* __restrict__ pool) {
+  extern __shared__ __align__(16) double smem[];
+  const int total_fields = list.prefix[list.nitems];
+  int staged_item = -1;
+  // Grid-stride over fields so that any grid size covers the work.
+  for (int f = blockIdx.x; f < total_fields; f += gridDim.x) {
+    const int item = item_of(list, f);
+    const KdItem& it = list.items[item];
+    const long long field_in_item = f - list.prefix[item];
+    load_field(it, it.in + field_in_item * it.in_stride, smem);
+    double* at = smem + 2 * it.stage;
+    if (item != staged_item) {
+      load_mats(it, at);
+      staged_item = item;
+    }
+    copy_async_wait();
+    __syncthreads();
+    run_item(it, it.nmats ? at : pool, it.out + field_in_item * it.out_stride, smem, smem + it.stage);
+    __syncthreads();
+  }
+}
+
+// Few fields: one LP_CL-CTA cluster per field.  Thread t of the cluster
+// computes outputs t, t + threads, ... of each pass (the first of them listed
+// in registers before the field has arrived) and stores them into all the
+// cluster's shared buffers (distributed shared memory), then one cluster
+// barrier; the last pass writes straight to global memory.  A field's FP64
+// work is spread over LP_CL SMs instead of one.
+template <int LP_CL, class List>
+__global__ void line_passes_cluster_kernel(const __grid_constant__ List list, const double* __restrict__ pool) {
+  namespace cg = cooperative_groups;
+  cg::cluster_group cluster = cg::this_cluster();
+  extern __shared__ __align__(16) double smem[];
+  const int rank = static_cast<int>(cluster.block_rank());
+  // no store into another CTA's buffers before that CTA runs
+  auto started = cluster.barrier_arrive();
+  const int f = blockIdx.x / LP_CL;
+  const int item = item_of(list, f);
+  const KdItem& it = list.items[item];
+  const long long field_in_item = f - list.prefix[item];
+  double* dst = it.out + field_in_item * it.out_stride;
+  double* X = smem;
+  double* Y = smem + it.stage;
+  double* at = smem + 2 * it.stage;
+  load_field(it, it.in + field_in_item * it.in_stride, X);
+  load_mats(it, at);
+  const int e0 = rank * blockDim.x + threadIdx.x, estride = LP_CL * blockDim.x;
+  KdOut first[3];
+#pragma unroll
+  for (int q = 0; q < 3; q++)
+    first[q] = q < it.npass && e0 < it.pass[q].nout ? load_out(it.pass[q].out + e0) : KdOut{0, 0, 0, 0};
+  copy_async_wait();
+  __syncthreads();
+  cluster.barrier_wait(std::move(started));
+  const double* mats = it.nmats ? at : pool;
+#pragma unroll
+  for (int q = 0; q < 3; q++) {
+    if (q >= it.npass) break;
+    const KdPass& p = it.pass[q];
+    const bool last = (q == it.npass - 1);
+    if (p.nbefore) {  // every CTA folds its own copy
+      fold_pairs(p.pairs, p.nbefore, X);
+      __syncthreads();
+    }
+    const bool straight = last && !p.nafter;
+    const double scale = last ? it.scale : 1.0;
+    KdOut o = first[q];
+    for (int e = e0; e < p.nout; e += estride) {
+      KdOut next = o;
+      if (e + estride < p.nout) next = load_out(p.out + e + estride);
+      double v = line_dot(o, mats, X);
+      if (scale != 1.0) v *= scale;
+      if (straight) {
+        dst[o.y0] = v;
+      } else {
+#pragma unroll
+        for (int r = 0; r < LP_CL; r++) cluster.map_shared_rank(Y, r)[o.y0] = v;
+      }
+      o = next;
+    }
+    if (straight) return;  // nobody writes into this CTA's buffers any more
+    cluster.sync();        // every CTA's Y is complete and nobody reads X any more
+    if (p.nafter) {
+      fold_pairs(p.pairs + p.nbefore, p.nafter, Y);
+      __syncthreads();
+    }
     double* tmp = X;
     X = Y;
     Y = tmp;
   }
-  if (it.npass == 0) {
-    if (rank == 0)
-      for (int e = threadIdx.x; e < n_in_elems; e += blockDim.x) dst[e] = bufA[e] * it.scale;
-  }
+  const int n_out_elems = output_size(it);  // the last stage has no padding
+  for (int e = e0; e < n_out_elems; e += estride) dst[e] = X[e];
+}
+
+// i % npts; the 64-bit remainder takes over a hundred instructions, so
+// indices below 2^32 go by the 32-bit one
+__device__ __forceinline__ long long point_of(long long i, long long npts) {
+  if (((i | npts) >> 32) == 0) return static_cast<unsigned>(i) % static_cast<unsigned>(npts);
+  return i % npts;
 }
 
 __global__ void ew_kernel(int op, long long npts, long long total, int ba, const double* __restrict__ a,
@@ -196,7 +246,7 @@ __global__ void ew_kernel(int op, long long npts, long long total, int ba, const
                           double beta) {
   for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < total;
        i += static_cast<long long>(gridDim.x) * blockDim.x) {
-    long long p = i % npts;
+    const long long p = total == npts ? i : point_of(i, npts);
     double x = (a != nullptr) ? a[ba == 1 ? p : i] : 0.0;
     double y = (b != nullptr) ? b[bb == 1 ? p : i] : 0.0;
     double r;
@@ -239,8 +289,8 @@ __global__ void gather_csr_kernel(const double* __restrict__ in, long long in_st
   long long total = static_cast<long long>(batch) * nrows;
   for (long long t = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; t < total;
        t += static_cast<long long>(gridDim.x) * blockDim.x) {
-    int r = static_cast<int>(t % nrows);
-    long long f = t / nrows;
+    const int r = static_cast<int>(point_of(t, nrows));
+    const long long f = (t >> 32) == 0 ? static_cast<unsigned>(t) / static_cast<unsigned>(nrows) : t / nrows;
     const double* src = in + f * in_stride;
     double acc = 0.0;
     for (int e = rowptr[r]; e < rowptr[r + 1]; e++) acc = fma(w[e], src[idx[e]], acc);
@@ -276,12 +326,12 @@ __global__ void absmax_kernel(const double* __restrict__ x, long long n, double*
   }
 }
 
-template <int CL>
-cudaError_t launch_lp_cluster(const KdItemList& list, int total_fields, size_t smem, const double* d_pool,
+template <int CL, class List>
+cudaError_t launch_lp_cluster(const List& list, int total_fields, size_t smem, const double* d_pool,
                               cudaStream_t s) {
   if (smem > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(line_passes_cluster_kernel<CL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         static_cast<int>(smem));
+    cudaError_t e = cudaFuncSetAttribute(line_passes_cluster_kernel<CL, List>,
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
     if (e != cudaSuccess) return e;
   }
   cudaLaunchConfig_t cfg = {};
@@ -296,8 +346,28 @@ cudaError_t launch_lp_cluster(const KdItemList& list, int total_fields, size_t s
   at[0].val.clusterDim.z = 1;
   cfg.attrs = at;
   cfg.numAttrs = 1;
-  cudaError_t e = cudaLaunchKernelEx(&cfg, line_passes_cluster_kernel<CL>, list, d_pool);
+  cudaError_t e = cudaLaunchKernelEx(&cfg, line_passes_cluster_kernel<CL, List>, list, d_pool);
   if (e != cudaSuccess) return e;
+  return cudaGetLastError();
+}
+
+template <class List>
+cudaError_t launch_list(const List& list, size_t smem, const double* d_pool, cudaStream_t s, LpShape shape) {
+  const int total_fields = list.prefix[list.nitems];
+  switch (shape.cluster) {
+    case 2: return launch_lp_cluster<2>(list, total_fields, smem, d_pool, s);
+    case 4: return launch_lp_cluster<4>(list, total_fields, smem, d_pool, s);
+    case 8: return launch_lp_cluster<8>(list, total_fields, smem, d_pool, s);
+    default: break;
+  }
+  if (smem > 48 * 1024) {
+    cudaError_t e = cudaFuncSetAttribute(line_passes_kernel<List>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         static_cast<int>(smem));
+    if (e != cudaSuccess) return e;
+  }
+  const int threads = (shape.threads == 64 || shape.threads == 256) ? shape.threads : 128;
+  int grid = total_fields < 152 * 8 ? total_fields : 152 * 8;
+  line_passes_kernel<List><<<grid, threads, smem, s>>>(list, d_pool);
   return cudaGetLastError();
 }
 
@@ -310,37 +380,39 @@ int grid_for(long long n, int threads) {
 
 }  // namespace
 
-LpShape lp_default_shape(int total_fields) {
+LpShape lp_default_shape(int total_fields, int stage) {
   LpShape sh;
-  if (total_fields <= LP_CLUSTER_MAX_FIELDS) sh.cluster = 8;
+  sh.threads = 256;
+  if (total_fields <= 32)
+    sh.cluster = (total_fields > 8 || stage < 1024) ? 4 : 8;
+  else if (total_fields <= 76 && stage >= 2048)
+    sh.cluster = 4;
   return sh;
 }
 
-cudaError_t launch_line_passes(const KdItemList& list, int smem_doubles, const double* d_pool, cudaStream_t s,
-                               LpShape shape) {
-  const int total_fields = list.prefix[list.nitems];
-  if (total_fields <= 0) return cudaSuccess;
-  size_t smem = static_cast<size_t>(smem_doubles) * 2 * sizeof(double);
-  switch (shape.cluster) {
-    case 2: return launch_lp_cluster<2>(list, total_fields, smem, d_pool, s);
-    case 4: return launch_lp_cluster<4>(list, total_fields, smem, d_pool, s);
-    case 8: return launch_lp_cluster<8>(list, total_fields, smem, d_pool, s);
-    default: break;
+cudaError_t launch_line_passes(const KdItemList& list, const double* d_pool, cudaStream_t s, LpShape shape) {
+  if (list.prefix[list.nitems] <= 0) return cudaSuccess;
+  // per item two stages of the field, the matrices behind them
+  size_t smem = 0;
+  for (int i = 0; i < list.nitems; i++) {
+    const size_t need = sizeof(double) * (2 * static_cast<size_t>(list.items[i].stage) + list.items[i].nmats);
+    if (need > smem) smem = need;
   }
-  if (smem > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(line_passes_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         static_cast<int>(smem));
-    if (e != cudaSuccess) return e;
+  if (list.nitems == 1) {
+    KdItemList1 one;
+    one.nitems = 1;
+    one.prefix[0] = list.prefix[0];
+    one.prefix[1] = list.prefix[1];
+    one.items[0] = list.items[0];
+    return launch_list(one, smem, d_pool, s, shape);
   }
-  const int threads = (shape.threads == 64 || shape.threads == 256) ? shape.threads : 128;
-  int grid = total_fields < 152 * 8 ? total_fields : 152 * 8;
-  line_passes_kernel<<<grid, threads, smem, s>>>(list, d_pool);
-  return cudaGetLastError();
+  return launch_list(list, smem, d_pool, s, shape);
 }
 
-cudaError_t launch_line_passes(const KdItemList& list, int smem_doubles, const double* d_pool,
-                               cudaStream_t s) {
-  return launch_line_passes(list, smem_doubles, d_pool, s, lp_default_shape(list.prefix[list.nitems]));
+cudaError_t launch_line_passes(const KdItemList& list, const double* d_pool, cudaStream_t s) {
+  int stage = 0;
+  for (int i = 0; i < list.nitems; i++) stage = list.items[i].stage > stage ? list.items[i].stage : stage;
+  return launch_line_passes(list, d_pool, s, lp_default_shape(list.prefix[list.nitems], stage));
 }
 
 cudaError_t launch_ew(int op, long long npts, int ba, const double* a, int bb, const double* b, double* out,

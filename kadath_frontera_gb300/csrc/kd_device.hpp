@@ -6,19 +6,26 @@
 
 namespace kd {
 
-// One 1-D pass of a separable operator over a 3-D block (r, theta, phi),
-// phi fastest.  The matrix applied to a line is looked up per line:
-//   dim 0 (r):     mat[j * mat_ld + k]   (basis depends on theta/phi indices)
-//   dim 1 (theta): mat[k]                (basis depends on the phi index)
-//   dim 2 (phi):   mat[0]
-// An entry < 0 means "this line's output is zero".  Offsets are in doubles
-// into the shared matrix pool; the matrix is row-major n_out x n_in.
+// One output of a line pass: sum_q m[m0 + q mstep] x[x0 + q xstep], q < count,
+// stored at y0.  Only the nonzero range of the matrix row is listed; count 0
+// stores a zero.  steps = count | mstep << 12 | xstep << 14.
+struct KdOut {
+  int x0, m0, y0;
+  unsigned steps;
+};
+
+// One 1-D pass of a separable operator over a 3-D block (r, theta, phi), phi
+// fastest, as the list of its outputs (ordered so that the outputs of a warp
+// have the same count) and of the mirrored pairs that are replaced by their
+// sum and difference in the pass's input (before) and output (after).
 struct KdPass {
   int dim;
   int n_in;
   int n_out;
-  int mat_ld;
-  const int* mat;
+  int nout;            // outputs
+  int nbefore, nafter; // pairs
+  const KdOut* out;
+  const int* pairs;    // first element | second << 16: before, then after
 };
 
 // A run of `batch` fields of identical shape processed by the same pass list.
@@ -29,7 +36,11 @@ struct KdItem {
   long long out_stride;
   int n0, n1, n2;        // input dims
   int npass;
+  int stage;             // doubles of the largest stage in shared memory
+  int pitch;             // row pitch (phi) of the input staged in shared memory
+  int nmats;             // doubles of the matrices staged in shared memory (0: read from the pool)
   double scale;          // applied to the final result
+  const double* mats;    // the matrices to stage, 16-byte aligned
   KdPass pass[3];
 };
 
@@ -43,6 +54,13 @@ struct KdItemList {
   KdItem items[KD_MAX_ITEMS];
 };
 
+// The same with one item: a tenth of the parameter bytes of a launch.
+struct KdItemList1 {
+  int nitems;
+  int prefix[2];
+  KdItem items[1];
+};
+
 // Launch shape of a line-pass launch: one CTA of `threads` threads per field
 // (cluster = 1), or a cluster of `cluster` CTAs (2, 4 or 8) of 128 threads
 // per field, each CTA computing every cluster-th block of a pass's outputs.
@@ -52,16 +70,21 @@ struct LpShape {
   int cluster = 1;
   int threads = 128;
 };
-// The rule without a tuning table: 8-CTA clusters up to 32 fields, else one
-// 128-thread CTA per field.
-LpShape lp_default_shape(int total_fields);
+// The rule without a tuning table, from the fields of the launch and the
+// doubles of the largest item's stage.  Up to 32 fields are bound by latency:
+// clusters of 8 CTAs, or of 4 where the field is small or the clusters no
+// longer all get SMs of their own (us per launch with 8 / 4 CTAs: one (9,5,4)
+// field 6.2 / 6.2, 30 of them 10.2 / 6.2; one (21,11,14) field 18.4 / 24.6, 30
+// of them 26.6 / 24.6).  Beyond that one 256-thread CTA per field (150 fields
+// of (15,11,12): 26.6 against 42.4 with 128 threads and 39.5 with clusters of
+// 4), except that large fields that leave half of the SMs idle keep clusters
+// of 4 (60 fields of (21,11,14): 34.0 against 43.0).
+LpShape lp_default_shape(int total_fields, int stage);
 
 // Runs the pass lists of all items with the given shape (default rule: the
 // overload without one).
-cudaError_t launch_line_passes(const KdItemList& list, int smem_doubles, const double* d_pool,
-                               cudaStream_t s, LpShape shape);
-cudaError_t launch_line_passes(const KdItemList& list, int smem_doubles, const double* d_pool,
-                               cudaStream_t s);
+cudaError_t launch_line_passes(const KdItemList& list, const double* d_pool, cudaStream_t s, LpShape shape);
+cudaError_t launch_line_passes(const KdItemList& list, const double* d_pool, cudaStream_t s);
 
 // Elementwise ops on fields of npts values. a has ba fields, b has bb fields
 // (ba, bb in {1, B}); out has max(ba, bb) fields.

@@ -17,9 +17,9 @@ void ew(Context* ctx, int op, long long npts, int ba, const double* a, int bb, c
   ctx->launches++;
 }
 
-void run_specs(Context* ctx, const std::vector<LinePassSpec>& specs, const double* in, double* out,
-               const int dims_in[3], long long in_stride, long long out_stride, int batch, double scale = 1.0) {
-  KdItem it = make_item(*ctx, specs, in, out, dims_in, in_stride, out_stride, scale);
+void run_plan(Context* ctx, const LinePlan& plan, const double* in, double* out, const int dims_in[3],
+              long long in_stride, long long out_stride, int batch) {
+  KdItem it = make_item(plan, in, out, dims_in, in_stride, out_stride, 1.0);
   ctx->run_items({it}, {batch});
 }
 
@@ -128,8 +128,7 @@ void DVal::coef() const {
   if (in_coef || zero) return;
   if (!base.def) throw KdError(KD_ERR_STATE, "Base not defined in Val_domain::coef");
   double* out = alloc(ctx, static_cast<long long>(batch) * ncoefs());
-  auto specs = coef_specs(*ctx, base, dom->np, dom->nc);
-  run_specs(ctx, specs, c, out, dom->np, npts(), ncoefs(), batch);
+  run_plan(ctx, coef_plan(*ctx, base, dom->np, dom->nc, false, batch), c, out, dom->np, npts(), ncoefs(), batch);
   cf = out;
   in_coef = true;
 }
@@ -138,8 +137,7 @@ void DVal::coef_i() const {
   if (in_conf || zero) return;
   if (!base.def) throw KdError(KD_ERR_STATE, "Base not defined in Val_domain::coef_i");
   double* out = alloc(ctx, static_cast<long long>(batch) * npts());
-  auto specs = coef_i_specs(*ctx, base, dom->np, dom->nc);
-  run_specs(ctx, specs, cf, out, dom->nc, ncoefs(), npts(), batch);
+  run_plan(ctx, coef_plan(*ctx, base, dom->np, dom->nc, true, batch), cf, out, dom->nc, ncoefs(), npts(), batch);
   c = out;
   in_conf = true;
 }
@@ -153,9 +151,9 @@ void DVal::compute_der_var() const {
     auto res = std::make_shared<DVal>(ctx, dom, batch);
     res->zero = false;
     res->base = base;
-    auto spec = ope_1d_spec(*ctx, OP_DER, var, base, dom->nc, res->base);
+    const LinePlan& plan = ope_1d_plan(*ctx, OP_DER, var, base, dom->nc, res->base);
     double* out = alloc(ctx, static_cast<long long>(batch) * ncoefs());
-    items.push_back(make_item(*ctx, {spec}, cf, out, dom->nc, ncoefs(), ncoefs(), 1.0));
+    items.push_back(make_item(plan, cf, out, dom->nc, ncoefs(), ncoefs(), 1.0));
     batches.push_back(batch);
     res->cf = out;
     res->in_coef = true;
@@ -457,9 +455,9 @@ DVal ope_coef(const DVal& so, int op, int dim) {
   DVal res(so.ctx, so.dom, so.batch);
   res.zero = false;
   res.base = so.base;
-  auto spec = ope_1d_spec(*so.ctx, op, dim, so.base, so.dom->nc, res.base);
+  const LinePlan& plan = ope_1d_plan(*so.ctx, op, dim, so.base, so.dom->nc, res.base);
   double* out = alloc(so.ctx, static_cast<long long>(so.batch) * so.ncoefs());
-  run_specs(so.ctx, {spec}, so.cf, out, so.dom->nc, so.ncoefs(), so.ncoefs(), so.batch);
+  run_plan(so.ctx, plan, so.cf, out, so.dom->nc, so.ncoefs(), so.ncoefs(), so.batch);
   res.cf = out;
   res.in_coef = true;
   return res;
@@ -479,10 +477,10 @@ static DVal mult_trig_phi(const DVal& so, int op) {
       else throw KdError(KD_ERR_UNSUPPORTED, "Unknown case in Domain_nucleus::mult_cos_phi");
     }
   Base tmp = res.base;
-  auto spec = ope_1d_spec(*so.ctx, op, 2, so.base, so.dom->nc, tmp);
+  const LinePlan& plan = ope_1d_plan(*so.ctx, op, 2, so.base, so.dom->nc, tmp);
   res.base.p = tmp.p;
   double* out = alloc(so.ctx, static_cast<long long>(so.batch) * so.ncoefs());
-  run_specs(so.ctx, {spec}, so.cf, out, so.dom->nc, so.ncoefs(), so.ncoefs(), so.batch);
+  run_plan(so.ctx, plan, so.cf, out, so.dom->nc, so.ncoefs(), so.ncoefs(), so.batch);
   res.cf = out;
   res.in_coef = true;
   return res;

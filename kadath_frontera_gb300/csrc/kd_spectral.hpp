@@ -50,6 +50,33 @@ std::vector<LinePassSpec> coef_i_specs(Context& ctx, const Base& base, const int
 // same domain: r, theta, then phi, each line through OP_RESAMPLE.
 std::vector<LinePassSpec> resample_specs(Context& ctx, const Base& base, const int nc_old[3], const int np_new[3]);
 
+// What a pass's table holds: its outputs, then its mirrored pairs.
+struct PassLists {
+  std::vector<KdOut> outs;
+  std::vector<int> before, after;
+};
+// The passes of a plan over a field of dims_in, their lists and the matrices
+// to stage (none when `stage` is off or they do not fit).  The caller puts the
+// lists and matrices into device memory and sets the plan's pointers.
+void compile_passes(Context& ctx, const std::vector<LinePassSpec>& specs, const int dims_in[3], bool fold, bool stage,
+                    LinePlan& plan, PassLists lists[3], std::vector<double>& mats);
+std::vector<int> pass_table(const PassLists& l);
+void set_pass_table(KdPass& p, const int* table);
+
+// Compiled pass lists, kept by the context by what they depend on (operator,
+// dims, every line's basis).  A transform of more than FOLD_MIN_FIELDS fields
+// combines mirrored entries (half the products, an extra barrier per pass: at
+// (13,9,4) one field takes 8.2 us without and 10.2 us with it, 2,580 fields 71
+// us with and 92 us without); the rule is on the fields of the call, not on the
+// launch's shape, so that the shape changes no result bit.
+constexpr long long FOLD_MIN_FIELDS = 32;
+const LinePlan& coef_plan(Context& ctx, const Base& base, const int np[3], const int nc[3], bool inverse,
+                          long long fields);
+// The operator's output basis table of `dim` is written to base_out.
+const LinePlan& ope_1d_plan(Context& ctx, int op, int dim, const Base& base, const int d[3], Base& base_out);
+KdItem make_item(const LinePlan& plan, const double* in, double* out, const int dims_in[3], long long in_stride,
+                 long long out_stride, double scale);
+
 // Turns pass specs into a kernel item (device tables resolved through ctx).
 KdItem make_item(Context& ctx, const std::vector<LinePassSpec>& specs, const double* in, double* out,
                  const int dims_in[3], long long in_stride, long long out_stride, double scale);

@@ -78,14 +78,7 @@ void regrid(Field& dst, Field& src) {
     list.prefix[0] = 0;
     list.prefix[1] = 1;
     list.items[0] = make_item(ctx, specs, v.cf, pn.c, nco, dmo.ncoefs(), dmn.npts(), 1.0);
-    int maxe = dmo.ncoefs();
-    int d[3] = {nco[0], nco[1], nco[2]};
-    for (const auto& sp : specs) {
-      d[sp.dim] = sp.n_out;
-      const int e = d[0] * d[1] * d[2];
-      if (e > maxe) maxe = e;
-    }
-    cuda_check(launch_line_passes(list, maxe, ctx.pool(), ctx.stream()), "regrid line passes");
+    cuda_check(launch_line_passes(list, ctx.pool(), ctx.stream()), "regrid line passes");
     ctx.launches++;
     cuda_check(cudaStreamSynchronize(ctx.stream()), "sync regrid");
     ctx.scratch().release_to(mark);
