@@ -1,0 +1,499 @@
+// Trailing update of the FP64 LU, C -= A * B, on the tcgen05 tensor cores by
+// exact products of 8-bit slices (the error-free splitting of Ozaki, Ogita,
+// Oishi and Rump, Numer. Algorithms 59, 2012, in fixed point).
+//
+// This GPU's FP64 pipe gives 1.1 TFLOP/s; its bf16 tensor cores 1,700 times
+// that.  Each operand entry becomes a 62-bit fixed-point number F relative to
+// the largest entry of its row of A (column of B), F = sum_s d_s 2^(8(8-s)),
+// s = 1..8, with d_s in [-128, 127]: eight bf16 matrices of integers.  The
+// product of slices i and j has integer entries, summed exactly in FP32: an
+// order o = i + j adds at most 8 pairs of k <= 128 products below 2^14, at
+// most 2^24 in all.  Orders 2..9 (36 of the 64 pairs) are kept, the rest is
+// below 2^-60 of the largest product.  Before splitting, row k of B is scaled
+// by a power of two to a largest entry in [1/2, 1) and column k of A by its
+// inverse, so that rows of B of very different sizes (a Jacobian's second
+// derivatives beside its boundary rows) do not cost each other digits.  The
+// split entries are off by 2^-63 of their row's largest one, against the
+// 2^-53 of every rounding of an FP64 product, and a tile's entry is rounded
+// twice (its 60-bit sum to double, the subtraction from C).
+//
+// One persistent CTA per SM, 128 x 64 tiles:
+//   warp 0   TMA loads of operand chunks: k = 32 of all eight slices of A and
+//            B (96 KB, 64-byte swizzle), two stages;
+//   warp 1   72 MMAs per chunk (M 128, N 64, K 16) into eight accumulators of
+//            64 TMEM columns, one per order: all 512 columns;
+//   warps 2-9 epilogue: the eight orders of an entry into one 64-bit integer,
+//            TMEM released, then C -= integer * 2^e (one conversion and one
+//            multiply-add on the FP64 pipe) beside the next tile's MMAs.
+// Bound: the MMAs' operand reads from shared memory (48 cycles per MMA of 32)
+// and the hand-over of the single set of accumulators.  128 x 64 tiles and not
+// 128 x 128: eight orders of 64 columns are all of TMEM, and one pass over the
+// operands serves all of them.
+// All updates of a factorisation, this kernel with its packing against the
+// library's FP64 GEMM: N = 8,000 19.7 against 319 ms (17 TFLOP/s of FP64
+// products), N = 12,331 64 against 1,173 ms; relative residuals of the solves
+// 1.2e-15 and 1.4e-15 with either.
+#include <cuda.h>
+#include <cuda_bf16.h>
+#include <cuda_runtime.h>
+
+#include <cstdint>
+#include <mutex>
+#include <string>
+
+#include "kd_gemm_tc.hpp"
+
+namespace kd {
+
+namespace {
+
+constexpr int S_SLICES = 8;
+constexpr int S_M = 128, S_N = 64, S_KC = 32;           // tile and k chunk
+constexpr int S_MAXK = 128;                              // exact sums: 8 pairs x 128 x 2^14 = 2^24
+constexpr int S_A_SLICE = S_M * S_KC * 2;                // bytes of one slice of a chunk
+constexpr int S_B_SLICE = S_N * S_KC * 2;
+constexpr int S_STAGE = S_SLICES * (S_A_SLICE + S_B_SLICE);
+constexpr int S_NST = 2;
+constexpr int S_THREADS = 320;
+constexpr size_t S_SMEM = 1024 + static_cast<size_t>(S_NST) * S_STAGE;
+constexpr unsigned long long S_WAIT_NS = 2000000000ull;
+constexpr int EXP_NONFINITE = 1 << 20;                   // scale of a row or column that holds Inf or NaN
+constexpr int EXP_ZERO = -(1 << 20);                     // scale of a zero row or column
+
+__device__ __forceinline__ uint32_t smem_addr(const void* p) {
+  return static_cast<uint32_t>(__cvta_generic_to_shared(p));
+}
+
+// Smallest E with |v| < 2^E; EXP_ZERO for zero (and subnormals, which are
+// taken as zero), EXP_NONFINITE for Inf and NaN.
+__device__ __forceinline__ int exponent_of(double v) {
+  const int e = static_cast<int>((static_cast<unsigned long long>(__double_as_longlong(v)) >> 52) & 0x7ff);
+  if (e == 0) return EXP_ZERO;
+  if (e == 0x7ff) return EXP_NONFINITE;
+  return e - 1022;
+}
+
+// v * 2^(62 - scale) rounded to an integer, for |v| < 2^scale.
+__device__ __forceinline__ long long fixed_point(double v, int scale) {
+  const unsigned long long b = static_cast<unsigned long long>(__double_as_longlong(v));
+  const int e = static_cast<int>((b >> 52) & 0x7ff);
+  if (e == 0 || e == 0x7ff) return 0;
+  const unsigned long long m = ((b & 0xfffffffffffffull) | 0x10000000000000ull) << 9;
+  const int shift = scale - (e - 1022);
+  long long f;
+  if (shift <= 0) f = static_cast<long long>(m);  // shift is never negative
+  else if (shift > 62) f = 0;
+  else f = static_cast<long long>((m + (1ull << (shift - 1))) >> shift);
+  return (b >> 63) ? -f : f;
+}
+
+// The eight digits of f, most significant first, as bf16.
+__device__ __forceinline__ void digits_of(long long f, __nv_bfloat16 (&d)[S_SLICES]) {
+  // adding 128 to the lower seven bytes makes each of them its digit + 128
+  const long long g = f + 0x0080808080808080ll;
+  d[0] = __float2bfloat16_rn(static_cast<float>(static_cast<int>(g >> 56)));
+#pragma unroll
+  for (int s = 1; s < S_SLICES; s++)
+    d[s] = __float2bfloat16_rn(static_cast<float>(static_cast<int>((g >> (8 * (7 - s))) & 255) - 128));
+}
+
+// xk[kk] = max over the columns of the exponents of row kk of B (k x n,
+// column-major); xk starts at EXP_ZERO.
+__global__ void slice_row_exponents(const double* __restrict__ B, long long ldb, int k, int n, int cols,
+                                    int* __restrict__ xk) {
+  const int kk = threadIdx.x;
+  if (kk >= k) return;
+  const int c0 = blockIdx.x * cols, c1 = min(n, c0 + cols);
+  int m = EXP_ZERO;
+#pragma unroll 8
+  for (int c = c0; c < c1; c++) {
+    const int e = exponent_of(B[static_cast<long long>(c) * ldb + kk]);
+    if (e != EXP_NONFINITE) m = max(m, e);
+  }
+  if (m != EXP_ZERO) atomicMax(xk + kk, m);
+}
+
+__global__ void slice_fill(int* __restrict__ v, int n, int x) {
+  if (static_cast<int>(threadIdx.x) < n) v[threadIdx.x] = x;
+}
+
+// Slices of B: out[s][column][kk] and the columns' scales; one warp a column.
+__global__ void slice_pack_b(const double* __restrict__ B, long long ldb, int k, int n, int kpad, int npad,
+                             const int* __restrict__ xk, __nv_bfloat16* __restrict__ out, int* __restrict__ scale) {
+  const int col = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (col >= npad) return;
+  double v[4];  // kk = 2 lane, 2 lane + 1, then + 64
+  int x[4], mx = EXP_ZERO;
+  bool bad = false;
+#pragma unroll
+  for (int q = 0; q < 4; q++) {
+    const int kk = 2 * lane + (q & 1) + 64 * (q >> 1);
+    v[q] = (col < n && kk < k) ? B[static_cast<long long>(col) * ldb + kk] : 0.0;
+    x[q] = kk < k ? xk[kk] : 0;
+    if (x[q] == EXP_ZERO) x[q] = 0;
+    const int e = exponent_of(v[q]);
+    if (e == EXP_NONFINITE) bad = true;
+    else if (e != EXP_ZERO) mx = max(mx, e - x[q]);
+  }
+  for (int o = 16; o > 0; o >>= 1) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+  bad = __any_sync(0xffffffffu, bad);
+  if (lane == 0) scale[col] = bad ? EXP_NONFINITE : mx;
+#pragma unroll
+  for (int p = 0; p < 2; p++) {
+    const int kk = 2 * lane + 64 * p;
+    if (kk >= kpad) continue;
+    __nv_bfloat16 d0[S_SLICES], d1[S_SLICES];
+    digits_of(fixed_point(v[2 * p], mx + x[2 * p]), d0);
+    digits_of(fixed_point(v[2 * p + 1], mx + x[2 * p + 1]), d1);
+#pragma unroll
+    for (int s = 0; s < S_SLICES; s++)
+      *reinterpret_cast<__nv_bfloat162*>(out + (static_cast<long long>(s) * npad + col) * kpad + kk) =
+          __nv_bfloat162(d0[s], d1[s]);
+  }
+}
+
+// Slices of A (m x k, column-major): out[s][row][kk] and the rows' scales; 32
+// rows a CTA, staged so that reads run along rows and writes along kk.
+constexpr int SA_ROWS = 32;
+__global__ void __launch_bounds__(256) slice_pack_a(const double* __restrict__ A, long long lda, int m, int k,
+                                                    int kpad, int mpad, const int* __restrict__ xk,
+                                                    __nv_bfloat16* __restrict__ out, int* __restrict__ scale) {
+  __shared__ double t[S_MAXK][SA_ROWS + 1];
+  __shared__ int x[S_MAXK], part[8][SA_ROWS], sc[SA_ROWS];
+  const int r0 = blockIdx.x * SA_ROWS, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  for (int e = threadIdx.x; e < S_MAXK; e += blockDim.x) {
+    const int v = e < k ? xk[e] : 0;
+    x[e] = v == EXP_ZERO ? 0 : v;
+  }
+  __syncthreads();
+  int mx = EXP_ZERO;
+  for (int kk = w; kk < kpad; kk += 8) {
+    const double v = (kk < k && r0 + lane < m) ? A[static_cast<long long>(kk) * lda + r0 + lane] : 0.0;
+    t[kk][lane] = v;
+    const int e = exponent_of(v);
+    if (e == EXP_NONFINITE) mx = EXP_NONFINITE;
+    else if (e != EXP_ZERO) mx = max(mx, e + x[kk]);
+  }
+  part[w][lane] = mx;
+  __syncthreads();
+  if (w == 0) {
+    for (int q = 1; q < 8; q++) mx = max(mx, part[q][lane]);
+    sc[lane] = mx;
+    scale[r0 + lane] = mx;
+  }
+  __syncthreads();
+  const int pairs = kpad / 2;
+  for (int e = threadIdx.x; e < SA_ROWS * pairs; e += blockDim.x) {
+    const int r = e / pairs, kk = 2 * (e - r * pairs), s0 = sc[r];
+    const bool some = s0 != EXP_NONFINITE && s0 != EXP_ZERO;
+    __nv_bfloat16 d0[S_SLICES], d1[S_SLICES];
+    digits_of(some ? fixed_point(t[kk][r], s0 - x[kk]) : 0, d0);
+    digits_of(some ? fixed_point(t[kk + 1][r], s0 - x[kk + 1]) : 0, d1);
+#pragma unroll
+    for (int s = 0; s < S_SLICES; s++)
+      *reinterpret_cast<__nv_bfloat162*>(out + (static_cast<long long>(s) * mpad + r0 + r) * kpad + kk) =
+          __nv_bfloat162(d0[s], d1[s]);
+  }
+}
+
+// ------------------------------------------------------------- the product --
+__device__ __forceinline__ unsigned long long s_now() {
+  unsigned long long t;
+  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+  return t;
+}
+
+// Bounded wait for phase `parity` of an mbarrier; false when it ran out.
+__device__ __forceinline__ bool s_wait(uint64_t* bar, uint32_t parity) {
+  const uint32_t a = smem_addr(bar);
+  uint32_t done = 0;
+  unsigned long long t0 = 0;
+  for (int spin = 0;; spin++) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}\n"
+        : "=r"(done)
+        : "r"(a), "r"(parity)
+        : "memory");
+    if (done) return true;
+    if (spin == 0) t0 = s_now();
+    else if ((spin & 255) == 0 && s_now() - t0 > S_WAIT_NS) return false;
+  }
+}
+
+__device__ __forceinline__ void s_load3(void* dst, const CUtensorMap* map, int x, int y, uint64_t* bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(
+          smem_addr(dst)),
+      "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(0), "r"(smem_addr(bar))
+      : "memory");
+}
+
+// K-major operand, rows of 64 bytes, 64-byte swizzle: 8-row groups 512 bytes
+// apart.
+__device__ __forceinline__ uint64_t sw64_desc(uint32_t saddr) {
+  uint64_t d = 0;
+  d |= static_cast<uint64_t>((saddr & 0x3FFFF) >> 4);
+  d |= static_cast<uint64_t>(1) << 16;
+  d |= static_cast<uint64_t>(512 >> 4) << 32;
+  d |= static_cast<uint64_t>(1) << 46;
+  d |= static_cast<uint64_t>(4) << 61;  // SWIZZLE_64B
+  return d;
+}
+
+// D = F32, A = B = BF16, both K-major.
+__device__ constexpr uint32_t bf16_idesc(int M, int N) {
+  return (1u << 4) | (1u << 7) | (1u << 10) | (static_cast<uint32_t>(N >> 3) << 17) |
+         (static_cast<uint32_t>(M >> 4) << 24);
+}
+
+__device__ __forceinline__ void tmem_load8(uint32_t addr, uint32_t (&r)[8]) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+               : "r"(addr));
+}
+
+__global__ void __launch_bounds__(S_THREADS, 1)
+    f64_update_sliced(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB,
+                      const int* __restrict__ ea, const int* __restrict__ fb, double* __restrict__ C, long long ldc,
+                      int m, int n, int nkc, int ntm, int ntiles, int* __restrict__ err) {
+  extern __shared__ __align__(1024) unsigned char s_raw[];
+  char* base = reinterpret_cast<char*>((reinterpret_cast<uintptr_t>(s_raw) + 1023) & ~uintptr_t(1023));
+  __shared__ uint64_t op_full[S_NST], op_empty[S_NST], acc_full, acc_empty, drained;
+  __shared__ uint32_t tmem_base_sh;
+  __shared__ int abort_flag;
+  volatile int* abort_v = &abort_flag;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (threadIdx.x == 0) {
+    abort_flag = 0;
+    for (int i = 0; i < S_NST; i++) {
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(&op_full[i])));
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(&op_empty[i])));
+    }
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(&acc_full)));
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(&drained)));
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 8;" ::"r"(smem_addr(&acc_empty)));  // the epilogue's warps
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&mapA)) : "memory");
+    asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&mapB)) : "memory");
+  }
+  if (warp == 1) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(&tmem_base_sh)),
+                 "r"(512));
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const uint32_t tmem = tmem_base_sh;
+
+  if (warp == 0) {
+    if (lane == 0) {  // ------------------------------------------- producer
+      int g = 0;
+      for (int tile = blockIdx.x; tile < ntiles && !*abort_v; tile += gridDim.x) {
+        const int tm = tile % ntm, tn = tile / ntm;
+        for (int kc = 0; kc < nkc; kc++, g++) {
+          const int st = g % S_NST, use = g / S_NST;
+          if (use > 0 && !s_wait(&op_empty[st], (use - 1) & 1)) {
+            *abort_v = 1;
+            break;
+          }
+          char* sp = base + st * S_STAGE;
+          asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_addr(&op_full[st])),
+                       "r"(S_STAGE)
+                       : "memory");
+          s_load3(sp, &mapA, kc * S_KC, tm * S_M, &op_full[st]);
+          s_load3(sp + S_SLICES * S_A_SLICE, &mapB, kc * S_KC, tn * S_N, &op_full[st]);
+        }
+      }
+      // no copy may be in flight when the CTA leaves
+      for (int st = 0; st < S_NST; st++) {
+        const int uses = (g + S_NST - 1 - st) / S_NST;
+        if (uses > 0 && !s_wait(&op_full[st], (uses - 1) & 1)) *abort_v = 1;
+      }
+    }
+  } else if (warp == 1) {
+    if (lane == 0) {  // ----------------------------------------- MMA issuer
+      const uint32_t idesc = bf16_idesc(S_M, S_N);
+      int it = 0, g = 0;
+      for (int tile = blockIdx.x; tile < ntiles && !*abort_v; tile += gridDim.x, it++) {
+        if (it > 0 && !s_wait(&acc_empty, (it - 1) & 1)) {
+          *abort_v = 1;
+          break;
+        }
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        bool ok = true;
+        for (int kc = 0; kc < nkc; kc++, g++) {
+          const int st = g % S_NST;
+          if (!s_wait(&op_full[st], (g / S_NST) & 1)) {
+            ok = false;
+            break;
+          }
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+          const uint32_t sa = smem_addr(base + st * S_STAGE), sb = sa + S_SLICES * S_A_SLICE;
+          const uint64_t a0 = sw64_desc(sa), b0 = sw64_desc(sb);
+          for (int o = 0; o < S_SLICES; o++) {  // order o + 2: slices i and o - i
+            const uint32_t d = tmem + static_cast<uint32_t>(o * S_N);
+            for (int i = 0; i <= o; i++) {
+              const uint64_t ad = a0 + static_cast<uint64_t>((i * S_A_SLICE) >> 4);
+              const uint64_t bd = b0 + static_cast<uint64_t>(((o - i) * S_B_SLICE) >> 4);
+#pragma unroll
+              for (int kk = 0; kk < S_KC / 16; kk++) {
+                const uint32_t accum = (kc | i | kk) ? 1u : 0u;
+                asm volatile(
+                    "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+                    "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(d),
+                    "l"(ad + static_cast<uint64_t>(2 * kk)), "l"(bd + static_cast<uint64_t>(2 * kk)), "r"(idesc),
+                    "r"(accum));
+              }
+            }
+          }
+          asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
+                           smem_addr(&op_empty[st]))
+                       : "memory");
+        }
+        if (!ok) {
+          *abort_v = 1;
+          break;
+        }
+        asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
+                         smem_addr(&acc_full))
+                     : "memory");
+      }
+      // nor an MMA when the tensor memory is freed
+      asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
+                       smem_addr(&drained))
+                   : "memory");
+      if (!s_wait(&drained, 0)) *abort_v = 1;
+    }
+  } else {  // ---------------------------------------------- epilogue (2-9)
+    const int quarter = warp & 3, half = (warp - 2) >> 2;
+    int it = 0;
+    for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x, it++) {
+      const int tm = tile % ntm, tn = tile / ntm;
+      if (!s_wait(&acc_full, it & 1) || *abort_v) {
+        *abort_v = 1;
+        break;
+      }
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      long long v[32];
+      const uint32_t t0 = tmem + (static_cast<uint32_t>(quarter * 32) << 16) + static_cast<uint32_t>(half * 32);
+#pragma unroll
+      for (int c8 = 0; c8 < 32; c8 += 8) {
+        uint32_t r[S_SLICES][8];
+#pragma unroll
+        for (int o = 0; o < S_SLICES; o++) tmem_load8(t0 + static_cast<uint32_t>(o * S_N + c8), r[o]);
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+        for (int q = 0; q < 8; q++) {
+          // orders 2..7 weigh 2^40 .. 1, orders 8 and 9 2^-8 and 2^-16
+          long long hi = 0;
+#pragma unroll
+          for (int o = 0; o < 6; o++) hi = (hi << 8) + __float2int_rn(__uint_as_float(r[o][q]));
+          const long long lo = (static_cast<long long>(__float2int_rn(__uint_as_float(r[6][q]))) << 8) +
+                               __float2int_rn(__uint_as_float(r[7][q]));
+          v[c8 + q] = hi + ((lo + 32768) >> 16);
+        }
+      }
+      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+      __syncwarp();
+      if (lane == 0)
+        asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_addr(&acc_empty)) : "memory");
+      // C -= v 2^(ea + fb - 52)
+      const int row = tm * S_M + quarter * 32 + lane;
+      const int col0 = tn * S_N + half * 32;
+      const int er = ea[row];
+      if (row < m) {
+        double* cp = C + static_cast<long long>(col0) * ldc + row;
+#pragma unroll
+        for (int c8 = 0; c8 < 32; c8 += 8) {
+          double c[8];
+#pragma unroll
+          for (int q = 0; q < 8; q++) c[q] = col0 + c8 + q < n ? cp[static_cast<long long>(c8 + q) * ldc] : 0.0;
+#pragma unroll
+          for (int q = 0; q < 8; q++) {
+            const int ec = fb[col0 + c8 + q];
+            const int e = er + ec - 52 + 1023;
+            if (er == EXP_NONFINITE || ec == EXP_NONFINITE) {
+              c[q] = nan("");
+            } else if (v[c8 + q] != 0) {  // never with a zero row or column
+              const double x = static_cast<double>(v[c8 + q]);
+              if (e > 0 && e < 2047)
+                c[q] = fma(-x, __longlong_as_double(static_cast<long long>(e) << 52), c[q]);
+              else
+                c[q] -= scalbn(x, e - 1023);
+            }
+          }
+#pragma unroll
+          for (int q = 0; q < 8; q++)
+            if (col0 + c8 + q < n) cp[static_cast<long long>(c8 + q) * ldc] = c[q];
+        }
+      }
+    }
+  }
+  __syncthreads();
+  if (threadIdx.x == 0 && *abort_v) atomicExch(err, 1);
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512));
+}
+
+// 3-D bf16 map of out[slice][row][kk]: boxes of 32 x rows x all slices.
+void make_slice_map(CUtensorMap* map, const void* ptr, int kpad, int rows, int box_rows) {
+  const cuuint64_t dims[3] = {static_cast<cuuint64_t>(kpad), static_cast<cuuint64_t>(rows),
+                              static_cast<cuuint64_t>(S_SLICES)};
+  const cuuint64_t strides[2] = {static_cast<cuuint64_t>(kpad) * 2, static_cast<cuuint64_t>(kpad) * 2 * rows};
+  const cuuint32_t box[3] = {S_KC, static_cast<cuuint32_t>(box_rows), S_SLICES};
+  const cuuint32_t estr[3] = {1, 1, 1};
+  auto fn = tensor_map_encoder();
+  if (!fn) throw KdError(KD_ERR_CUDA, "cuTensorMapEncodeTiled is not available");
+  const CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(ptr), dims, strides, box, estr,
+                        CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                        CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) throw KdError(KD_ERR_CUDA, "cuTensorMapEncodeTiled failed (" + std::to_string(r) + ")");
+}
+
+}  // namespace
+
+bool f64_sliced_update_possible(int k) { return k > 0 && k <= S_MAXK && tensor_map_encoder() != nullptr; }
+
+void f64_sliced_update(Context* ctx, int m, int n, int k, const double* A, long long lda, const double* B,
+                       long long ldb, double* C, long long ldc) {
+  if (m <= 0 || n <= 0 || k <= 0) return;
+  cudaStream_t s = ctx->stream();
+  const int kpad = (k + S_KC - 1) / S_KC * S_KC;
+  const int mpad = (m + S_M - 1) / S_M * S_M, npad = (n + S_N - 1) / S_N * S_N;
+  // slices, then the scales (rows of A, columns of B), then the row scaling of B
+  const size_t abytes = static_cast<size_t>(S_SLICES) * mpad * kpad * 2, bbytes = static_cast<size_t>(S_SLICES) * npad * kpad * 2;
+  char* wa = static_cast<char*>(ctx->workspace(Context::WS_TC_A, abytes + sizeof(int) * mpad));
+  char* wb = static_cast<char*>(ctx->workspace(Context::WS_TC_B, bbytes + sizeof(int) * (static_cast<size_t>(npad) + S_MAXK)));
+  auto* as = reinterpret_cast<__nv_bfloat16*>(wa);
+  auto* bs = reinterpret_cast<__nv_bfloat16*>(wb);
+  int* ea = reinterpret_cast<int*>(wa + abytes);
+  int* fb = reinterpret_cast<int*>(wb + bbytes);
+  int* xk = fb + npad;
+  bool fresh = false;
+  int* err = static_cast<int*>(ctx->workspace(Context::WS_TC_FLAG, sizeof(int), &fresh));
+  if (fresh) cuda_check(cudaMemsetAsync(err, 0, sizeof(int), s), "memset err");
+  static std::once_flag attr;
+  std::call_once(attr, [] {
+    cuda_check(cudaFuncSetAttribute(f64_update_sliced, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    static_cast<int>(S_SMEM)),
+               "cudaFuncSetAttribute(sliced update)");
+  });
+  slice_fill<<<1, S_MAXK, 0, s>>>(xk, S_MAXK, EXP_ZERO);
+  const int cols = 32;
+  slice_row_exponents<<<(n + cols - 1) / cols, S_MAXK, 0, s>>>(B, ldb, k, n, cols, xk);
+  slice_pack_b<<<(npad + 7) / 8, 256, 0, s>>>(B, ldb, k, n, kpad, npad, xk, bs, fb);
+  slice_pack_a<<<mpad / SA_ROWS, 256, 0, s>>>(A, lda, m, k, kpad, mpad, xk, as, ea);
+  CUtensorMap mA, mB;
+  make_slice_map(&mA, as, kpad, mpad, S_M);
+  make_slice_map(&mB, bs, kpad, npad, S_N);
+  const int ntm = mpad / S_M, ntiles = ntm * (npad / S_N);
+  const int grid = ntiles < ctx->sms() ? ntiles : ctx->sms();
+  f64_update_sliced<<<grid, S_THREADS, S_SMEM, s>>>(mA, mB, ea, fb, C, ldc, m, n, kpad / S_KC, ntm, ntiles, err);
+  ctx->launches += 5;
+  cuda_check(cudaGetLastError(), "sliced FP64 trailing update");
+}
+
+}  // namespace kd

@@ -516,29 +516,11 @@ __global__ void __launch_bounds__(P_THREADS, 1)
   if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(256));
 }
 
-// cuTensorMapEncodeTiled through the runtime's driver entry point (no
-// link-time dependency on the driver library).
-using EncodeTiledFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                                   const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
-                                   CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-EncodeTiledFn encode_fn() {
-  static EncodeTiledFn fn = nullptr;
-  static std::once_flag once;
-  std::call_once(once, [] {
-    void* p = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &p, 12000, cudaEnableDefault, &q) == cudaSuccess &&
-        q == cudaDriverEntryPointSuccess)
-      fn = reinterpret_cast<EncodeTiledFn>(p);
-  });
-  return fn;
-}
-
 // 2-D FP32 tensor map: inner extent `inner` (contiguous), `outer` rows
 // `stride_bytes` apart, box box0 x box1.
 void make_map(CUtensorMap* m, const void* ptr, long long inner, long long outer, long long stride_bytes, int box0,
               int box1, bool swizzle128) {
-  EncodeTiledFn fn = encode_fn();
+  TensorMapEncoder fn = tensor_map_encoder();
   if (!fn) throw KdError(KD_ERR_CUDA, "cuTensorMapEncodeTiled is not available");
   cuuint64_t dims[2] = {static_cast<cuuint64_t>(inner), static_cast<cuuint64_t>(outer)};
   cuuint64_t strides[1] = {static_cast<cuuint64_t>(stride_bytes)};
@@ -559,13 +541,26 @@ int grid_for(long long n) {
 
 }  // namespace
 
+TensorMapEncoder tensor_map_encoder() {
+  static TensorMapEncoder fn = nullptr;
+  static std::once_flag once;
+  std::call_once(once, [] {
+    void* p = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &p, 12000, cudaEnableDefault, &q) == cudaSuccess &&
+        q == cudaDriverEntryPointSuccess)
+      fn = reinterpret_cast<TensorMapEncoder>(p);
+  });
+  return fn;
+}
+
 bool tf32_gemm_supported(int k) { return k > 0 && k <= TC_MAXK; }
 
 bool tf32x3_gemm_possible(int k, const float* C, long long ldc, int m, int c_rows_writable) {
   const int kpad = ((k + TC_KBLK - 1) / TC_KBLK) * TC_KBLK;
   // the persistent pipeline's conditions (it streams k, so k may reach TC_MAXK_P)
   return k > 0 && kpad <= TC_MAXK_P && reinterpret_cast<uintptr_t>(C) % 16 == 0 && ldc % 4 == 0 &&
-         (m + 3) / 4 * 4 <= c_rows_writable && encode_fn() != nullptr;
+         (m + 3) / 4 * 4 <= c_rows_writable && tensor_map_encoder() != nullptr;
 }
 
 int tf32_update_max_clusters16() {
@@ -630,7 +625,7 @@ void tf32_gemm_update(Context* ctx, int m, int n, int k, const float* A, long lo
   // to 4 may be written (with their unchanged values or zeros), so the
   // persistent path needs them to be scratch (c_rows_writable).
   const int m4 = (m + 3) / 4 * 4;
-  if (reinterpret_cast<uintptr_t>(C) % 16 == 0 && ldc % 4 == 0 && m4 <= c_rows_writable && encode_fn()) {
+  if (reinterpret_cast<uintptr_t>(C) % 16 == 0 && ldc % 4 == 0 && m4 <= c_rows_writable && tensor_map_encoder()) {
     // persistent TMA pipeline
     CUtensorMap mA, mB, mAl, mBl, mC;
     make_map(&mA, at, kpad, mpad, static_cast<long long>(kpad) * 4, TC_KBLK, TC_M, true);

@@ -3,6 +3,7 @@
 // (FP32 accumulation in tensor memory); otherwise a plain FP32 product.
 #pragma once
 #include <cublas_v2.h>
+#include <cuda.h>
 
 #include "kd_context.hpp"
 
@@ -35,5 +36,19 @@ bool tf32x3_gemm_possible(int k, const float* C, long long ldc, int m, int c_row
 // Returns (and clears) the flag a CTA sets when its wait for the tensor-core
 // results ran out of polls.
 int tf32_gemm_error_flag(Context* ctx);
+
+// C -= A * B in FP64 (column-major, k <= 128) by exact products of 8-bit
+// slices on the tensor cores (kd_gemm_f64.cu); a wait that ran out sets the
+// flag that tf32_gemm_error_flag reads.
+bool f64_sliced_update_possible(int k);
+void f64_sliced_update(Context* ctx, int m, int n, int k, const double* A, long long lda, const double* B,
+                       long long ldb, double* C, long long ldc);
+
+// cuTensorMapEncodeTiled through the runtime's driver entry point (no
+// link-time dependency on the driver library); null when there is none.
+using TensorMapEncoder = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
+                                      const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
+                                      CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+TensorMapEncoder tensor_map_encoder();
 
 }  // namespace kd
