@@ -27,39 +27,112 @@ namespace kd {
 
 namespace {
 
-// A12 := L11^{-1} A12, L11 unit lower (nb x nb at (j0, j0)), A12 = rows
-// [j0, j0+nb) of columns [c0, c1).  One thread per column, TRSM_COLS columns
-// per CTA; L11 and the column tile live in shared memory.
-constexpr int TRSM_COLS = 64;
-template <class T>
-__global__ void trsm_unit_lower(T* __restrict__ A, long long ld, int j0, int nbk, int c0, int c1) {
-  extern __shared__ unsigned char smraw[];
-  double* L = reinterpret_cast<double*>(smraw);     // nbk x nbk, row-major L[i*nbk+k]
-  double* X = L + nbk * nbk;                        // nbk x TRSM_COLS, X[i*TRSM_COLS + c]
-  int cbase = c0 + blockIdx.x * TRSM_COLS;
-  for (int e = threadIdx.x; e < nbk * nbk; e += blockDim.x) {
-    int i = e % nbk, k = e / nbk;  // column-major read of L11
-    L[i * nbk + k] = static_cast<double>(A[static_cast<long long>(j0 + k) * ld + j0 + i]);
-  }
-  for (int e = threadIdx.x; e < nbk * TRSM_COLS; e += blockDim.x) {
-    int i = e % nbk, c = e / nbk;
-    int col = cbase + c;
-    X[i * TRSM_COLS + c] = (col < c1) ? static_cast<double>(A[static_cast<long long>(col) * ld + j0 + i]) : 0.0;
-  }
-  __syncthreads();
-  int c = threadIdx.x;
-  if (c < TRSM_COLS) {
-    for (int i = 1; i < nbk; i++) {
-      double s = X[i * TRSM_COLS + c];
-      for (int k = 0; k < i; k++) s -= L[i * nbk + k] * X[k * TRSM_COLS + c];
-      X[i * TRSM_COLS + c] = s;
+// A CTA's candidate for one column of a grid panel.
+struct PanelRecord {
+  unsigned long long key;  // of its modulus
+  unsigned long long row;
+};
+
+// U12 = L11^-1 A12 (L11 unit lower, jb <= 96) for FP64 factors, 16 columns a
+// CTA.  By 32-row chunks: the chunk's own triangle with 8 lanes a column (rows
+// l, l + 8, l + 16, l + 24; each finished entry broadcast by a shuffle), then
+// its products with the rows below as a register-tiled product, every entry
+// summed in column order as by plain substitution.
+// Bound: the FP64 pipe (4,560 multiply-adds a column); three CTAs an SM.  One
+// thread a column on 64-column CTAs, as before, was bound by its chain of
+// dependent multiply-adds instead (0.23 ms at any width).
+constexpr int TD_COLS = 16, TD_THREADS = 128, TD_LD = 97;
+constexpr size_t TD_SMEM = sizeof(double) * (6 * 32 * 32 + TD_COLS * TD_LD);
+__global__ void __launch_bounds__(TD_THREADS) trsm_chunk_f64(double* __restrict__ A, long long ld, int j0, int jb,
+                                                             int c0, int c1) {
+  extern __shared__ __align__(16) double td_sm[];
+  double* LT = td_sm;                // block (rb, kb) of L11, transposed: [k][r]
+  double* X = td_sm + 6 * 32 * 32;   // X[c * TD_LD + row]
+  const int tid = threadIdx.x, cb = c0 + blockIdx.x * TD_COLS;
+  for (int blk = 0; blk < 6; blk++) {
+    const int rb = blk < 1 ? 0 : blk < 3 ? 1 : 2, kb = blk - rb * (rb + 1) / 2;
+    double v[8];
+#pragma unroll
+    for (int u = 0; u < 8; u++) {
+      const int e = tid + u * TD_THREADS, r = rb * 32 + (e & 31), k = kb * 32 + (e >> 5);
+      v[u] = (r < jb && k < jb) ? A[static_cast<long long>(j0 + k) * ld + j0 + r] : 0.0;
     }
+#pragma unroll
+    for (int u = 0; u < 8; u++) LT[blk * 1024 + tid + u * TD_THREADS] = v[u];
+  }
+  for (int e = tid; e < TD_COLS * 96; e += TD_THREADS) {
+    const int c = e / 96, i = e - c * 96;
+    X[c * TD_LD + i] = (i < jb && cb + c < c1) ? A[static_cast<long long>(cb + c) * ld + j0 + i] : 0.0;
   }
   __syncthreads();
-  for (int e = threadIdx.x; e < nbk * TRSM_COLS; e += blockDim.x) {
-    int i = e % nbk, cc = e / nbk;
-    int col = cbase + cc;
-    if (col < c1) A[static_cast<long long>(col) * ld + j0 + i] = static_cast<T>(X[i * TRSM_COLS + cc]);
+  const int l = tid & 7, col = tid >> 3, lane = tid & 31;
+  for (int c = 0; c < 3; c++) {
+    if (c * 32 >= jb) break;
+    {
+      const double* L = LT + (c * (c + 1) / 2 + c) * 1024;
+      double* xc = X + col * TD_LD + c * 32;
+      double x[4];
+#pragma unroll
+      for (int q = 0; q < 4; q++) x[q] = xc[l + 8 * q];
+#pragma unroll
+      for (int k = 0; k < 31; k++) {
+        const double xk = __shfl_sync(0xffffffffu, x[k >> 3], (lane & 24) | (k & 7));
+#pragma unroll
+        for (int q = k >> 3; q < 4; q++)
+          if (q > (k >> 3) || l > (k & 7)) x[q] = fma(-L[k * 32 + l + 8 * q], xk, x[q]);
+      }
+#pragma unroll
+      for (int q = 0; q < 4; q++) xc[l + 8 * q] = x[q];
+    }
+    __syncthreads();
+    const double* xk = X + c * 32;
+    if (c == 0) {  // rows 32..95: 4 rows x 2 columns a thread
+      const int r = (tid & 15) * 4, cc = (tid >> 4) * 2, rb = 1 + (r >> 5);
+      const double* L = LT + (rb * (rb + 1) / 2) * 1024 + (r & 31);
+      double acc[2][4];
+#pragma unroll
+      for (int u = 0; u < 2; u++)
+#pragma unroll
+        for (int q = 0; q < 4; q++) acc[u][q] = X[(cc + u) * TD_LD + 32 + r + q];
+#pragma unroll 4
+      for (int k = 0; k < 32; k++) {
+        const double2 a = *reinterpret_cast<const double2*>(L + k * 32), b = *reinterpret_cast<const double2*>(L + k * 32 + 2);
+#pragma unroll
+        for (int u = 0; u < 2; u++) {
+          const double x = xk[(cc + u) * TD_LD + k];
+          acc[u][0] = fma(-a.x, x, acc[u][0]);
+          acc[u][1] = fma(-a.y, x, acc[u][1]);
+          acc[u][2] = fma(-b.x, x, acc[u][2]);
+          acc[u][3] = fma(-b.y, x, acc[u][3]);
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < 2; u++)
+#pragma unroll
+        for (int q = 0; q < 4; q++) X[(cc + u) * TD_LD + 32 + r + q] = acc[u][q];
+    } else if (c == 1) {  // rows 64..95: 4 rows x 1 column a thread
+      const int r = (tid & 7) * 4, cc = tid >> 3;
+      const double* L = LT + (2 * 3 / 2 + 1) * 1024 + r;
+      double acc[4];
+#pragma unroll
+      for (int q = 0; q < 4; q++) acc[q] = X[cc * TD_LD + 64 + r + q];
+#pragma unroll 4
+      for (int k = 0; k < 32; k++) {
+        const double2 a = *reinterpret_cast<const double2*>(L + k * 32), b = *reinterpret_cast<const double2*>(L + k * 32 + 2);
+        const double x = xk[cc * TD_LD + k];
+        acc[0] = fma(-a.x, x, acc[0]);
+        acc[1] = fma(-a.y, x, acc[1]);
+        acc[2] = fma(-b.x, x, acc[2]);
+        acc[3] = fma(-b.y, x, acc[3]);
+      }
+#pragma unroll
+      for (int q = 0; q < 4; q++) X[cc * TD_LD + 64 + r + q] = acc[q];
+    }
+    __syncthreads();
+  }
+  for (int e = tid; e < TD_COLS * 96; e += TD_THREADS) {
+    const int c = e / 96, i = e - c * 96;
+    if (i < jb && cb + c < c1) A[static_cast<long long>(cb + c) * ld + j0 + i] = X[c * TD_LD + i];
   }
 }
 
@@ -776,8 +849,8 @@ DenseLU::DenseLU(Context* ctx) : ctx_(ctx) {
   cuda_check(cudaDeviceGetAttribute(&nsm_, cudaDevAttrMultiProcessorCount, dev), "SM count");
   // panel exchange slots (sized for FP64 rows), barrier counter, error flag,
   // then the row-move list of one panel
-  const size_t slot_bytes = sizeof(double) * (2 * 128 * static_cast<size_t>(nsm_) + 2 * nsm_ + 2 * 128) +
-                            sizeof(int) * 2 * static_cast<size_t>(nsm_) + 32;
+  const size_t slot_bytes = sizeof(double) * (2 * 128 * static_cast<size_t>(nsm_) + 2 * 128) +
+                            sizeof(PanelRecord) * 2 * static_cast<size_t>(nsm_) + 32;
   const size_t map_bytes = sizeof(int) * (1 + 4 * 128) + 60;  // + padding to 16 bytes
   cuda_check(cudaMalloc(&slot_mem_, slot_bytes + map_bytes + 32), "cudaMalloc(panel slots)");
   cuda_check(cudaMemsetAsync(slot_mem_, 0, slot_bytes + map_bytes + 32, ctx_->stream()), "memset panel slots");
@@ -944,32 +1017,43 @@ __global__ void panel_cluster_kernel(T* __restrict__ A, long long ld, int N, int
 // ---- panel over the whole GPU (cooperative launch) ------------------------
 // CTA b owns rows [j0 + b*per, j0 + (b+1)*per) of the panel and keeps them in
 // shared memory, column-major (tile[k*per + r]), for the whole panel.  Per
-// column j, ONE grid barrier:
-//   before it, every CTA publishes its local arg-max |a(i, j)| with the full
-//   panel row of that candidate, and the CTA owning row j publishes row j
-//   (double-buffered slots, indexed by the column's parity);
-//   after it, every CTA reduces the candidates in the same order (largest
-//   modulus, ties to the lowest row, as idamax), reads the winning row as the
-//   pivot row, the owner of the pivot row takes row j in its place, the owner
-//   of row j takes the pivot row, and each CTA scales and rank-1-updates its
-//   own rows.
-// Slot reuse is safe: a CTA writes slot (jj & 1) at column jj only after
-// barrier jj-1, by which every CTA has finished reading that slot (column
-// jj-2).  Cross-CTA data is read with L1-bypassing loads.
-constexpr int GP_THREADS = 256;
+// column j one exchange:
+//   warp 0 finds the CTA's arg-max |a(i, j)|, stores that candidate's full
+//   panel row (the CTA owning row j also row j; double-buffered slots, indexed
+//   by the column's parity) and its record {modulus, row}, and arrives at a
+//   counter;
+//   when all have arrived, one lane per CTA reads the records, every CTA
+//   reduces them to the same winner (largest modulus, ties to the lowest row,
+//   as idamax) and reads the winning row as the pivot row; the owner of the
+//   pivot row takes row j in its place, the owner of row j takes the pivot row,
+//   and each CTA scales and rank-1-updates its own rows.
+// Slot reuse is safe: a CTA writes slot (jj & 1) at column jj only after all
+// have arrived at column jj-1, by which every CTA has finished reading that
+// slot (column jj-2).  Cross-CTA data is read with L1-bypassing loads.
+// Bound: latency.  Of about 9,000 cycles a column (FP64, 40 rows a CTA) the
+// update takes 2,700 (1,500 of the FP64 pipe), storing and arriving 1,350, the
+// counter 1,400, records 700, the pivot row 1,100.  Moduli are compared as
+// integers and reduced by redux (FP64 compares made the two arg-max 1,300
+// cycles each), the reciprocal is formed once beside the row's load and not by
+// every warp, and the row moves are listed here: 692 -> 405 us per FP64 panel at
+// N = 8,000, FP32 panels of up to 40,081 rows 412 -> 327 us on average.  Polling
+// all records instead of one counter was slower (560 us): 152 CTAs reading
+// 152 records each keep the L2 slices busy that hold them.
+constexpr int GP_THREADS = 512;
+constexpr int GP_POLL_WARPS = 6;  // one lane a CTA: at most 192 CTAs
 constexpr int GP_MIN_ROWS = 32;
 constexpr size_t GP_MAX_SMEM = 200 * 1024;
+constexpr size_t GP_MIN_SMEM = 8 * 1024;
 
 template <class T>
 struct PanelSlots {
-  T* cand_rows;     // [2][nblk][jb]
-  double* cand_v;   // [2][nblk]
-  int* cand_i;      // [2][nblk]
-  T* jrow;          // [2][jb]
-  unsigned* bar;    // arrival counter, zeroed before the launch
-  int* err;         // set when a barrier wait runs out
-  unsigned long long wait_ns;  // limit of one barrier wait (Context::grid_wait_ns)
-  unsigned stall;   // added to every barrier target (Context::stall_waits)
+  T* cand_rows;      // [2][nblk][jb]
+  PanelRecord* rec;  // [2][nblk]
+  T* jrow;           // [2][jb]
+  int* err;          // set when a wait runs out
+  unsigned long long wait_ns;  // limit of one wait (Context::grid_wait_ns)
+  unsigned* count;   // arrivals, zeroed before the launch
+  unsigned stall;    // added to every arrival target (Context::stall_waits)
 };
 
 __device__ __forceinline__ unsigned long long globaltimer_ns() {
@@ -978,72 +1062,45 @@ __device__ __forceinline__ unsigned long long globaltimer_ns() {
   return t;
 }
 
-// Grid-wide barrier of a cooperative launch (all CTAs resident): the CTA's
-// writes are published by thread 0's release increment (after the block
-// barrier), the other CTAs' writes acquired by its polling loads.  Returns
-// false, with *err set, when the counter did not reach `target` within
-// limit_ns; the caller then leaves its loops.
-__device__ bool grid_barrier(unsigned* bar, unsigned target, int* err, int* s_ok, unsigned long long limit_ns) {
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    asm volatile("red.release.gpu.global.add.u32 [%0], %1;" ::"l"(bar), "r"(1u) : "memory");
-    const unsigned long long t0 = globaltimer_ns();
-    int ok = 1;
-    for (unsigned it = 0;; it++) {
-      unsigned v;
-      asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(bar) : "memory");
-      if (v >= target) break;
-      if ((it & 31) == 31 && globaltimer_ns() - t0 > limit_ns) {
-        ok = 0;
-        atomicExch(err, 1);
-        break;
-      }
-      __nanosleep(20);
-    }
-    *s_ok = ok;
-  }
-  __syncthreads();
-  return *s_ok != 0;
-}
-
 template <class V>
 __device__ __forceinline__ bool better(V v, int i, V bv, int bi) {
   return v > bv || (v == bv && i < bi);
 }
 
-// Block-wide arg-max of (v, i) carrying a tag; every thread gets the result.
-template <class V>
-__device__ void block_argmax(V& v, int& i, int& tag, V* rv, int* ri, int* rt) {
-  for (int o = 16; o > 0; o >>= 1) {
-    V ov = __shfl_xor_sync(0xffffffffu, v, o);
-    int oi = __shfl_xor_sync(0xffffffffu, i, o);
-    int ot = __shfl_xor_sync(0xffffffffu, tag, o);
-    if (better(ov, oi, v, i)) {
-      v = ov;
-      i = oi;
-      tag = ot;
-    }
-  }
-  const int w = threadIdx.x >> 5;
-  if ((threadIdx.x & 31) == 0) {
-    rv[w] = v;
-    ri[w] = i;
-    rt[w] = tag;
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    for (int q = 1; q < static_cast<int>(blockDim.x >> 5); q++)
-      if (better(rv[q], ri[q], rv[0], ri[0])) {
-        rv[0] = rv[q];
-        ri[0] = ri[q];
-        rt[0] = rt[q];
-      }
-  }
-  __syncthreads();
-  v = rv[0];
-  i = ri[0];
-  tag = rt[0];
-  __syncthreads();
+// The modulus of v as an integer that orders the same way: 0 for NaN (never a
+// pivot), else its bits + 1.  Integer compares, because an FP64 compare costs
+// an FP64 instruction.
+__device__ __forceinline__ unsigned long long modulus_key(double v) {
+  const unsigned long long k = static_cast<unsigned long long>(__double_as_longlong(v)) & 0x7fffffffffffffffull;
+  return k > 0x7ff0000000000000ull ? 0ull : k + 1;
+}
+__device__ __forceinline__ unsigned long long modulus_key(float v) {
+  const unsigned k = __float_as_uint(v) & 0x7fffffffu;
+  return k > 0x7f800000u ? 0ull : static_cast<unsigned long long>(k) + 1;
+}
+constexpr unsigned long long KEY_OF_ZERO = 1;
+
+// Largest key, ties to the lowest row.
+struct Candidate {
+  unsigned long long key;
+  int row;
+};
+__device__ __forceinline__ Candidate better_of(const Candidate& a, const Candidate& b) {
+  return (b.key > a.key || (b.key == a.key && b.row < a.row)) ? b : a;
+}
+// The best of a warp, in every lane: three integer reductions in hardware.
+__device__ __forceinline__ Candidate warp_best(const Candidate& c) {
+  const unsigned hi = static_cast<unsigned>(c.key >> 32), lo = static_cast<unsigned>(c.key);
+  const unsigned mh = __reduce_max_sync(0xffffffffu, hi);
+  const unsigned ml = __reduce_max_sync(0xffffffffu, hi == mh ? lo : 0u);
+  const int row = __reduce_min_sync(0xffffffffu, hi == mh && lo == ml ? c.row : 0x7fffffff);
+  return Candidate{static_cast<unsigned long long>(mh) << 32 | ml, row};
+}
+__device__ __forceinline__ void modulus_of(unsigned long long key, double& v) {
+  v = __longlong_as_double(static_cast<long long>(key - 1));
+}
+__device__ __forceinline__ void modulus_of(unsigned long long key, float& v) {
+  v = __uint_as_float(static_cast<unsigned>(key - 1));
 }
 
 // Double-float arithmetic (a value is an unevaluated sum hi + lo of two
@@ -1477,112 +1534,6 @@ __global__ void __launch_bounds__(256) trsv_chain(const T* __restrict__ A, long 
   }
 }
 
-template <class T>
-__global__ void __launch_bounds__(GP_THREADS) panel_grid_kernel(T* __restrict__ A, long long ld, int N, int j0, int jb,
-                                                                int per, int* __restrict__ ipiv,
-                                                                int* __restrict__ info, PanelSlots<T> ps) {
-  extern __shared__ __align__(16) unsigned char gp_raw[];
-  T* tile = reinterpret_cast<T*>(gp_raw);
-  __shared__ T prow[128];
-  __shared__ T rv[GP_THREADS / 32];
-  __shared__ int ri[GP_THREADS / 32], rt[GP_THREADS / 32];
-  __shared__ int s_ok;
-  const int nblk = gridDim.x, b = blockIdx.x, tid = threadIdx.x, bd = blockDim.x;
-  const int r0 = j0 + b * per;
-  const int r1 = (r0 + per < N) ? r0 + per : N;
-  const int nr = r1 - r0;
-  for (int e = tid; e < jb * nr; e += bd) {
-    int k = e / nr, r = e % nr;
-    tile[k * per + r] = A[static_cast<long long>(j0 + k) * ld + r0 + r];
-    }
-  __syncthreads();
-  for (int jj = 0; jj < jb; jj++) {
-    const int j = j0 + jj;
-    const int slot = jj & 1;
-    // 1. local candidate
-    T best = T(-1);
-    int bi = N, tag = 0;
-    for (int i = (r0 > j ? r0 : j) + tid; i < r1; i += bd) {
-      T v = fabs(tile[jj * per + i - r0]);
-      if (better(v, i, best, bi)) {
-        best = v;
-        bi = i;
-      }
-    }
-    block_argmax(best, bi, tag, rv, ri, rt);
-    // 2. publish it (and row j when this CTA owns it)
-    T* mine = ps.cand_rows + (static_cast<size_t>(slot) * nblk + b) * jb;
-    if (bi < N)
-      for (int k = tid; k < jb; k += bd) mine[k] = tile[k * per + bi - r0];
-    if (tid == 0) {
-      ps.cand_v[slot * nblk + b] = static_cast<double>(best);
-      ps.cand_i[slot * nblk + b] = bi;
-    }
-    if (j >= r0 && j < r1)
-      for (int k = tid; k < jb; k += bd) ps.jrow[slot * jb + k] = tile[k * per + j - r0];
-    // 3. one barrier per column
-    if (!grid_barrier(ps.bar, static_cast<unsigned>(nblk) * (jj + 1) + ps.stall, ps.err, &s_ok, ps.wait_ns)) return;
-    // 4. every CTA reduces the candidates identically
-    best = T(-1);
-    bi = N;
-    tag = -1;
-    for (int t = tid; t < nblk; t += bd) {
-      T v = static_cast<T>(__ldcg(ps.cand_v + slot * nblk + t));
-      int ii = __ldcg(ps.cand_i + slot * nblk + t);
-      if (better(v, ii, best, bi)) {
-        best = v;
-        bi = ii;
-        tag = t;
-      }
-    }
-    block_argmax(best, bi, tag, rv, ri, rt);
-    int gi = bi;
-    if (gi >= N) {  // nothing usable below the diagonal: no swap
-      gi = j;
-      tag = -1;
-    }
-    if (b == 0 && tid == 0) {
-      ipiv[j] = gi;
-      if (!(best > T(0)) && *info == 0) *info = j + 1;  // zero (or NaN) pivot
-    }
-    // 5. pivot row, row exchange
-    const T* src = (tag >= 0) ? ps.cand_rows + (static_cast<size_t>(slot) * nblk + tag) * jb : ps.jrow + slot * jb;
-    for (int k = tid; k < jb; k += bd) prow[k] = __ldcg(src + k);
-    if (gi != j && gi >= r0 && gi < r1)
-      for (int k = tid; k < jb; k += bd) tile[k * per + gi - r0] = __ldcg(ps.jrow + slot * jb + k);
-    __syncthreads();
-    if (j >= r0 && j < r1)
-      for (int k = tid; k < jb; k += bd) tile[k * per + j - r0] = prow[k];
-    // 6. scale the column below the pivot, rank-1 update of the rest
-    const T piv = prow[jj];
-    const int rs = (r0 > j + 1) ? r0 : j + 1;
-    __syncthreads();
-    if (piv != T(0) && rs < r1) {
-      const T inv = T(1) / piv;
-      for (int i = rs + tid; i < r1; i += bd) tile[jj * per + i - r0] *= inv;
-      __syncthreads();
-      // thread -> (row, column phase): rows along the low 7 bits (conflict-free
-      // shared memory), columns strided by the number of phases
-      const int nrr = r1 - rs;
-      const int nph = bd >> 7, ph = tid >> 7;
-      for (int i0 = 0; i0 < nrr; i0 += 128) {
-        const int ii = i0 + (tid & 127);
-        if (ii < nrr) {
-          const int li = rs - r0 + ii;
-          const T l = tile[jj * per + li];
-          for (int k = jj + 1 + ph; k < jb; k += nph)
-            tile[k * per + li] = fma(-l, prow[k], tile[k * per + li]);
-        }
-      }
-    }
-    __syncthreads();
-  }
-  for (int e = tid; e < jb * nr; e += bd) {
-    int k = e / nr, r = e % nr;
-    A[static_cast<long long>(j0 + k) * ld + r0 + r] = tile[k * per + r];
-  }
-}
-
 // The row exchanges of one panel (pivots piv[0 .. jb), rows j0 .. ) as a
 // list of moves row dst[t] <- row src[t] over the rows they touch (at most
 // 2 jb): rows j0 .. j0+jb-1 first, then the pivot rows below the panel in
@@ -1641,6 +1592,150 @@ __global__ void build_swap_map(const int* __restrict__ ipiv, int j0, int jb, int
   for (int t = threadIdx.x; t < jb; t += 32) piv[t] = ipiv[j0 + t];
   __syncwarp();
   swap_map_warp(piv, j0, jb, map, rows, content, hkey, hidx, &cnt);
+}
+
+template <class T>
+__global__ void __launch_bounds__(GP_THREADS) panel_grid_kernel(T* __restrict__ A, long long ld, int N, int j0, int jb,
+                                                                int per, int* __restrict__ ipiv,
+                                                                int* __restrict__ info, int* __restrict__ map,
+                                                                PanelSlots<T> ps) {
+  extern __shared__ __align__(16) unsigned char gp_raw[];
+  T* tile = reinterpret_cast<T*>(gp_raw);
+  __shared__ T prow[128];  // the pivot row
+  __shared__ T s_inv;
+  __shared__ Candidate s_best[GP_POLL_WARPS];
+  __shared__ int s_fail, s_piv[128];
+  const int nblk = gridDim.x, b = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int r0 = j0 + b * per;
+  const int r1 = (r0 + per < N) ? r0 + per : N;
+  const int nr = r1 - r0;
+  if (tid == 0) s_fail = 0;
+  for (int k = warp; k < jb; k += GP_THREADS / 32)
+    for (int r = lane; r < nr; r += 32) tile[k * per + r] = A[static_cast<long long>(j0 + k) * ld + r0 + r];
+  __syncthreads();
+  for (int jj = 0; jj < jb; jj++) {
+    const int j = j0 + jj, slot = jj & 1;
+    if (warp == 0) {
+      // 1. local candidate
+      Candidate c{0, N};
+      for (int i = (r0 > j ? r0 : j) + lane; i < r1; i += 32)
+        c = better_of(c, Candidate{modulus_key(tile[jj * per + i - r0]), i});
+      c = warp_best(c);
+      if (c.key == 0) c.row = N;
+      // 2. publish its row (and row j when this CTA owns it), then the record
+      T* mine = ps.cand_rows + (static_cast<size_t>(slot) * nblk + b) * jb;
+      if (c.row < N)
+        for (int k = lane; k < jb; k += 32) mine[k] = tile[k * per + c.row - r0];
+      if (j >= r0 && j < r1)
+        for (int k = lane; k < jb; k += 32) ps.jrow[slot * jb + k] = tile[k * per + j - r0];
+      __syncwarp();
+      if (lane == 0) {
+        ps.rec[slot * nblk + b] = PanelRecord{c.key, static_cast<unsigned long long>(c.row)};
+        asm volatile("red.release.gpu.global.add.u32 [%0], %1;" ::"l"(ps.count), "r"(1u) : "memory");
+      }
+    }
+    // 3. all arrivals seen: every CTA's record, one a lane
+    if (warp == 0 && lane == 0) {
+      const unsigned want = static_cast<unsigned>(nblk) * (jj + 1) + ps.stall;
+      unsigned long long t0 = 0;
+      for (unsigned it = 0;; it++) {
+        unsigned v;
+        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(ps.count) : "memory");
+        if (v >= want) break;
+        if (it == 0) t0 = globaltimer_ns();
+        else if ((it & 31) == 31 && globaltimer_ns() - t0 > ps.wait_ns) {
+          s_fail = 1;
+          break;
+        }
+      }
+    }
+    __syncthreads();
+    if (s_fail) {
+      if (tid == 0) {
+        atomicExch(ps.err, 1);
+        if (b == 0) map[0] = 0;  // no row moves
+      }
+      return;
+    }
+    if (warp < GP_POLL_WARPS) {
+      Candidate c{0, N};
+      const int t = warp * 32 + lane;
+      if (t < nblk) {
+        const ulonglong2 r = __ldcg(reinterpret_cast<const ulonglong2*>(ps.rec + slot * nblk + t));
+        c = Candidate{r.x, static_cast<int>(r.y)};
+      }
+      c = warp_best(c);
+      if (lane == 0) s_best[warp] = c;
+    }
+    __syncthreads();
+    Candidate best = s_best[0];
+#pragma unroll
+    for (int w = 1; w < GP_POLL_WARPS; w++) best = better_of(best, s_best[w]);
+    // nothing usable below the diagonal: no swap
+    const int gi = best.key != 0 ? best.row : j;
+    // 4. the pivot row into prow (the part left of the diagonal only where
+    // the row goes) and the row exchange: nobody reads rows j and gi of the
+    // tile between these barriers
+    const int from = best.key != 0 ? (gi - j0) / per : 0;
+    const T* src = best.key != 0 ? ps.cand_rows + (static_cast<size_t>(slot) * nblk + from) * jb : ps.jrow + slot * jb;
+    const bool own_j = j >= r0 && j < r1;
+    if (tid < jb) {
+      if (tid >= jj || own_j) {
+        const T pk = __ldcg(src + tid);
+        prow[tid] = pk;
+        if (own_j) tile[tid * per + j - r0] = pk;
+      }
+    } else if (tid >= 128 && tid < 128 + jb) {
+      if (gi != j && gi >= r0 && gi < r1) tile[(tid - 128) * per + gi - r0] = __ldcg(ps.jrow + slot * jb + tid - 128);
+    } else if (tid == 256) {  // the reciprocal, from the key, beside the row's load
+      T v = T(0);
+      if (best.key > KEY_OF_ZERO) modulus_of(best.key, v);
+      s_inv = v != T(0) ? T(1) / v : T(0);
+      s_piv[jj] = gi;
+      if (b == 0) {
+        ipiv[j] = gi;
+        if (best.key <= KEY_OF_ZERO && *info == 0) *info = j + 1;  // zero (or NaN) pivot
+      }
+    }
+    __syncthreads();
+    // 5. scale the column below the pivot, rank-1 update of the rest
+    const T inv = prow[jj] < T(0) ? -s_inv : s_inv;
+    const int rs = (r0 > j + 1) ? r0 : j + 1;
+    if (inv != T(0) && rs < r1) {
+      for (int i = rs + tid; i < r1; i += GP_THREADS) tile[jj * per + i - r0] *= inv;
+      __syncthreads();
+      // warps over (64-row group, column phase): rows along the lanes
+      // (conflict-free shared memory), two per lane
+      const int nrr = r1 - rs, ngr = (nrr + 63) / 64, nph = (GP_THREADS / 32) / (ngr < GP_THREADS / 32 ? ngr : GP_THREADS / 32);
+      const int nwu = ngr < GP_THREADS / 32 ? ngr : GP_THREADS / 32;  // row groups worked on at a time
+      const int wg = warp % nwu, ph = warp / nwu;
+      if (ph < nph)
+        for (int gq = wg; gq < ngr; gq += nwu) {
+          const int i0 = gq * 64 + lane, i1 = i0 + 32;
+          const bool u0 = i0 < nrr, u1 = i1 < nrr;
+          T* c0 = tile + (rs - r0) + i0;
+          T* c1 = c0 + 32;
+          const T l0 = u0 ? c0[jj * per] : T(0), l1 = u1 ? c1[jj * per] : T(0);
+          for (int k = jj + 1 + ph; k < jb; k += nph) {
+            const T p = prow[k];
+            if (u0) c0[k * per] = fma(-l0, p, c0[k * per]);
+            if (u1) c1[k * per] = fma(-l1, p, c1[k * per]);
+          }
+        }
+    }
+    __syncthreads();
+  }
+  for (int k = warp; k < jb; k += GP_THREADS / 32)
+    for (int r = lane; r < nr; r += 32) A[static_cast<long long>(j0 + k) * ld + r0 + r] = tile[k * per + r];
+  // the panel's row moves for the swaps outside it (the tile is free now)
+  if (b == 0) {
+    __syncthreads();
+    if (warp == 0) {
+      int* rows = reinterpret_cast<int*>(gp_raw);
+      swap_map_warp(s_piv, j0, jb, map, rows, rows + 256, rows + 512, rows + 512 + SWAP_HASH,
+                    rows + 512 + 2 * SWAP_HASH);
+    }
+  }
 }
 
 // ---- panel on one 16-CTA cluster (FP32 factors) --------------------------
@@ -2061,6 +2156,7 @@ static int cluster_panel_width(int rows, int min_w = 32) {
 static bool grid_panel_fits(int rows, int jb, int nsm, size_t elem) {
   int nblk = (rows + GP_MIN_ROWS - 1) / GP_MIN_ROWS;
   if (nblk > nsm) nblk = nsm;
+  if (nblk > 32 * GP_POLL_WARPS) nblk = 32 * GP_POLL_WARPS;
   const int per = (rows + nblk - 1) / nblk;
   return static_cast<size_t>(per) * jb * elem <= GP_MAX_SMEM;
 }
@@ -2152,15 +2248,17 @@ __global__ void laswp_map(T* __restrict__ A, long long ld, int N, int j0, int jb
 }
 
 template <class T>
-static bool panel_grid(Context* ctx, T* A, long long ld, int N, int j0, int jb, int* ipiv, int* info, int nsm,
-                       const PanelSlots<T>& slots) {
+static bool panel_grid(Context* ctx, T* A, long long ld, int N, int j0, int jb, int* ipiv, int* info, int* map,
+                       int nsm, const PanelSlots<T>& slots) {
   const int rows = N - j0;
   int nblk = (rows + GP_MIN_ROWS - 1) / GP_MIN_ROWS;
   if (nblk > nsm) nblk = nsm;
+  if (nblk > 32 * GP_POLL_WARPS) nblk = 32 * GP_POLL_WARPS;
   const int per = (rows + nblk - 1) / nblk;
   nblk = (rows + per - 1) / per;
-  const size_t smem = static_cast<size_t>(per) * jb * sizeof(T);
+  size_t smem = static_cast<size_t>(per) * jb * sizeof(T);
   if (smem > GP_MAX_SMEM) return false;
+  if (smem < GP_MIN_SMEM) smem = GP_MIN_SMEM;  // the row moves are listed there at the end
   static std::once_flag attr;
   std::call_once(attr, [] {
     cuda_check(cudaFuncSetAttribute(panel_grid_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -2168,7 +2266,7 @@ static bool panel_grid(Context* ctx, T* A, long long ld, int N, int j0, int jb, 
                "cudaFuncSetAttribute(panel)");
   });
   cudaStream_t s = ctx->stream();
-  cuda_check(cudaMemsetAsync(slots.bar, 0, sizeof(unsigned), s), "memset barrier");
+  cuda_check(cudaMemsetAsync(slots.count, 0, sizeof(unsigned), s), "memset arrivals");
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(nblk, 1, 1);
   cfg.blockDim = dim3(GP_THREADS, 1, 1);
@@ -2179,7 +2277,7 @@ static bool panel_grid(Context* ctx, T* A, long long ld, int N, int j0, int jb, 
   at[0].val.cooperative = 1;
   cfg.attrs = at;
   cfg.numAttrs = 1;
-  cuda_check(cudaLaunchKernelEx(&cfg, panel_grid_kernel<T>, A, ld, N, j0, jb, per, ipiv, info, slots),
+  cuda_check(cudaLaunchKernelEx(&cfg, panel_grid_kernel<T>, A, ld, N, j0, jb, per, ipiv, info, map, slots),
              "panel grid kernel");
   ctx->launches += 1;
   return true;
@@ -2187,7 +2285,8 @@ static bool panel_grid(Context* ctx, T* A, long long ld, int N, int j0, int jb, 
 
 template <class T>
 // Factors one panel; returns true when the panel kernel also wrote the
-// panel's row-move list into swap_map (the FP32 cluster path).
+// panel's row-move list into swap_map (not the cluster that works in global
+// memory).
 static bool panel_factor(Context* ctx, T* A, long long ld, int N, int j0, int jb, int* ipiv, int* info, int nsm,
                          void* slot_mem, int* swap_map) {
   cudaStream_t s = ctx->stream();
@@ -2198,13 +2297,11 @@ static bool panel_factor(Context* ctx, T* A, long long ld, int N, int j0, int jb
     char* p = static_cast<char*>(slot_mem);
     slots.cand_rows = reinterpret_cast<T*>(p);
     p += sizeof(double) * 2 * 128 * static_cast<size_t>(nsm);
-    slots.cand_v = reinterpret_cast<double*>(p);
-    p += sizeof(double) * 2 * static_cast<size_t>(nsm);
+    slots.rec = reinterpret_cast<PanelRecord*>(p);
+    p += sizeof(PanelRecord) * 2 * static_cast<size_t>(nsm);
     slots.jrow = reinterpret_cast<T*>(p);
     p += sizeof(double) * 2 * 128;
-    slots.cand_i = reinterpret_cast<int*>(p);
-    p += sizeof(int) * 2 * static_cast<size_t>(nsm);
-    slots.bar = reinterpret_cast<unsigned*>(p);
+    slots.count = reinterpret_cast<unsigned*>(p);
     slots.err = reinterpret_cast<int*>(p + 16);
     slots.wait_ns = ctx->grid_wait_ns;
     slots.stall = ctx->stall_waits ? 1u : 0u;
@@ -2212,7 +2309,7 @@ static bool panel_factor(Context* ctx, T* A, long long ld, int N, int j0, int jb
   if constexpr (std::is_same<T, float>::value) {
     if (panel_cluster16(ctx, A, ld, N, j0, jb, ipiv, info, swap_map, slots.err, slots.wait_ns, slots.stall)) return true;
   }
-  if (panel_grid<T>(ctx, A, ld, N, j0, jb, ipiv, info, nsm < ctx->sms() ? nsm : ctx->sms(), slots)) return false;
+  if (panel_grid<T>(ctx, A, ld, N, j0, jb, ipiv, info, swap_map, nsm < ctx->sms() ? nsm : ctx->sms(), slots)) return true;
   // Panels too tall for the shared memory of the GPU: one 8-CTA cluster
   // working on the panel in global memory.
   cudaLaunchConfig_t cfg = {};
@@ -2258,18 +2355,18 @@ static void trsm_and_swaps(Context* ctx, T* A, long long ld, int N, int j0, int 
     ctx->launches += 1;
   }
   if (j0 + jb < N) {
-    size_t smem = sizeof(double) * (static_cast<size_t>(jb) * jb + static_cast<size_t>(jb) * TRSM_COLS);
-    static std::once_flag attr_set;
-    std::call_once(attr_set,
-                   [] { cudaFuncSetAttribute(trsm_unit_lower<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024); });
     if constexpr (std::is_same<T, float>::value) {
-      if (jb <= 96) {
-        launch_trsm_chunk(ctx, A, ld, j0, jb, j0 + jb, N);
-        return;
-      }
+      launch_trsm_chunk(ctx, A, ld, j0, jb, j0 + jb, N);
+    } else {
+      static std::once_flag attr_set;
+      std::call_once(attr_set, [] {
+        cuda_check(cudaFuncSetAttribute(trsm_chunk_f64, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                        static_cast<int>(TD_SMEM)),
+                   "cudaFuncSetAttribute(trsm)");
+      });
+      trsm_chunk_f64<<<blocks(N - j0 - jb, TD_COLS), TD_THREADS, TD_SMEM, s>>>(A, ld, j0, jb, j0 + jb, N);
+      ctx->launches += 1;
     }
-    trsm_unit_lower<T><<<blocks(N - j0 - jb, TRSM_COLS), TRSM_COLS, smem, s>>>(A, ld, j0, jb, j0 + jb, N);
-    ctx->launches += 1;
   }
   cuda_check(cudaGetLastError(), "laswp/trsm kernels");
 }
