@@ -926,25 +926,32 @@ int kd_fields_val_points(int nfields, kd_field* const* fields, long long npts, c
     if (npts == 0) return;
     kd::Context& c = *fields[0]->sp->ctx->c;
     cudaStream_t s = c.stream();
-    double *d_xyz = nullptr, *d_out = nullptr;
-    kd::cuda_check(cudaMalloc(&d_xyz, sizeof(double) * 3 * npts), "cudaMalloc(points)");
-    if (cudaMalloc(&d_out, sizeof(double) * nfields * npts) != cudaSuccess) {
-      cudaFree(d_xyz);
-      throw kd::KdError(KD_ERR_CUDA, "cudaMalloc(values)");
+    const size_t nin = 3 * static_cast<size_t>(npts), nout = static_cast<size_t>(nfields) * npts;
+    // small calls stage in the context's arena; large ones allocate and give back
+    constexpr size_t ARENA_DOUBLES = size_t(4) << 20;
+    struct Owned {
+      double* p = nullptr;
+      ~Owned() { cudaFree(p); }
+    } owned;
+    kd::DeviceArena& ar = c.scratch();
+    const size_t mark = ar.mark();
+    struct Release {
+      kd::DeviceArena& a;
+      size_t m;
+      ~Release() { a.release_to(m); }
+    } release{ar, mark};
+    double* d_xyz;
+    if (nin + nout <= ARENA_DOUBLES) {
+      d_xyz = ar.alloc_doubles(nin + nout);
+    } else {
+      kd::cuda_check(cudaMalloc(&owned.p, sizeof(double) * (nin + nout)), "cudaMalloc(points)");
+      d_xyz = owned.p;
     }
-    try {
-      kd::cuda_check(cudaMemcpyAsync(d_xyz, xyz, sizeof(double) * 3 * npts, cudaMemcpyHostToDevice, s), "H2D points");
-      kd::fields_val_points(&c, list, npts, d_xyz, d_out);
-      kd::cuda_check(cudaMemcpyAsync(out, d_out, sizeof(double) * nfields * npts, cudaMemcpyDeviceToHost, s),
-                     "D2H values");
-      kd::cuda_check(cudaStreamSynchronize(s), "sync");
-    } catch (...) {
-      cudaFree(d_xyz);
-      cudaFree(d_out);
-      throw;
-    }
-    cudaFree(d_xyz);
-    cudaFree(d_out);
+    double* d_out = d_xyz + nin;
+    kd::cuda_check(cudaMemcpyAsync(d_xyz, xyz, sizeof(double) * nin, cudaMemcpyHostToDevice, s), "H2D points");
+    kd::fields_val_points(&c, list, npts, d_xyz, d_out);
+    kd::cuda_check(cudaMemcpyAsync(out, d_out, sizeof(double) * nout, cudaMemcpyDeviceToHost, s), "D2H values");
+    kd::cuda_check(cudaStreamSynchronize(s), "sync");
   });
 }
 
