@@ -1,10 +1,12 @@
 #include "kd_context.hpp"
+#include "kd_spectral.hpp"
 
 #include <algorithm>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
 #include <fstream>
+#include <iterator>
 #include <sstream>
 
 namespace kd {
@@ -108,6 +110,7 @@ void* Context::workspace(int slot, size_t bytes, bool* fresh) {
 }
 
 void Context::fork(int n) {
+  if (batch_.on) return;  // one stream, ordered by levels
   if (n < 1) n = 1;
   if (!fork_ev_) cuda_check(cudaEventCreateWithFlags(&fork_ev_, cudaEventDisableTiming), "cudaEventCreate");
   while (static_cast<int>(side_.size()) < n) {
@@ -123,7 +126,10 @@ void Context::fork(int n) {
   nfork_ = n;
 }
 
-void Context::use(int i) { cur_ = (i < 0 || nfork_ == 0) ? stream_ : side_[i % nfork_]; }
+void Context::use(int i) {
+  if (batch_.on) return;
+  cur_ = (i < 0 || nfork_ == 0) ? stream_ : side_[i % nfork_];
+}
 
 void Context::join() {
   for (int i = 0; i < nfork_; i++) {
@@ -132,6 +138,149 @@ void Context::join() {
   }
   nfork_ = 0;
   cur_ = stream_;
+}
+
+bool Context::begin_batch() {
+  if (prof_on_ || batch_.on || nfork_ > 0) return false;
+  batch_.on = true;
+  return true;
+}
+
+void Context::drop_batch() {
+  batch_.on = false;
+  batch_.ops.clear();
+  batch_.level.clear();
+  batch_.buffers.clear();
+  batch_.rows.clear();
+}
+
+void Context::end_batch() {
+  if (!batch_.on) return;
+  batch_.on = false;
+  flush_batch();
+}
+
+int Context::level_of(std::initializer_list<const void*> reads, const void* write) {
+  int level = 0;
+  for (const void* r : reads) {
+    if (!r) continue;
+    auto it = batch_.buffers.find(r);
+    if (it != batch_.buffers.end()) level = std::max(level, it->second.written + 1);
+  }
+  auto it = batch_.buffers.find(write);
+  if (it != batch_.buffers.end()) level = std::max(level, std::max(it->second.written, it->second.read) + 1);
+  return level;
+}
+
+void Context::mark(std::initializer_list<const void*> reads, const void* write, int level) {
+  for (const void* r : reads)
+    if (r) {
+      Levels& l = batch_.buffers[r];
+      l.read = std::max(l.read, level);
+    }
+  batch_.buffers[write].written = level;
+}
+
+bool Context::defer_item(const LinePlan& plan, const double* in, double* out) {
+  // larger fields keep their launches of a cluster per field: one CTA would
+  // take longer than the launch it saves (60 us for a (25,13,14) transform)
+  if (!batch_.on || plan.stage > 3000) return false;
+  if (!plan.dev) {
+    if (capturing) return false;
+    const KdItem it = make_item(plan, nullptr, nullptr, plan.dims_in, 0, 0, 1.0);
+    std::vector<int> raw(sizeof(KdItem) / sizeof(int));
+    std::memcpy(raw.data(), &it, sizeof(KdItem));
+    plan.dev = reinterpret_cast<const KdItem*>(table(raw));
+  }
+  KdOpRec o{};
+  o.kind = KD_OP_LINE;
+  o.smem = 2 * plan.stage + plan.nmats;
+  o.p[0] = plan.dev;
+  o.p[1] = in;
+  o.p[2] = out;
+  const int level = level_of({in}, out);
+  mark({in}, out, level);
+  batch_.ops.push_back(o);
+  batch_.level.push_back(level);
+  return true;
+}
+
+bool Context::defer_ew(int op, long long npts, const double* a, const double* b, double* out, double alpha,
+                       double beta) {
+  if (!batch_.on || npts > 4096) return false;
+  KdOpRec o{};
+  o.kind = KD_OP_EW;
+  o.sub = op;
+  o.n = static_cast<int>(npts);
+  o.p[0] = a;
+  o.p[1] = b;
+  o.p[2] = out;
+  o.alpha = alpha;
+  o.beta = beta;
+  const int level = level_of({a, b}, out);
+  mark({a, b}, out, level);
+  batch_.ops.push_back(o);
+  batch_.level.push_back(level);
+  return true;
+}
+
+bool Context::defer_gather(const double* in, int nrows, const int* rowptr, const int* idx, const double* w,
+                           double* out, long long osr, double alpha, int accumulate) {
+  if (!batch_.on || osr != 1 || nrows <= 0) return false;
+  KdOpRec o{};
+  o.kind = KD_OP_GATHER;
+  o.sub = accumulate;
+  o.n = nrows;
+  o.p[0] = in;
+  o.p[1] = out;
+  o.p[2] = rowptr;
+  o.p[3] = idx;
+  o.p[4] = w;
+  o.alpha = alpha;
+  o.osr = osr;
+  int level = level_of({in}, out);
+  // rows that an earlier gather of the batch wrote: after it
+  const double* end = out + nrows;
+  const double* first = out;
+  auto it = batch_.rows.lower_bound(out);
+  if (it != batch_.rows.begin()) {
+    auto before = std::prev(it);
+    if (before->second.end > out) it = before;
+  }
+  while (it != batch_.rows.end() && it->first < end) {
+    level = std::max(level, it->second.level + 1);
+    first = std::min(first, it->first);
+    end = std::max(end, it->second.end);
+    it = batch_.rows.erase(it);
+  }
+  batch_.rows[first] = Range{end, level};
+  mark({in}, out, level);
+  batch_.ops.push_back(o);
+  batch_.level.push_back(level);
+  return true;
+}
+
+void Context::flush_batch() {
+  if (batch_.ops.empty()) return;
+  const int n = static_cast<int>(batch_.ops.size());
+  int top = 0;
+  for (int l : batch_.level) top = std::max(top, l);
+  std::vector<int> at(top + 2, 0);
+  for (int l : batch_.level) at[l + 1]++;
+  for (int l = 0; l <= top; l++) at[l + 1] += at[l];
+  std::vector<KdOpRec> sorted(n);
+  std::vector<int> next(at.begin(), at.end() - 1);
+  for (int i = 0; i < n; i++) sorted[next[batch_.level[i]]++] = batch_.ops[i];
+  batch_.ops.clear();
+  batch_.level.clear();
+  batch_.buffers.clear();
+  batch_.rows.clear();
+  const double* dp = pool();
+  for (int l = 0; l <= top; l++)
+    for (int i = at[l]; i < at[l + 1]; i += KD_MAX_OPS) {
+      cuda_check(launch_ops(sorted.data() + i, std::min(KD_MAX_OPS, at[l + 1] - i), dp, cur_), "operation list kernel");
+      launches++;
+    }
 }
 
 const double* Context::pool() {

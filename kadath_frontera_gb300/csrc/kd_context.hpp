@@ -4,6 +4,8 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <exception>
+#include <initializer_list>
 #include <map>
 #include <stdexcept>
 #include <string>
@@ -72,6 +74,8 @@ struct LinePlan {
   const double* mats = nullptr;
   KdPass pass[3] = {};
   std::vector<int> out_base;
+  int dims_in[3] = {0, 0, 0};
+  mutable const KdItem* dev = nullptr;  // device copy, made when a batch first needs it
 };
 
 class Context {
@@ -96,8 +100,15 @@ class Context {
   void set_sm_budget(int n) { sm_budget_ = n; }
   // The stream work is issued on: the context's main stream, or one of the
   // side streams between fork() and join().
-  cudaStream_t stream() const { return cur_; }
-  cudaStream_t main_stream() const { return stream_; }
+  // (Work collected by a batch is launched first.)
+  cudaStream_t stream() {
+    if (!batch_.ops.empty()) flush_batch();
+    return cur_;
+  }
+  cudaStream_t main_stream() {
+    if (!batch_.ops.empty()) flush_batch();
+    return stream_;
+  }
   // Side streams for independent work (the per-domain equations of a value
   // pass): fork() makes n side streams wait for the main stream's work so
   // far, use(i) issues on side stream i % n (i < 0: the main stream), join()
@@ -105,6 +116,22 @@ class Context {
   void fork(int n);
   void use(int i);
   void join();
+
+  // Between begin_batch() and end_batch() single-field operations (the defer_*
+  // calls below) are collected instead of launched, each with the level that
+  // the operations it depends on give it; a flush launches level by level, one
+  // CTA per operation, on the main stream.  Any other use of a stream flushes
+  // first, so launches in between keep their order.  fork() and use() do
+  // nothing meanwhile.  Not nested; off in profile mode, whose categories time
+  // single launches.
+  bool begin_batch();  // false when none was begun
+  void end_batch();
+  void drop_batch();
+  void flush_batch();
+  bool defer_item(const LinePlan& plan, const double* in, double* out);
+  bool defer_ew(int op, long long npts, const double* a, const double* b, double* out, double alpha, double beta);
+  bool defer_gather(const double* in, int nrows, const int* rowptr, const int* idx, const double* w, double* out,
+                    long long osr, double alpha, int accumulate);
 
   MatrixBank& bank() { return bank_; }
   // Makes sure every matrix in the bank is present in the device pool.
@@ -221,6 +248,25 @@ class Context {
     }
   };
   std::unordered_map<std::vector<int>, LinePlan, KeyHash> plans_;
+  // Collected operations.  Arena buffers are disjoint and used whole, so a
+  // buffer is known by its first address; gathers also write parts of one
+  // vector, whose ranges are kept in order.
+  struct Levels {
+    int written = -1, read = -1;
+  };
+  struct Range {
+    const double* end;
+    int level;
+  };
+  struct Batch {
+    bool on = false;
+    std::vector<KdOpRec> ops;
+    std::vector<int> level;
+    std::unordered_map<const void*, Levels> buffers;
+    std::map<const double*, Range> rows;
+  } batch_;
+  int level_of(std::initializer_list<const void*> reads, const void* write);
+  void mark(std::initializer_list<const void*> reads, const void* write, int level);
   std::map<std::vector<double>, double*> dtables_;
   DeviceArena scratch_;
   DeviceArena* active_scratch_ = &scratch_;
@@ -236,6 +282,21 @@ struct ProfScope {
   double work;
   ProfScope(Context* ctx, int category, double w) : c(ctx), cat(category), work(w) { c->prof_begin(cat); }
   ~ProfScope() { c->prof_end(cat, work); }
+};
+
+// A batch for its lifetime (none where a stream is forked or profiled).  When
+// an exception leaves it, what was collected is dropped: its outputs are
+// garbage to nobody, since the pass that collected it has failed.
+struct BatchScope {
+  Context* c;
+  bool mine;
+  int pending;
+  explicit BatchScope(Context* ctx) : c(ctx), mine(ctx->begin_batch()), pending(std::uncaught_exceptions()) {}
+  ~BatchScope() noexcept(false) {
+    if (!mine) return;
+    if (std::uncaught_exceptions() > pending) c->drop_batch();
+    else c->end_batch();
+  }
 };
 
 // Builds the pass description of a 1-D operator along `dim` for a field of

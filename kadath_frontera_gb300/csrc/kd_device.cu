@@ -241,6 +241,39 @@ __device__ __forceinline__ long long point_of(long long i, long long npts) {
   return i % npts;
 }
 
+__device__ __forceinline__ double ew_value(int op, double x, double y, double alpha, double beta) {
+  double r;
+  switch (op) {
+    case EW_ADD: r = x + y; break;
+    case EW_SUB: r = x - y; break;
+    case EW_MUL: r = x * y; break;
+    case EW_DIV: r = x / y; break;
+    case EW_AXPBY: r = alpha * x + beta * y; break;
+    case EW_SCALE: r = alpha * x; break;
+    case EW_ADDC: r = x + alpha; break;
+    case EW_CSUB: r = alpha - x; break;
+    case EW_CDIV: r = alpha / x; break;
+    case EW_POWD: r = pow(x, alpha); break;
+    case EW_EXP: r = exp(x); break;
+    case EW_LOG: r = log(x); break;
+    case EW_SQRT: r = sqrt(x); break;
+    case EW_SIN: r = sin(x); break;
+    case EW_COS: r = cos(x); break;
+    case EW_NEG: r = -x; break;
+    case EW_FILL: r = alpha; break;
+    case EW_COPY: r = x; break;
+    case EW_POWI: r = pow(x, alpha); break;
+    case EW_ATAN: r = atan(x); break;
+    case EW_MULC_ADD: r = x * y * alpha; break;
+    case EW_DIVC: r = x / alpha; break;
+    case EW_COSH: r = cosh(x); break;
+    case EW_SINH: r = sinh(x); break;
+    case EW_ATANH: r = atanh(x); break;
+    default: r = 0.0; break;
+  }
+  return r;
+}
+
 __global__ void ew_kernel(int op, long long npts, long long total, int ba, const double* __restrict__ a,
                           int bb, const double* __restrict__ b, double* __restrict__ out, double alpha,
                           double beta) {
@@ -249,36 +282,7 @@ __global__ void ew_kernel(int op, long long npts, long long total, int ba, const
     const long long p = total == npts ? i : point_of(i, npts);
     double x = (a != nullptr) ? a[ba == 1 ? p : i] : 0.0;
     double y = (b != nullptr) ? b[bb == 1 ? p : i] : 0.0;
-    double r;
-    switch (op) {
-      case EW_ADD: r = x + y; break;
-      case EW_SUB: r = x - y; break;
-      case EW_MUL: r = x * y; break;
-      case EW_DIV: r = x / y; break;
-      case EW_AXPBY: r = alpha * x + beta * y; break;
-      case EW_SCALE: r = alpha * x; break;
-      case EW_ADDC: r = x + alpha; break;
-      case EW_CSUB: r = alpha - x; break;
-      case EW_CDIV: r = alpha / x; break;
-      case EW_POWD: r = pow(x, alpha); break;
-      case EW_EXP: r = exp(x); break;
-      case EW_LOG: r = log(x); break;
-      case EW_SQRT: r = sqrt(x); break;
-      case EW_SIN: r = sin(x); break;
-      case EW_COS: r = cos(x); break;
-      case EW_NEG: r = -x; break;
-      case EW_FILL: r = alpha; break;
-      case EW_COPY: r = x; break;
-      case EW_POWI: r = pow(x, alpha); break;
-      case EW_ATAN: r = atan(x); break;
-      case EW_MULC_ADD: r = x * y * alpha; break;
-      case EW_DIVC: r = x / alpha; break;
-      case EW_COSH: r = cosh(x); break;
-      case EW_SINH: r = sinh(x); break;
-      case EW_ATANH: r = atanh(x); break;
-      default: r = 0.0; break;
-    }
-    out[i] = r;
+    out[i] = ew_value(op, x, y, alpha, beta);
   }
 }
 
@@ -324,6 +328,71 @@ __global__ void absmax_kernel(const double* __restrict__ x, long long n, double*
       atomicMax(reinterpret_cast<unsigned long long*>(out), __double_as_longlong(m));
     }
   }
+}
+
+// One operation per CTA (KdOpRec): the operations of one level of a pass.
+// Bound: the latency of a launch and of one operation; a value pass of the
+// (13,9,4) star has 4,800 operations on 27 levels, which as launches of their
+// own cost the host 2.7 us each.  Residual 13.2 -> 2.0 ms (the host's evaluation
+// of the expression trees), replayed from its graph 4.65 -> 0.40 ms.
+template <int N>
+struct KdOpList {
+  int n;
+  KdOpRec ops[N];
+};
+template <int N>
+__global__ void __launch_bounds__(256) op_list_kernel(const __grid_constant__ KdOpList<N> list,
+                                                      const double* __restrict__ pool) {
+  extern __shared__ __align__(16) double smem[];
+  __shared__ __align__(8) unsigned char item_raw[sizeof(KdItem)];
+  const KdOpRec& o = list.ops[blockIdx.x];
+  if (o.kind == KD_OP_LINE) {
+    static_assert(sizeof(KdItem) % 8 == 0 && sizeof(KdItem) <= 8 * 256, "copied by one round of 8-byte loads");
+    if (threadIdx.x < sizeof(KdItem) / 8)
+      reinterpret_cast<unsigned long long*>(item_raw)[threadIdx.x] =
+          __ldg(static_cast<const unsigned long long*>(o.p[0]) + threadIdx.x);
+    __syncthreads();
+    const KdItem& it = *reinterpret_cast<const KdItem*>(item_raw);
+    load_field(it, static_cast<const double*>(o.p[1]), smem);
+    double* at = smem + 2 * it.stage;
+    load_mats(it, at);
+    copy_async_wait();
+    __syncthreads();
+    run_item(it, it.nmats ? at : pool, static_cast<double*>(const_cast<void*>(o.p[2])), smem, smem + it.stage);
+  } else if (o.kind == KD_OP_EW) {
+    const double* a = static_cast<const double*>(o.p[0]);
+    const double* b = static_cast<const double*>(o.p[1]);
+    double* out = static_cast<double*>(const_cast<void*>(o.p[2]));
+    for (int i = threadIdx.x; i < o.n; i += blockDim.x)
+      out[i] = ew_value(o.sub, a ? a[i] : 0.0, b ? b[i] : 0.0, o.alpha, o.beta);
+  } else {
+    const double* in = static_cast<const double*>(o.p[0]);
+    double* out = static_cast<double*>(const_cast<void*>(o.p[1]));
+    const int* rowptr = static_cast<const int*>(o.p[2]);
+    const int* idx = static_cast<const int*>(o.p[3]);
+    const double* w = static_cast<const double*>(o.p[4]);
+    for (int r = threadIdx.x; r < o.n; r += blockDim.x) {
+      double acc = 0.0;
+      for (int e = rowptr[r]; e < rowptr[r + 1]; e++) acc = fma(w[e], in[idx[e]], acc);
+      double* dst = out + r * o.osr;
+      if (o.sub) *dst += o.alpha * acc;
+      else *dst = o.alpha * acc;
+    }
+  }
+}
+
+template <int N>
+cudaError_t launch_op_list(const KdOpRec* ops, int n, size_t smem, const double* d_pool, cudaStream_t s) {
+  KdOpList<N> list;
+  list.n = n;
+  for (int i = 0; i < n; i++) list.ops[i] = ops[i];
+  if (smem > 48 * 1024) {
+    const cudaError_t e =
+        cudaFuncSetAttribute(op_list_kernel<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+    if (e != cudaSuccess) return e;
+  }
+  op_list_kernel<N><<<n, 256, smem, s>>>(list, d_pool);
+  return cudaGetLastError();
 }
 
 template <int CL, class List>
@@ -379,6 +448,17 @@ int grid_for(long long n, int threads) {
 }
 
 }  // namespace
+
+cudaError_t launch_ops(const KdOpRec* ops, int n, const double* d_pool, cudaStream_t s) {
+  if (n <= 0) return cudaSuccess;
+  size_t smem = 0;
+  for (int i = 0; i < n; i++)
+    if (sizeof(double) * ops[i].smem > smem) smem = sizeof(double) * ops[i].smem;
+  // parameters are copied with every launch: the smallest list that holds them
+  if (n <= 12) return launch_op_list<12>(ops, n, smem, d_pool, s);
+  if (n <= 80) return launch_op_list<80>(ops, n, smem, d_pool, s);
+  return launch_op_list<KD_MAX_OPS>(ops, n, smem, d_pool, s);
+}
 
 LpShape lp_default_shape(int total_fields, int stage) {
   LpShape sh;

@@ -61,6 +61,22 @@ struct KdItemList1 {
   KdItem items[1];
 };
 
+// Single-field operations collected by a pass and launched level by level
+// (Context::begin_batch): one CTA per operation, up to KD_MAX_OPS of them with
+// no dependence on one another in a launch.
+constexpr int KD_MAX_OPS = 400;  // 32,008 bytes of the 32,764 that kernel parameters may take
+enum KdOpKind : int { KD_OP_LINE = 0, KD_OP_EW = 1, KD_OP_GATHER = 2 };
+struct KdOpRec {
+  int kind;
+  int sub;           // elementwise operation; gather: accumulate
+  int n;             // elementwise: points; gather: rows
+  int smem;          // line passes: doubles of shared memory
+  const void* p[5];  // line: item (its in and out unused), in, out; ew: a, b, out; gather: in, out, rowptr, idx, w
+  double alpha, beta;
+  long long osr;     // gather: stride of the output rows
+};
+cudaError_t launch_ops(const KdOpRec* ops, int n, const double* d_pool, cudaStream_t s);
+
 // Launch shape of a line-pass launch: one CTA of `threads` threads per field
 // (cluster = 1), or a cluster of `cluster` CTAs (2, 4 or 8) of 128 threads
 // per field, each CTA computing every cluster-th block of a pass's outputs.

@@ -11,6 +11,7 @@ double* alloc(Context* ctx, long long n) { return ctx->scratch().alloc_doubles(s
 void ew(Context* ctx, int op, long long npts, int ba, const double* a, int bb, const double* b, double* out,
         double alpha = 0.0, double beta = 0.0) {
   int nf = ba > bb ? ba : bb;
+  if (nf <= 1 && ctx->defer_ew(op, npts, a, b, out, alpha, beta)) return;
   ProfScope ps(ctx, Context::PROF_EW,
                8.0 * npts * ((a ? ba : 0) + (b ? bb : 0) + nf));
   cuda_check(launch_ew(op, npts, ba, a, bb, b, out, alpha, beta, ctx->stream()), "elementwise kernel");
@@ -19,6 +20,7 @@ void ew(Context* ctx, int op, long long npts, int ba, const double* a, int bb, c
 
 void run_plan(Context* ctx, const LinePlan& plan, const double* in, double* out, const int dims_in[3],
               long long in_stride, long long out_stride, int batch) {
+  if (batch == 1 && ctx->defer_item(plan, in, out)) return;
   KdItem it = make_item(plan, in, out, dims_in, in_stride, out_stride, 1.0);
   ctx->run_items({it}, {batch});
 }
@@ -153,14 +155,16 @@ void DVal::compute_der_var() const {
     res->base = base;
     const LinePlan& plan = ope_1d_plan(*ctx, OP_DER, var, base, dom->nc, res->base);
     double* out = alloc(ctx, static_cast<long long>(batch) * ncoefs());
-    items.push_back(make_item(plan, cf, out, dom->nc, ncoefs(), ncoefs(), 1.0));
-    batches.push_back(batch);
+    if (batch != 1 || !ctx->defer_item(plan, cf, out)) {
+      items.push_back(make_item(plan, cf, out, dom->nc, ncoefs(), ncoefs(), 1.0));
+      batches.push_back(batch);
+    }
     res->cf = out;
     res->in_coef = true;
     (*arr)[var] = res;
   }
   // The three derivatives run in one launch.
-  ctx->run_items(items, batches);
+  if (!items.empty()) ctx->run_items(items, batches);
   dvar_ = arr;
 }
 

@@ -251,6 +251,7 @@ void compile_passes(Context& ctx, const std::vector<LinePassSpec>& specs, const 
                     LinePlan& plan, PassLists lists[3], std::vector<double>& mats) {
   if (specs.empty() || specs.size() > 3) throw KdError(KD_ERR_ARG, "one to three passes per item");
   plan.npass = static_cast<int>(specs.size());
+  for (int i = 0; i < 3; i++) plan.dims_in[i] = dims_in[i];
   auto stage_of = [&](bool padded) {
     int d[3] = {dims_in[0], dims_in[1], dims_in[2]};
     long long m = static_cast<long long>(d[0]) * d[1] * row_pitch(d[2], padded);

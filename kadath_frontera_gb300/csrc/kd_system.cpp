@@ -827,6 +827,11 @@ void System::export_term(const Equation& eq, const Term& t, bool der, int side_d
                                                           : export_table(d, v.base, 1, side_bound);
       if (tab.nrows != tv.nrows) throw KdError(KD_ERR_STATE, "tangent basis changes the number of conditions");
       long long in_stride = (v.batch == 1 && batch > 1) ? 0 : v.ncoefs();
+      if (batch == 1 && ctx->defer_gather(v.cf, tab.nrows, tab.rowptr, tab.idx, tab.w, out + row * osr, osr, alpha,
+                                          accumulate ? 1 : 0)) {
+        row += tv.nrows;
+        continue;
+      }
       ProfScope ps(ctx, Context::PROF_GATHER, 8.0 * batch * (tab.nnz + 2.0 * tab.nrows));
       cuda_check(launch_gather_csr(v.cf, in_stride, batch, tab.nrows, tab.rowptr, tab.idx, tab.w, out + row * osr,
                                    osf, osr, alpha, accumulate ? 1 : 0, ctx->stream()),
@@ -1075,6 +1080,8 @@ void System::residual_pass(double* d_F, bool record) {
   // The equations of different domains are independent (fields are only
   // read, temporaries come from the pass's arena): one side stream per
   // domain, so that their small kernels overlap on the GPU.
+  // Where the pass is collected into levels instead, fork and use do nothing.
+  BatchScope batch(ctx);
   struct Fork {
     Context* c;
     Fork(Context* c_, int n) : c(c_) { c->fork(n); }
@@ -1407,6 +1414,7 @@ void System::dres_dcst(int cst, double* d_y) {
   st.seed_cst = cst;
   st.vcache = &vcache_;
   cuda_check(cudaMemsetAsync(d_y, 0, sizeof(double) * N, ctx->stream()), "memset y");
+  BatchScope batch(ctx);
   for (auto& eq : eqs_) export_tangent(eq, st, d_y, 0, 1);
   export_int_ders(st, -1, d_y, 1, 1);
 }
@@ -1562,6 +1570,7 @@ void System::jx(const double* d_x, double* d_y) {
   st.jx_doubles = &xd;
   st.vcache = &vcache_;
   cuda_check(cudaMemsetAsync(d_y, 0, sizeof(double) * N, ctx->stream()), "memset y");
+  BatchScope batch(ctx);
   for (auto& eq : eqs_) export_tangent(eq, st, d_y, 0, 1);
   export_int_ders(st, -1, d_y, 1, 1);
 }

@@ -609,8 +609,10 @@ class OpeFunctional : public Ope {
       cuda_check(cudaMemsetAsync(out, 0, sizeof(double) * v.batch, ctx->stream()), "memset functional");
       return out;
     }
-    cuda_check(launch_gather_csr(src, stride, v.batch, 1, ctx->table(rp), ctx->table(idx), ctx->dtable(wt), out, 1, 0,
-                                 1.0, 0, ctx->stream()),
+    const int *d_rp = ctx->table(rp), *d_idx = ctx->table(idx);
+    const double* d_w = ctx->dtable(wt);
+    if (v.batch == 1 && ctx->defer_gather(src, 1, d_rp, d_idx, d_w, out, 1, 1.0, 0)) return out;
+    cuda_check(launch_gather_csr(src, stride, v.batch, 1, d_rp, d_idx, d_w, out, 1, 0, 1.0, 0, ctx->stream()),
                "functional gather");
     ctx->launches++;
     return out;
