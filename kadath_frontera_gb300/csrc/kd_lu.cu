@@ -1743,92 +1743,67 @@ __global__ void __launch_bounds__(GP_THREADS) panel_grid_kernel(T* __restrict__ 
 // shared memory: CTA r of the cluster keeps rows [j0 + r*per, ...) of the
 // panel in its shared memory, row by row (stride cp_row_stride(jb) floats,
 // so that a row's 16-column inner block is four aligned 128-bit words and
-// eight consecutive rows hit distinct banks).  Per column, one block
-// barrier and one cluster barrier:
+// eight consecutive rows hit distinct banks).  While a 16-column inner block is
+// worked on, its columns live in the registers of the rows' threads.  Per
+// column, one block barrier and one exchange:
 //  - every thread already holds its best candidate for the column (found
-//    while updating it in the previous column step); a warp reduction and
-//    one block barrier give the CTA's candidate;
-//  - warp 0 pushes (value, row, the row's inner block) into every CTA's
-//    receive slot, and warp 1 of the owner of row j pushes row j's inner
-//    block; the CTA keeps its candidate's full row and row j locally;
-//  - after the cluster barrier every warp picks the winner from its own
+//    while updating it in the previous column step); a warp reduction, the
+//    winner's block columns through shared memory and one block barrier give
+//    the CTA's candidate;
+//  - warp 0 pushes (value, the row's inner block) and warp 2 the row number
+//    into every CTA's receive slot, and warp 1 of the owner of row j pushes
+//    row j's inner block; the CTA keeps its candidate's full row (copied by
+//    warp 2 first) and row j locally;
+//  - when its slot is complete every warp picks the winner from its own
 //    receive slot (same order everywhere); each thread then swaps, scales
-//    and updates the inner block of its rows in registers and tracks its
-//    candidate for column j + 1, all in one pass;
+//    and updates the inner block of its rows and tracks its candidate for
+//    column j + 1, all in one pass; the multipliers go to the tile;
 //  - the other columns of the two swapped rows are fetched from the owners'
-//    shared memory off the critical path (they are read again only after
-//    the next cluster barrier).
+//    shared memory off the critical path.
 // Receive slots, candidate rows and row j are double-buffered by column
-// parity: a CTA can only overwrite a slot after every CTA has passed the
-// next cluster barrier, i.e. has finished reading it.
+// parity: a CTA can only overwrite a slot after every CTA has pushed the next
+// column, i.e. has finished reading it.
+// Bound: latency, about 3,200 cycles a column (376 rows a CTA, 96 columns): the
+// CTA's candidate 550, pushing 600, waiting 500, the winner 250, the column step
+// 430, the block ends 720.  With the block in shared memory a step took 850 (its
+// bandwidth), arg-max by shuffles instead of redux 900 more, the U12 columns of a
+// block end through shared memory 300, and the candidate's row copy before the
+// pushes of the same warp 100: 224 -> 151 us per panel at N = 6,001, 235 -> 151 us
+// on average at N = 12,331.
 constexpr int CP_CL = 16;
-constexpr int CP_THREADS = 384;  // 251 rows per CTA and warp-level reductions over 12 warps (512 and 768 were slower)
+constexpr int CP_THREADS = 512;  // most; see cp_threads
 constexpr int CP_WARPS = CP_THREADS / 32;
 constexpr size_t CP_MAX_SMEM = 212 * 1024;
+// Threads for `per` rows a CTA: whole rounds of the rows, at most 448 a round
+// (771 rows: two rounds of 416 instead of three of 384), no fewer than 256.
+constexpr int cp_threads(int per) {
+  const int rounds = (per + 447) / 448, t = ((per + rounds - 1) / rounds + 31) / 32 * 32;
+  return t < 256 ? 256 : t;
+}
 constexpr int CP_IB = 16;  // inner block: columns updated per column step
 
 // Row stride (floats) of the panel in shared memory: whole 16-column inner
 // blocks plus 4, i.e. an odd number of 16-byte words.
 __host__ __device__ constexpr int cp_row_stride(int jb) { return ((jb + 15) / 16) * 16 + 4; }
 
+// |v| as an integer of the same order: 0 for NaN (never a pivot), else its bits
+// + 1.  Arg-max are then two redux instructions (largest key, lowest row).
+__device__ __forceinline__ unsigned cp_key(float v) {
+  const unsigned k = __float_as_uint(v) & 0x7fffffffu;
+  return k > 0x7f800000u ? 0u : k + 1u;
+}
+__device__ __forceinline__ void cp_warp_best(unsigned& key, int& row) {
+  const unsigned m = __reduce_max_sync(0xffffffffu, key);
+  row = __reduce_min_sync(0xffffffffu, key == m ? row : 0x7fffffff);
+  key = m;
+}
+
 struct CpSlot {
   float4 seg[CP_CL][CP_IB / 4];  // candidate rows' inner blocks, by source CTA
   float4 jseg[CP_IB / 4];        // row j's inner block
-  float v[CP_CL];                // candidate |values|, by source CTA
+  unsigned v[CP_CL];             // keys of the candidates, by source CTA
   int i[CP_CL];                  // candidate rows (N: none), by source CTA
 };
-
-// One column step on this thread's rows of the inner block, for column Q0
-// of the block: swap (row j <- pivot row, row gi <- row j), scale column
-// Q0, update columns Q0+1..15, and the thread's candidate for column Q0+1.
-// Q0 is a template parameter so that the column selections cost nothing.
-template <int Q0>
-__device__ __forceinline__ void cp_column_step(float* __restrict__ tile, int S, int b0, int r0, int nr, int j, int gi,
-                                               int nb, const float (&ps)[CP_IB], const float4* jseg4, float inv,
-                                               bool nonzero, int N, float& best, int& bi) {
-  best = -1.0f;
-  bi = N;
-  for (int li = threadIdx.x; li < nr; li += blockDim.x) {
-    const int i = r0 + li;
-    if (i < j) continue;
-    float4* row = reinterpret_cast<float4*>(tile + static_cast<size_t>(li) * S + b0);
-    if (i == j) {  // row j becomes the pivot row (inner block)
-#pragma unroll
-      for (int c = 0; c < CP_IB / 4; c++) row[c] = make_float4(ps[4 * c], ps[4 * c + 1], ps[4 * c + 2], ps[4 * c + 3]);
-      continue;
-    }
-    // the row's inner block in registers (row gi takes row j's)
-    const float4* in = (i == gi) ? jseg4 : row;
-    float t[CP_IB];
-#pragma unroll
-    for (int c = 0; c < CP_IB / 4; c++) {
-      const float4 x = in[c];
-      t[4 * c] = x.x;
-      t[4 * c + 1] = x.y;
-      t[4 * c + 2] = x.z;
-      t[4 * c + 3] = x.w;
-    }
-    if (nonzero) {
-      const float l = t[Q0] * inv;
-      t[Q0] = l;
-#pragma unroll
-      for (int q = Q0 + 1; q < CP_IB; q++) t[q] = fmaf(-l, ps[q], t[q]);
-    }
-    if (Q0 + 1 < CP_IB && Q0 + 1 < nb) {
-      const float v = fabsf(t[(Q0 + 1) % CP_IB]);
-      if (better(v, i, best, bi)) {
-        best = v;
-        bi = i;
-      }
-    }
-    // columns before Q0 only change in the swapped rows
-    constexpr int cfirst = Q0 / 4;
-    const int cstart = (i == gi) ? 0 : cfirst;
-#pragma unroll
-    for (int c = 0; c < CP_IB / 4; c++)
-      if (c >= cstart) row[c] = make_float4(t[4 * c], t[4 * c + 1], t[4 * c + 2], t[4 * c + 3]);
-  }
-}
 
 // The per-column exchange of the cluster panel: each CTA's candidate (and the
 // owner's row j) go to every CTA's receive slot by st.async, which completes
@@ -1876,7 +1851,8 @@ __device__ __forceinline__ bool cp_wait(unsigned long long* bar, unsigned parity
   }
 }
 
-__global__ void __launch_bounds__(CP_THREADS) panel_cluster16_kernel(float* __restrict__ A, long long ld, int N,
+template <int RPT>
+__global__ void __launch_bounds__(CP_THREADS, 1) panel_cluster16_kernel(float* __restrict__ A, long long ld, int N,
                                                                      int j0, int jb, int per,
                                                                      int* __restrict__ ipiv,
                                                                      int* __restrict__ info,
@@ -1892,8 +1868,9 @@ __global__ void __launch_bounds__(CP_THREADS) panel_cluster16_kernel(float* __re
   __shared__ __align__(16) float jrow[2][128];
   __shared__ __align__(16) CpSlot recv[2];
   __shared__ __align__(16) float ublk[CP_IB][128];  // rows of the current inner block (L11 | A12 -> U12)
-  __shared__ float wv[CP_WARPS];
+  __shared__ unsigned wv[CP_WARPS];
   __shared__ int wi[CP_WARPS];
+  __shared__ __align__(16) float4 wseg[CP_WARPS][CP_IB / 4], jbuf[CP_IB / 4];  // the warps' candidates, row j
   __shared__ __align__(8) unsigned long long xmb[2];  // the exchange's mbarriers, one per receive slot
   const int S = cp_row_stride(jb);
   const int rank = static_cast<int>(cluster.block_rank());
@@ -1923,28 +1900,53 @@ __global__ void __launch_bounds__(CP_THREADS) panel_cluster16_kernel(float* __re
   for (int b0 = 0; b0 < jb; b0 += CP_IB) {
     const int be = (b0 + CP_IB < jb) ? b0 + CP_IB : jb;
     const int nb = be - b0;
-    // this thread's candidate for the block's first column
-    float best = -1.0f;
+    // The inner block of this thread's rows stays in registers for the
+    // block's columns, t[r][0] being the current column (each step shifts the
+    // rest down); and the thread's candidate for the block's first column.
+    float t[RPT][CP_IB];
+    unsigned best = 0;
     int bi = N;
-    for (int li = tid; li < nr; li += bd) {
-      const int i = r0 + li;
-      if (i < j0 + b0) continue;
-      const float v = fabsf(tile[li * S + b0]);
-      if (better(v, i, best, bi)) {
-        best = v;
-        bi = i;
+#pragma unroll
+    for (int r = 0; r < RPT; r++) {
+      const int li = tid + r * bd;
+#pragma unroll
+      for (int c = 0; c < CP_IB / 4; c++) {
+        float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (li < nr) x = *reinterpret_cast<const float4*>(tile + static_cast<size_t>(li) * S + b0 + 4 * c);
+        t[r][4 * c] = x.x;
+        t[r][4 * c + 1] = x.y;
+        t[r][4 * c + 2] = x.z;
+        t[r][4 * c + 3] = x.w;
+      }
+      if (li < nr && r0 + li >= j0 + b0) {
+        const unsigned key = cp_key(t[r][0]);
+        if (key > best) {  // rows ascend: ties stay with the lower one
+          best = key;
+          bi = r0 + li;
+        }
       }
     }
     for (int jj = b0; jj < be; jj++) {
       const int j = j0 + jj;
       const int slot = jj & 1;
       const int q0 = jj - b0;  // column jj within the inner block
-      for (int o = 16; o > 0; o >>= 1) {
-        const float ov = __shfl_xor_sync(0xffffffffu, best, o);
-        const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-        if (better(ov, oi, best, bi)) {
-          best = ov;
-          bi = oi;
+      {
+        const int own = bi;
+        cp_warp_best(best, bi);
+        const bool cand = best != 0 && own == bi;
+#pragma unroll
+        for (int r = 0; r < RPT; r++) {
+          const int i = r0 + tid + r * bd;
+          if (cand && i == bi) {
+#pragma unroll
+            for (int c = 0; c < CP_IB / 4; c++)
+              wseg[warp][c] = make_float4(t[r][4 * c], t[r][4 * c + 1], t[r][4 * c + 2], t[r][4 * c + 3]);
+          }
+          if (i == j && tid + r * bd < nr) {
+#pragma unroll
+            for (int c = 0; c < CP_IB / 4; c++)
+              jbuf[c] = make_float4(t[r][4 * c], t[r][4 * c + 1], t[r][4 * c + 2], t[r][4 * c + 3]);
+          }
         }
       }
       if (lane == 0) {
@@ -1952,37 +1954,39 @@ __global__ void __launch_bounds__(CP_THREADS) panel_cluster16_kernel(float* __re
         wi[warp] = bi;
       }
       __syncthreads();  // also orders the previous column step's tile writes
-      if (warp == 0) {
-        float cv = (lane < CP_WARPS) ? wv[lane] : -1.0f;
-        int ci = (lane < CP_WARPS) ? wi[lane] : N;
-        for (int o = 16; o > 0; o >>= 1) {
-          const float ov = __shfl_xor_sync(0xffffffffu, cv, o);
-          const int oi = __shfl_xor_sync(0xffffffffu, ci, o);
-          if (better(ov, oi, cv, ci)) {
-            cv = ov;
-            ci = oi;
+      if (warp == 0 || warp == 2) {
+        unsigned cv = (lane < (bd >> 5)) ? wv[lane] : 0u;
+        int ci = (lane < (bd >> 5)) ? wi[lane] : N;
+        const unsigned wkey = cv;
+        const int wrow = ci;
+        cp_warp_best(cv, ci);
+        if (warp == 0) {
+          const int from = __ffs(__ballot_sync(0xffffffffu, wkey == cv && wrow == ci)) - 1;
+          const float4* src = wseg[from < CP_WARPS ? from : 0];  // any words when there is no candidate
+          // (destination CTA, half of the inner block)
+          for (int e = lane; e < 2 * ncl; e += 32) {
+            const unsigned d = static_cast<unsigned>(e >> 1);
+            const int c0 = (e & 1) * 2;
+            const unsigned bar = cp_mapa(cp_smem(&xmb[slot]), d);
+            cp_push4(cp_mapa(cp_smem(&recv[slot].seg[rank][c0]), d), src[c0], bar);
+            cp_push4(cp_mapa(cp_smem(&recv[slot].seg[rank][c0 + 1]), d), src[c0 + 1], bar);
+            if ((e & 1) == 0) cp_push1(cp_mapa(cp_smem(&recv[slot].v[rank]), d), cv, bar);
           }
-        }
-        const int crow = (ci < N) ? ci - r0 : 0;  // row 0's words stand in when there is no candidate
-        if (ci < N)
-          for (int k = lane; k < jb; k += 32) cand_row[slot][k] = tile[crow * S + k];
-        __syncwarp();  // the whole row copy before any lane's (releasing) push
-        const float4* src = reinterpret_cast<const float4*>(tile + static_cast<size_t>(crow) * S + b0);
-        for (int e = lane; e < 2 * ncl; e += 32) {  // (destination CTA, half of the inner block)
-          const unsigned d = static_cast<unsigned>(e >> 1);
-          const int c0 = (e & 1) * 2;
-          const unsigned bar = cp_mapa(cp_smem(&xmb[slot]), d);
-          cp_push4(cp_mapa(cp_smem(&recv[slot].seg[rank][c0]), d), src[c0], bar);
-          cp_push4(cp_mapa(cp_smem(&recv[slot].seg[rank][c0 + 1]), d), src[c0 + 1], bar);
-          if ((e & 1) == 0) {
-            cp_push1(cp_mapa(cp_smem(&recv[slot].v[rank]), d), __float_as_uint(cv), bar);
-            cp_push1(cp_mapa(cp_smem(&recv[slot].i[rank]), d), static_cast<unsigned>(ci), bar);
-          }
+        } else {
+          // the candidate's other columns, then its row number: the (releasing)
+          // push of the number comes after the whole row copy
+          if (cv == 0) ci = N;
+          if (ci < N)
+            for (int k = lane; k < jb; k += 32) cand_row[slot][k] = tile[static_cast<size_t>(ci - r0) * S + k];
+          __syncwarp();
+          if (lane < ncl)
+            cp_push1(cp_mapa(cp_smem(&recv[slot].i[rank]), lane), static_cast<unsigned>(ci),
+                     cp_mapa(cp_smem(&xmb[slot]), lane));
         }
       } else if (warp == 1 && j >= r0 && j < r1) {
         for (int k = lane; k < jb; k += 32) jrow[slot][k] = tile[(j - r0) * S + k];
         __syncwarp();
-        const float4* src = reinterpret_cast<const float4*>(tile + static_cast<size_t>(j - r0) * S + b0);
+        const float4* src = jbuf;
         for (int e = lane; e < 2 * ncl; e += 32) {
           const unsigned d = static_cast<unsigned>(e >> 1);
           const int c0 = (e & 1) * 2;
@@ -1997,23 +2001,13 @@ __global__ void __launch_bounds__(CP_THREADS) panel_cluster16_kernel(float* __re
       if (tid == 0 && !dead) cp_arm(&xmb[slot], xbytes);
       // the winner, from this CTA's own receive slot: every warp reduces the
       // candidates across its lanes (same result everywhere)
-      float gv = -1.0f;
-      int gi = N, tag = -1;
-      if (lane < ncl) {
-        gv = recv[slot].v[lane];
-        gi = recv[slot].i[lane];
-        tag = lane;
-      }
-      for (int o = 16; o > 0; o >>= 1) {
-        const float ov = __shfl_xor_sync(0xffffffffu, gv, o);
-        const int oi = __shfl_xor_sync(0xffffffffu, gi, o);
-        const int ot = __shfl_xor_sync(0xffffffffu, tag, o);
-        if (better(ov, oi, gv, gi)) {
-          gv = ov;
-          gi = oi;
-          tag = ot;
-        }
-      }
+      const unsigned mine = lane < ncl ? recv[slot].v[lane] : 0u;
+      unsigned gv = mine;
+      int gi = lane < ncl ? recv[slot].i[lane] : N;
+      const int row = gi;
+      cp_warp_best(gv, gi);
+      // the CTA it came from (rows are distinct)
+      int tag = __ffs(__ballot_sync(0xffffffffu, mine == gv && row == gi)) - 1;
       // nothing usable below the diagonal: no swap.  (A winner is always a
       // row at or below j; a thread whose exchange wait ran out may read a
       // stale slot, and the row-move list must still hold rows of the panel.)
@@ -2024,7 +2018,7 @@ __global__ void __launch_bounds__(CP_THREADS) panel_cluster16_kernel(float* __re
       if (rank == 0 && tid == 0) {
         ipiv[j] = gi;
         pivs[jj] = gi;
-        if (!(gv > 0.0f) && *info == 0) *info = j + 1;  // zero (or NaN) pivot
+        if (gv <= 1u && *info == 0) *info = j + 1;  // zero (or NaN) pivot
       }
       // the pivot row's inner block
       const float4* p4 = (tag >= 0) ? recv[slot].seg[tag] : recv[slot].jseg;
@@ -2037,32 +2031,60 @@ __global__ void __launch_bounds__(CP_THREADS) panel_cluster16_kernel(float* __re
         ps[4 * c + 2] = x.z;
         ps[4 * c + 3] = x.w;
       }
-      float piv = ps[0];
+      const float piv = ps[0];
+      const bool nonzero = piv != 0.0f;
+      const float inv = nonzero ? 1.0f / piv : 0.0f;
+      // the column step on this thread's rows: row gi takes row j's block, the
+      // multiplier goes to its place in the tile, the rest is updated and
+      // shifted down; and the thread's candidate for the next column
+      best = 0;
+      bi = N;
 #pragma unroll
-      for (int q = 1; q < CP_IB; q++)
-        if (q == q0) piv = ps[q];
-      const float inv = (piv != 0.0f) ? 1.0f / piv : 0.0f;
-      const float4* jseg4 = recv[slot].jseg;
-      switch (q0) {
-#define KD_CP_CASE(Q) \
-  case Q: cp_column_step<Q>(tile, S, b0, r0, nr, j, gi, nb, ps, jseg4, inv, piv != 0.0f, N, best, bi); break;
-        KD_CP_CASE(0) KD_CP_CASE(1) KD_CP_CASE(2) KD_CP_CASE(3) KD_CP_CASE(4) KD_CP_CASE(5) KD_CP_CASE(6)
-        KD_CP_CASE(7) KD_CP_CASE(8) KD_CP_CASE(9) KD_CP_CASE(10) KD_CP_CASE(11) KD_CP_CASE(12) KD_CP_CASE(13)
-        KD_CP_CASE(14) KD_CP_CASE(15)
-#undef KD_CP_CASE
-        default: break;
+      for (int r = 0; r < RPT; r++) {
+        const int li = tid + r * bd, i = r0 + li;
+        if (li >= nr || i <= j) continue;
+        if (i == gi) {
+#pragma unroll
+          for (int c = 0; c < CP_IB / 4; c++) {
+            const float4 x = recv[slot].jseg[c];
+            t[r][4 * c] = x.x;
+            t[r][4 * c + 1] = x.y;
+            t[r][4 * c + 2] = x.z;
+            t[r][4 * c + 3] = x.w;
+          }
+        }
+        const float l = nonzero ? t[r][0] * inv : t[r][0];
+        tile[static_cast<size_t>(li) * S + jj] = l;
+        if (nonzero) {
+#pragma unroll
+          for (int q = 1; q < CP_IB; q++) t[r][q - 1] = fmaf(-l, ps[q], t[r][q]);
+        } else {
+#pragma unroll
+          for (int q = 1; q < CP_IB; q++) t[r][q - 1] = t[r][q];
+        }
+        t[r][CP_IB - 1] = 0.0f;
+        if (q0 + 1 < nb) {
+          const unsigned key = cp_key(t[r][0]);
+          if (key > best) {
+            best = key;
+            bi = i;
+          }
+        }
       }
+      // row j becomes the pivot row: its columns jj .. be - 1
+      if (j >= r0 && j < r1 && tid < be - jj)
+        tile[static_cast<size_t>(j - r0) * S + jj + tid] = reinterpret_cast<const float*>(p4)[tid];
       // the swapped rows' other columns, from the owners' shared memory
       if (gi != j) {
         if (gi >= r0 && gi < r1) {
           const float* src = cluster.map_shared_rank(&jrow[slot][0], (j - j0) / per);
           for (int k = tid; k < jb; k += bd)
-            if (k < b0 || k >= be) tile[(gi - r0) * S + k] = src[k];
+            if (k < jj || k >= be) tile[(gi - r0) * S + k] = src[k];
         }
         if (j >= r0 && j < r1) {
           const float* src = cluster.map_shared_rank(&cand_row[slot][0], tag);
           for (int k = tid; k < jb; k += bd)
-            if (k < b0 || k >= be) tile[(j - r0) * S + k] = src[k];
+            if (k < jj || k >= be) tile[(j - r0) * S + k] = src[k];
         }
       }
     }
@@ -2071,20 +2093,40 @@ __global__ void __launch_bounds__(CP_THREADS) panel_cluster16_kernel(float* __re
       // diagonal); every CTA fetches them whole and forms
       // U12 = L11^{-1} A12 for columns be..jb-1.
       cluster.sync();
-      for (int e = tid; e < nb * jb; e += bd) {
-        const int t = e / jb, k = e % jb;
-        const int row = j0 + b0 + t;
-        const int owner = (row - j0) / per;
-        const float* ot = cluster.map_shared_rank(tile, owner);
-        ublk[t][k] = ot[static_cast<long long>(row - (j0 + owner * per)) * S + k];
+      // (the columns from b0 on, by 16-byte words, all loads before the stores;
+      // nb == CP_IB here, and padding columns come along)
+      {
+        const int words = S / 4 - 1 - b0 / 4, total = CP_IB * words;
+        float4 w[2];
+#pragma unroll
+        for (int u = 0; u < 2; u++) {
+          const int e = tid + u * bd;
+          if (e < total) {
+            const int t = e / words, k4 = e - t * words, row = b0 + t, owner = row / per;
+            w[u] = *reinterpret_cast<const float4*>(cluster.map_shared_rank(tile, owner) +
+                                                    static_cast<size_t>(row - owner * per) * S + b0 + 4 * k4);
+          }
+        }
+#pragma unroll
+        for (int u = 0; u < 2; u++) {
+          const int e = tid + u * bd;
+          if (e < total) *reinterpret_cast<float4*>(&ublk[e / words][b0 + 4 * (e % words)]) = w[u];
+        }
       }
       __syncthreads();
-      for (int k = be + tid; k < jb; k += bd)  // one column of U12 per thread
-        for (int t = 1; t < nb; t++) {
-          float acc = ublk[t][k];
-          for (int q = 0; q < t; q++) acc = fmaf(-ublk[t][b0 + q], ublk[q][k], acc);
+      for (int k = be + tid; k < jb; k += bd) {  // one column of U12 per thread, in registers
+        float u[CP_IB];
+#pragma unroll
+        for (int t = 0; t < CP_IB; t++) u[t] = ublk[t][k];
+#pragma unroll
+        for (int t = 1; t < CP_IB; t++) {
+          float acc = u[t];
+#pragma unroll
+          for (int q = 0; q < t; q++) acc = fmaf(-ublk[t][b0 + q], u[q], acc);
+          u[t] = acc;
           ublk[t][k] = acc;
         }
+      }
       cluster.sync();  // remote reads of the block rows are done
       // owners store U12; rows below the block get the rank-16 update, one
       // row per thread with its 16 multipliers in registers and four
@@ -2175,13 +2217,14 @@ static bool panel_cluster16(Context* ctx, float* A, long long ld, int N, int j0,
   const int per = (rows + ncl - 1) / ncl;
   const size_t smem = static_cast<size_t>(per) * cp_row_stride(jb) * sizeof(float);
   if (smem > CP_MAX_SMEM) return false;
-  static int usable = 0;
+  static bool usable = false;
   static std::once_flag probe;
   std::call_once(probe, [] {
-    if (cudaFuncSetAttribute(panel_cluster16_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) ==
-            cudaSuccess &&
-        cudaFuncSetAttribute(panel_cluster16_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             static_cast<int>(CP_MAX_SMEM)) == cudaSuccess) {
+    auto prepare = [](auto* kernel) {
+      if (cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
+          cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(CP_MAX_SMEM)) !=
+              cudaSuccess)
+        return false;
       cudaLaunchConfig_t q = {};
       q.gridDim = dim3(CP_CL, 1, 1);
       q.blockDim = dim3(CP_THREADS, 1, 1);
@@ -2194,15 +2237,16 @@ static bool panel_cluster16(Context* ctx, float* A, long long ld, int N, int j0,
       q.attrs = qa;
       q.numAttrs = 1;
       int nclusters = 0;
-      if (cudaOccupancyMaxActiveClusters(&nclusters, panel_cluster16_kernel, &q) == cudaSuccess && nclusters > 0)
-        usable = 1;
-    }
+      return cudaOccupancyMaxActiveClusters(&nclusters, kernel, &q) == cudaSuccess && nclusters > 0;
+    };
+    usable = prepare(panel_cluster16_kernel<1>) && prepare(panel_cluster16_kernel<2>) &&
+             prepare(panel_cluster16_kernel<4>);
     cudaGetLastError();  // clear a refused attribute or query
   });
   if (!usable) return false;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(ncl, 1, 1);
-  cfg.blockDim = dim3(CP_THREADS, 1, 1);
+  cfg.blockDim = dim3(cp_threads(per), 1, 1);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = ctx->stream();
   cudaLaunchAttribute at[1];
@@ -2212,8 +2256,10 @@ static bool panel_cluster16(Context* ctx, float* A, long long ld, int N, int j0,
   at[0].val.clusterDim.z = 1;
   cfg.attrs = at;
   cfg.numAttrs = 1;
-  cuda_check(cudaLaunchKernelEx(&cfg, panel_cluster16_kernel, A, ld, N, j0, jb, per, ipiv, info, swap_map, err, wait_ns,
-                                stall),
+  const int rpt = (per + static_cast<int>(cfg.blockDim.x) - 1) / static_cast<int>(cfg.blockDim.x);
+  auto* kernel = rpt == 1 ? panel_cluster16_kernel<1> : rpt == 2 ? panel_cluster16_kernel<2> : panel_cluster16_kernel<4>;
+  if (rpt > 4) return false;
+  cuda_check(cudaLaunchKernelEx(&cfg, kernel, A, ld, N, j0, jb, per, ipiv, info, swap_map, err, wait_ns, stall),
              "panel cluster kernel");
   ctx->launches += 1;
   return true;

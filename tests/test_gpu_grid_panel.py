@@ -58,3 +58,23 @@ def test_zero_column_is_reported(ctx, col):
     with pytest.raises(KadathError) as e:
         _solve(ctx, a)
     assert e.value.status == 3  # KD_ERR_SINGULAR
+
+
+@pytest.mark.parametrize("n", [2, 33, 95, 97, 200, 450, 897, 1300, 3600])
+def test_cluster_panel_pivots_as_lapack(ctx, n):
+    """The FP32 cluster panel (clusters of 2 to 16 CTAs, one or two rows a thread,
+    last panels of any width) on a matrix of small integers, whose first pivots are
+    exact in FP32 as in LAPACK: the solves then need few refinements."""
+    from kadath_frontera_gb300.kadath import DenseLU, KD_LU_FP32_IR
+    rng = np.random.default_rng(n)
+    a = rng.integers(-4, 5, (n, n)).astype(float) + 3.0 * n ** 0.5 * np.diag(rng.choice([-1.0, 1.0], n))
+    x = rng.standard_normal(n)
+    b = a @ x
+    da, db = torch.tensor(a.T.copy(), device="cuda"), torch.tensor(b, device="cuda")
+    torch.cuda.synchronize()
+    lu = DenseLU(ctx)
+    lu.factor(da.data_ptr(), n, n, KD_LU_FP32_IR)
+    lu.solve(db.data_ptr())
+    # refined to 1e-14 relative residual; the condition number is below 1e3
+    assert np.linalg.norm(db.cpu().numpy() - x) <= 1e-10 * np.linalg.norm(x)
+    assert lu.stats()["refine_iters"] <= 6
