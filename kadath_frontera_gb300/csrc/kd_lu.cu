@@ -291,6 +291,46 @@ __device__ __forceinline__ double pow2_inverse(double m) {
   return ldexp(1.0, 1 - e);  // 2^-(e-1): scaled max in [1, 2)
 }
 
+// The equilibration and the FP32 working copy move powers of two about: on
+// integers, because an FP64 multiply, compare or maximum takes 16 cycles of an
+// SM per warp (the copy of a 12,331 x 12,331 matrix took 1.5 ms with five FP64
+// instructions an entry, 0.3 ms of which are its bytes).
+// |v| as bits (ordered like it), 0 for NaN.
+__device__ __forceinline__ unsigned long long modulus_bits(double v) {
+  const unsigned long long b = static_cast<unsigned long long>(__double_as_longlong(v)) & 0x7fffffffffffffffull;
+  return b > 0x7ff0000000000000ull ? 0ull : b;
+}
+// v * 2^k, exact like the product.  The rare case is a call, not inlined: the
+// loops below hold sixteen of them.
+__device__ __noinline__ double times_pow2_rare(double v, int k) { return scalbn(v, k); }  // subnormal, Inf, NaN, out of range
+__device__ __forceinline__ double times_pow2(double v, int k) {
+  const int hi = __double2hiint(v), lo = __double2loint(v);
+  const int e = (hi >> 20) & 0x7ff;
+  if (static_cast<unsigned>(e - 1) < 0x7feu && static_cast<unsigned>(e + k - 1) < 0x7feu)
+    return __hiloint2double(hi + (k << 20), lo);
+  if (((hi & 0x7fffffff) | lo) == 0) return v;
+  return times_pow2_rare(v, k);
+}
+// v * 2^k rounded to FP32: where the result is a normal float, the top 23
+// mantissa bits rounded to nearest even by hand, since the conversion also
+// runs at the FP64 rate (it bounded the copy: 0.65 ms, its bytes 0.28 ms).
+__device__ __noinline__ float pow2_to_float_rare(double v, int k) { return static_cast<float>(scalbn(v, k)); }
+__device__ __forceinline__ float pow2_to_float(double v, int k) {
+  const unsigned hi = static_cast<unsigned>(__double2hiint(v)), lo = static_cast<unsigned>(__double2loint(v));
+  const int e = static_cast<int>((hi >> 20) & 0x7ffu), ef = e + k - 1023 + 127;  // the float's exponent field
+  if (static_cast<unsigned>(e - 1) < 0x7feu && static_cast<unsigned>(ef - 1) < 0xfeu) {
+    const unsigned f = (hi & 0x80000000u) | (static_cast<unsigned>(ef) << 23) | ((hi & 0xfffffu) << 3) | (lo >> 29);
+    // the 29 bits cut off, against half a unit: up if above, or equal and f odd
+    return __uint_as_float(f + (((lo & 0x1fffffffu) + (f & 1u) > 0x10000000u) ? 1u : 0u));
+  }
+  if (((hi & 0x7fffffffu) | lo) == 0u) return __uint_as_float(hi);
+  return pow2_to_float_rare(v, k);
+}
+// k of a scale 2^k
+__device__ __forceinline__ int pow2_exponent(double s) {
+  return ((__double2hiint(s) >> 20) & 0x7ff) - 1023;
+}
+
 // Maxima of |A_ij| over column chunks, merged with atomicMax on the bit
 // patterns of non-negative doubles (order-independent, deterministic).
 __global__ void row_absmax_kernel(const double* __restrict__ A, long long ld, int N, int chunk,
@@ -299,9 +339,17 @@ __global__ void row_absmax_kernel(const double* __restrict__ A, long long ld, in
   if (i >= N) return;
   const int c0 = blockIdx.y * chunk;
   const int c1 = (c0 + chunk < N) ? c0 + chunk : N;
-  double m = 0.0;
-  for (int j = c0; j < c1; j++) m = fmax(m, fabs(A[static_cast<long long>(j) * ld + i]));
-  atomicMax(rmax + i, static_cast<unsigned long long>(__double_as_longlong(m)));
+  unsigned long long m = 0;
+  int j = c0;
+  for (; j + 8 <= c1; j += 8) {
+    unsigned long long v[8];
+#pragma unroll
+    for (int u = 0; u < 8; u++) v[u] = modulus_bits(A[static_cast<long long>(j + u) * ld + i]);
+#pragma unroll
+    for (int u = 0; u < 8; u++) m = max(m, v[u]);
+  }
+  for (; j < c1; j++) m = max(m, modulus_bits(A[static_cast<long long>(j) * ld + i]));
+  atomicMax(rmax + i, m);
 }
 
 __global__ void row_scale_kernel(const unsigned long long* __restrict__ rmax, int N, double* __restrict__ rs) {
@@ -309,27 +357,81 @@ __global__ void row_scale_kernel(const unsigned long long* __restrict__ rmax, in
   if (i < N) rs[i] = pow2_inverse(__longlong_as_double(static_cast<long long>(rmax[i])));
 }
 
-// One CTA per column: c_j from max_i |r_i A_ij|, then the scaled FP32 column.
-__global__ void col_scale_convert_kernel(const double* __restrict__ A, long long lda, const double* __restrict__ rs,
-                                         int N, double* __restrict__ cs, float* __restrict__ B, long long ldb) {
-  __shared__ double red[32];
+// One CTA per column: c_j from max_i |r_i A_ij|, then the scaled FP32 column,
+// its rows in the order perm when one is given.  rs null: no scales.  The
+// converted column is put in order in shared memory where it fits (KEEP): rows
+// gathered from global memory cost a 32-byte sector each.  Memory's share of
+// 12,331 rows is 0.28 ms; measured 0.51 ms in order and 0.78 ms permuted (the
+// column kept as doubles, half as many CTAs an SM: 1.9 ms; FP64 products and
+// comparisons and a global gather: 1.5 ms each).
+constexpr int SC_THREADS = 512;
+constexpr size_t SC_MAX_SMEM = 220 * 1024;
+template <bool KEEP>
+__global__ void __launch_bounds__(SC_THREADS) scale_convert_kernel(const double* __restrict__ A, long long lda,
+                                                                   const double* __restrict__ rs, int N,
+                                                                   double* __restrict__ cs, float* __restrict__ B,
+                                                                   long long ldb, const int* __restrict__ perm) {
+  extern __shared__ float kept[];  // the converted column, rows in A's order
+  __shared__ unsigned long long red[SC_THREADS / 32];
+  constexpr int U = 8;
   const int j = blockIdx.x;
   const double* col = A + static_cast<long long>(j) * lda;
-  double m = 0.0;
-  for (int i = threadIdx.x; i < N; i += blockDim.x) m = fmax(m, fabs(rs[i] * col[i]));
-  for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = m;
-  __syncthreads();
-  if (threadIdx.x < 32) {
-    m = (threadIdx.x < (blockDim.x >> 5)) ? red[threadIdx.x] : 0.0;
-    for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
-    if (threadIdx.x == 0) red[0] = m;
+  int kc = 0;
+  if (rs) {
+    unsigned long long m = 0;
+    for (int i0 = threadIdx.x; i0 < N; i0 += U * SC_THREADS) {
+      double v[U], r[U];
+#pragma unroll
+      for (int u = 0; u < U; u++) {
+        const int i = i0 + u * SC_THREADS;
+        v[u] = i < N ? col[i] : 0.0;
+        r[u] = i < N ? rs[i] : 1.0;
+      }
+#pragma unroll
+      for (int u = 0; u < U; u++) m = max(m, modulus_bits(times_pow2(v[u], pow2_exponent(r[u]))));
+    }
+    for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = m;
+    __syncthreads();
+#pragma unroll
+    for (int w = 0; w < SC_THREADS / 32; w++) m = max(m, red[w]);
+    const double c = pow2_inverse(__longlong_as_double(static_cast<long long>(m)));
+    if (threadIdx.x == 0) cs[j] = c;
+    kc = pow2_exponent(c);
   }
-  __syncthreads();
-  const double c = pow2_inverse(red[0]);
-  if (threadIdx.x == 0) cs[j] = c;
   float* out = B + static_cast<long long>(j) * ldb;
-  for (int i = threadIdx.x; i < N; i += blockDim.x) out[i] = static_cast<float>(rs[i] * col[i] * c);
+  for (int i0 = threadIdx.x; i0 < N; i0 += U * SC_THREADS) {
+    double v[U], r[U];
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      const int i = i0 + u * SC_THREADS;
+      const int p = (!KEEP && perm && i < N) ? perm[i] : i;
+      v[u] = i < N ? col[p] : 0.0;
+      r[u] = (rs && i < N) ? rs[p] : 1.0;
+    }
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      const int i = i0 + u * SC_THREADS;
+      const float f = pow2_to_float(v[u], pow2_exponent(r[u]) + kc);
+      if (i < N) {
+        if (KEEP)
+          kept[i] = f;
+        else
+          out[i] = f;
+      }
+    }
+  }
+  if (KEEP) {
+    __syncthreads();
+    for (int i0 = threadIdx.x; i0 < N; i0 += U * SC_THREADS) {
+      int p[U];
+#pragma unroll
+      for (int u = 0; u < U; u++) p[u] = i0 + u * SC_THREADS < N ? perm[i0 + u * SC_THREADS] : 0;
+#pragma unroll
+      for (int u = 0; u < U; u++)
+        if (i0 + u * SC_THREADS < N) out[i0 + u * SC_THREADS] = kept[p[u]];
+    }
+  }
 }
 
 // ---- panel of a static-pivot factorisation (FP32, rows in pivot order) ----
@@ -580,51 +682,9 @@ __global__ void __launch_bounds__(NP_THREADS) panel_nopiv_kernel(float* __restri
   }
 }
 
-// The FP32 working copy with its rows in a given order:
-// B[i][j] = r_{p(i)} A[p(i)][j] c_j, c_j = 2^-round(log2 max_i |r_i A_ij|)
-// (the same column scales as col_scale_convert_kernel, whose maximum does
-// not depend on the row order).  rs == nullptr: no scaling.
-__global__ void convert_rows_kernel(const double* __restrict__ A, long long lda, const double* __restrict__ rs,
-                                    int N, double* __restrict__ cs, float* __restrict__ B, long long ldb,
-                                    const int* __restrict__ perm) {
-  __shared__ double red[32];
-  const int j = blockIdx.x;
-  const double* col = A + static_cast<long long>(j) * lda;
-  double c = 1.0;
-  if (rs) {
-    double m = 0.0;
-    for (int i = threadIdx.x; i < N; i += blockDim.x) m = fmax(m, fabs(rs[i] * col[i]));
-    for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = m;
-    __syncthreads();
-    if (threadIdx.x < 32) {
-      m = (threadIdx.x < (blockDim.x >> 5)) ? red[threadIdx.x] : 0.0;
-      for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
-      if (threadIdx.x == 0) red[0] = m;
-    }
-    __syncthreads();
-    c = pow2_inverse(red[0]);
-    if (threadIdx.x == 0) cs[j] = c;
-  }
-  float* out = B + static_cast<long long>(j) * ldb;
-  for (int i = threadIdx.x; i < N; i += blockDim.x) {
-    const int p = perm[i];
-    out[i] = static_cast<float>((rs ? rs[p] : 1.0) * col[p] * c);
-  }
-}
-
 __global__ void scale_vec_kernel(double* __restrict__ x, const double* __restrict__ s, int N) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < N) x[i] *= s[i];
-}
-
-__global__ void d2s(const double* __restrict__ A, long long lda, float* __restrict__ B, long long ldb, int N) {
-  long long total = static_cast<long long>(N) * N;
-  for (long long t = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; t < total;
-       t += static_cast<long long>(gridDim.x) * blockDim.x) {
-    long long c = t / N, r = t % N;
-    B[c * ldb + r] = static_cast<float>(A[c * lda + r]);
-  }
 }
 
 // ---- triangular solves on one right-hand side (blocked by TB rows) --------
@@ -637,18 +697,6 @@ __global__ void iota_kernel(int* __restrict__ v, int n) {
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) v[i] = i;
 }
 
-// perm such that (P b)[i] = b[perm[i]] for the sequential row swaps ipiv.
-__global__ void build_perm(const int* __restrict__ ipiv, int N, int* __restrict__ perm) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  for (int i = 0; i < N; i++) perm[i] = i;
-  for (int j = 0; j < N; j++) {
-    int p = ipiv[j];
-    int t = perm[j];
-    perm[j] = perm[p];
-    perm[p] = t;
-  }
-}
-
 __global__ void gather_perm(const double* __restrict__ b, const int* __restrict__ perm, int N, double* __restrict__ out) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < N) out[i] = b[perm[i]];
@@ -659,47 +707,64 @@ __global__ void scatter_perm(const double* __restrict__ z, const int* __restrict
   if (i < N) out[perm[i]] = z[i];
 }
 
-// One CTA per TB x TB diagonal block: inverse of its unit-lower part (L) and
-// of its upper part (U), row-major, zero padded to TB x TB.  Thread c builds
-// column c of each inverse by substitution in FP64.
+// Inverse of the unit-lower (blockIdx.y 0) or upper part (1) of one TB x TB
+// diagonal block, row-major, zero padded to TB x TB; with FP32 factors also as
+// (hi, lo) float pairs.  Eight lanes a column, rows l + 8 q each; a finished
+// entry is broadcast by a shuffle and a warp starts at the first row of its four
+// columns.  Bound: the FP64 pipe.  (One thread a column took 140 us, a chain of
+// 2,000 dependent multiply-adds.)
+constexpr int ID_THREADS = TB * 8;
 template <class T>
-__global__ void invert_diag_blocks(const T* __restrict__ A, long long ld, int N, double* __restrict__ Linv,
-                                   double* __restrict__ Uinv) {
+__global__ void __launch_bounds__(ID_THREADS) invert_diag_blocks(const T* __restrict__ A, long long ld, int N,
+                                                                 double* __restrict__ Linv, double* __restrict__ Uinv,
+                                                                 float2* __restrict__ Linv2,
+                                                                 float2* __restrict__ Uinv2) {
   extern __shared__ double sm[];
-  double* D = sm;                 // D[i*TB + k]
-  double* XL = sm + TB * TB;      // XL[i*TB + c]
-  double* XU = sm + 2 * TB * TB;  // XU[i*TB + c]
-  const int blk = blockIdx.x;
+  double* D = sm;              // D[k * TB + i]: entry (i, k), rows reversed in both directions for U
+  double* X = sm + TB * TB;    // X[c * (TB + 1) + i]
+  __shared__ double rd[TB];
+  const int blk = blockIdx.x, upper = blockIdx.y;
   const int r0 = blk * TB;
   const int n = (N - r0 < TB) ? N - r0 : TB;
-  for (int e = threadIdx.x; e < TB * TB; e += blockDim.x) {
-    int i = e / TB, k = e % TB;
-    D[e] = (i < n && k < n) ? static_cast<double>(A[static_cast<long long>(r0 + k) * ld + r0 + i]) : 0.0;
-    XL[e] = 0.0;
-    XU[e] = 0.0;
+  // the upper part read from its last row and column on is a lower one
+  for (int e = threadIdx.x; e < TB * TB; e += ID_THREADS) {
+    const int i = e % TB, k = e / TB, si = upper ? n - 1 - i : i, sk = upper ? n - 1 - k : k;
+    const double v = (i < n && k < n && i >= k) ? static_cast<double>(A[static_cast<long long>(r0 + sk) * ld + r0 + si]) : 0.0;
+    D[e] = v;
+    if (i == k) rd[i] = (upper && i < n) ? 1.0 / v : 1.0;
   }
   __syncthreads();
-  const int c = threadIdx.x;
-  if (c < n) {
-    XL[c * TB + c] = 1.0;
-    for (int i = c + 1; i < n; i++) {
-      double s = 0.0;
-      for (int k = c; k < i; k++) s += D[i * TB + k] * XL[k * TB + c];
-      XL[i * TB + c] = -s;
-    }
-    XU[c * TB + c] = 1.0 / D[c * TB + c];
-    for (int i = c - 1; i >= 0; i--) {
-      double s = 0.0;
-      for (int k = i + 1; k <= c; k++) s += D[i * TB + k] * XU[k * TB + c];
-      XU[i * TB + c] = -s / D[i * TB + i];
+  const int l = threadIdx.x & 7, c = threadIdx.x >> 3, lane = threadIdx.x & 31;
+  double x[8];
+#pragma unroll
+  for (int q = 0; q < 8; q++) x[q] = (l + 8 * q == c) ? 1.0 : 0.0;
+  const int k0 = c & ~3;  // first column of the warp
+#pragma unroll
+  for (int kq = 0; kq < 8; kq++) {
+    if (8 * kq + 7 < k0) continue;
+    for (int kr = 0; kr < 8; kr++) {
+      const int k = 8 * kq + kr;
+      if (k < k0) continue;
+      const double xk = __shfl_sync(0xffffffffu, x[kq], (lane & 24) | kr) * rd[k];
+      if (l == kr) x[kq] = xk;
+#pragma unroll
+      for (int q = kq; q < 8; q++)
+        if (q > kq || l > kr) x[q] = fma(-D[k * TB + l + 8 * q], xk, x[q]);
     }
   }
+#pragma unroll
+  for (int q = 0; q < 8; q++) X[c * (TB + 1) + l + 8 * q] = x[q];
   __syncthreads();
-  double* lo = Linv + static_cast<size_t>(blk) * TB * TB;
-  double* uo = Uinv + static_cast<size_t>(blk) * TB * TB;
-  for (int e = threadIdx.x; e < TB * TB; e += blockDim.x) {
-    lo[e] = XL[e];
-    uo[e] = XU[e];
+  double* out = (upper ? Uinv : Linv) + static_cast<size_t>(blk) * TB * TB;
+  float2* out2 = upper ? Uinv2 : Linv2;
+  for (int e = threadIdx.x; e < TB * TB; e += ID_THREADS) {
+    const int i = e / TB, k = e % TB;  // row, column of the block
+    const double v = (i < n && k < n) ? (upper ? X[(n - 1 - k) * (TB + 1) + n - 1 - i] : X[k * (TB + 1) + i]) : 0.0;
+    out[e] = v;
+    if constexpr (std::is_same<T, float>::value) {
+      const float h = static_cast<float>(v);
+      out2[static_cast<size_t>(blk) * TB * TB + e] = make_float2(h, static_cast<float>(v - static_cast<double>(h)));
+    }
   }
 }
 
@@ -1123,16 +1188,6 @@ __device__ __forceinline__ DF df_add(DF a, DF b) {
   e += a.l + b.l;
   const float r = s + e;
   return {r, e - (r - s)};
-}
-
-// FP64 inverse blocks as (hi, lo) FP32 pairs: hi = fl32(d), lo = fl32(d - hi).
-__global__ void split_df_kernel(const double* __restrict__ d, float2* __restrict__ out, long long n) {
-  for (long long t = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; t < n;
-       t += static_cast<long long>(gridDim.x) * blockDim.x) {
-    const double v = d[t];
-    const float h = static_cast<float>(v);
-    out[t] = make_float2(h, static_cast<float>(v - static_cast<double>(h)));
-  }
 }
 
 // ---- triangular sweeps -----------------------------------------------------
@@ -2269,11 +2324,24 @@ static bool panel_cluster16(Context* ctx, float* A, long long ld, int N, int j0,
 // per column: all sources are read into registers before any write.
 constexpr int SWAP_PER_LANE = 8;  // 2 jb <= 256 = 32 x 8 moves
 template <class T>
-__global__ void laswp_map(T* __restrict__ A, long long ld, int N, int j0, int jb, const int* __restrict__ map) {
+__global__ void laswp_map(T* __restrict__ A, long long ld, int N, int j0, int jb, const int* __restrict__ map,
+                          int* __restrict__ perm) {
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   const int ncol = N - jb;
-  if (warp >= ncol) return;
+  if (warp > ncol) return;
+  if (warp == ncol) {  // the pivot order (P b)[i] = b[perm[i]] moves like a column
+    const int n = map[0];
+    int v[SWAP_PER_LANE];
+#pragma unroll
+    for (int q = 0; q < SWAP_PER_LANE; q++)
+      if (lane + 32 * q < n) v[q] = perm[map[1 + 2 * jb + lane + 32 * q]];
+    __syncwarp();
+#pragma unroll
+    for (int q = 0; q < SWAP_PER_LANE; q++)
+      if (lane + 32 * q < n) perm[map[1 + lane + 32 * q]] = v[q];
+    return;
+  }
   const int c = (warp < j0) ? warp : warp + jb;
   T* col = A + static_cast<long long>(c) * ld;
   const int n = map[0];
@@ -2389,17 +2457,15 @@ static void launch_trsm_chunk(Context* ctx, float* A, long long ld, int j0, int 
 
 template <class T>
 static void trsm_and_swaps(Context* ctx, T* A, long long ld, int N, int j0, int jb, const int* ipiv, int* map,
-                           bool map_ready) {
+                           bool map_ready, int* perm) {
   cudaStream_t s = ctx->stream();
   ProfScope ps(ctx, Context::PROF_LU_SWAP_TRSM, 2.0 * sizeof(T) * jb * (N - j0 - jb));
-  if (N > jb) {
-    if (!map_ready) {
-      build_swap_map<<<1, 32, 0, s>>>(ipiv, j0, jb, map);
-      ctx->launches += 1;
-    }
-    laswp_map<T><<<blocks(static_cast<long long>(N - jb) * 32, 256), 256, 0, s>>>(A, ld, N, j0, jb, map);
+  if (!map_ready) {
+    build_swap_map<<<1, 32, 0, s>>>(ipiv, j0, jb, map);
     ctx->launches += 1;
   }
+  laswp_map<T><<<blocks(static_cast<long long>(N - jb + 1) * 32, 256), 256, 0, s>>>(A, ld, N, j0, jb, map, perm);
+  ctx->launches += 1;
   if (j0 + jb < N) {
     if constexpr (std::is_same<T, float>::value) {
       launch_trsm_chunk(ctx, A, ld, j0, jb, j0 + jb, N);
@@ -2430,7 +2496,7 @@ void DenseLU::factor_fp64(double* A, long long ld, int N) {
   for (int j0 = 0; j0 < N; j0 += NB) {
     int jb = (N - j0 < NB) ? N - j0 : NB;
     const bool map_ready = panel_factor<double>(ctx_, A, ld, N, j0, jb, ipiv_, d_info_, nsm_, slot_mem_, swap_map_);
-    trsm_and_swaps<double>(ctx_, A, ld, N, j0, jb, ipiv_, swap_map_, map_ready);
+    trsm_and_swaps<double>(ctx_, A, ld, N, j0, jb, ipiv_, swap_map_, map_ready, perm_);
     int m = N - j0 - jb;
     if (m > 0) {
       // A22 -= A21 * A12
@@ -2488,7 +2554,7 @@ void DenseLU::factor_f32(float* A, long long ld, int N, bool tf32) {
       ctx_->join();
       side_pending = false;
     }
-    trsm_and_swaps<float>(ctx_, A, ld, N, j0, jb, ipiv_, swap_map_, map_ready);
+    trsm_and_swaps<float>(ctx_, A, ld, N, j0, jb, ipiv_, swap_map_, map_ready, perm_);
     const int m = N - j0 - jb;
     if (m <= 0) break;
     const int j0n = j0 + jb, jbn = width(j0n);
@@ -2623,6 +2689,25 @@ void DenseLU::factor_mixed(double* A, long long ld, int N, int mode, const int* 
   double* cs = eq_buf_ + N;
   unsigned long long* rmax = reinterpret_cast<unsigned long long*>(eq_buf_ + 2 * static_cast<size_t>(N));
   cudaStream_t st = ctx_->stream();
+  const size_t column = sizeof(float) * static_cast<size_t>(N);
+  const bool keep = perm && column <= SC_MAX_SMEM;
+  if (keep) {
+    static std::once_flag attr;
+    std::call_once(attr, [] {
+      cuda_check(cudaFuncSetAttribute(scale_convert_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      static_cast<int>(SC_MAX_SMEM)),
+                 "cudaFuncSetAttribute(working copy)");
+      cuda_check(cudaFuncSetAttribute(scale_convert_kernel<true>, cudaFuncAttributePreferredSharedMemoryCarveout,
+                                      cudaSharedmemCarveoutMaxShared),
+                 "cudaFuncSetAttribute(working copy)");
+    });
+  }
+  auto convert = [&](const double* r, double* c) {
+    if (keep)
+      scale_convert_kernel<true><<<N, SC_THREADS, column, st>>>(A, ld, r, N, c, A32_, ld32_, perm);
+    else
+      scale_convert_kernel<false><<<N, SC_THREADS, 0, st>>>(A, ld, r, N, c, A32_, ld32_, perm);
+  };
   if (equilibrate) {
     cuda_check(cudaMemsetAsync(rmax, 0, sizeof(unsigned long long) * N, st), "memset row max");
     const int rb = blocks(N, 256);
@@ -2632,27 +2717,22 @@ void DenseLU::factor_mixed(double* A, long long ld, int N, int mode, const int* 
     nch = (N + chunk - 1) / chunk;
     row_absmax_kernel<<<dim3(rb, nch), 256, 0, st>>>(A, ld, N, chunk, rmax);
     row_scale_kernel<<<rb, 256, 0, st>>>(rmax, N, rs);
-    if (perm)
-      convert_rows_kernel<<<N, 256, 0, st>>>(A, ld, rs, N, cs, A32_, ld32_, perm);
-    else
-      col_scale_convert_kernel<<<N, 256, 0, st>>>(A, ld, rs, N, cs, A32_, ld32_);
+    convert(rs, cs);
     ctx_->launches += 3;
-  } else if (perm) {
-    convert_rows_kernel<<<N, 256, 0, st>>>(A, ld, nullptr, N, nullptr, A32_, ld32_, perm);
-    ctx_->launches++;
   } else {
-    d2s<<<152 * 8, 256, 0, st>>>(A, ld, A32_, ld32_, N);
+    convert(nullptr, nullptr);
     ctx_->launches++;
   }
   scaled_ = equilibrate;
   iota_kernel<<<blocks(N, 256), 256, 0, st>>>(ipiv_, N);
+  if (!perm) iota_kernel<<<blocks(N, 256), 256, 0, st>>>(perm_, N);
   ctx_->launches++;
   if (perm) {
     factor_f32_nopiv(A32_, ld32_, N, mode == LU_TF32_IR);
-    prepare_solves<float>(A32_, ld32_, N, true);
+    prepare_solves<float>(A32_, ld32_, N);
   } else {
     factor_f32(A32_, ld32_, N, mode == LU_TF32_IR);
-    prepare_solves<float>(A32_, ld32_, N, false);
+    prepare_solves<float>(A32_, ld32_, N);
   }
   nopiv_ = perm != nullptr;
 }
@@ -2676,13 +2756,23 @@ void DenseLU::factor(double* A, long long ld, int N, int mode) {
     cuda_check(cudaMalloc(&ipiv_, sizeof(int) * N), "cudaMalloc(ipiv)");
     ipiv_cap_ = N;
   }
+  if (static_cast<size_t>(N) > perm_cap_) {
+    cudaFree(perm_);
+    cudaFree(tri_work_);
+    cuda_check(cudaMalloc(&perm_, sizeof(int) * N), "cudaMalloc(perm)");
+    // two FP64 vectors, then two FP32 vectors (the chained sweeps' copies)
+    cuda_check(cudaMalloc(&tri_work_, sizeof(double) * 3 * (((static_cast<size_t>(N) + 31) / 32) * 32)),
+               "cudaMalloc(tri work)");
+    perm_cap_ = N;
+  }
   stats = LuStats();
   stats.flops = static_cast<long long>(2.0 / 3.0 * double(N) * N * N);
   iota_kernel<<<blocks(N, 256), 256, 0, ctx_->stream()>>>(ipiv_, N);
   ctx_->launches++;
   if (mode == LU_FP64) {
+    iota_kernel<<<blocks(N, 256), 256, 0, ctx_->stream()>>>(perm_, N);
     factor_fp64(A, ld, N);
-    prepare_solves<double>(A, ld, N, false);
+    prepare_solves<double>(A, ld, N);
     nopiv_ = false;
   } else {
     ld32_ = ((static_cast<long long>(N) + 31) / 32) * 32;  // 128-byte aligned columns
@@ -2839,7 +2929,7 @@ void DenseLU::ensure_bsave() {
 // After factorisation: pivots as one permutation, inverses of the 64 x 64
 // diagonal blocks of L (unit lower) and U.
 template <class T>
-void DenseLU::prepare_solves(const T* LU, long long ld, int N, bool keep_perm) {
+void DenseLU::prepare_solves(const T* LU, long long ld, int N) {
   cudaStream_t s = ctx_->stream();
   const int nblk = (N + TB - 1) / TB;
   size_t need = static_cast<size_t>(nblk) * TB * TB;
@@ -2855,30 +2945,14 @@ void DenseLU::prepare_solves(const T* LU, long long ld, int N, bool keep_perm) {
     cuda_check(cudaMalloc(&dinv2_u_, need * sizeof(float2)), "cudaMalloc(Uinv pairs)");
     dinv_cap_ = need;
   }
-  if (static_cast<size_t>(N) > perm_cap_) {
-    cudaFree(perm_);
-    cudaFree(tri_work_);
-    cuda_check(cudaMalloc(&perm_, sizeof(int) * N), "cudaMalloc(perm)");
-    // two FP64 vectors, then two FP32 vectors (the chained sweeps' copies)
-    cuda_check(cudaMalloc(&tri_work_, sizeof(double) * 3 * (((static_cast<size_t>(N) + 31) / 32) * 32)),
-               "cudaMalloc(tri work)");
-    perm_cap_ = N;
-  }
-  if (!keep_perm) build_perm<<<1, 1, 0, s>>>(ipiv_, N, perm_);
-  size_t smem = sizeof(double) * 3 * TB * TB;
+  constexpr size_t smem = sizeof(double) * (TB * TB + TB * (TB + 1));
   static std::once_flag attr_set;
-  std::call_once(attr_set, [smem] {
+  std::call_once(attr_set, [] {
     cudaFuncSetAttribute(invert_diag_blocks<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
     cudaFuncSetAttribute(invert_diag_blocks<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
   });
-  invert_diag_blocks<T><<<nblk, TB, smem, s>>>(LU, ld, N, dinv_l_, dinv_u_);
-  if constexpr (std::is_same<T, float>::value) {
-    const long long n2 = static_cast<long long>(nblk) * TB * TB;
-    split_df_kernel<<<blocks(n2, 256) < 152 * 8 ? blocks(n2, 256) : 152 * 8, 256, 0, s>>>(dinv_l_, dinv2_l_, n2);
-    split_df_kernel<<<blocks(n2, 256) < 152 * 8 ? blocks(n2, 256) : 152 * 8, 256, 0, s>>>(dinv_u_, dinv2_u_, n2);
-    ctx_->launches += 2;
-  }
-  ctx_->launches += 2;
+  invert_diag_blocks<T><<<dim3(nblk, 2), ID_THREADS, smem, s>>>(LU, ld, N, dinv_l_, dinv_u_, dinv2_l_, dinv2_u_);
+  ctx_->launches++;
   cuda_check(cudaGetLastError(), "solve preparation");
 }
 

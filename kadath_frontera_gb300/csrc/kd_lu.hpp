@@ -103,7 +103,7 @@ class DenseLU {
   template <class T>
   void tri_solve(const T* LU, long long ld, int N, double* b, int trans);
   template <class T>
-  void prepare_solves(const T* LU, long long ld, int N, bool keep_perm);
+  void prepare_solves(const T* LU, long long ld, int N);
   void factor_f32_nopiv(float* A, long long ld, int N, bool tf32);
   void factor_mixed(double* A, long long ld, int N, int mode, const int* perm);
   int read_info();
