@@ -62,36 +62,79 @@ __host__ __device__ constexpr uint32_t tf32_idesc(int M, int N) {
          (static_cast<uint32_t>(M >> 4) << 24);
 }
 
-// Packs a column-major panel into a K-major, zero-padded buffer:
-//   out[r * kpad + kk] = src(r, kk) for r < rows, kk < k; 0 elsewhere.
-// src(r, kk) = col_major ? src[kk * ld + r] : src[r * ld + kk].
-// out_lo != nullptr: also the TF32 rounding of the remainder (v - hi), so
-// that hi + lo carries about 21 significant bits (3xTF32 products).
-__global__ void pack_kmajor(const float* __restrict__ src, long long ld, int rows, int k, int col_major,
-                            float* __restrict__ out, float* __restrict__ out_lo, int rows_pad, int kpad) {
-  long long total = static_cast<long long>(rows_pad) * kpad;
-  for (long long t = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; t < total;
-       t += static_cast<long long>(gridDim.x) * blockDim.x) {
-    int r, kk;
-    if (col_major) {  // read coalesced along r
-      r = static_cast<int>(t % rows_pad);
-      kk = static_cast<int>(t / rows_pad);
-    } else {          // read coalesced along kk
-      kk = static_cast<int>(t % kpad);
-      r = static_cast<int>(t / kpad);
+// Packs both operands of an update into K-major, zero-padded buffers, rounded
+// to TF32 (the tensor cores would truncate):
+//   at[r * kpad + kk] = A[kk * lda + r]   r < m, kk < k; 0 up to mpad, kpad
+//   bt[r * kpad + kk] = B[r * ldb + kk]   r < n, kk < k; 0 up to npad, kpad
+// lo != 0: also the TF32 rounding of the remainder (v - hi) right after each
+// buffer's hi part, so that hi + lo carries about 21 significant bits (3xTF32
+// products).  One CTA a tile of 64 rows x 32 kk: A's tile is read down its
+// columns and transposed in shared memory, all loads of a thread in flight and
+// 16-byte stores.  A launch an operand with an element a thread in a grid-
+// stride loop took 2 x 7.7 us on average over the 12,331-row factorisation
+// (64-bit divisions, stores 4 * kpad bytes apart); this takes 4.7 us, its bytes
+// about 2 of them.
+constexpr int PK_THREADS = 256;
+constexpr int PK_ROWS = 64;
+static_assert(TC_M % PK_ROWS == 0 && TC_N % PK_ROWS == 0 && TC_KBLK == 32, "tiles divide the padded operands");
+__device__ __forceinline__ float tf32_round(float v) {
+  uint32_t r;
+  asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(r) : "f"(v));
+  return __uint_as_float(r);
+}
+__global__ void __launch_bounds__(PK_THREADS) pack_operands(const float* __restrict__ A, long long lda, int m, int mpad,
+                                                            float* __restrict__ at, const float* __restrict__ B,
+                                                            long long ldb, int n, int npad, float* __restrict__ bt,
+                                                            int k, int kpad, int lo, int b_vec) {
+  __shared__ float tile[PK_ROWS][TC_KBLK + 1];
+  const int nkb = kpad / TC_KBLK, ta = mpad / PK_ROWS * nkb;
+  const int tid = threadIdx.x;
+  const bool isA = static_cast<int>(blockIdx.x) < ta;
+  const int t = isA ? blockIdx.x : blockIdx.x - ta;
+  const int r0 = t / nkb * PK_ROWS, k0 = t % nkb * TC_KBLK;
+  float4 v[2];  // row r0 + (tid + 256 u) / 8, columns k0 + 4 (tid % 8) ...
+  if (isA) {
+    const int r = tid & (PK_ROWS - 1), kq = tid / PK_ROWS;
+    float x[8];
+#pragma unroll
+    for (int u = 0; u < 8; u++) {
+      const int kk = k0 + kq + 4 * u;
+      x[u] = (r0 + r < m && kk < k) ? A[static_cast<long long>(kk) * lda + r0 + r] : 0.0f;
     }
-    float v = 0.0f;
-    if (r < rows && kk < k) v = col_major ? src[static_cast<long long>(kk) * ld + r] : src[static_cast<long long>(r) * ld + kk];
-    // round to the nearest TF32 value (the tensor cores would truncate)
-    uint32_t rounded;
-    asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(rounded) : "f"(v));
-    const float hi = __uint_as_float(rounded);
-    out[static_cast<long long>(r) * kpad + kk] = hi;
-    if (out_lo) {
-      uint32_t rlo;
-      asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(rlo) : "f"(v - hi));
-      out_lo[static_cast<long long>(r) * kpad + kk] = __uint_as_float(rlo);
+#pragma unroll
+    for (int u = 0; u < 8; u++) tile[r][kq + 4 * u] = x[u];
+    __syncthreads();
+#pragma unroll
+    for (int u = 0; u < 2; u++) {
+      const float* q = &tile[(tid + PK_THREADS * u) >> 3][(tid & 7) * 4];
+      v[u] = make_float4(q[0], q[1], q[2], q[3]);
     }
+  } else {
+#pragma unroll
+    for (int u = 0; u < 2; u++) {
+      const int r = r0 + ((tid + PK_THREADS * u) >> 3), kk = k0 + (tid & 7) * 4;
+      const float* q = B + static_cast<long long>(r) * ldb + kk;
+      if (b_vec && r < n && kk + 4 <= k) {
+        v[u] = *reinterpret_cast<const float4*>(q);
+      } else {
+        v[u].x = (r < n && kk < k) ? q[0] : 0.0f;
+        v[u].y = (r < n && kk + 1 < k) ? q[1] : 0.0f;
+        v[u].z = (r < n && kk + 2 < k) ? q[2] : 0.0f;
+        v[u].w = (r < n && kk + 3 < k) ? q[3] : 0.0f;
+      }
+    }
+  }
+  float* out = isA ? at : bt;
+  const long long half = static_cast<long long>(isA ? mpad : npad) * kpad;
+#pragma unroll
+  for (int u = 0; u < 2; u++) {
+    const int r = r0 + ((tid + PK_THREADS * u) >> 3), kk = k0 + (tid & 7) * 4;
+    float* q = out + static_cast<long long>(r) * kpad + kk;
+    const float4 h = make_float4(tf32_round(v[u].x), tf32_round(v[u].y), tf32_round(v[u].z), tf32_round(v[u].w));
+    *reinterpret_cast<float4*>(q) = h;
+    if (lo)
+      *reinterpret_cast<float4*>(q + half) = make_float4(tf32_round(v[u].x - h.x), tf32_round(v[u].y - h.y),
+                                                         tf32_round(v[u].z - h.z), tf32_round(v[u].w - h.w));
   }
 }
 
@@ -617,9 +660,10 @@ void tf32_gemm_update(Context* ctx, int m, int n, int k, const float* A, long lo
   float* bt_lo = bt + need_b;
   // A is column-major m x k (contiguous along m); B is column-major k x n
   // (contiguous along k).
-  pack_kmajor<<<grid_for(need_a), 256, 0, s>>>(A, lda, m, k, 1, at, split3 ? at_lo : nullptr, mpad, kpad);
-  pack_kmajor<<<grid_for(need_b), 256, 0, s>>>(B, ldb, n, k, 0, bt, split3 ? bt_lo : nullptr, npad, kpad);
-  ctx->launches += 2;
+  const int b_vec = reinterpret_cast<uintptr_t>(B) % 16 == 0 && ldb % 4 == 0;
+  pack_operands<<<(mpad + npad) / PK_ROWS * (kpad / TC_KBLK), PK_THREADS, 0, s>>>(
+      A, lda, m, mpad, at, B, ldb, n, npad, bt, k, kpad, split3 ? 1 : 0, b_vec);
+  ctx->launches += 1;
   const int nkb = kpad / TC_KBLK;
   // TMA clips the stored rows at 16-byte granularity: rows up to m rounded
   // to 4 may be written (with their unchanged values or zeros), so the
