@@ -708,7 +708,7 @@ __global__ void scatter_perm(const double* __restrict__ z, const int* __restrict
 }
 
 // Inverse of the unit-lower (blockIdx.y 0) or upper part (1) of one TB x TB
-// diagonal block, row-major, zero padded to TB x TB; with FP32 factors also as
+// diagonal block, row-major, zero padded to TB x TB; with FP32 factors as
 // (hi, lo) float pairs.  Eight lanes a column, rows l + 8 q each; a finished
 // entry is broadcast by a shuffle and a warp starts at the first row of its four
 // columns.  Bound: the FP64 pipe.  (One thread a column took 140 us, a chain of
@@ -760,7 +760,7 @@ __global__ void __launch_bounds__(ID_THREADS) invert_diag_blocks(const T* __rest
   for (int e = threadIdx.x; e < TB * TB; e += ID_THREADS) {
     const int i = e / TB, k = e % TB;  // row, column of the block
     const double v = (i < n && k < n) ? (upper ? X[(n - 1 - k) * (TB + 1) + n - 1 - i] : X[k * (TB + 1) + i]) : 0.0;
-    out[e] = v;
+    if constexpr (std::is_same<T, double>::value) out[e] = v;
     if constexpr (std::is_same<T, float>::value) {
       const float h = static_cast<float>(v);
       out2[static_cast<size_t>(blk) * TB * TB + e] = make_float2(h, static_cast<float>(v - static_cast<double>(h)));
@@ -941,6 +941,8 @@ DenseLU::~DenseLU() {
   cudaFree(dinv_u_);
   cudaFree(dinv2_l_);
   cudaFree(dinv2_u_);
+  cudaFree(group_x_l_);
+  cudaFree(group_x_u_);
   cudaFree(perm_);
   cudaFree(tri_work_);
   cudaFree(bsave_);
@@ -1216,6 +1218,361 @@ __device__ __forceinline__ unsigned wait_progress(const unsigned* progress, unsi
   }
 }
 
+// ---- sweeps over FP32 factors ----
+// Groups of TG consecutive 64-row blocks (from row 0 on), whose triangle is
+// inverted as a whole after the factorisation: with G its inverse,
+// x_g = G (b_g - sum of the products with earlier groups).
+constexpr int TG = 2;
+constexpr int TG_ROWS = TG * TB;
+constexpr int TG_LD = TB + 1;  // row stride of the staged blocks: conflict-free reads down a column
+
+// Off-diagonal 64 x 64 block of the inverse of every group's triangle, as
+// (hi, lo) float pairs, row-major: X = -D1 T10 D0 of L (blockIdx.y 0), of U the
+// same with the order of the blocks reversed, from the diagonal blocks'
+// inverses D.  Two products of 64^3, four rows and columns a thread, in
+// double-float like the D.  Bound: FP32 instructions, about 12 a term.
+constexpr int GI_LD = TB + 4;  // 16-byte aligned rows
+constexpr int GI_PLANE = TB * GI_LD;
+constexpr size_t GI_SMEM = 7 * static_cast<size_t>(GI_PLANE) * sizeof(float);
+// acc (sum, lost) += L R, L of hi and (LOW) lo planes, R of both
+template <bool LOW>
+__device__ __forceinline__ void gi_product(float2 (&acc)[4][4], const float* __restrict__ L,
+                                           const float* __restrict__ R, int ty, int tx) {
+#pragma unroll 4
+  for (int k = 0; k < TB; k++) {
+    const float4 h4 = *reinterpret_cast<const float4*>(R + k * GI_LD + 4 * tx);
+    const float4 l4 = *reinterpret_cast<const float4*>(R + GI_PLANE + k * GI_LD + 4 * tx);
+    const float rh[4] = {h4.x, h4.y, h4.z, h4.w}, rl[4] = {l4.x, l4.y, l4.z, l4.w};
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+      const float lh = L[(4 * ty + i) * GI_LD + k];
+      const float ll = LOW ? L[GI_PLANE + (4 * ty + i) * GI_LD + k] : 0.0f;
+#pragma unroll
+      for (int j = 0; j < 4; j++) {
+        const float p = lh * rh[j];
+        float low = fmaf(lh, rl[j], fmaf(lh, rh[j], -p));
+        if (LOW) low = fmaf(ll, rh[j], low);
+        const float s = acc[i][j].x, n = s + p, z = n - s;
+        acc[i][j].y += ((s - (n - z)) + (p - z)) + low;
+        acc[i][j].x = n;
+      }
+    }
+  }
+}
+__global__ void __launch_bounds__(256) invert_groups(const float* __restrict__ A, long long ld, int N,
+                                                     const float2* __restrict__ Linv2,
+                                                     const float2* __restrict__ Uinv2, float2* __restrict__ Lx,
+                                                     float2* __restrict__ Ux) {
+  extern __shared__ __align__(16) float gi[];  // planes of 64 x GI_LD
+  float* D[TG] = {gi, gi + 2 * GI_PLANE};       // hi, lo; in the order of elimination
+  float* S = gi + 4 * GI_PLANE;                 // T D0: hi, lo
+  float* T = gi + 6 * GI_PLANE;
+  const int g = blockIdx.x, upper = blockIdx.y, tid = threadIdx.x;
+  const int nblk = (N + TB - 1) / TB;
+  const int ty = tid >> 4, tx = tid & 15;
+  const float2* Dinv2 = upper ? Uinv2 : Linv2;
+  float2* out = (upper ? Ux : Lx) + static_cast<size_t>(g) * TB * TB;
+  auto natural = [&](int o) { return TG * g + (upper ? TG - 1 - o : o); };  // block of elimination step o
+#pragma unroll
+  for (int o = 0; o < TG; o++) {
+    const int b = natural(o);
+#pragma unroll 8
+    for (int e = tid; e < TB * TB; e += 256) {
+      const float2 d = b < nblk ? Dinv2[static_cast<size_t>(b) * TB * TB + e] : make_float2(0.f, 0.f);
+      float* at = D[o] + (e / TB) * GI_LD + e % TB;
+      at[0] = d.x;
+      at[GI_PLANE] = d.y;
+    }
+  }
+  const int r0 = natural(1) * TB, k0 = natural(0) * TB;
+#pragma unroll 8
+  for (int e = tid; e < TB * TB; e += 256) {
+    const int i = e % TB, k = e / TB;
+    T[i * GI_LD + k] = (r0 + i < N && k0 + k < N) ? A[static_cast<long long>(k0 + k) * ld + r0 + i] : 0.0f;
+  }
+  __syncthreads();
+  float2 s[4][4] = {};
+  gi_product<false>(s, T, D[0], ty, tx);
+#pragma unroll
+  for (int i = 0; i < 4; i++)
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+      const float n = s[i][j].x + s[i][j].y;
+      float* at = S + (4 * ty + i) * GI_LD + 4 * tx + j;
+      at[0] = n;
+      at[GI_PLANE] = s[i][j].y - (n - s[i][j].x);
+    }
+  __syncthreads();
+  float2 v[4][4] = {};
+  gi_product<true>(v, D[1], S, ty, tx);
+#pragma unroll
+  for (int i = 0; i < 4; i++)
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+      const float n = v[i][j].x + v[i][j].y;
+      out[(4 * ty + i) * TB + 4 * tx + j] = make_float2(-n, -(v[i][j].y - (n - v[i][j].x)));
+    }
+}
+
+// A whole sweep in one cooperative launch; CTA c owns the groups c, c + grid,
+// ... in sweep order.  Bound: the chain from group to group, whose links are the
+// way of the last x through L2, its products and G's product; the tiles over
+// earlier groups are loaded a group ahead.  The FP32 copy of x is its own
+// signal: yf enters as all ones (a NaN that no x is stored as) and a thread
+// waits for its entries to change, which saves the release, the acquire and one
+// more way to L2; only the CTA whose turn is next polls without a pause.  Sums
+// are double-float (G and the right-hand side as float pairs, about 48 bits) of
+// FP32 products with x in sums of 8 terms: FP64 adds and conversions would run
+// at the FP64 rate.  TRANS: the transposed factor.  Inside the group the rows
+// run in sweep order (reversed when descending): G is lower triangular in all
+// four sweeps.  Every CTA is resident and a group waits for earlier ones only.
+// N = 12,331: 0.177 ms a sweep (97 groups, about 3,700 cycles a link: 2,000 in
+// the order of the arithmetic, 1,250 of them G's product, and the way through
+// L2); 192-row groups chained block by block with a released counter 0.351 ms.
+// Tried: G's product formed ahead for all but the last x, whose share then went
+// through G in FP32: faster still, but matrices with ill-conditioned diagonal
+// blocks took more refinement.  4-byte loads of the tiles: 6,000 cycles a link.
+constexpr int TG_PART = 161;
+// place of a row's partial sums: without bank conflicts for 16 lanes of rows
+// 4 s + a each, for 16 lanes of one row, and for 8 consecutive rows read in pairs
+__device__ __forceinline__ int tg_place(int row) { return (row >> 6) * 80 + (row & 3) * 20 + ((row & 63) >> 2); }
+constexpr unsigned TG_EMPTY = 0xffffffffu;
+__device__ __forceinline__ uint4 ld_relaxed_v4(const float* p) {
+  uint4 v;
+  asm volatile("ld.relaxed.gpu.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
+  return v;
+}
+struct TgShared {
+  float2 D[TG][TB * TG_LD];   // diagonal blocks of G, (hi, lo)
+  float2 X[TB * TG_LD];       // block (1, 0)
+  float2 part[16][TG_PART];   // sums of 16 threads a row, then of 8 warps
+  float2 b[TG_ROWS];          // right-hand side, natural row order
+  float2 v[TG_ROWS];          // in sweep order
+  int abort;
+};
+template <bool TRANS>
+__global__ void __launch_bounds__(256, 1) trsv_group(const float* __restrict__ A, long long ld, int N,
+                                                     const double* __restrict__ b, double* __restrict__ y,
+                                                     float* yf, const float2* __restrict__ Dinv2,
+                                                     const float2* __restrict__ Xinv, int ascending, int* err,
+                                                     unsigned long long wait_ns, unsigned stall) {
+  static_assert(TG == 2 && TG_ROWS == 128, "two threads a row");
+  extern __shared__ __align__(16) unsigned char tg_raw[];
+  TgShared& sh = *reinterpret_cast<TgShared*>(tg_raw);
+  const int nblk = (N + TB - 1) / TB, ng = (nblk + TG - 1) / TG;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  // This thread's 16 entries of a 64 x 64 tile: four columns from 4 slot on and
+  // four rows; four 16-byte loads, 256 contiguous bytes a half-warp.
+  const int slot = TRANS ? lane & 15 : 2 * warp + (lane >> 4), c0 = 4 * slot;
+  auto tile_row = [&](int a) { return TRANS ? 8 * warp + 2 * a + (lane >> 4) : 4 * (lane & 15) + a; };
+  const int i0 = lane, i1 = TB - 1 - lane;  // G: two rows of each block, columns warp + 8 i
+  const int rown = tid >> 1, half = tid & 1;
+  auto group = [&](int pos) { return ascending ? pos : ng - 1 - pos; };
+  auto order = [&](int i) { return ascending ? i : TG_ROWS - 1 - i; };  // natural row of a group <-> sweep order
+  auto df = [](float2 f) { return DF{f.x, f.y}; };
+  auto both = [](DF a) {  // the sum of a pair of threads
+    return df_add(a, {__shfl_xor_sync(0xffffffffu, a.h, 1), __shfl_xor_sync(0xffffffffu, a.l, 1)});
+  };
+  if (tid == 0) sh.abort = 0;
+  __syncthreads();
+  for (int pos = blockIdx.x; pos < ng; pos += gridDim.x) {
+    const int R0 = group(pos) * TG_ROWS;
+    bool inside = true;  // no row of this thread past the matrix
+#pragma unroll
+    for (int a = 0; a < 4; a++) inside = inside && R0 + TB + tile_row(a) < N;
+    float t[TG][TG][16];  // [block of columns][block of rows][4 row + column]
+    auto load_tile = [&](int p) {
+      const int p0 = group(p) * TG_ROWS;
+#pragma unroll
+      for (int cb = 0; cb < TG; cb++) {
+        const int k0 = p0 + cb * TB + c0;
+        // the working copy's columns are 128-byte aligned, k0 and the first row multiples of 4
+        if (inside && k0 + 4 <= N) {
+          const float* src = TRANS ? A + static_cast<long long>(R0 + tile_row(0)) * ld + k0
+                                   : A + static_cast<long long>(k0) * ld + R0 + tile_row(0);
+          const long long next = TRANS ? 2 * ld : ld;  // to the thread's next row, or its next column
+#pragma unroll
+          for (int rb = 0; rb < TG; rb++) {
+            const float* q = src + (TRANS ? static_cast<long long>(rb) * TB * ld : rb * TB);
+#pragma unroll
+            for (int u = 0; u < 4; u++) {
+              const float4 v = __ldg(reinterpret_cast<const float4*>(q));
+              constexpr int s1 = TRANS ? 1 : 4, su = TRANS ? 4 : 1;
+              t[cb][rb][su * u] = v.x;
+              t[cb][rb][su * u + s1] = v.y;
+              t[cb][rb][su * u + 2 * s1] = v.z;
+              t[cb][rb][su * u + 3 * s1] = v.w;
+              q += next;
+            }
+          }
+        } else {
+#pragma unroll
+          for (int rb = 0; rb < TG; rb++)
+#pragma unroll
+            for (int a = 0; a < 4; a++)
+#pragma unroll
+              for (int j = 0; j < 4; j++) {
+                const int row = R0 + rb * TB + tile_row(a), k = k0 + j;
+                t[cb][rb][4 * a + j] =
+                    (row < N && k < N) ? A[TRANS ? static_cast<long long>(row) * ld + k : static_cast<long long>(k) * ld + row]
+                                       : 0.f;
+              }
+        }
+      }
+    };
+    if (pos > 0) load_tile(0);
+    for (int nb = 0; nb < TG; nb++) {  // natural block nb of the group
+      const int blk = group(pos) * TG + nb, ob = ascending ? nb : TG - 1 - nb;
+#pragma unroll 8
+      for (int e = tid; e < TB * TB; e += 256) {
+        const float2 d = blk < nblk ? Dinv2[static_cast<size_t>(blk) * TB * TB + e] : make_float2(0.f, 0.f);
+        int r = TRANS ? e % TB : e / TB, c = TRANS ? e / TB : e % TB;
+        if (!ascending) r = TB - 1 - r, c = TB - 1 - c;
+        sh.D[ob][r * TG_LD + c] = d;
+      }
+    }
+#pragma unroll 8
+    for (int e = tid; e < TB * TB; e += 256) {
+      int r = TRANS ? e % TB : e / TB, c = TRANS ? e / TB : e % TB;
+      if (!ascending) r = TB - 1 - r, c = TB - 1 - c;
+      sh.X[r * TG_LD + c] = Xinv[static_cast<size_t>(group(pos)) * TB * TB + e];
+    }
+    if (tid < TG_ROWS) {
+      const double bv = R0 + tid < N ? b[R0 + tid] : 0.0;
+      const float h = static_cast<float>(bv);
+      sh.b[tid] = make_float2(h, static_cast<float>(bv - static_cast<double>(h)));
+    }
+    DF acc[TG][4];
+#pragma unroll
+    for (int r = 0; r < TG; r++)
+#pragma unroll
+      for (int a = 0; a < 4; a++) acc[r][a] = {0.f, 0.f};
+    __syncthreads();
+    float2 g0[2][4], g1[2][8], gx[2][8];  // this thread's entries of G
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
+      const int c = warp + 8 * i;
+#pragma unroll
+      for (int ob = 0; ob < TG; ob++) {
+        if (i < 4) g0[ob][i] = sh.D[ob][i0 * TG_LD + c];  // row i0 < 32 ends before column 32
+        g1[ob][i] = sh.D[ob][i1 * TG_LD + c];
+      }
+      gx[0][i] = sh.X[i0 * TG_LD + c];
+      gx[1][i] = sh.X[i1 * TG_LD + c];
+    }
+    // products with the x of position p, then the tile over the next one
+    auto step = [&](int p) {
+      float x[TG][4];
+      unsigned long long t_first = 0;
+      for (unsigned it = 0;; it++) {
+        bool here = stall == 0;
+#pragma unroll
+        for (int cb = 0; cb < TG; cb++) {
+          const int k0 = group(p) * TG_ROWS + cb * TB + c0;
+          // yf is 128-byte aligned and as long as N rounded up to 32, k0 a multiple of 4
+          uint4 v = make_uint4(0u, 0u, 0u, 0u);
+          if (k0 < N) v = ld_relaxed_v4(yf + k0);
+          if (k0 + 1 >= N) v.y = 0u;
+          if (k0 + 2 >= N) v.z = 0u;
+          if (k0 + 3 >= N) v.w = 0u;
+          here = here && v.x != TG_EMPTY && v.y != TG_EMPTY && v.z != TG_EMPTY && v.w != TG_EMPTY;
+          x[cb][0] = __uint_as_float(v.x);
+          x[cb][1] = __uint_as_float(v.y);
+          x[cb][2] = __uint_as_float(v.z);
+          x[cb][3] = __uint_as_float(v.w);
+        }
+        if (__all_sync(0xffffffffu, here)) break;
+        if (p + 1 < pos) __nanosleep(400);
+        if ((it & 15) == 15) {
+          const unsigned long long now = globaltimer_ns();
+          if (t_first == 0) t_first = now;
+          if (__any_sync(0xffffffffu, now - t_first > wait_ns)) return false;
+        }
+      }
+#pragma unroll
+      for (int r = 0; r < TG; r++)
+#pragma unroll
+        for (int a = 0; a < 4; a++) {
+          float sum = 0.f;
+#pragma unroll
+          for (int cb = 0; cb < TG; cb++)
+#pragma unroll
+            for (int j = 0; j < 4; j++) sum = fmaf(t[cb][r][4 * a + j], x[cb][j], sum);
+          acc[r][a] = df_add(acc[r][a], {sum, 0.f});
+        }
+      if (p + 1 < pos) load_tile(p + 1);
+      return true;
+    };
+    bool ok = true;
+    for (int p = 0; p < pos && ok; p++) ok = step(p);
+    if (!ok) sh.abort = 1;
+#pragma unroll
+    for (int r = 0; r < TG; r++)
+#pragma unroll
+      for (int a = 0; a < 4; a++) sh.part[slot][tg_place(r * TB + tile_row(a))] = make_float2(acc[r][a].h, acc[r][a].l);
+    __syncthreads();
+    if (sh.abort) {
+      if (tid == 0) atomicExch(err, 1);
+      return;
+    }
+    {  // v = b - sums: two threads a row
+      DF h[8];
+#pragma unroll
+      for (int k = 0; k < 8; k++) h[k] = df(sh.part[8 * half + k][tg_place(rown)]);
+#pragma unroll
+      for (int w = 4; w > 0; w >>= 1)
+#pragma unroll
+        for (int k = 0; k < w; k++) h[k] = df_add(h[k], h[k + w]);
+      const DF sum = both(h[0]);
+      const DF v = df_add(df(sh.b[rown]), {-sum.h, -sum.l});
+      if (half == 0) sh.v[order(rown)] = make_float2(v.h, v.l);
+    }
+    __syncthreads();
+    // x = G v: rows i0 and i1 of each block over the columns warp + 8 i
+#pragma unroll
+    for (int ob = 0; ob < TG; ob++) {
+      float s[2] = {0.f, 0.f}, e[2] = {0.f, 0.f};  // sums, and what their roundings lost
+      auto term = [&](int k, float2 d, float2 v) {
+        const float p = d.x * v.x;
+        const float low = fmaf(d.y, v.x, fmaf(d.x, v.y, fmaf(d.x, v.x, -p)));
+        const float n = s[k] + p, z = n - s[k];
+        e[k] += ((s[k] - (n - z)) + (p - z)) + low;
+        s[k] = n;
+      };
+#pragma unroll
+      for (int i = 0; i < 8; i++) {
+        const int c = warp + 8 * i;
+        const float2 v = sh.v[ob * TB + c];
+        if (i < 4) term(0, g0[ob][i], v);
+        term(1, g1[ob][i], v);
+      }
+      if (ob == 1) {
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
+          const int c = warp + 8 * i;
+          const float2 v = sh.v[c];
+          term(0, gx[0][i], v);
+          term(1, gx[1][i], v);
+        }
+      }
+      sh.part[warp][ob * TB + i0] = make_float2(s[0], e[0]);
+      sh.part[warp][ob * TB + i1] = make_float2(s[1], e[1]);
+    }
+    __syncthreads();
+    const DF x = both(df_add(df_add(df(sh.part[4 * half][rown]), df(sh.part[4 * half + 1][rown])),
+                             df_add(df(sh.part[4 * half + 2][rown]), df(sh.part[4 * half + 3][rown]))));
+    const int row = R0 + order(rown);
+    if (half == 0 && row < N) {
+      const unsigned bits = __float_as_uint(x.h);
+      asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(yf + row), "r"(bits == TG_EMPTY ? 0x7fffffffu : bits)
+                   : "memory");
+      y[row] = static_cast<double>(x.h) + static_cast<double>(x.l);
+    }
+    __syncthreads();  // the staged blocks and part are read no more
+  }
+}
+
+// ---- sweeps over FP64 factors ----
 // A whole sweep in one cooperative launch, CH_R consecutive blocks per group
 // and one group at a time per CTA: CTA c owns the groups c, c + grid, ..., group g the sweep
 // positions g R .. g R + R - 1.  While earlier groups are worked on it
@@ -1230,52 +1587,30 @@ __device__ __forceinline__ unsigned wait_progress(const unsigned* progress, unsi
 // critical path.  A group waits for lower groups only, and every CTA is
 // resident, so the lowest unfinished group can always go on.
 //
-// Bound: the chain of dependent blocks (about 1.8 us each), not the factor's
-// bytes.  Matrices of more than R * 64 rows per SM (29,184 on 152 SMs) give
-// a CTA several groups: while the other CTAs' groups chain (456 blocks,
-// about 0.8 ms) it reads its next group's factor rows (22 MB in all SMs per
-// block column), so the chain stays the bound there too.
+// Bound: the chain of dependent blocks, not the factor's bytes.
 // TRANS sweeps solve with the transposed factor: the tile of output block p
 // and finished block pi is the stored block (pi, p), whose columns are the
-// output rows, so a thread reads 16 consecutive entries of one column
-// (64 contiguous bytes with FP32 factors).
+// output rows, so a thread reads 16 consecutive entries of one column.
 constexpr int CH_R = 3;
-constexpr int CH_DST = TB + 1;  // row stride of the staged Dinv blocks (8-byte entries: conflict-free row reads)
+constexpr int CH_DST = TB + 1;  // row stride of the staged Dinv blocks (conflict-free row reads)
 constexpr int CH_LST = TB + 1;  // column stride of the staged internal blocks (transposed staging without conflicts)
 // dynamic shared memory: the internal L blocks, then Dinv of the own blocks
-// (8 bytes an entry: a (hi, lo) float pair or a double)
-template <class T>
-constexpr size_t chain_smem() {
-  return static_cast<size_t>(CH_R * (CH_R - 1) / 2) * TB * CH_LST * sizeof(T) +
-         static_cast<size_t>(CH_R) * TB * CH_DST * 8;
-}
+constexpr size_t CH_SMEM = (static_cast<size_t>(CH_R * (CH_R - 1) / 2) * TB * CH_LST +
+                            static_cast<size_t>(CH_R) * TB * CH_DST) * sizeof(double);
 
-// With FP32 factors every value a thread multiplies is a float: the
-// producer stores x twice (y in FP64, yf in FP32), phase A and the internal
-// products read the FP32 copy, and the sums go in double-float.  (On this
-// GPU FP64 adds and FP64 <-> FP32 conversions run at the FP64 rate, a few
-// per clock per SM: one conversion per product would cost more than the
-// products.)
-template <class T, bool TRANS>
-__global__ void __launch_bounds__(256) trsv_chain(const T* __restrict__ A, long long ld, int N,
+template <bool TRANS>
+__global__ void __launch_bounds__(256) trsv_chain(const double* __restrict__ A, long long ld, int N,
                                                   const double* __restrict__ b, double* __restrict__ y,
-                                                  float* __restrict__ yf, const double* __restrict__ Dinv,
-                                                  const float2* __restrict__ Dinv2, int lower, unsigned* progress,
+                                                  const double* __restrict__ Dinv, int lower, unsigned* progress,
                                                   int* err, unsigned long long wait_ns, unsigned stall) {
-  constexpr bool kF = std::is_same<T, float>::value;
   extern __shared__ __align__(16) unsigned char ch_raw[];
-  T* Lin = reinterpret_cast<T*>(ch_raw);  // internal blocks (r2, r1), r1 < r2: column-major, stride CH_LST
+  double* Lin = reinterpret_cast<double*>(ch_raw);  // internal blocks (r2, r1), r1 < r2: column-major, stride CH_LST
   // Dinv of the own blocks, row-major 64 x 64 each with row stride CH_DST
-  unsigned char* dsm = ch_raw + static_cast<size_t>(CH_R * (CH_R - 1) / 2) * TB * CH_LST * sizeof(T);
-  float2* D2s = reinterpret_cast<float2*>(dsm);
-  double* Dds = reinterpret_cast<double*>(dsm);
+  double* Dds = Lin + static_cast<size_t>(CH_R * (CH_R - 1) / 2) * TB * CH_LST;
   __shared__ double bsm[CH_R][TB];
   __shared__ double part[4][TB];
-  __shared__ float parth[4][TB], partl[4][TB];
-  __shared__ float vh[TB], vl[TB];
   __shared__ double vd[TB];
   __shared__ double xs[TB];
-  __shared__ float xsf[TB];
   __shared__ int s_abort;
   const int nblk = (N + TB - 1) / TB;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -1289,7 +1624,6 @@ __global__ void __launch_bounds__(256) trsv_chain(const T* __restrict__ A, long 
   // 16-byte vector loads of x only from an aligned y (callers pass offset
   // vectors, e.g. a work vector at an odd offset N)
   const bool y_aligned = (reinterpret_cast<unsigned long long>(y) & 15ull) == 0;
-  const bool yf_aligned = kF && (reinterpret_cast<unsigned long long>(yf) & 15ull) == 0;
   for (int p0 = blockIdx.x * CH_R; p0 < nblk; p0 += gridDim.x * CH_R) {
   const int np = (nblk - p0 < CH_R) ? nblk - p0 : CH_R;
   // Stage what the own blocks need besides the x of earlier blocks: the
@@ -1299,14 +1633,14 @@ __global__ void __launch_bounds__(256) trsv_chain(const T* __restrict__ A, long 
   for (int r2 = 1; r2 < np; r2++)
     for (int r1 = 0; r1 < r2; r1++) {
       const int kr = blk(p0 + r2), kc = blk(p0 + r1);
-      T* dst = Lin + static_cast<size_t>(tri(r2, r1)) * TB * CH_LST;
+      double* dst = Lin + static_cast<size_t>(tri(r2, r1)) * TB * CH_LST;
       for (int e0 = 0; e0 < TB * TB; e0 += 16 * 256) {
-        T v[16];
+        double v[16];
 #pragma unroll
         for (int u = 0; u < 16; u++) {
           const int e = e0 + u * 256 + tid;
           const int row = (TRANS ? kc : kr) * TB + e % TB, col = (TRANS ? kr : kc) * TB + e / TB;
-          v[u] = (row < N && col < N) ? A[static_cast<long long>(col) * ld + row] : T(0);
+          v[u] = (row < N && col < N) ? A[static_cast<long long>(col) * ld + row] : 0.0;
         }
 #pragma unroll
         for (int u = 0; u < 16; u++) {  // entry (i, j) of the block at dst[j * CH_LST + i]
@@ -1320,26 +1654,14 @@ __global__ void __launch_bounds__(256) trsv_chain(const T* __restrict__ A, long 
     for (int e0 = 0; e0 < TB * TB; e0 += 16 * 256) {
       // entry e = row * TB + col of the block goes to row * CH_DST + col
       // (TRANS: the transposed inverse, to col * CH_DST + row)
-      if constexpr (std::is_same<T, float>::value) {
-        float2 v[16];
+      double v[16];
 #pragma unroll
-        for (int u = 0; u < 16; u++) v[u] = Dinv2[src + e0 + u * 256 + tid];
+      for (int u = 0; u < 16; u++) v[u] = Dinv[src + e0 + u * 256 + tid];
 #pragma unroll
-        for (int u = 0; u < 16; u++) {
-          const int e = e0 + u * 256 + tid;
-          D2s[static_cast<size_t>(r) * TB * CH_DST + (TRANS ? (e % TB) * CH_DST + e / TB : (e / TB) * CH_DST + e % TB)] =
-              v[u];
-        }
-      } else {
-        double v[16];
-#pragma unroll
-        for (int u = 0; u < 16; u++) v[u] = Dinv[src + e0 + u * 256 + tid];
-#pragma unroll
-        for (int u = 0; u < 16; u++) {
-          const int e = e0 + u * 256 + tid;
-          Dds[static_cast<size_t>(r) * TB * CH_DST + (TRANS ? (e % TB) * CH_DST + e / TB : (e / TB) * CH_DST + e % TB)] =
-              v[u];
-        }
+      for (int u = 0; u < 16; u++) {
+        const int e = e0 + u * 256 + tid;
+        Dds[static_cast<size_t>(r) * TB * CH_DST + (TRANS ? (e % TB) * CH_DST + e / TB : (e / TB) * CH_DST + e % TB)] =
+            v[u];
       }
     }
     if (tid < TB) {
@@ -1348,20 +1670,12 @@ __global__ void __launch_bounds__(256) trsv_chain(const T* __restrict__ A, long 
     }
   }
   __syncthreads();
-  double acc[CH_R];  // FP64 factors
-  DF accf[CH_R];     // FP32 factors
+  double acc[CH_R];
 #pragma unroll
-  for (int r = 0; r < CH_R; r++) {
-    acc[r] = 0.0;
-    accf[r] = {0.f, 0.f};
-  }
-  // phase A: the finished blocks of earlier CTAs.  With FP32 factors the L
-  // tile of the next block is loaded while the current one is used (it
-  // does not depend on x), so the factor's HBM latency overlaps the
-  // progress waits and the x loads.
+  for (int r = 0; r < CH_R; r++) acc[r] = 0.0;
+  // phase A: the finished blocks of earlier CTAs
   bool ok = true;
-  constexpr bool kAhead = sizeof(T) == 4;  // FP64 tiles would not fit twice in registers
-  T a[CH_R][16], an[kAhead ? CH_R : 1][16];
+  double a[CH_R][16];
   // rows of this thread in its CTA's blocks (N when past the matrix)
   int rowof[CH_R];
 #pragma unroll
@@ -1369,47 +1683,32 @@ __global__ void __launch_bounds__(256) trsv_chain(const T* __restrict__ A, long 
     const int row = blk(p0 + r) * TB + rr;
     rowof[r] = (r < np && row < N) ? row : N;
   }
-  auto load_tile = [&](int pi, T(&dst)[CH_R][16]) {
+  auto load_tile = [&](int pi) {
     const int cb = blk(pi) * TB + c0;
     if constexpr (TRANS) {
-      // entries cb .. cb + 15 of column rowof[r]; the FP32 copy's columns
-      // are 128-byte aligned and cb is a multiple of 16
-      const bool vec = kF && cb + 16 <= N && (ld & 3) == 0 && (reinterpret_cast<unsigned long long>(A) & 15ull) == 0;
+      // entries cb .. cb + 15 of column rowof[r]
 #pragma unroll
       for (int r = 0; r < CH_R; r++) {
-        const T* q = A + static_cast<long long>(rowof[r] < N ? rowof[r] : 0) * ld + cb;
-        if (rowof[r] < N && vec) {
-          if constexpr (kF) {
+        const double* src = A + static_cast<long long>(rowof[r] < N ? rowof[r] : 0) * ld + cb;
 #pragma unroll
-            for (int j = 0; j < 4; j++) {
-              const float4 v = __ldg(reinterpret_cast<const float4*>(q) + j);
-              dst[r][4 * j] = v.x;
-              dst[r][4 * j + 1] = v.y;
-              dst[r][4 * j + 2] = v.z;
-              dst[r][4 * j + 3] = v.w;
-            }
-          }
-        } else {
-#pragma unroll
-          for (int j = 0; j < 16; j++) dst[r][j] = (rowof[r] < N && cb + j < N) ? q[j] : T(0);
-        }
+        for (int j = 0; j < 16; j++) a[r][j] = (rowof[r] < N && cb + j < N) ? src[j] : 0.0;
       }
       return;
     }
-    const T* colp = A + static_cast<long long>(cb) * ld;
+    const double* colp = A + static_cast<long long>(cb) * ld;
     if (cb + 16 <= N) {  // whole column quarter inside the matrix: no column predicates
 #pragma unroll
       for (int r = 0; r < CH_R; r++) {
         if (rowof[r] < N) {
-          const T* q = colp + rowof[r];
+          const double* src = colp + rowof[r];
 #pragma unroll
           for (int j = 0; j < 16; j++) {
-            dst[r][j] = *q;
-            q += ld;
+            a[r][j] = *src;
+            src += ld;
           }
         } else {
 #pragma unroll
-          for (int j = 0; j < 16; j++) dst[r][j] = T(0);
+          for (int j = 0; j < 16; j++) a[r][j] = 0.0;
         }
       }
     } else {
@@ -1417,23 +1716,12 @@ __global__ void __launch_bounds__(256) trsv_chain(const T* __restrict__ A, long 
       for (int r = 0; r < CH_R; r++)
 #pragma unroll
         for (int j = 0; j < 16; j++)
-          dst[r][j] = (rowof[r] < N && cb + j < N) ? colp[static_cast<long long>(j) * ld + rowof[r]] : T(0);
+          a[r][j] = (rowof[r] < N && cb + j < N) ? colp[static_cast<long long>(j) * ld + rowof[r]] : 0.0;
     }
   };
-  if constexpr (kAhead) {
-    if (p0 > 0) load_tile(0, an);
-  }
   for (int pi = 0; pi < p0; pi++) {
     const int cb = blk(pi) * TB + c0;
-    if constexpr (kAhead) {
-#pragma unroll
-      for (int r = 0; r < CH_R; r++)
-#pragma unroll
-        for (int j = 0; j < 16; j++) a[r][j] = an[r][j];
-      if (pi + 1 < p0) load_tile(pi + 1, an);
-    } else {
-      load_tile(pi, a);
-    }
+    load_tile(pi);
     if (static_cast<unsigned>(pi) >= avail) {
       const unsigned v = wait_progress(progress, static_cast<unsigned>(pi) + 1 + stall, wait_ns);
       if (v == 0) {
@@ -1442,44 +1730,25 @@ __global__ void __launch_bounds__(256) trsv_chain(const T* __restrict__ A, long 
       }
       avail = v - stall;  // positions known finished
     }
-    T xq[16];
-    if constexpr (kF) {
-      if (yf_aligned && cb + 16 <= N) {  // yf + cb is then 16-byte aligned (cb is a multiple of 16)
-        const float4* y4 = reinterpret_cast<const float4*>(yf + cb);
-#pragma unroll
-        for (int j = 0; j < 4; j++) {
-          const float4 v = __ldcg(y4 + j);
-          xq[4 * j] = v.x;
-          xq[4 * j + 1] = v.y;
-          xq[4 * j + 2] = v.z;
-          xq[4 * j + 3] = v.w;
-        }
-      } else {
-#pragma unroll
-        for (int j = 0; j < 16; j++) xq[j] = (cb + j < N) ? __ldcg(yf + cb + j) : 0.f;
-      }
-    } else if (y_aligned && cb + 16 <= N) {  // y + cb is then 16-byte aligned (cb is a multiple of 16)
+    double xq[16];
+    if (y_aligned && cb + 16 <= N) {  // y + cb is then 16-byte aligned (cb is a multiple of 16)
       const double2* y2 = reinterpret_cast<const double2*>(y + cb);
 #pragma unroll
       for (int j = 0; j < 8; j++) {
         const double2 v = __ldcg(y2 + j);
-        xq[2 * j] = static_cast<T>(v.x);
-        xq[2 * j + 1] = static_cast<T>(v.y);
+        xq[2 * j] = v.x;
+        xq[2 * j + 1] = v.y;
       }
     } else {
 #pragma unroll
-      for (int j = 0; j < 16; j++) xq[j] = static_cast<T>((cb + j < N) ? __ldcg(y + cb + j) : 0.0);
+      for (int j = 0; j < 16; j++) xq[j] = (cb + j < N) ? __ldcg(y + cb + j) : 0.0;
     }
 #pragma unroll
     for (int r = 0; r < CH_R; r++) {
-      T sum = T(0);
+      double sum = 0.0;
 #pragma unroll
       for (int j = 0; j < 16; j++) sum = fma(a[r][j], xq[j], sum);
-      if constexpr (kF) {
-        accf[r] = df_add(accf[r], {static_cast<float>(sum), 0.f});
-      } else {
-        acc[r] += static_cast<double>(sum);
-      }
+      acc[r] += sum;
     }
   }
   if (!ok) s_abort = 1;
@@ -1490,77 +1759,34 @@ __global__ void __launch_bounds__(256) trsv_chain(const T* __restrict__ A, long 
     const int k = blk(p0 + r);
     const int r0 = k * TB;
     const int n = (N - r0 < TB) ? N - r0 : TB;
-    if constexpr (kF) {
-      parth[q][rr] = accf[r].h;
-      partl[q][rr] = accf[r].l;
-    } else {
-      part[q][rr] = acc[r];
-    }
+    part[q][rr] = acc[r];
     __syncthreads();
     if (s_abort) {
       if (tid == 0) atomicExch(err, 1);
       return;
     }
     if (tid < TB) {
-      double sacc;
-      if constexpr (kF) {
-        const DF a = df_add({parth[0][tid], partl[0][tid]}, {parth[1][tid], partl[1][tid]});
-        const DF c = df_add({parth[2][tid], partl[2][tid]}, {parth[3][tid], partl[3][tid]});
-        const DF t = df_add(a, c);
-        sacc = static_cast<double>(t.h) + static_cast<double>(t.l);
-      } else {
-        sacc = (part[0][tid] + part[1][tid]) + (part[2][tid] + part[3][tid]);
-      }
-      const double v = (tid < n) ? bsm[r][tid] - sacc : 0.0;
-      vd[tid] = v;
-      const float hv = static_cast<float>(v);
-      vh[tid] = hv;
-      vl[tid] = static_cast<float>(v - static_cast<double>(hv));
+      const double sacc = (part[0][tid] + part[1][tid]) + (part[2][tid] + part[3][tid]);
+      vd[tid] = (tid < n) ? bsm[r][tid] - sacc : 0.0;
     }
     __syncthreads();
     // x = Dinv v: thread (h, q, lane) forms row rr over columns c0 .. c0 + 15
     // (two accumulators), the four column quarters are added in shared
     // memory in a fixed order
     const size_t drow = static_cast<size_t>(r) * TB * CH_DST + static_cast<size_t>(rr) * CH_DST + c0;
-    if constexpr (std::is_same<T, float>::value) {
-      DF s0 = {0.f, 0.f}, s1 = {0.f, 0.f};
+    double s0 = 0.0, s1 = 0.0;
 #pragma unroll
-      for (int j = 0; j < 16; j += 2) {
-        const float2 d0 = D2s[drow + j], d1 = D2s[drow + j + 1];
-        s0 = df_add(s0, df_mul(d0.x, d0.y, vh[c0 + j], vl[c0 + j]));
-        s1 = df_add(s1, df_mul(d1.x, d1.y, vh[c0 + j + 1], vl[c0 + j + 1]));
-      }
-      const DF sq = df_add(s0, s1);
-      parth[q][rr] = sq.h;
-      partl[q][rr] = sq.l;
-    } else {
-      double s0 = 0.0, s1 = 0.0;
-#pragma unroll
-      for (int j = 0; j < 16; j += 2) {
-        s0 = fma(Dds[drow + j], vd[c0 + j], s0);
-        s1 = fma(Dds[drow + j + 1], vd[c0 + j + 1], s1);
-      }
-      part[q][rr] = s0 + s1;
+    for (int j = 0; j < 16; j += 2) {
+      s0 = fma(Dds[drow + j], vd[c0 + j], s0);
+      s1 = fma(Dds[drow + j + 1], vd[c0 + j + 1], s1);
     }
+    part[q][rr] = s0 + s1;
     __syncthreads();
     if (tid < TB) {
-      double x;
-      if constexpr (std::is_same<T, float>::value) {
-        const DF a = df_add({parth[0][tid], partl[0][tid]}, {parth[1][tid], partl[1][tid]});
-        const DF c = df_add({parth[2][tid], partl[2][tid]}, {parth[3][tid], partl[3][tid]});
-        const DF t = df_add(a, c);
-        x = static_cast<double>(t.h) + static_cast<double>(t.l);
-      } else {
-        x = (part[0][tid] + part[1][tid]) + (part[2][tid] + part[3][tid]);
-      }
+      double x = (part[0][tid] + part[1][tid]) + (part[2][tid] + part[3][tid]);
       if (tid >= n) x = 0.0;
       xs[tid] = x;
       if (tid < n) y[r0 + tid] = x;
-      if constexpr (kF) {
-        const float xf = static_cast<float>(x);
-        xsf[tid] = xf;
-        if (tid < n) yf[r0 + tid] = xf;
-      }
     }
     __syncthreads();
     // release after the block barrier: the barrier orders every thread's
@@ -1572,17 +1798,11 @@ __global__ void __launch_bounds__(256) trsv_chain(const T* __restrict__ A, long 
 #pragma unroll
     for (int r2 = r + 1; r2 < CH_R; r2++) {
       if (r2 >= np) break;
-      const T* L = Lin + static_cast<size_t>(tri(r2, r)) * TB * CH_LST;
-      T sum = T(0);
-      if constexpr (kF) {
+      const double* L = Lin + static_cast<size_t>(tri(r2, r)) * TB * CH_LST;
+      double sum = 0.0;
 #pragma unroll
-        for (int j = 0; j < 16; j++) sum = fmaf(L[(c0 + j) * CH_LST + rr], xsf[c0 + j], sum);
-        accf[r2] = df_add(accf[r2], {sum, 0.f});
-      } else {
-#pragma unroll
-        for (int j = 0; j < 16; j++) sum = fma(L[(c0 + j) * CH_LST + rr], static_cast<T>(xs[c0 + j]), sum);
-        acc[r2] += static_cast<double>(sum);
-      }
+      for (int j = 0; j < 16; j++) sum = fma(L[(c0 + j) * CH_LST + rr], xs[c0 + j], sum);
+      acc[r2] += sum;
     }
   }
   __syncthreads();  // the staged blocks are read no more: the next group's may overwrite them
@@ -2827,54 +3047,68 @@ void DenseLU::tri_solve(const T* LU, long long ld, int N, double* b, int trans) 
   const size_t rnd = ((static_cast<size_t>(N) + 31) / 32) * 32;
   double* w1 = tri_work_;
   double* w2 = tri_work_ + rnd;  // 256-byte aligned second vector
+  constexpr bool kF = std::is_same<T, float>::value;
   static std::once_flag ch_attr;
   std::call_once(ch_attr, [] {
     auto smem = [](auto* kernel, size_t bytes) {
       cuda_check(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes)),
                  "cudaFuncSetAttribute(chain sweep)");
     };
-    smem(trsv_chain<float, false>, chain_smem<float>());
-    smem(trsv_chain<float, true>, chain_smem<float>());
-    smem(trsv_chain<double, false>, chain_smem<double>());
-    smem(trsv_chain<double, true>, chain_smem<double>());
+    if constexpr (kF) {
+      smem(trsv_group<false>, sizeof(TgShared));
+      smem(trsv_group<true>, sizeof(TgShared));
+    } else {
+      smem(trsv_chain<false>, CH_SMEM);
+      smem(trsv_chain<true>, CH_SMEM);
+    }
   });
-  // one group of CH_R blocks per CTA while the device holds that many CTAs;
+  // one group of blocks per CTA while the device holds that many CTAs;
   // more groups go round the context's SMs.  The sums' order does not depend
   // on the grid, so concurrent and serial solves agree bit for bit.
-  const int gch = (nblk + CH_R - 1) / CH_R;
+  constexpr int R = kF ? TG : CH_R;
+  const int gch = (nblk + R - 1) / R;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(gch <= nsm_ ? gch : ctx_->sms(), 1, 1);
   cfg.blockDim = dim3(256, 1, 1);
-  cfg.dynamicSmemBytes = chain_smem<T>();
+  cfg.dynamicSmemBytes = kF ? sizeof(TgShared) : CH_SMEM;
   cfg.stream = s;
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeCooperative;
   at[0].val.cooperative = 1;
   cfg.attrs = at;
   cfg.numAttrs = 1;
-  cuda_check(cudaMemsetAsync(tri_bar_, 0, 2 * sizeof(unsigned), s), "memset sweep progress");
-  const float2* dl2 = std::is_same<T, float>::value ? dinv2_l_ : nullptr;
-  const float2* du2 = std::is_same<T, float>::value ? dinv2_u_ : nullptr;
-  // FP32 copies of the two sweeps' outputs (FP32 factors only)
-  float* yf1 = std::is_same<T, float>::value ? reinterpret_cast<float*>(tri_work_ + 2 * rnd) : nullptr;
-  float* yf2 = std::is_same<T, float>::value ? yf1 + rnd : nullptr;
   const unsigned stall = ctx_->stall_waits ? 1u : 0u;
-  auto sweep = [&](auto* kernel, const double* in, double* out, float* outf, const double* dinv, const float2* dinv2,
-                   int lower, unsigned* progress, const char* what) {
+  // FP32 copies of the two sweeps' outputs (FP32 factors only)
+  float* yf = reinterpret_cast<float*>(tri_work_ + 2 * rnd);
+  if constexpr (kF)
+    cuda_check(cudaMemsetAsync(yf, 0xff, 2 * rnd * sizeof(float), s), "memset sweep outputs");
+  else
+    cuda_check(cudaMemsetAsync(tri_bar_, 0, 2 * sizeof(unsigned), s), "memset sweep progress");
+  // sweep number k over L (or its transpose) or U
+  auto sweep = [&](int k, bool over_l, const double* in, double* out, const char* what) {
     ProfScope ps(ctx_, Context::PROF_LU_SOLVE, sweep_bytes);
-    cuda_check(cudaLaunchKernelEx(&cfg, kernel, LU, ld, N, in, out, outf, dinv, dinv2, lower, progress, panel_err_,
-                                  ctx_->grid_wait_ns, stall),
-               what);
+    const int ascending = k == 0 ? 1 : 0;
+    if constexpr (kF) {
+      cuda_check(cudaLaunchKernelEx(&cfg, trans ? trsv_group<true> : trsv_group<false>, LU, ld, N, in, out,
+                                    yf + k * rnd, over_l ? dinv2_l_ : dinv2_u_, over_l ? group_x_l_ : group_x_u_,
+                                    ascending, panel_err_, ctx_->grid_wait_ns, stall),
+                 what);
+    } else {
+      cuda_check(cudaLaunchKernelEx(&cfg, trans ? trsv_chain<true> : trsv_chain<false>, LU, ld, N, in, out,
+                                    over_l ? dinv_l_ : dinv_u_, ascending, tri_bar_ + k, panel_err_,
+                                    ctx_->grid_wait_ns, stall),
+                 what);
+    }
   };
   if (!trans) {
     // L y = P b, then U x = y
     gather_perm<<<blocks(N, 256), 256, 0, s>>>(b, perm_, N, w1);
-    sweep(trsv_chain<T, false>, w1, w2, yf1, dinv_l_, dl2, 1, tri_bar_, "forward sweep");
-    sweep(trsv_chain<T, false>, w2, b, yf2, dinv_u_, du2, 0, tri_bar_ + 1, "backward sweep");
+    sweep(0, true, w1, w2, "forward sweep");
+    sweep(1, false, w2, b, "backward sweep");
   } else {
     // A^T = U^T L^T P: U^T y = b (forward), L^T z = y (backward), x = P^T z
-    sweep(trsv_chain<T, true>, b, w2, yf1, dinv_u_, du2, 1, tri_bar_, "forward transposed sweep");
-    sweep(trsv_chain<T, true>, w2, w1, yf2, dinv_l_, dl2, 0, tri_bar_ + 1, "backward transposed sweep");
+    sweep(0, false, b, w2, "forward transposed sweep");
+    sweep(1, true, w2, w1, "backward transposed sweep");
     scatter_perm<<<blocks(N, 256), 256, 0, s>>>(w1, perm_, N, b);
   }
   ctx_->launches += 3;
@@ -2953,6 +3187,27 @@ void DenseLU::prepare_solves(const T* LU, long long ld, int N) {
   });
   invert_diag_blocks<T><<<dim3(nblk, 2), ID_THREADS, smem, s>>>(LU, ld, N, dinv_l_, dinv_u_, dinv2_l_, dinv2_u_);
   ctx_->launches++;
+  if constexpr (std::is_same<T, float>::value) {
+    const int ng = (nblk + TG - 1) / TG;
+    const size_t gx = static_cast<size_t>(ng) * TB * TB;
+    if (gx > group_x_cap_) {
+      cudaFree(group_x_l_);
+      cudaFree(group_x_u_);
+      group_x_l_ = group_x_u_ = nullptr;
+      group_x_cap_ = 0;
+      cuda_check(cudaMalloc(&group_x_l_, gx * sizeof(float2)), "cudaMalloc(group inverses)");
+      cuda_check(cudaMalloc(&group_x_u_, gx * sizeof(float2)), "cudaMalloc(group inverses)");
+      group_x_cap_ = gx;
+    }
+    static std::once_flag gi_attr;
+    std::call_once(gi_attr, [] {
+      cuda_check(cudaFuncSetAttribute(invert_groups, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      static_cast<int>(GI_SMEM)),
+                 "cudaFuncSetAttribute(group inverses)");
+    });
+    invert_groups<<<dim3(ng, 2), 256, GI_SMEM, s>>>(LU, ld, N, dinv2_l_, dinv2_u_, group_x_l_, group_x_u_);
+    ctx_->launches++;
+  }
   cuda_check(cudaGetLastError(), "solve preparation");
 }
 

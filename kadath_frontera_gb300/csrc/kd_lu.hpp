@@ -119,6 +119,9 @@ class DenseLU {
   float2* dinv2_l_ = nullptr;  // the same as (hi, lo) FP32 pairs (sweeps with FP32 factors)
   float2* dinv2_u_ = nullptr;
   size_t dinv_cap_ = 0;
+  float2* group_x_l_ = nullptr;  // off-diagonal blocks of the inverses of the 192-row groups (FP32 factors)
+  float2* group_x_u_ = nullptr;
+  size_t group_x_cap_ = 0;
   int* perm_ = nullptr;       // pivots as one permutation
   double* tri_work_ = nullptr;
   size_t perm_cap_ = 0;
