@@ -769,9 +769,13 @@ __global__ void __launch_bounds__(ID_THREADS) invert_diag_blocks(const T* __rest
 }
 
 // y = alpha A x + beta b (FP64, column-major).  The columns are split into
-// chunks so that the grid covers the GPU: gemv_partial writes one partial
-// sum per (chunk, row), gemv_finish adds them in chunk order (deterministic).
+// chunks: gemv_partial writes one partial sum per (chunk, row), gemv_finish
+// adds them in chunk order (deterministic).  Bound: the FP64 pipe (an FP64
+// multiply-add takes a warp 16 cycles of its SM: 0.26 ms for N = 12,331, the
+// matrix's bytes 0.18 ms), so every SM needs the same share: 16 CTAs an SM
+// while the chunks allow it (four an SM left some SMs with five: 0.31 ms).
 constexpr int GEMV_ROWS = 256;
+constexpr int GEMV_MAX_CHUNKS = 64;
 __global__ void __launch_bounds__(GEMV_ROWS) gemv_partial(const double* __restrict__ A, long long ld, int N,
                                                           const double* __restrict__ x, int chunk,
                                                           double* __restrict__ part) {
@@ -816,6 +820,7 @@ __global__ void gemv_finish(const double* __restrict__ part, int nchunk, int N, 
   const int row = blockIdx.x * blockDim.x + threadIdx.x;
   if (row >= N) return;
   double s = 0.0;
+#pragma unroll 8
   for (int c = 0; c < nchunk; c++) s += part[static_cast<size_t>(c) * N + row];
   y[row] = alpha * s + (b ? beta * b[row] : 0.0);
 }
@@ -823,7 +828,7 @@ __global__ void gemv_finish(const double* __restrict__ part, int nchunk, int N, 
 // y = alpha A^T x + beta b: one warp per column of A (a row of A^T), the
 // column read coalesced, lane partial sums reduced by xor shuffles (fixed
 // order).
-constexpr int GEMVT_WARPS = 8;
+constexpr int GEMVT_WARPS = 2;  // small CTAs: the SMs' shares differ by a column or two
 __global__ void __launch_bounds__(GEMVT_WARPS * 32) gemv_t_kernel(const double* __restrict__ A, long long ld, int N,
                                                                  const double* __restrict__ x, double alpha,
                                                                  double beta, const double* __restrict__ b,
@@ -834,6 +839,16 @@ __global__ void __launch_bounds__(GEMVT_WARPS * 32) gemv_t_kernel(const double* 
   const double* a = A + static_cast<long long>(col) * ld;
   double s0 = 0.0, s1 = 0.0;
   int k = lane;
+  for (; k + 7 * 32 < N; k += 8 * 32) {  // eight loads in flight
+    double v[8];
+#pragma unroll
+    for (int u = 0; u < 8; u++) v[u] = __ldcs(a + k + 32 * u);
+#pragma unroll
+    for (int u = 0; u < 8; u += 2) {
+      s0 = fma(v[u], x[k + 32 * u], s0);
+      s1 = fma(v[u + 1], x[k + 32 * u + 32], s1);
+    }
+  }
   for (; k + 32 < N; k += 64) {
     s0 = fma(a[k], x[k], s0);
     s1 = fma(a[k + 32], x[k + 32], s1);
@@ -3223,12 +3238,13 @@ void DenseLU::gemv(const double* x, double* y, double alpha, double beta, const 
     return;
   }
   const int rb = blocks(N, GEMV_ROWS);
-  int nchunk = (4 * nsm_ + rb - 1) / rb;  // the device's SMs: the split of the sums stays fixed
-  if (nchunk > 32) nchunk = 32;
+  int nchunk = (16 * nsm_ + rb - 1) / rb;  // the device's SMs: the split of the sums stays fixed
+  if (nchunk > GEMV_MAX_CHUNKS) nchunk = GEMV_MAX_CHUNKS;
+  if (nchunk > (N + 15) / 16) nchunk = (N + 15) / 16;  // shorter chunks cost more in gemv_finish than they save
   if (nchunk < 1) nchunk = 1;
   const int chunk = (N + nchunk - 1) / nchunk;
   nchunk = (N + chunk - 1) / chunk;
-  const size_t need = static_cast<size_t>(32) * N;
+  const size_t need = static_cast<size_t>(GEMV_MAX_CHUNKS) * N;
   if (need > part_cap_) {
     cudaFree(part_);
     cuda_check(cudaMalloc(&part_, need * sizeof(double)), "cudaMalloc(gemv partials)");
