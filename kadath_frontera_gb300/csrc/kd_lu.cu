@@ -2690,17 +2690,25 @@ static void launch_trsm_chunk(Context* ctx, float* A, long long ld, int j0, int 
   cuda_check(cudaGetLastError(), "trsm kernel");
 }
 
+// The row exchanges of a factored panel in every other column.
 template <class T>
-static void trsm_and_swaps(Context* ctx, T* A, long long ld, int N, int j0, int jb, const int* ipiv, int* map,
-                           bool map_ready, int* perm) {
+static void exchange_rows(Context* ctx, T* A, long long ld, int N, int j0, int jb, const int* ipiv, int* map,
+                          bool map_ready, int* perm) {
   cudaStream_t s = ctx->stream();
-  ProfScope ps(ctx, Context::PROF_LU_SWAP_TRSM, 2.0 * sizeof(T) * jb * (N - j0 - jb));
   if (!map_ready) {
     build_swap_map<<<1, 32, 0, s>>>(ipiv, j0, jb, map);
     ctx->launches += 1;
   }
   laswp_map<T><<<blocks(static_cast<long long>(N - jb + 1) * 32, 256), 256, 0, s>>>(A, ld, N, j0, jb, map, perm);
   ctx->launches += 1;
+}
+
+template <class T>
+static void trsm_and_swaps(Context* ctx, T* A, long long ld, int N, int j0, int jb, const int* ipiv, int* map,
+                           bool map_ready, int* perm) {
+  cudaStream_t s = ctx->stream();
+  ProfScope ps(ctx, Context::PROF_LU_SWAP_TRSM, 2.0 * sizeof(T) * jb * (N - j0 - jb));
+  exchange_rows<T>(ctx, A, ld, N, j0, jb, ipiv, map, map_ready, perm);
   if (j0 + jb < N) {
     if constexpr (std::is_same<T, float>::value) {
       launch_trsm_chunk(ctx, A, ld, j0, jb, j0 + jb, N);
@@ -2768,11 +2776,60 @@ void DenseLU::factor_f32(float* A, long long ld, int N, bool tf32) {
     if (cluster_panel_width(rows, 64) > 0) return true;
     return !grid_panel_fits(rows, 96, nsm_eff, sizeof(float)) && cluster_panel_width(rows) > 0;
   };
+  // A panel on the grid has no look-ahead, so it may as well be two: 192 columns
+  // as two halves of 96, the right one brought up to date between them, and one
+  // trailing update with k = 192 for both, which streams the trailing matrix
+  // through HBM half as often.  N = 40,081: updates 362 -> 294 ms with all of the
+  // right halves' extra products, the factorisation 519 -> 452 ms.  (Cluster
+  // panels stay at 96 or 64: their updates run beside the next panel.)
+  const int NW = 2 * NB;
+  auto wide = [&](int rows) {
+    return tf32 && tf32_terms == 3 && rows > NW && !on_cluster(rows) &&
+           grid_panel_fits(rows, NB, nsm_eff, sizeof(float)) &&
+           tf32x3_gemm_possible(NW, A, ld, 4, 4);  // panels start at multiples of 4, so A stands for every C
+  };
   auto width = [&](int j0) {
     const int rows = N - j0;
     int w = NB;
     if (on_cluster(rows)) w = cluster_panel_width(rows);
+    else if (wide(rows)) w = NW;
     return (rows < w) ? rows : w;
+  };
+  auto at = [&](int row, int col) { return A + static_cast<long long>(col) * ld + row; };
+  auto panel = [&](int j0, int jb) {
+    return panel_factor<float>(ctx_, A, ld, N, j0, jb, ipiv_, d_info_, nsm_, slot_mem_, swap_map_);
+  };
+  // Factors the panel of jb columns; of a wide one both halves, with the left
+  // half's row exchanges in every column.
+  auto factor_panel = [&](int j0, int jb) {
+    const bool left = panel(j0, jb <= NB ? jb : NB);
+    if (jb <= NB) return left;
+    {
+      ProfScope ps(ctx_, Context::PROF_LU_SWAP_TRSM, 2.0 * sizeof(float) * NB * (N - j0 - NB));
+      exchange_rows<float>(ctx_, A, ld, N, j0, NB, ipiv_, swap_map_, left, perm_);
+      launch_trsm_chunk(ctx_, A, ld, j0, NB, j0 + NB, j0 + jb);
+    }
+    gemm_update_f32(ctx_, blas_, N - j0 - NB, jb - NB, NB, at(j0 + NB, j0), ld, at(j0, j0 + NB), ld,
+                    at(j0 + NB, j0 + NB), ld, tf32, static_cast<int>(ld - j0 - NB), tf32_terms);
+    return panel(j0 + NB, jb - NB);
+  };
+  // The (right half's) row exchanges and U12 = L11^-1 A12 over the trailing columns.
+  auto finish_panel = [&](int j0, int jb, bool ready) {
+    if (jb <= NB) {
+      trsm_and_swaps<float>(ctx_, A, ld, N, j0, jb, ipiv_, swap_map_, ready, perm_);
+      return;
+    }
+    const int c0 = j0 + jb;
+    {
+      ProfScope ps(ctx_, Context::PROF_LU_SWAP_TRSM, 2.0 * sizeof(float) * NB * (N - c0));
+      exchange_rows<float>(ctx_, A, ld, N, j0 + NB, jb - NB, ipiv_, swap_map_, ready, perm_);
+      if (c0 < N) launch_trsm_chunk(ctx_, A, ld, j0, NB, c0, N);
+    }
+    if (c0 >= N) return;
+    gemm_update_f32(ctx_, blas_, jb - NB, N - c0, NB, at(j0 + NB, j0), ld, at(j0, c0), ld, at(j0 + NB, c0), ld, tf32,
+                    jb - NB, tf32_terms);
+    ProfScope ps(ctx_, Context::PROF_LU_SWAP_TRSM, 2.0 * sizeof(float) * (jb - NB) * (N - c0));
+    launch_trsm_chunk(ctx_, A, ld, j0 + NB, jb - NB, c0, N);
   };
   // Look-ahead (tensor-core update only): the columns of the next panel are
   // updated first, then the rest of the trailing update runs on a side
@@ -2782,14 +2839,14 @@ void DenseLU::factor_f32(float* A, long long ld, int N, bool tf32) {
   // the update: look-ahead only when the next panel fits a cluster.
   const bool lookahead = tf32 && tf32_update_max_clusters16() >= 2;
   int j0 = 0, jb = width(0);
-  bool map_ready = panel_factor<float>(ctx_, A, ld, N, j0, jb, ipiv_, d_info_, nsm_, slot_mem_, swap_map_);
+  bool map_ready = factor_panel(j0, jb);
   bool side_pending = false;
   for (;;) {
     if (side_pending) {
       ctx_->join();
       side_pending = false;
     }
-    trsm_and_swaps<float>(ctx_, A, ld, N, j0, jb, ipiv_, swap_map_, map_ready, perm_);
+    finish_panel(j0, jb, map_ready);
     const int m = N - j0 - jb;
     if (m <= 0) break;
     const int j0n = j0 + jb, jbn = width(j0n);
@@ -2809,7 +2866,7 @@ void DenseLU::factor_f32(float* A, long long ld, int N, bool tf32) {
     } else {
       gemm_update_f32(ctx_, blas_, m, m, jb, A21, ld, A12, ld, A22, ld, tf32, writable, tf32_terms);
     }
-    map_ready = panel_factor<float>(ctx_, A, ld, N, j0n, jbn, ipiv_, d_info_, nsm_, slot_mem_, swap_map_);
+    map_ready = factor_panel(j0n, jbn);
     j0 = j0n;
     jb = jbn;
   }
