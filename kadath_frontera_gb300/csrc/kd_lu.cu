@@ -440,13 +440,26 @@ __global__ void __launch_bounds__(SC_THREADS) scale_convert_kernel(const double*
 // A11 = L11 U11 without exchanges, then L21 = A21 U11^-1.  Every CTA factors
 // the (at most 96 x 96) diagonal block itself in shared memory -- redundant,
 // but it removes every grid-wide synchronisation -- and then solves
-// x U11 = a for NP_THREADS rows of A21, one row per thread with the row in
-// registers.  The last CTA to finish writes L11 \ U11 back.  A zero or non-finite pivot sets
+// x U11 = a for its share of A21's rows, two rows a thread.  The last CTA to
+// read the diagonal block writes L11 \ U11 back.  A zero or non-finite pivot sets
 // *info (the caller then factors with partial pivoting instead).
 constexpr int NP_NB = 96;
 constexpr int NP_LD = NP_NB + 4;  // row stride: 16-byte aligned rows, read four elements at a time by L21
 constexpr int NP_THREADS = 256;
-constexpr int NP_XS_BYTES = (NP_NB - 32) * NP_THREADS * 4;  // the solved chunks 0 and 1 of every thread's row
+// L21: two rows a thread.  The 16-byte reads of U11 take the shared memory four
+// cycles each whatever they feed: with one row a thread they were the bound
+// (35,000 cycles for 256 rows); with four a warp is alone on its scheduler and
+// waits for them (36,000 for 128).  A thread's rows of the panel wait in its own
+// column of dynamic shared memory, copied there while the diagonal block is
+// factored.
+// Measured, N = 12,331, beside the trailing update: a panel 82,000 -> 60,000
+// cycles below 5,000 rows (L21 35,000 -> 23,000, diagonal block 25,000 -> 19,600,
+// write-back 8,000 -> 0) and 110,000 - 180,000 -> 84,000 above 10,000; the whole
+// factorisation in a reused order 17.1 -> 15.9 ms.
+constexpr int NP_L21_THREADS = 192;
+constexpr int NP_L21_ROWS = 2 * NP_L21_THREADS;  // rows of A21 a round
+constexpr int NP_XS_BYTES = NP_NB * NP_L21_THREADS * 8;
+constexpr int NP_MIN_ROWS = 128;  // of a CTA: fewer would not be faster
 constexpr int NP_MAX_CTAS = 38;  // SMs outside the seven 16-CTA clusters of a GB300's trailing update: 152 - 112 = 40
 static_assert(NP_THREADS == 256 && NP_NB == 96, "three 32-column blocks; 16 x 16 threads tile the trailing blocks");
 
@@ -483,39 +496,98 @@ __device__ __forceinline__ void np_trailing(float* __restrict__ U, int o, int ti
 // Eight elimination steps k0 .. k0+7 of a 32 x 32 diagonal block held by
 // one warp, lane l holding row l with its values shifted so that d[0] is
 // column k (see panel_nopiv_kernel).  From step k0 on at most W = 32 - k0
-// columns are live, so only W - 1 values of the pivot row are broadcast.
-// rp enters as __frcp_rn of step k0's pivot and leaves as the next one's;
-// each step stores the element of column k that became final.
+// columns are live.  The pivot row goes to the other lanes through shared
+// memory (prow, one of two in turn), 16 bytes at a time.  A multiplier is the
+// quotient q = d r corrected by q (1 - p r), r about 1 / p: as accurate as the
+// product with a rounded reciprocal, and without the branch of __frcp_rn, behind
+// which a lone warp waits (28,000 cycles for the 96 steps).  (r, 1 - p r) enter
+// for step k0 and leave for the next one; every lane works them out with the
+// pivot's owner's operations from three shuffles.  Each step stores the element
+// of column k that became final.
+__device__ __forceinline__ float2 np_reciprocal(float p) {
+  float r;
+  asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(p));
+  return make_float2(r, fmaf(-p, r, 1.0f));
+}
+__device__ __forceinline__ float np_quotient(float d, float2 rp) {
+  const float q = d * rp.x;
+  return fmaf(q, rp.y, q);
+}
 template <int W>
-__device__ __forceinline__ void np_diag_steps(float (&d)[32], float& rp, float* __restrict__ urow,
-                                              float* __restrict__ rpv, int lane, int k0) {
+__device__ __forceinline__ void np_diag_steps(float (&d)[32], float2& rp, float* __restrict__ urow, float* prow,
+                                              int lane, int k0) {
 #pragma unroll 1
   for (int k = k0; k < k0 + 8; k++) {
-    float pr[W];  // the pivot row (lane k's values)
+    float* row = prow + (k & 1) * 32;
+    if (lane == k) {
 #pragma unroll
-    for (int j = 1; j < W; j++) pr[j] = __shfl_sync(0xffffffffu, d[j], k);
+      for (int j = 0; j < W; j += 4) *reinterpret_cast<float4*>(row + j) = make_float4(d[j], d[j + 1], d[j + 2], d[j + 3]);
+    }
+    __syncwarp();
+    const float p1 = __shfl_sync(0xffffffffu, d[1], k);
+    const float a0 = __shfl_sync(0xffffffffu, d[0], (k + 1) & 31), a1 = __shfl_sync(0xffffffffu, d[1], (k + 1) & 31);
     // rows up to k (the finished ones and the pivot row) take a zero
     // multiplier: their multiply-adds leave them as they are
-    const float lm = (lane > k) ? d[0] * rp : 0.0f;
-    if (lane == 0) rpv[k] = rp;
+    const float q = np_quotient(d[0], rp);
+    const float lm = (lane > k) ? q : 0.0f;
     urow[k] = (lane > k) ? lm : d[0];
-    // the next pivot first, so that its reciprocal overlaps this step
-    d[0] = fmaf(-lm, pr[1], d[1]);
-    const float rpn = __frcp_rn(__shfl_sync(0xffffffffu, d[0], (k + 1) & 31));
+    rp = np_reciprocal(fmaf(-np_quotient(a0, rp), p1, a1));
+    float pr[W];
 #pragma unroll
-    for (int j = 2; j < W; j++) d[j - 1] = fmaf(-lm, pr[j], d[j]);
+    for (int j = 0; j < W; j += 4) {
+      const float4 v = *reinterpret_cast<const float4*>(row + j);
+      pr[j] = v.x;
+      pr[j + 1] = v.y;
+      pr[j + 2] = v.z;
+      pr[j + 3] = v.w;
+    }
+#pragma unroll
+    for (int j = 1; j < W; j++) d[j - 1] = fmaf(-lm, pr[j], d[j]);
     d[W - 1] = 0.0f;
-    rp = rpn;
   }
 }
 
+// two FP32 multiply-adds in one instruction
+__device__ __forceinline__ unsigned long long pack2(float lo, float hi) {
+  unsigned long long v;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(lo), "f"(hi));
+  return v;
+}
+__device__ __forceinline__ float2 unpack2(unsigned long long v) {
+  float2 f;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(f.x), "=f"(f.y) : "l"(v));
+  return f;
+}
+__device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
+  unsigned long long d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+
 __global__ void __launch_bounds__(NP_THREADS) panel_nopiv_kernel(float* __restrict__ A, long long ld, int N, int j0,
-                                                                 int jb, int rpt, int* __restrict__ info,
+                                                                 int jb, int rows, int* __restrict__ info,
                                                                  unsigned* __restrict__ done) {
   __shared__ __align__(16) float U[NP_NB * NP_LD];
   __shared__ float rdiag[NP_NB];
   __shared__ float rpv[NP_NB];  // __frcp_rn of the pivots
+  __shared__ __align__(16) float prow[2 * 32];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  // rows first .. end of A21 are this CTA's; A's columns are 128-byte aligned
+  // and padded to a multiple of 32 rows, first is a multiple of 4
+  const int first = j0 + jb + blockIdx.x * rows, end = min(first + rows, N);
+  const int lt = tid - (NP_THREADS - NP_L21_THREADS);  // L21's threads: all warps but the first two
+  extern __shared__ __align__(16) float2 np_xs[];  // [column][thread]: two rows
+  auto fetch = [&](int row) {
+    if (lt >= 0 && row < end) {
+      const float* src = A + static_cast<long long>(j0) * ld + row;
+      for (int k = 0; k < jb; k++, src += ld)
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(static_cast<unsigned>(
+                         __cvta_generic_to_shared(np_xs + k * NP_L21_THREADS + lt))),
+                     "l"(src)
+                     : "memory");
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
   {
     // all 36 loads of the thread in flight before the shared stores
     constexpr int NV = NP_NB * NP_NB / NP_THREADS;
@@ -534,35 +606,49 @@ __global__ void __launch_bounds__(NP_THREADS) panel_nopiv_kernel(float* __restri
       U[(e % NP_NB) * NP_LD + e / NP_NB] = v[q];
     }
   }
+  fetch(first + 2 * lt);
+  // L11 \ U11 goes back to A only when every CTA has read the diagonal block:
+  // the last CTA to have read it writes it (each holds the same factors), with
+  // the two warps that have no rows of L21, and resets the counter for the next
+  // panel.  CTAs need not be resident together, as they are beside the trailing
+  // update on a side stream.
+  __shared__ int np_last;
   __syncthreads();
+  if (tid == NP_THREADS - 1) {  // not of the warp that factors the diagonal block
+    __threadfence();
+    np_last = (atomicAdd(done, 1u) == gridDim.x - 1) ? 1 : 0;
+    __threadfence();
+    if (np_last) *done = 0u;
+  }
   // Blocked right-looking elimination in shared memory, by 32-column
   // blocks o = 0, 32, 64 (identity padding past jb stays identity):
   //  (a) warp 0 factors the diagonal block in registers, lane l holding row
-  //      o + l; step k broadcasts the pivot row by shuffles, no barrier;
+  //      o + l, no barrier;
   //  (b) threads 0..rest-1 solve the block row U12 by columns and threads
   //      128..128+rest-1 the block column L21 by rows;
   //  (c) all threads apply the rank-32 update to the trailing block, a
   //      register tile each.
-  // Every element receives its multiply-adds in increasing k and every
-  // multiplier is (value) * __frcp_rn(pivot), the unblocked right-looking
-  // elimination's own operations in its own order: the factors are the same.
+  // Every element receives its multiply-adds in increasing k, like in the
+  // unblocked right-looking elimination.
   // The loop over k of (a) stays rolled: one warp running unrolled
   // straight-line code once per launch waits on instruction fetch most of
   // the time.  So that registers are never indexed by k, each step shifts
   // the lane's values down by one (column o + k is always d[0]) and stores
   // the element that became final.
-#pragma unroll
+#pragma unroll 1
   for (int o = 0; o < NP_NB; o += 32) {
     if (warp == 0) {
       float d[32];  // row o + lane, columns o + k + j
 #pragma unroll
       for (int j = 0; j < 32; j++) d[j] = U[(o + lane) * NP_LD + o + j];
       float* urow = U + (o + lane) * NP_LD + o;
-      float rp = __frcp_rn(__shfl_sync(0xffffffffu, d[0], 0));  // the correctly rounded 1 / pivot
-      np_diag_steps<32>(d, rp, urow, rpv + o, lane, 0);
-      np_diag_steps<24>(d, rp, urow, rpv + o, lane, 8);
-      np_diag_steps<16>(d, rp, urow, rpv + o, lane, 16);
-      np_diag_steps<8>(d, rp, urow, rpv + o, lane, 24);
+      float2 rp = np_reciprocal(__shfl_sync(0xffffffffu, d[0], 0));
+      np_diag_steps<32>(d, rp, urow, prow, lane, 0);
+      np_diag_steps<24>(d, rp, urow, prow, lane, 8);
+      np_diag_steps<16>(d, rp, urow, prow, lane, 16);
+      np_diag_steps<8>(d, rp, urow, prow, lane, 24);
+      __syncwarp();
+      rpv[o + lane] = __frcp_rn(urow[lane]);  // the correctly rounded 1 / pivot
     }
     __syncthreads();
     const int rest = NP_NB - o - 32;
@@ -605,81 +691,92 @@ __global__ void __launch_bounds__(NP_THREADS) panel_nopiv_kernel(float* __restri
     rdiag[tid] = 1.0f / d;
   }
   __syncthreads();
-  // L21: x U11 = a for each of this thread's rpt rows (CTA b owns rows
-  // j0 + jb + [b rpt NP_THREADS, (b + 1) rpt NP_THREADS)), by 32-column
-  // chunks with the chunk in registers: a chunk first takes off the products
-  // with the finished chunks (kept in the thread's column of np_xs, dynamic
-  // shared memory, rather than re-read from global memory), then is solved
-  // against its 32 x 32 diagonal block of U11, then written back.
-  extern __shared__ float np_xs[];  // [64][NP_THREADS]
-  for (int rr = 0; rr < rpt; rr++) {
-  const int row = j0 + jb + (blockIdx.x * rpt + rr) * NP_THREADS + tid;
-  if (row >= N) break;
-  float* arow = A + static_cast<long long>(j0) * ld + row;  // element k at arow[k * ld]
-#pragma unroll
-  for (int c = 0; c < NP_NB / 32; c++) {
-    if (c * 32 >= jb) break;
-    float x[32];
-#pragma unroll
-    for (int j = 0; j < 32; j++) x[j] = (c * 32 + j < jb) ? arow[static_cast<long long>(c * 32 + j) * ld] : 0.0f;
-#pragma unroll
-    for (int cp = 0; cp < c; cp++) {
+  if (np_last && lt < 0) {
 #pragma unroll 8
-      for (int kk = 0; kk < 32; kk++) {
-        const float yk = np_xs[(cp * 32 + kk) * NP_THREADS + tid];
-        const float4* urow = reinterpret_cast<const float4*>(U + (cp * 32 + kk) * NP_LD + c * 32);
+    for (int e = tid; e < NP_NB * NP_NB; e += NP_THREADS - NP_L21_THREADS) {
+      const int i = e % NP_NB, k = e / NP_NB;
+      if (i < jb && k < jb) A[static_cast<long long>(j0 + k) * ld + j0 + i] = U[i * NP_LD + k];
+    }
+  }
+  // L21: x U11 = a for two rows a thread, by 32-column chunks with the chunk in
+  // registers (pairs of columns): a chunk first takes off the products with the
+  // finished chunks, then is solved against its 32 x 32 diagonal block of U11,
+  // then written back.  The loop over the chunks stays rolled, for the
+  // instruction cache's sake.
+  for (int r0 = first; r0 < end; r0 += NP_L21_ROWS) {
+    const int row = r0 + 2 * lt;
+    if (r0 != first) fetch(row);
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    if (lt < 0 || row >= end) continue;
+    float2* xs = np_xs + lt;
+#pragma unroll 1
+    for (int c = 0; c < jb; c += 32) {
+      unsigned long long x[2][16];
 #pragma unroll
-        for (int j4 = 0; j4 < 8; j4++) {
-          const float4 u = urow[j4];
-          x[4 * j4] = fmaf(-yk, u.x, x[4 * j4]);
-          x[4 * j4 + 1] = fmaf(-yk, u.y, x[4 * j4 + 1]);
-          x[4 * j4 + 2] = fmaf(-yk, u.z, x[4 * j4 + 2]);
-          x[4 * j4 + 3] = fmaf(-yk, u.w, x[4 * j4 + 3]);
+      for (int p = 0; p < 16; p++) {
+        float2 lo = make_float2(0.f, 0.f), hi = lo;
+        if (c + 2 * p < jb) lo = xs[(c + 2 * p) * NP_L21_THREADS];
+        if (c + 2 * p + 1 < jb) hi = xs[(c + 2 * p + 1) * NP_L21_THREADS];
+        x[0][p] = pack2(lo.x, hi.x);
+        x[1][p] = pack2(lo.y, hi.y);
+      }
+#pragma unroll 4
+      for (int k = 0; k < c; k++) {
+        const float2 y = xs[k * NP_L21_THREADS];
+        const unsigned long long n0 = pack2(-y.x, -y.x), n1 = pack2(-y.y, -y.y);
+        const ulonglong2* u = reinterpret_cast<const ulonglong2*>(U + k * NP_LD + c);
+#pragma unroll
+        for (int q = 0; q < 8; q++) {
+          const ulonglong2 v = u[q];
+          x[0][2 * q] = fma2(n0, v.x, x[0][2 * q]);
+          x[0][2 * q + 1] = fma2(n0, v.y, x[0][2 * q + 1]);
+          x[1][2 * q] = fma2(n1, v.x, x[1][2 * q]);
+          x[1][2 * q + 1] = fma2(n1, v.y, x[1][2 * q + 1]);
         }
       }
-    }
 #pragma unroll
-    for (int kk = 0; kk < 32; kk++) {
-      x[kk] *= rdiag[c * 32 + kk];
-      const float xk = x[kk];
-      const float4* urow = reinterpret_cast<const float4*>(U + (c * 32 + kk) * NP_LD + c * 32);
+      for (int k = 0; k < 32; k++) {
+        const float rd = rdiag[c + k];
+        const ulonglong2* u = reinterpret_cast<const ulonglong2*>(U + (c + k) * NP_LD + c);
+        unsigned long long n[2];
 #pragma unroll
-      for (int j4 = (kk + 1) / 4; j4 < 8; j4++) {
-        const float4 u = urow[j4];
-        if (4 * j4 > kk) x[4 * j4] = fmaf(-xk, u.x, x[4 * j4]);
-        if (4 * j4 + 1 > kk) x[4 * j4 + 1] = fmaf(-xk, u.y, x[4 * j4 + 1]);
-        if (4 * j4 + 2 > kk) x[4 * j4 + 2] = fmaf(-xk, u.z, x[4 * j4 + 2]);
-        if (4 * j4 + 3 > kk) x[4 * j4 + 3] = fmaf(-xk, u.w, x[4 * j4 + 3]);
+        for (int r = 0; r < 2; r++) {
+          const float2 f = unpack2(x[r][k / 2]);
+          const float xk = ((k & 1) ? f.y : f.x) * rd;
+          n[r] = pack2(-xk, -xk);
+          if (k & 1)
+            x[r][k / 2] = pack2(f.x, xk);
+          else
+            x[r][k / 2] = pack2(xk, fmaf(-xk, U[(c + k) * NP_LD + c + k + 1], f.y));
+        }
+#pragma unroll
+        for (int q = (k / 2 + 1) / 2; q < 8; q++) {
+          const ulonglong2 v = u[q];
+#pragma unroll
+          for (int r = 0; r < 2; r++) {
+            if (2 * q > k / 2) x[r][2 * q] = fma2(n[r], v.x, x[r][2 * q]);
+            x[r][2 * q + 1] = fma2(n[r], v.y, x[r][2 * q + 1]);
+          }
+        }
+      }
+      float* dst = A + static_cast<long long>(j0 + c) * ld + row;
+#pragma unroll
+      for (int p = 0; p < 16; p++) {
+        const float2 f0 = unpack2(x[0][p]), f1 = unpack2(x[1][p]);
+        const float2 lo = make_float2(f0.x, f1.x), hi = make_float2(f0.y, f1.y);
+        if (c + 2 * p < jb) {
+          *reinterpret_cast<float2*>(dst) = lo;
+          xs[(c + 2 * p) * NP_L21_THREADS] = lo;
+        }
+        if (c + 2 * p + 1 < jb) {
+          *reinterpret_cast<float2*>(dst + ld) = hi;
+          xs[(c + 2 * p + 1) * NP_L21_THREADS] = hi;
+        }
+        dst += 2 * ld;
       }
     }
-#pragma unroll
-    for (int j = 0; j < 32; j++)
-      if (c * 32 + j < jb) arow[static_cast<long long>(c * 32 + j) * ld] = x[j];
-    if (c < NP_NB / 32 - 1) {
-#pragma unroll
-      for (int j = 0; j < 32; j++) np_xs[(c * 32 + j) * NP_THREADS + tid] = x[j];
-    }
   }
-  }
-  // L11 \ U11 goes back to A only when every CTA has read the diagonal
-  // block: the last CTA to finish writes it (each holds the same factors)
-  // and resets the counter for the next panel.  CTAs need not be resident
-  // together, as they are beside the trailing update on a side stream.
-  __shared__ int np_last;
-  __syncthreads();
-  if (tid == 0) {
-    __threadfence();
-    np_last = (atomicAdd(done, 1u) == gridDim.x - 1) ? 1 : 0;
-    __threadfence();
-  }
-  __syncthreads();
-  if (np_last) {
-    for (int e = tid; e < jb * jb; e += NP_THREADS) {
-      const int i = e % jb, k = e / jb;
-      A[static_cast<long long>(j0 + k) * ld + j0 + i] = U[i * NP_LD + k];
-    }
-    if (tid == 0) *done = 0u;
-  }
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
 }
 
 __global__ void scale_vec_kernel(double* __restrict__ x, const double* __restrict__ s, int N) {
@@ -2891,17 +2988,17 @@ void DenseLU::factor_f32_nopiv(float* A, long long ld, int N, bool tf32) {
   auto panel = [&](int j0, int jb) {
     const int m = N - j0 - jb;
     ProfScope ps(ctx_, Context::PROF_LU_PANEL_STATIC, 2.0 * sizeof(float) * jb * (N - j0));
-    // at most NP_MAX_CTAS CTAs (several 256-row groups each): the SMs left
-    // beside the trailing update's 16-CTA clusters
-    const int groups = m > 0 ? blocks(m, NP_THREADS) : 1;
-    const int rpt = (groups + NP_MAX_CTAS - 1) / NP_MAX_CTAS;
-    const int grid = (groups + rpt - 1) / rpt;
+    // at most NP_MAX_CTAS CTAs: the SMs left beside the trailing update's
+    // 16-CTA clusters; equal shares in whole 128-byte lines
+    int rows = ((m + NP_MAX_CTAS - 1) / NP_MAX_CTAS + 31) / 32 * 32;
+    if (rows < NP_MIN_ROWS) rows = NP_MIN_ROWS;
+    const int grid = m > 0 ? blocks(m, rows) : 1;
     static std::once_flag attr;
     std::call_once(attr, [] {
       cuda_check(cudaFuncSetAttribute(panel_nopiv_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, NP_XS_BYTES),
                  "panel_nopiv smem");
     });
-    panel_nopiv_kernel<<<grid, NP_THREADS, NP_XS_BYTES, ctx_->stream()>>>(A, ld, N, j0, jb, rpt, d_info_, np_done_);
+    panel_nopiv_kernel<<<grid, NP_THREADS, NP_XS_BYTES, ctx_->stream()>>>(A, ld, N, j0, jb, rows, d_info_, np_done_);
     ctx_->launches++;
   };
   auto trsm = [&](int j0, int jb, int c0, int c1) {
