@@ -779,11 +779,6 @@ __global__ void __launch_bounds__(NP_THREADS) panel_nopiv_kernel(float* __restri
   asm volatile("cp.async.wait_group 0;" ::: "memory");
 }
 
-__global__ void scale_vec_kernel(double* __restrict__ x, const double* __restrict__ s, int N) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < N) x[i] *= s[i];
-}
-
 // ---- triangular solves on one right-hand side (blocked by TB rows) --------
 constexpr int TB = 64;
 
@@ -794,14 +789,21 @@ __global__ void iota_kernel(int* __restrict__ v, int n) {
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) v[i] = i;
 }
 
-__global__ void gather_perm(const double* __restrict__ b, const int* __restrict__ perm, int N, double* __restrict__ out) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < N) out[i] = b[perm[i]];
+// out = P (scale b), and out = scale (P^T z); scale null: 1
+__global__ void gather_perm(const double* __restrict__ b, const int* __restrict__ perm,
+                            const double* __restrict__ scale, int N, double* __restrict__ out) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= N) return;
+  const int p = perm[i];
+  out[i] = scale ? b[p] * scale[p] : b[p];
 }
 
-__global__ void scatter_perm(const double* __restrict__ z, const int* __restrict__ perm, int N, double* __restrict__ out) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < N) out[perm[i]] = z[i];
+__global__ void scatter_perm(const double* __restrict__ z, const int* __restrict__ perm,
+                             const double* __restrict__ scale, int N, double* __restrict__ out) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= N) return;
+  const int p = perm[i];
+  out[p] = scale ? z[i] * scale[p] : z[i];
 }
 
 // Inverse of the unit-lower (blockIdx.y 0) or upper part (1) of one TB x TB
@@ -912,14 +914,27 @@ __global__ void __launch_bounds__(GEMV_ROWS) gemv_partial(const double* __restri
   part[static_cast<size_t>(blockIdx.y) * N + row] = (s0 + s1) + (s2 + s3);
 }
 
-__global__ void gemv_finish(const double* __restrict__ part, int nchunk, int N, double alpha, double beta,
-                            const double* __restrict__ b, double* __restrict__ y) {
-  const int row = blockIdx.x * blockDim.x + threadIdx.x;
-  if (row >= N) return;
+// Eight threads a row, a share of the chunks each (50 chunks one after the
+// other took 10 us, as much as the rest of a GMRES step's vector work).
+constexpr int GEMV_SHARES = 8;
+__global__ void __launch_bounds__(32 * GEMV_SHARES) gemv_finish(const double* __restrict__ part, int nchunk, int N,
+                                                                double alpha, double beta,
+                                                                const double* __restrict__ b, double* __restrict__ y) {
+  __shared__ double sums[GEMV_SHARES][32];
+  const int lane = threadIdx.x & 31, share = threadIdx.x >> 5;
+  const int row = blockIdx.x * 32 + lane;
   double s = 0.0;
+  if (row < N) {
 #pragma unroll 8
-  for (int c = 0; c < nchunk; c++) s += part[static_cast<size_t>(c) * N + row];
-  y[row] = alpha * s + (b ? beta * b[row] : 0.0);
+    for (int c = share; c < nchunk; c += GEMV_SHARES) s += part[static_cast<size_t>(c) * N + row];
+  }
+  sums[share][lane] = s;
+  __syncthreads();
+  if (share == 0 && row < N) {
+#pragma unroll
+    for (int k = 1; k < GEMV_SHARES; k++) s += sums[k][lane];
+    y[row] = alpha * s + (b ? beta * b[row] : 0.0);
+  }
 }
 
 // y = alpha A^T x + beta b: one warp per column of A (a row of A^T), the
@@ -957,47 +972,86 @@ __global__ void __launch_bounds__(GEMVT_WARPS * 32) gemv_t_kernel(const double* 
 }
 
 // ---- vector algebra of GMRES (fixed reduction order: bitwise reproducible) --
+// Bound by latency and launches: few, and each with enough loads in flight.
 constexpr int VA_THREADS = 256;
+constexpr int VD_THREADS = 1024;
 
-// h[i] = V_i . w for the k basis vectors V_i = V + i N: one CTA per i.
-__global__ void basis_dots(const double* __restrict__ V, int N, int k, const double* __restrict__ w,
-                           double* __restrict__ h) {
-  __shared__ double part[VA_THREADS];
-  const int i = blockIdx.x;
-  const double* v = V + static_cast<size_t>(i) * N;
-  double acc = 0.0;
-  for (int t = threadIdx.x; t < N; t += VA_THREADS) acc = fma(v[t], w[t], acc);
-  part[threadIdx.x] = acc;
+// The sum over a CTA of THREADS threads, in thread 0.
+template <int THREADS>
+__device__ __forceinline__ double block_sum(double v) {
+  __shared__ double part[THREADS / 32];
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = v;
   __syncthreads();
-  for (int st = VA_THREADS / 2; st > 0; st >>= 1) {
-    if (static_cast<int>(threadIdx.x) < st) part[threadIdx.x] += part[threadIdx.x + st];
-    __syncthreads();
-  }
-  if (threadIdx.x == 0 && i < k) h[i] = part[0];
+  if (threadIdx.x >= 32) return 0.0;
+  v = threadIdx.x < THREADS / 32 ? part[threadIdx.x] : 0.0;
+  for (int o = THREADS / 64; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
 }
 
-// w -= sum_i h[i] V_i over the k basis vectors.
-__global__ void basis_subtract(const double* __restrict__ V, int N, int k, const double* __restrict__ h,
-                               double* __restrict__ w) {
+// h[i] = V_i . w for the k basis vectors V_i = V + i N: one CTA per i (N =
+// 12,331: 4 us; 256 threads and one load at a time 14).
+__global__ void __launch_bounds__(VD_THREADS) basis_dots(const double* __restrict__ V, int N,
+                                                         const double* __restrict__ w, double* __restrict__ h) {
+  const double* v = V + static_cast<size_t>(blockIdx.x) * N;
+  double acc = 0.0;
+  int t = threadIdx.x;
+  for (; t + 3 * VD_THREADS < N; t += 4 * VD_THREADS) {
+    double a[4], b[4];
+#pragma unroll
+    for (int u = 0; u < 4; u++) {
+      a[u] = v[t + u * VD_THREADS];
+      b[u] = w[t + u * VD_THREADS];
+    }
+#pragma unroll
+    for (int u = 0; u < 4; u++) acc = fma(a[u], b[u], acc);
+  }
+  for (; t < N; t += VD_THREADS) acc = fma(v[t], w[t], acc);
+  acc = block_sum<VD_THREADS>(acc);
+  if (threadIdx.x == 0) h[blockIdx.x] = acc;
+}
+
+// w -= sum_i h[i] V_i over the k basis vectors; with norms, also each CTA's
+// sum of w^2 (added on the host, in their order).
+__global__ void __launch_bounds__(VA_THREADS) basis_subtract(const double* __restrict__ V, int N, int k,
+                                                             const double* __restrict__ h, double* __restrict__ w,
+                                                             double* __restrict__ norms) {
+  const int t = blockIdx.x * VA_THREADS + threadIdx.x;
+  double v = 0.0;
+  if (t < N) {
+    double acc = 0.0;
+#pragma unroll 4
+    for (int i = 0; i < k; i++) acc = fma(h[i], V[static_cast<size_t>(i) * N + t], acc);
+    v = w[t] - acc;
+    w[t] = v;
+  }
+  if (norms) {
+    v = block_sum<VA_THREADS>(v * v);
+    if (threadIdx.x == 0) norms[blockIdx.x] = v;
+  }
+}
+
+// Each CTA's sum of x^2.
+__global__ void __launch_bounds__(VA_THREADS) sum_squares(const double* __restrict__ x, int N,
+                                                          double* __restrict__ norms) {
+  const int t = blockIdx.x * VA_THREADS + threadIdx.x;
+  const double v = t < N ? x[t] : 0.0;
+  const double sum = block_sum<VA_THREADS>(v * v);
+  if (threadIdx.x == 0) norms[blockIdx.x] = sum;
+}
+
+// y = sum_i c_i V_i over k vectors, added to y when accumulate is set.
+constexpr int COMBINE_MAX = 32;
+struct CombineCoefs {
+  double c[COMBINE_MAX];
+};
+__global__ void basis_combine(const double* __restrict__ V, int N, int k, const __grid_constant__ CombineCoefs c,
+                              double* __restrict__ y, int accumulate) {
   const int t = blockIdx.x * VA_THREADS + threadIdx.x;
   if (t >= N) return;
-  double acc = 0.0;
-  for (int i = 0; i < k; i++) acc = fma(h[i], V[static_cast<size_t>(i) * N + t], acc);
-  w[t] -= acc;
-}
-
-// out = sum_t x[t]^2 (a single CTA, fixed order).
-__global__ void sum_squares(const double* __restrict__ x, int N, double* __restrict__ out) {
-  __shared__ double part[VA_THREADS];
-  double acc = 0.0;
-  for (int t = threadIdx.x; t < N; t += VA_THREADS) acc = fma(x[t], x[t], acc);
-  part[threadIdx.x] = acc;
-  __syncthreads();
-  for (int st = VA_THREADS / 2; st > 0; st >>= 1) {
-    if (static_cast<int>(threadIdx.x) < st) part[threadIdx.x] += part[threadIdx.x + st];
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) *out = part[0];
+  double acc = accumulate ? y[t] : 0.0;
+  for (int i = 0; i < k; i++) acc = fma(c.c[i], V[static_cast<size_t>(i) * N + t], acc);
+  y[t] = acc;
 }
 
 // y = alpha x, or y += alpha x when accumulate is set.
@@ -1437,7 +1491,8 @@ __global__ void __launch_bounds__(256) invert_groups(const float* __restrict__ A
 // FP32 products with x in sums of 8 terms: FP64 adds and conversions would run
 // at the FP64 rate.  TRANS: the transposed factor.  Inside the group the rows
 // run in sweep order (reversed when descending): G is lower triangular in all
-// four sweeps.  Every CTA is resident and a group waits for earlier ones only.
+// four sweeps.  b enters times bscale, y leaves times yscale (null: 1).  Every CTA
+// is resident and a group waits for earlier ones only.
 // N = 12,331: 0.177 ms a sweep (97 groups, about 3,700 cycles a link: 2,000 in
 // the order of the arithmetic, 1,250 of them G's product, and the way through
 // L2); 192-row groups chained block by block with a released counter 0.351 ms.
@@ -1464,8 +1519,10 @@ struct TgShared {
 };
 template <bool TRANS>
 __global__ void __launch_bounds__(256, 1) trsv_group(const float* __restrict__ A, long long ld, int N,
-                                                     const double* __restrict__ b, double* __restrict__ y,
-                                                     float* yf, const float2* __restrict__ Dinv2,
+                                                     const double* __restrict__ b,
+                                                     const double* __restrict__ bscale, double* __restrict__ y,
+                                                     const double* __restrict__ yscale, float* yf,
+                                                     const float2* __restrict__ Dinv2,
                                                      const float2* __restrict__ Xinv, int ascending, int* err,
                                                      unsigned long long wait_ns, unsigned stall) {
   static_assert(TG == 2 && TG_ROWS == 128, "two threads a row");
@@ -1550,7 +1607,8 @@ __global__ void __launch_bounds__(256, 1) trsv_group(const float* __restrict__ A
       sh.X[r * TG_LD + c] = Xinv[static_cast<size_t>(group(pos)) * TB * TB + e];
     }
     if (tid < TG_ROWS) {
-      const double bv = R0 + tid < N ? b[R0 + tid] : 0.0;
+      double bv = R0 + tid < N ? b[R0 + tid] : 0.0;
+      if (bscale && R0 + tid < N) bv *= bscale[R0 + tid];
       const float h = static_cast<float>(bv);
       sh.b[tid] = make_float2(h, static_cast<float>(bv - static_cast<double>(h)));
     }
@@ -1678,7 +1736,8 @@ __global__ void __launch_bounds__(256, 1) trsv_group(const float* __restrict__ A
       const unsigned bits = __float_as_uint(x.h);
       asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(yf + row), "r"(bits == TG_EMPTY ? 0x7fffffffu : bits)
                    : "memory");
-      y[row] = static_cast<double>(x.h) + static_cast<double>(x.l);
+      const double sum = static_cast<double>(x.h) + static_cast<double>(x.l);
+      y[row] = yscale ? sum * yscale[row] : sum;
     }
     __syncthreads();  // the staged blocks and part are read no more
   }
@@ -3208,7 +3267,8 @@ void DenseLU::factor(double* A, long long ld, int N, int mode) {
 // diagonal blocks: one launch per block computes the block's unknowns as a
 // small GEMV and subtracts their contribution from the remaining rows.
 template <class T>
-void DenseLU::tri_solve(const T* LU, long long ld, int N, double* b, int trans) {
+void DenseLU::tri_solve(const T* LU, long long ld, int N, const double* b, double* x, int trans, const double* bscale,
+                        const double* xscale) {
   cudaStream_t s = ctx_->stream();
   // work of one sweep: the triangle of the factors it reads
   const double sweep_bytes = 0.5 * sizeof(T) * N * static_cast<double>(N);
@@ -3254,13 +3314,14 @@ void DenseLU::tri_solve(const T* LU, long long ld, int N, double* b, int trans) 
   else
     cuda_check(cudaMemsetAsync(tri_bar_, 0, 2 * sizeof(unsigned), s), "memset sweep progress");
   // sweep number k over L (or its transpose) or U
-  auto sweep = [&](int k, bool over_l, const double* in, double* out, const char* what) {
+  auto sweep = [&](int k, bool over_l, const double* in, const double* iscale, double* out, const double* oscale,
+                   const char* what) {
     ProfScope ps(ctx_, Context::PROF_LU_SOLVE, sweep_bytes);
     const int ascending = k == 0 ? 1 : 0;
     if constexpr (kF) {
-      cuda_check(cudaLaunchKernelEx(&cfg, trans ? trsv_group<true> : trsv_group<false>, LU, ld, N, in, out,
-                                    yf + k * rnd, over_l ? dinv2_l_ : dinv2_u_, over_l ? group_x_l_ : group_x_u_,
-                                    ascending, panel_err_, ctx_->grid_wait_ns, stall),
+      cuda_check(cudaLaunchKernelEx(&cfg, trans ? trsv_group<true> : trsv_group<false>, LU, ld, N, in, iscale, out,
+                                    oscale, yf + k * rnd, over_l ? dinv2_l_ : dinv2_u_,
+                                    over_l ? group_x_l_ : group_x_u_, ascending, panel_err_, ctx_->grid_wait_ns, stall),
                  what);
     } else {
       cuda_check(cudaLaunchKernelEx(&cfg, trans ? trsv_chain<true> : trsv_chain<false>, LU, ld, N, in, out,
@@ -3271,38 +3332,29 @@ void DenseLU::tri_solve(const T* LU, long long ld, int N, double* b, int trans) 
   };
   if (!trans) {
     // L y = P b, then U x = y
-    gather_perm<<<blocks(N, 256), 256, 0, s>>>(b, perm_, N, w1);
-    sweep(0, true, w1, w2, "forward sweep");
-    sweep(1, false, w2, b, "backward sweep");
+    gather_perm<<<blocks(N, 256), 256, 0, s>>>(b, perm_, bscale, N, w1);
+    sweep(0, true, w1, nullptr, w2, nullptr, "forward sweep");
+    sweep(1, false, w2, nullptr, x, xscale, "backward sweep");
   } else {
     // A^T = U^T L^T P: U^T y = b (forward), L^T z = y (backward), x = P^T z
-    sweep(0, false, b, w2, "forward transposed sweep");
-    sweep(1, true, w2, w1, "backward transposed sweep");
-    scatter_perm<<<blocks(N, 256), 256, 0, s>>>(w1, perm_, N, b);
+    sweep(0, false, b, bscale, w2, nullptr, "forward transposed sweep");
+    sweep(1, true, w2, nullptr, w1, nullptr, "backward transposed sweep");
+    scatter_perm<<<blocks(N, 256), 256, 0, s>>>(w1, perm_, xscale, N, x);
   }
   ctx_->launches += 3;
   cuda_check(cudaGetLastError(), "triangular solve");
 }
 
 void DenseLU::solve_fp64(const double* LU, long long ld, int N, double* b, int trans) {
-  tri_solve<double>(LU, ld, N, b, trans);
+  tri_solve<double>(LU, ld, N, b, b, trans, nullptr, nullptr);
 }
 
-void DenseLU::solve_f32(double* b, int trans) {
+void DenseLU::solve_f32(const double* b, double* x, int trans) {
   // M^-1 b = D_c (LU)^-1 (D_r b) with the equilibrated factors LU of
   // P D_r A D_c; transposed, M^-T b = D_r (LU)^-T (D_c b)
-  cudaStream_t st = ctx_->stream();
   const double* first = trans ? eq_buf_ + N_ : eq_buf_;
   const double* last = trans ? eq_buf_ : eq_buf_ + N_;
-  if (scaled_) {
-    scale_vec_kernel<<<blocks(N_, 256), 256, 0, st>>>(b, first, N_);
-    ctx_->launches++;
-  }
-  tri_solve<float>(A32_, ld32_, N_, b, trans);
-  if (scaled_) {
-    scale_vec_kernel<<<blocks(N_, 256), 256, 0, st>>>(b, last, N_);
-    ctx_->launches++;
-  }
+  tri_solve<float>(A32_, ld32_, N_, b, x, trans, scaled_ ? first : nullptr, scaled_ ? last : nullptr);
 }
 
 // A sweep that gave up is reported first (its garbage also stops the
@@ -3405,7 +3457,7 @@ void DenseLU::gemv(const double* x, double* y, double alpha, double beta, const 
     part_cap_ = need;
   }
   gemv_partial<<<dim3(rb, nchunk), GEMV_ROWS, 0, s>>>(A_, ld_, N, x, chunk, part_);
-  gemv_finish<<<blocks(N, 256), 256, 0, s>>>(part_, nchunk, N, alpha, beta, b, y);
+  gemv_finish<<<blocks(N, 32), 32 * GEMV_SHARES, 0, s>>>(part_, nchunk, N, alpha, beta, b, y);
   ctx_->launches += 2;
 }
 
@@ -3419,21 +3471,21 @@ void DenseLU::gmres_ir(double* b, int trans) {
   const int N = N_;
   const int m = gmres_max_iter;
   cudaStream_t s = ctx_->stream();
-  const size_t hn_at = 2 * static_cast<size_t>(m + 1);  // projections of both passes, then |w|^2
-  ensure_work(static_cast<size_t>(N) * (m + 4) + hn_at + 1);
-  if (hproj_cap_ < hn_at + 1) {
+  const int nb = blocks(N, VA_THREADS);
+  const size_t hn_at = 2 * static_cast<size_t>(m + 1);  // projections of both passes, then the CTAs' shares of |w|^2
+  ensure_work(static_cast<size_t>(N) * (m + 4) + hn_at + nb);
+  if (hproj_cap_ < hn_at + nb) {
     if (hproj_) cudaFreeHost(hproj_);
     hproj_ = nullptr;
     hproj_cap_ = 0;
-    cuda_check(cudaMallocHost(&hproj_, (hn_at + 1) * sizeof(double)), "cudaMallocHost(projections)");
-    hproj_cap_ = hn_at + 1;
+    cuda_check(cudaMallocHost(&hproj_, (hn_at + nb) * sizeof(double)), "cudaMallocHost(projections)");
+    hproj_cap_ = hn_at + nb;
   }
   double* V = work_;  // m + 1 basis vectors
   double* w = work_ + static_cast<size_t>(N) * (m + 1);
   double* x = w + N;
   double* r = x + N;
-  double* dproj = r + N;  // [0, m+1): first pass, [m+1, 2m+2): second pass, [2m+2]: |w|^2
-  const int nb = blocks(N, VA_THREADS);
+  double* dproj = r + N;  // [0, m+1): first pass, [m+1, 2m+2): second pass, then |w|^2's shares
   auto copy_scaled = [&](const double* src, double alpha, double* dst) {
     scaled_copy<<<nb, VA_THREADS, 0, s>>>(N, alpha, src, dst, 0);
     ctx_->launches++;
@@ -3442,18 +3494,24 @@ void DenseLU::gmres_ir(double* b, int trans) {
     scaled_copy<<<nb, VA_THREADS, 0, s>>>(N, alpha, src, dst, 1);
     ctx_->launches++;
   };
+  auto host_norm = [&] {
+    double sum = 0.0;
+    for (int i = 0; i < nb; i++) sum += hproj_[hn_at + i];
+    return std::sqrt(sum);
+  };
   auto norm = [&](const double* v) {
-    sum_squares<<<1, VA_THREADS, 0, s>>>(v, N, dproj + hn_at);
+    sum_squares<<<nb, VA_THREADS, 0, s>>>(v, N, dproj + hn_at);
     ctx_->launches++;
-    cuda_check(cudaMemcpyAsync(hproj_ + hn_at, dproj + hn_at, sizeof(double), cudaMemcpyDeviceToHost, s),
+    cuda_check(cudaMemcpyAsync(hproj_ + hn_at, dproj + hn_at, nb * sizeof(double), cudaMemcpyDeviceToHost, s),
                "D2H norm");
     cuda_check(cudaStreamSynchronize(s), "sync norm");
-    return std::sqrt(hproj_[hn_at]);
+    return host_norm();
   };
   cuda_check(cudaMemsetAsync(x, 0, sizeof(double) * N, s), "memset x");
   const double bnorm = norm(b);
   if (bnorm == 0) return;
   int total_it = 0;
+  bool checked = false;
   for (int restart = 0; restart < gmres_restarts; restart++) {
     // r = b - A x (x = 0 on the first cycle: r = b, no matvec)
     if (restart == 0) {
@@ -3464,15 +3522,17 @@ void DenseLU::gmres_ir(double* b, int trans) {
     }
     const double beta = norm(r);
     stats.final_rel_residual = beta / bnorm;
-    if (beta / bnorm < gmres_tol) break;
+    if (beta / bnorm < gmres_tol) {
+      checked = true;  // of this very x
+      break;
+    }
     std::vector<double> H(static_cast<size_t>(m + 1) * m, 0.0), cs(m), sn(m), g(m + 1, 0.0);
     g[0] = beta;
     copy_scaled(r, 1.0 / beta, V);
     int k = 0;
     for (; k < m; k++) {
       // w = A M^-1 v_k
-      copy_scaled(V + static_cast<size_t>(k) * N, 1.0, r);
-      solve_f32(r, trans);
+      solve_f32(V + static_cast<size_t>(k) * N, r, trans);
       {
         ProfScope ps(ctx_, Context::PROF_GMRES, 8.0 * double(N) * N);
         gemv(r, w, 1.0, 0.0, nullptr, trans);
@@ -3481,16 +3541,14 @@ void DenseLU::gmres_ir(double* b, int trans) {
       const int kk = k + 1;
       for (int pass = 0; pass < 2; pass++) {
         double* h = dproj + static_cast<size_t>(pass) * (m + 1);
-        basis_dots<<<kk, VA_THREADS, 0, s>>>(V, N, kk, w, h);
-        basis_subtract<<<nb, VA_THREADS, 0, s>>>(V, N, kk, h, w);
+        basis_dots<<<kk, VD_THREADS, 0, s>>>(V, N, w, h);
+        basis_subtract<<<nb, VA_THREADS, 0, s>>>(V, N, kk, h, w, pass ? dproj + hn_at : nullptr);
         ctx_->launches += 2;
       }
-      sum_squares<<<1, VA_THREADS, 0, s>>>(w, N, dproj + hn_at);
-      ctx_->launches++;
-      cuda_check(cudaMemcpyAsync(hproj_, dproj, (hn_at + 1) * sizeof(double), cudaMemcpyDeviceToHost, s),
+      cuda_check(cudaMemcpyAsync(hproj_, dproj, (hn_at + nb) * sizeof(double), cudaMemcpyDeviceToHost, s),
                  "D2H projections");
       cuda_check(cudaStreamSynchronize(s), "sync projections");
-      const double hn = std::sqrt(hproj_[hn_at]);
+      const double hn = host_norm();
       for (int i = 0; i <= k; i++) H[static_cast<size_t>(i) * m + k] = hproj_[i] + hproj_[m + 1 + i];
       H[static_cast<size_t>(k + 1) * m + k] = hn;
       if (hn > 0) copy_scaled(w, 1.0 / hn, V + static_cast<size_t>(k + 1) * N);
@@ -3520,16 +3578,24 @@ void DenseLU::gmres_ir(double* b, int trans) {
       for (int j = i + 1; j < k; j++) sum -= H[i * m + j] * y[j];
       y[i] = sum / H[i * m + i];
     }
-    cuda_check(cudaMemsetAsync(r, 0, sizeof(double) * N, s), "memset r");
-    for (int i = 0; i < k; i++) add_scaled(V + static_cast<size_t>(i) * N, y[i], r);
-    solve_f32(r, trans);
+    if (k == 0) cuda_check(cudaMemsetAsync(w, 0, sizeof(double) * N, s), "memset w");
+    for (int i0 = 0; i0 < k; i0 += COMBINE_MAX) {
+      CombineCoefs c;
+      const int n = std::min(COMBINE_MAX, k - i0);
+      for (int i = 0; i < n; i++) c.c[i] = y[i0 + i];
+      basis_combine<<<nb, VA_THREADS, 0, s>>>(V + static_cast<size_t>(i0) * N, N, n, c, w, i0 > 0);
+      ctx_->launches++;
+    }
+    solve_f32(w, r, trans);
     add_scaled(r, 1.0, x);
   }
-  {
-    ProfScope ps(ctx_, Context::PROF_GMRES, 8.0 * double(N) * N);
-    gemv(x, r, -1.0, 1.0, b, trans);
+  if (!checked) {
+    {
+      ProfScope ps(ctx_, Context::PROF_GMRES, 8.0 * double(N) * N);
+      gemv(x, r, -1.0, 1.0, b, trans);
+    }
+    stats.final_rel_residual = norm(r) / bnorm;
   }
-  stats.final_rel_residual = norm(r) / bnorm;
   stats.refine_iters = total_it;
   cuda_check(cudaMemcpyAsync(b, x, sizeof(double) * N, cudaMemcpyDeviceToDevice, s), "copy x");
 }

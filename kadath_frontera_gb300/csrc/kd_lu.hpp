@@ -99,9 +99,10 @@ class DenseLU {
   void factor_fp64(double* A, long long ld, int N);
   void factor_f32(float* A, long long ld, int N, bool tf32);
   void solve_fp64(const double* LU, long long ld, int N, double* b, int trans);
-  void solve_f32(double* b, int trans = 0);  // applies the FP32 factors to an FP64 vector
+  void solve_f32(const double* b, double* x, int trans = 0);  // x = M^-1 b with the FP32 factors, FP64 vectors
   template <class T>
-  void tri_solve(const T* LU, long long ld, int N, double* b, int trans);
+  void tri_solve(const T* LU, long long ld, int N, const double* b, double* x, int trans, const double* bscale,
+                 const double* xscale);
   template <class T>
   void prepare_solves(const T* LU, long long ld, int N);
   void factor_f32_nopiv(float* A, long long ld, int N, bool tf32);
