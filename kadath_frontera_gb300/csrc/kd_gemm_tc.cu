@@ -260,14 +260,13 @@ __global__ void __launch_bounds__(TC_THREADS) tf32_update_kernel(const float* __
 // ---------------------------------------------------------------------------
 // Persistent, warp-specialised version (used when C allows TMA: 16-byte
 // aligned base, ldc a multiple of 4 floats).  One CTA per SM walks the
-// 128 x 128 tiles of C (tile t -> CTA t % grid):
+// 128 x 128 (or 128 x 256) tiles of C (tile t -> CTA t % grid):
 //   warp 0  producer: TMA loads of the tile's operand blocks (128-byte
-//           swizzled, K-major) and of C in 128 x 32 chunks through a ring of
-//           four shared-memory slots;
-//   warp 1  allocates 256 TMEM columns (two 128-column accumulators) and
-//           issues the MMAs of a tile into one accumulator while the
-//           epilogue drains the other;
-//   warps 2-5 epilogue: per C chunk, tcgen05.ld of 32 accumulator columns,
+//           swizzled, K-major); warp 6 those of C in chunks of 32 (16)
+//           columns through a ring of shared-memory slots;
+//   warp 1  allocates two accumulators in TMEM and issues the MMAs of a tile
+//           into one of them while the epilogue drains the other;
+//   warps 2-5 epilogue: per C chunk, tcgen05.ld of its accumulator columns,
 //           C -= acc in shared memory, TMA store of the chunk.
 // Every mbarrier wait gives up after GP_TC_WAIT_NS; the CTA then sets the
 // error flag, lets its roles fall out of their loops and frees its TMEM.
@@ -275,8 +274,8 @@ __global__ void __launch_bounds__(TC_THREADS) tf32_update_kernel(const float* __
 constexpr int P_THREADS = 224;
 constexpr int P_CSLOTS = 8;                              // most C chunks in flight
 constexpr int P_NST = 2;                                 // operand stages (one k-block each)
-constexpr int P_CCOLS = 32;                              // columns per C chunk
-constexpr int P_CHUNK_BYTES = TC_M * P_CCOLS * 4;        // 16 KiB
+// columns per C chunk: 16 KiB chunks, 8 KiB ones where the operands leave room for few
+__host__ __device__ constexpr int p_ccols(int tn) { return tn == 256 ? 16 : 32; }
 constexpr int P_OPBLK_BYTES = 128 * 128;                 // 128 rows x 32 TF32
 constexpr unsigned long long P_WAIT_NS = 2000000000ull;  // 2 s
 constexpr size_t P_MAX_SMEM = 226 * 1024;  // + 1 KiB static shared memory = the 227 KiB per-CTA limit
@@ -359,6 +358,10 @@ __device__ __forceinline__ void tf32_mma(uint32_t d, uint64_t ad, uint64_t bd, u
       "l"(ad), "l"(bd), "r"(idesc), "r"(accum));
 }
 
+// TN: columns of a tile, 128 or 256.  The wider tile reads a quarter less of the
+// operands for the same products (see the rule beside the launch); its two
+// accumulators fill the SM's 512 columns of tensor memory.
+template <int TN>
 __global__ void __launch_bounds__(P_THREADS, 1)
     tf32_update_persistent(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB,
                            const __grid_constant__ CUtensorMap mapAlo, const __grid_constant__ CUtensorMap mapBlo,
@@ -368,8 +371,11 @@ __global__ void __launch_bounds__(P_THREADS, 1)
   char* base = reinterpret_cast<char*>((reinterpret_cast<uintptr_t>(p_raw) + 1023) & ~uintptr_t(1023));
   // P_NST operand stages, each one k-block of A, B (and their lo parts):
   // the k-blocks of consecutive tiles stream through them
-  const int nplanes = split3 ? 4 : 2;
-  const int stage_bytes = nplanes * P_OPBLK_BYTES;
+  constexpr int CC = p_ccols(TN), CB = TC_M * CC * 4;
+  constexpr int NB = TN / 128;                        // 128-row blocks of a B tile
+  constexpr int HALF = (1 + NB) * P_OPBLK_BYTES;      // A and B of one part
+  static_assert(TN % 128 == 0 && TC_N == 128, "B tiles are whole 128-row boxes");
+  const int stage_bytes = (split3 ? 2 : 1) * HALF;
   char* sC = base + P_NST * stage_bytes;  // ring of ncs C chunks
   __shared__ uint64_t op_full[P_NST], op_empty[P_NST], acc_full[2], acc_empty[2], c_full[P_CSLOTS],
       c_empty[P_CSLOTS];
@@ -400,7 +406,7 @@ __global__ void __launch_bounds__(P_THREADS, 1)
   }
   if (warp == 1) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base_sh)),
-                 "r"(256));
+                 "r"(2 * TN));
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -422,10 +428,14 @@ __global__ void __launch_bounds__(P_THREADS, 1)
           char* sp = base + st * stage_bytes;
           p_expect_tx(&op_full[st], static_cast<uint32_t>(stage_bytes));
           p_tma_load(sp, &mapA, kb * TC_KBLK, tm * TC_M, &op_full[st]);
-          p_tma_load(sp + P_OPBLK_BYTES, &mapB, kb * TC_KBLK, tn * TC_N, &op_full[st]);
+#pragma unroll
+          for (int q = 0; q < NB; q++)
+            p_tma_load(sp + (1 + q) * P_OPBLK_BYTES, &mapB, kb * TC_KBLK, tn * TN + q * 128, &op_full[st]);
           if (split3) {
-            p_tma_load(sp + 2 * P_OPBLK_BYTES, &mapAlo, kb * TC_KBLK, tm * TC_M, &op_full[st]);
-            p_tma_load(sp + 3 * P_OPBLK_BYTES, &mapBlo, kb * TC_KBLK, tn * TC_N, &op_full[st]);
+            p_tma_load(sp + HALF, &mapAlo, kb * TC_KBLK, tm * TC_M, &op_full[st]);
+#pragma unroll
+            for (int q = 0; q < NB; q++)
+              p_tma_load(sp + HALF + (1 + q) * P_OPBLK_BYTES, &mapBlo, kb * TC_KBLK, tn * TN + q * 128, &op_full[st]);
           }
         }
       }
@@ -436,21 +446,21 @@ __global__ void __launch_bounds__(P_THREADS, 1)
       int cchunk = 0;
       for (int tile = blockIdx.x; tile < ntiles && !*abort_v; tile += gridDim.x) {
         const int tm = tile % ntm, tn = tile / ntm;
-        for (int ch = 0; ch < TC_N / P_CCOLS; ch++, cchunk++) {
+        for (int ch = 0; ch < TN / CC; ch++, cchunk++) {
           const int slot = cchunk % ncs, use = cchunk / ncs;
           if (use > 0 && !p_wait(&c_empty[slot], (use - 1) & 1)) {
             *abort_v = 1;
             break;
           }
-          p_expect_tx(&c_full[slot], P_CHUNK_BYTES);
-          p_tma_load_stream(sC + slot * P_CHUNK_BYTES, &mapC, tm * TC_M, tn * TC_N + ch * P_CCOLS, &c_full[slot],
+          p_expect_tx(&c_full[slot], CB);
+          p_tma_load_stream(sC + slot * CB, &mapC, tm * TC_M, tn * TN + ch * CC, &c_full[slot],
                             pol);
         }
       }
     }
   } else if (warp == 1) {
     if (lane == 0) {  // ------------------------------------------- MMA issuer
-      const uint32_t idesc = tf32_idesc(TC_M, TC_N);
+      const uint32_t idesc = tf32_idesc(TC_M, TN);
       int it = 0, g = 0;
       for (int tile = blockIdx.x; tile < ntiles && !*abort_v; tile += gridDim.x, it++) {
         const int acc = it & 1, use = it >> 1;
@@ -458,7 +468,7 @@ __global__ void __launch_bounds__(P_THREADS, 1)
           *abort_v = 1;
           break;
         }
-        const uint32_t d = tmem + static_cast<uint32_t>(acc * TC_N);
+        const uint32_t d = tmem + static_cast<uint32_t>(acc * TN);
         bool ok = true;
         for (int kb = 0; kb < nkb; kb++, g++) {
           const int st = g % P_NST;
@@ -474,8 +484,8 @@ __global__ void __launch_bounds__(P_THREADS, 1)
             const uint64_t bd = sw128_desc(sp + P_OPBLK_BYTES) + koff;
             uint32_t accum = (kb | k) ? 1u : 0u;
             if (split3) {  // small terms first: lo*hi, hi*lo, then hi*hi
-              const uint64_t ald = sw128_desc(sp + 2 * P_OPBLK_BYTES) + koff;
-              const uint64_t bld = sw128_desc(sp + 3 * P_OPBLK_BYTES) + koff;
+              const uint64_t ald = sw128_desc(sp + HALF) + koff;
+              const uint64_t bld = sw128_desc(sp + HALF + P_OPBLK_BYTES) + koff;
               tf32_mma(d, ald, bd, idesc, accum);
               tf32_mma(d, ad, bld, idesc, 1u);
               accum = 1u;
@@ -509,16 +519,16 @@ __global__ void __launch_bounds__(P_THREADS, 1)
       asm volatile("bar.sync 1, 128;" ::: "memory");
       if (epi_abort) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      for (int ch = 0; ch < TC_N / P_CCOLS; ch++, cchunk++) {
+      for (int ch = 0; ch < TN / CC; ch++, cchunk++) {
         const int slot = cchunk % ncs;
         if (et == 0 && !p_wait(&c_full[slot], (cchunk / ncs) & 1)) epi_abort = 1;
         asm volatile("bar.sync 1, 128;" ::: "memory");
         if (epi_abort) break;
-        float* cs = reinterpret_cast<float*>(sC + slot * P_CHUNK_BYTES);  // [column][row]
-        for (int c16 = 0; c16 < P_CCOLS; c16 += 16) {
+        float* cs = reinterpret_cast<float*>(sC + slot * CB);  // [column][row]
+        for (int c16 = 0; c16 < CC; c16 += 16) {
           uint32_t r[16];
           const uint32_t taddr = tmem + (static_cast<uint32_t>(quarter * 32) << 16) +
-                                 static_cast<uint32_t>(acc * TC_N + ch * P_CCOLS + c16);
+                                 static_cast<uint32_t>(acc * TN + ch * CC + c16);
           asm volatile(
               "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, "
               "[%16];"
@@ -534,14 +544,14 @@ __global__ void __launch_bounds__(P_THREADS, 1)
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
         asm volatile("bar.sync 1, 128;" ::: "memory");
         if (et == 0) {
-          p_tma_store_stream(&mapC, cs, tm * TC_M, tn * TC_N + ch * P_CCOLS, p_evict_first());
+          p_tma_store_stream(&mapC, cs, tm * TC_M, tn * TN + ch * CC, p_evict_first());
           asm volatile("cp.async.bulk.commit_group;" ::: "memory");
           // one store stays in flight: the previous chunk's slot is free
           // once its store has read it
           asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
           if (pend_slot >= 0) p_arrive(&c_empty[pend_slot]);
           pend_slot = slot;
-          if (ch == TC_N / P_CCOLS - 1) p_arrive(&acc_empty[acc]);  // all 128 threads are past their loads
+          if (ch == TN / CC - 1) p_arrive(&acc_empty[acc]);  // all 128 threads are past their loads
         }
       }
       if (epi_abort) break;
@@ -556,7 +566,7 @@ __global__ void __launch_bounds__(P_THREADS, 1)
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(256));
+  if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(2 * TN));
 }
 
 // 2-D FP32 tensor map: inner extent `inner` (contiguous), `outer` rows
@@ -573,13 +583,6 @@ void make_map(CUtensorMap* m, const void* ptr, long long inner, long long outer,
                   CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE,
                   CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) throw KdError(KD_ERR_CUDA, "cuTensorMapEncodeTiled failed (" + std::to_string(r) + ")");
-}
-
-
-int grid_for(long long n) {
-  long long g = (n + 255) / 256;
-  if (g > 152 * 8) g = 152 * 8;
-  return static_cast<int>(g < 1 ? 1 : g);
 }
 
 }  // namespace
@@ -610,9 +613,12 @@ int tf32_update_max_clusters16() {
   static int maxc = 0;
   static std::once_flag once;
   std::call_once(once, [] {
-    if (cudaFuncSetAttribute(tf32_update_persistent, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
-        cudaFuncSetAttribute(tf32_update_persistent, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             static_cast<int>(P_MAX_SMEM)) != cudaSuccess) {
+    auto prepare = [](auto* kernel) {
+      return cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+             cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  static_cast<int>(P_MAX_SMEM)) == cudaSuccess;
+    };
+    if (!prepare(tf32_update_persistent<128>) || !prepare(tf32_update_persistent<256>)) {
       cudaGetLastError();
       return;
     }
@@ -628,11 +634,22 @@ int tf32_update_max_clusters16() {
     q.attrs = qa;
     q.numAttrs = 1;
     int n = 0;
-    if (cudaOccupancyMaxActiveClusters(&n, tf32_update_persistent, &q) == cudaSuccess) maxc = n;
+    if (cudaOccupancyMaxActiveClusters(&n, tf32_update_persistent<256>, &q) == cudaSuccess) maxc = n;
     cudaGetLastError();
   });
   return maxc;
 }
+
+// When an update takes 256-column tiles: 3xTF32 with k above 128 on the whole
+// GPU, with at least two tiles an SM.  There the operands' way from L2 is the
+// bound (85 KB a k-block and 128 x 128 tile, C included, against 826 cycles of
+// MMA), and the wider tile needs a quarter less of them: all updates of 40,081
+// rows 294 -> 253 ms.  Its operand stages leave 32 KB for C, four chunks of 16
+// columns (two of 32: 340 ms).  With k = 96 C's stream is the bound and wants
+// the longer ring; as clusters on 112 SMs beside a panel L2 serves fewer SMs,
+// and the wider tile loses (12,331 rows in a reused order 15.9 -> 16.8 ms).
+constexpr int WIDE_MIN_K = 128;
+constexpr int WIDE_MIN_WAVES = 2;
 
 void tf32_gemm_update(Context* ctx, int m, int n, int k, const float* A, long long lda, const float* B, long long ldb,
                       float* C, long long ldc, int c_rows_writable, int terms, int clusters, int max_ctas) {
@@ -676,25 +693,35 @@ void tf32_gemm_update(Context* ctx, int m, int n, int k, const float* A, long lo
     make_map(&mB, bt, kpad, npad, static_cast<long long>(kpad) * 4, TC_KBLK, TC_N, true);
     make_map(&mAl, at_lo, kpad, mpad, static_cast<long long>(kpad) * 4, TC_KBLK, TC_M, true);
     make_map(&mBl, bt_lo, kpad, npad, static_cast<long long>(kpad) * 4, TC_KBLK, TC_N, true);
-    make_map(&mC, C, m, n, ldc * 4, TC_M, P_CCOLS, false);
+    
     static int nsm = 0;
     static std::once_flag pattr;
     std::call_once(pattr, [] {
       int dev = 0;
       cuda_check(cudaGetDevice(&dev), "cudaGetDevice");
       cuda_check(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev), "SM count");
-      cuda_check(cudaFuncSetAttribute(tf32_update_persistent, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      static_cast<int>(P_MAX_SMEM)),
-                 "cudaFuncSetAttribute(tf32 persistent)");
+      for (auto* kernel : {tf32_update_persistent<128>, tf32_update_persistent<256>})
+        cuda_check(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                        static_cast<int>(P_MAX_SMEM)),
+                   "cudaFuncSetAttribute(tf32 persistent)");
     });
+    const int ntm = mpad / TC_M;
+    const int cap_sms = ctx->sms() < nsm ? ctx->sms() : nsm;
+    const bool wide = split3 && clusters == 0 && kpad > WIDE_MIN_K && n >= 1024 &&
+                      static_cast<long long>(ntm) * ((n + 255) / 256) >= WIDE_MIN_WAVES * cap_sms;
+    const int tn = wide ? 256 : TC_N;
+    const int ccols = p_ccols(tn), chunk_bytes = TC_M * ccols * 4;
+    make_map(&mC, C, m, n, ldc * 4, TC_M, ccols, false);
+    auto* kernel = wide ? tf32_update_persistent<256> : tf32_update_persistent<128>;
     // shared memory: P_NST operand stages of one k-block each (x2 for the
     // lo parts), then as many C chunks as fit, up to P_CSLOTS
-    const size_t ops = static_cast<size_t>(P_NST) * (split3 ? 4 : 2) * P_OPBLK_BYTES;
-    int ncs = static_cast<int>((P_MAX_SMEM - 1024 - ops) / P_CHUNK_BYTES);
+    const size_t ops = static_cast<size_t>(P_NST) * (split3 ? 2 : 1) * (1 + tn / 128) * P_OPBLK_BYTES;
+    int ncs = static_cast<int>((P_MAX_SMEM - 1024 - ops) / chunk_bytes);
     if (ncs > P_CSLOTS) ncs = P_CSLOTS;
-    const size_t psmem = 1024 + ops + static_cast<size_t>(ncs) * P_CHUNK_BYTES;
-    if (psmem > P_MAX_SMEM) throw KdError(KD_ERR_UNSUPPORTED, "tcgen05 update: operands do not fit in shared memory");
-    const int ntm = mpad / TC_M, ntiles = ntm * (npad / TC_N);
+    const size_t psmem = 1024 + ops + static_cast<size_t>(ncs) * chunk_bytes;
+    if (psmem > P_MAX_SMEM || ncs < 2)
+      throw KdError(KD_ERR_UNSUPPORTED, "tcgen05 update: operands do not fit in shared memory");
+    const int ntiles = ntm * ((n + tn - 1) / tn);
     const int maxc = clusters ? tf32_update_max_clusters16() : 0;
     if (maxc >= 2) {
       // 16-CTA clusters (the CTAs share nothing): one fewer than fit, or all
@@ -713,16 +740,16 @@ void tf32_gemm_update(Context* ctx, int m, int n, int k, const float* A, long lo
       at[0].val.clusterDim.z = 1;
       cfg.attrs = at;
       cfg.numAttrs = 1;
-      cuda_check(cudaLaunchKernelEx(&cfg, tf32_update_persistent, mA, mB, mAl, mBl, mC, nkb, ntm, ntiles,
+      cuda_check(cudaLaunchKernelEx(&cfg, kernel, mA, mB, mAl, mBl, mC, nkb, ntm, ntiles,
                                     split3 ? 1 : 0, ncs, err),
                  "tcgen05 trailing update (clusters)");
       ctx->launches += 1;
       return;
     }
-    int cap = ctx->sms() < nsm ? ctx->sms() : nsm;
+    int cap = cap_sms;
     if (max_ctas > 0 && max_ctas < cap) cap = max_ctas;
     const int grid = ntiles < cap ? ntiles : cap;
-    tf32_update_persistent<<<grid, P_THREADS, psmem, s>>>(mA, mB, mAl, mBl, mC, nkb, ntm, ntiles, split3 ? 1 : 0, ncs,
+    kernel<<<grid, P_THREADS, psmem, s>>>(mA, mB, mAl, mBl, mC, nkb, ntm, ntiles, split3 ? 1 : 0, ncs,
                                                           err);
     ctx->launches += 1;
     cuda_check(cudaGetLastError(), "tcgen05 trailing update (persistent)");
