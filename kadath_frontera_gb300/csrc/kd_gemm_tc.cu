@@ -266,12 +266,16 @@ __global__ void __launch_bounds__(TC_THREADS) tf32_update_kernel(const float* __
 //           columns through a ring of shared-memory slots;
 //   warp 1  allocates two accumulators in TMEM and issues the MMAs of a tile
 //           into one of them while the epilogue drains the other;
-//   warps 2-5 epilogue: per C chunk, tcgen05.ld of its accumulator columns,
-//           C -= acc in shared memory, TMA store of the chunk.
+//   warps 2-5 and 7-10 epilogue: per C chunk, tcgen05.ld of its accumulator
+//           columns, C -= acc in shared memory, TMA store of the chunk.  A chunk
+//           takes its group about 600 cycles and 33 a column, waits and barriers
+//           mostly, which one group could not hide behind a wide tile's MMAs.
 // Every mbarrier wait gives up after GP_TC_WAIT_NS; the CTA then sets the
 // error flag, lets its roles fall out of their loops and frees its TMEM.
-// warps: 0 operand producer, 1 MMA issuer, 2-5 epilogue, 6 C producer
-constexpr int P_THREADS = 224;
+// warps: 0 operand producer, 1 MMA issuer, 2-5 epilogue, 6 C producer, 7-10
+// second epilogue group
+constexpr int P_THREADS = 352;
+constexpr int P_EPI = 2;  // epilogue groups of four warps, taking the C chunks in turn
 constexpr int P_CSLOTS = 8;                              // most C chunks in flight
 constexpr int P_NST = 2;                                 // operand stages (one k-block each)
 // columns per C chunk: 16 KiB chunks, 8 KiB ones where the operands leave room for few
@@ -380,20 +384,20 @@ __global__ void __launch_bounds__(P_THREADS, 1)
   __shared__ uint64_t op_full[P_NST], op_empty[P_NST], acc_full[2], acc_empty[2], c_full[P_CSLOTS],
       c_empty[P_CSLOTS];
   __shared__ uint32_t tmem_base_sh;
-  __shared__ int abort_flag, epi_abort;
+  __shared__ int abort_flag, epi_abort[P_EPI];
   volatile int* abort_v = &abort_flag;  // written by one role, polled by the others
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
   if (threadIdx.x == 0) {
     abort_flag = 0;
-    epi_abort = 0;
+    for (int i = 0; i < P_EPI; i++) epi_abort[i] = 0;
     for (int i = 0; i < P_NST; i++) {
       asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&op_full[i])));
       asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&op_empty[i])));
     }
     for (int i = 0; i < 2; i++) {
       asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&acc_full[i])));
-      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&acc_empty[i])));
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(&acc_empty[i])), "n"(P_EPI));
     }
     for (int i = 0; i < P_CSLOTS; i++) {
       asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&c_full[i])));
@@ -506,24 +510,29 @@ __global__ void __launch_bounds__(P_THREADS, 1)
                      : "memory");
       }
     }
-  } else {  // ---------------------------------------------- epilogue (2-5)
-    const int et = threadIdx.x - 64;      // 0..127
-    const int quarter = warp & 3;         // TMEM lanes this warp may read
-    const int row = quarter * 32 + lane;  // tile row
-    int it = 0, cchunk = 0;
-    int pend_slot = -1;  // slot whose TMA store may still be reading it (thread et == 0)
+  } else {  // ------------------------------------- epilogue (2-5 and 7-10)
+    const int grp = warp > 6 ? 1 : 0;
+    const int et = threadIdx.x - (grp ? 224 : 64);  // 0..127
+    const int quarter = warp & 3;                   // TMEM lanes this warp may read
+    const int row = quarter * 32 + lane;            // tile row
+    volatile int* out_v = &epi_abort[grp];          // this group's own, so that its threads leave together
+    auto group_sync = [&] { asm volatile("bar.sync %0, 128;" ::"r"(1 + grp) : "memory"); };
+    int it = 0;
+    constexpr int CHUNKS = TN / CC;
+    static_assert(CHUNKS % P_EPI == 0, "a group's chunks are the same in every tile");
     for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x, it++) {
       const int tm = tile % ntm, tn = tile / ntm;
       const int acc = it & 1;
-      if (et == 0 && (*abort_v || !p_wait(&acc_full[acc], (it >> 1) & 1))) epi_abort = 1;
-      asm volatile("bar.sync 1, 128;" ::: "memory");
-      if (epi_abort) break;
+      if (et == 0 && (*abort_v || !p_wait(&acc_full[acc], (it >> 1) & 1))) *out_v = 1;
+      group_sync();
+      if (*out_v) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      for (int ch = 0; ch < TN / CC; ch++, cchunk++) {
+      for (int ch = grp; ch < CHUNKS; ch += P_EPI) {
+        const int cchunk = it * CHUNKS + ch;
         const int slot = cchunk % ncs;
-        if (et == 0 && !p_wait(&c_full[slot], (cchunk / ncs) & 1)) epi_abort = 1;
-        asm volatile("bar.sync 1, 128;" ::: "memory");
-        if (epi_abort) break;
+        if (et == 0 && !p_wait(&c_full[slot], (cchunk / ncs) & 1)) *out_v = 1;
+        group_sync();
+        if (*out_v) break;
         float* cs = reinterpret_cast<float*>(sC + slot * CB);  // [column][row]
         for (int c16 = 0; c16 < CC; c16 += 16) {
           uint32_t r[16];
@@ -542,27 +551,22 @@ __global__ void __launch_bounds__(P_THREADS, 1)
         // generic-proxy writes -> visible to the TMA store
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-        asm volatile("bar.sync 1, 128;" ::: "memory");
+        group_sync();
         if (et == 0) {
           p_tma_store_stream(&mapC, cs, tm * TC_M, tn * TN + ch * CC, p_evict_first());
           asm volatile("cp.async.bulk.commit_group;" ::: "memory");
-          // one store stays in flight: the previous chunk's slot is free
-          // once its store has read it
-          asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
-          if (pend_slot >= 0) p_arrive(&c_empty[pend_slot]);
-          pend_slot = slot;
-          if (ch == TN / CC - 1) p_arrive(&acc_empty[acc]);  // all 128 threads are past their loads
+          if (ch + P_EPI >= CHUNKS) p_arrive(&acc_empty[acc]);  // all 128 threads are past their loads
+          // the slot is free once the store has read it; the other group works meanwhile
+          asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+          p_arrive(&c_empty[slot]);
         }
       }
-      if (epi_abort) break;
+      if (*out_v) break;
     }
-    if (et == 0) {
-      asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
-      if (pend_slot >= 0) p_arrive(&c_empty[pend_slot]);
-    }
+    if (et == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
   }
   __syncthreads();
-  if (threadIdx.x == 0 && (*abort_v || epi_abort)) atomicExch(err, 1);
+  if (threadIdx.x == 0 && (*abort_v || epi_abort[0] || epi_abort[1])) atomicExch(err, 1);
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -640,14 +644,15 @@ int tf32_update_max_clusters16() {
   return maxc;
 }
 
-// When an update takes 256-column tiles: 3xTF32 with k above 128 on the whole
-// GPU, with at least two tiles an SM.  There the operands' way from L2 is the
-// bound (85 KB a k-block and 128 x 128 tile, C included, against 826 cycles of
-// MMA), and the wider tile needs a quarter less of them: all updates of 40,081
-// rows 294 -> 253 ms.  Its operand stages leave 32 KB for C, four chunks of 16
-// columns (two of 32: 340 ms).  With k = 96 C's stream is the bound and wants
-// the longer ring; as clusters on 112 SMs beside a panel L2 serves fewer SMs,
-// and the wider tile loses (12,331 rows in a reused order 15.9 -> 16.8 ms).
+// When an update takes 256-column tiles: 3xTF32 with k above 128 and at least
+// two tiles an SM.  There the operands' way from L2 is the bound (85 KB a k-block
+// and 128 x 128 tile, C included, against 826 cycles of MMA), and the wider tile
+// needs a quarter less of them: all updates of 40,081 rows 294 -> 234 ms, the
+// factorisation of 12,331 rows in a reused order, whose updates run as clusters
+// on 112 SMs beside the panels, 16.0 -> 15.75 ms.  Its operand stages leave 32 KB
+// for C: four chunks of 16 columns (two of 32: 340 ms, eight of 8: 360 ms, both
+// with one epilogue group, which with four of 16 took 253 ms).  With k = 96 C's
+// stream is the bound and wants the longer ring.
 constexpr int WIDE_MIN_K = 128;
 constexpr int WIDE_MIN_WAVES = 2;
 
@@ -707,7 +712,7 @@ void tf32_gemm_update(Context* ctx, int m, int n, int k, const float* A, long lo
     });
     const int ntm = mpad / TC_M;
     const int cap_sms = ctx->sms() < nsm ? ctx->sms() : nsm;
-    const bool wide = split3 && clusters == 0 && kpad > WIDE_MIN_K && n >= 1024 &&
+    const bool wide = split3 && kpad > WIDE_MIN_K && n >= 1024 &&
                       static_cast<long long>(ntm) * ((n + 255) / 256) >= WIDE_MIN_WAVES * cap_sms;
     const int tn = wide ? 256 : TC_N;
     const int ccols = p_ccols(tn), chunk_bytes = TC_M * ccols * 4;
@@ -718,8 +723,9 @@ void tf32_gemm_update(Context* ctx, int m, int n, int k, const float* A, long lo
     const size_t ops = static_cast<size_t>(P_NST) * (split3 ? 2 : 1) * (1 + tn / 128) * P_OPBLK_BYTES;
     int ncs = static_cast<int>((P_MAX_SMEM - 1024 - ops) / chunk_bytes);
     if (ncs > P_CSLOTS) ncs = P_CSLOTS;
+    ncs -= ncs % P_EPI;  // a group's chunks keep to its own slots
     const size_t psmem = 1024 + ops + static_cast<size_t>(ncs) * chunk_bytes;
-    if (psmem > P_MAX_SMEM || ncs < 2)
+    if (psmem > P_MAX_SMEM || ncs < P_EPI)
       throw KdError(KD_ERR_UNSUPPORTED, "tcgen05 update: operands do not fit in shared memory");
     const int ntiles = ntm * ((n + tn - 1) / tn);
     const int maxc = clusters ? tf32_update_max_clusters16() : 0;
