@@ -1354,10 +1354,11 @@ __device__ __forceinline__ DF df_add(DF a, DF b) {
 
 // ---- triangular sweeps -----------------------------------------------------
 // Block k of the solution, x_k = Dinv_k (b_k - sum_i T_ki x_i) over the
-// 64-row blocks i before k in sweep order.  Finished blocks are announced
-// through one progress counter (release max by the producer, acquire loads
-// by the consumers), the number of sweep positions whose x is in y.  Every
-// wait is bounded by wait_ns: on timeout the CTA sets *err and leaves.
+// 64-row blocks i before k in sweep order.  With FP64 factors finished blocks
+// are announced through one progress counter (release max by the producer,
+// acquire loads by the consumers), the number of sweep positions whose x is in
+// y; with FP32 factors x is its own signal.  Every wait is bounded by wait_ns:
+// on timeout the CTA sets *err and leaves.
 __device__ __forceinline__ unsigned ld_acquire_u32(const unsigned* p) {
   unsigned v;
   asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
@@ -3257,9 +3258,9 @@ void DenseLU::factor(double* A, long long ld, int N, int mode) {
   stats.static_pivots = nopiv_ ? 1 : 0;
 }
 
-// Triangular solves by 64-row blocks with precomputed inverses of the
-// diagonal blocks: one launch per block computes the block's unknowns as a
-// small GEMV and subtracts their contribution from the remaining rows.
+// x = xscale (LU)^-1 (bscale b), or with the transposed factors: two sweeps,
+// one launch each, and the pivot order's permutation.  Scales null: 1 (FP64
+// factors: always).
 template <class T>
 void DenseLU::tri_solve(const T* LU, long long ld, int N, const double* b, double* x, int trans, const double* bscale,
                         const double* xscale) {

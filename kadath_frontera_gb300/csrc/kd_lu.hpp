@@ -115,9 +115,9 @@ class DenseLU {
   int pivoted_iters_ = 1000;  // refinement iterations with the last pivoted factors
   double* bsave_ = nullptr;   // right-hand side kept for a re-solve
   size_t bsave_cap_ = 0;
-  double* dinv_l_ = nullptr;  // inverses of the 64 x 64 diagonal blocks
+  double* dinv_l_ = nullptr;  // inverses of the 64 x 64 diagonal blocks (FP64 factors)
   double* dinv_u_ = nullptr;
-  float2* dinv2_l_ = nullptr;  // the same as (hi, lo) FP32 pairs (sweeps with FP32 factors)
+  float2* dinv2_l_ = nullptr;  // the same as (hi, lo) FP32 pairs (FP32 factors)
   float2* dinv2_u_ = nullptr;
   size_t dinv_cap_ = 0;
   float2* group_x_l_ = nullptr;  // off-diagonal blocks of the inverses of the 192-row groups (FP32 factors)
