@@ -1,6 +1,7 @@
 // Trailing update of the FP64 LU, C -= A * B, on the tcgen05 tensor cores by
 // exact products of 8-bit slices (the error-free splitting of Ozaki, Ogita,
-// Oishi and Rump, Numer. Algorithms 59, 2012, in fixed point).
+// Oishi and Rump, Numer. Algorithms 59, 2012, in fixed point), entry by entry
+// only where that loses nothing against a product in FP64.
 //
 // This GPU's FP64 pipe gives 1.1 TFLOP/s; its bf16 tensor cores 1,700 times
 // that.  Each operand entry becomes a 62-bit fixed-point number F relative to
@@ -8,31 +9,48 @@
 // s = 1..8, with d_s in [-128, 127]: eight bf16 matrices of integers.  The
 // product of slices i and j has integer entries, summed exactly in FP32: an
 // order o = i + j adds at most 8 pairs of k <= 128 products below 2^14, at
-// most 2^24 in all.  Orders 2..9 (36 of the 64 pairs) are kept, the rest is
-// below 2^-60 of the largest product.  Before splitting, row k of B is scaled
-// by a power of two to a largest entry in [1/2, 1) and column k of A by its
-// inverse, so that rows of B of very different sizes (a Jacobian's second
-// derivatives beside its boundary rows) do not cost each other digits.  The
-// split entries are off by 2^-63 of their row's largest one, against the
-// 2^-53 of every rounding of an FP64 product, and a tile's entry is rounded
-// twice (its 60-bit sum to double, the subtraction from C).
+// most 2^24 in all.  Orders 2..9 (36 of the 64 pairs) are kept.  Before
+// splitting, row k of B is scaled by a power of two to a largest entry in
+// [1/2, 1) and column k of A by its inverse, so that rows of B of very different
+// sizes (a Jacobian's second derivatives beside its boundary rows) do not cost
+// each other digits.
+//
+// Error.  With R the bound 2^(row's scale + column's scale) of the products of
+// an entry, the orders left out and the rounding of the digits come to about
+// 2^-59 R (96 random digits; the 2^-63 of each entry's last digit is less), and
+// the sum is rounded to FP64 once.  An FP64 product errs by about 2^-53 of
+// sum_k |a_k b_k|, and the subtraction by 2^-53 of the result, so an entry is
+// taken from the slices only where one of the two is at least 2^-4 R or so:
+//   three or more k have |a_k| >= 2^-3 and |b_k| >= 2^-3 of their row's and
+//   column's scale (bit masks made while packing), or
+//   the sum itself, or the updated entry, is at least 2^-4 R in size.
+// Every other entry, and every entry of a row or column with Inf or NaN, is left
+// as it is and listed, and sum_listed forms it in FP64, term by term in the order
+// of k over the k that are nonzero in both operands, as a plain product would.
+// Unknowns in different units need that: where one row of B is small in every
+// column but those of its own group, the sums in that group's columns are far
+// below R (groups 40 binades apart: componentwise backward errors of 1e-8 to 1e-2
+// with the slices alone, 7e-16 now and with LAPACK).  Sparse Jacobians too: of the
+// star's entries 0.4 % (index notation) to 2.4 % are listed.
 //
 // One persistent CTA per SM, 128 x 64 tiles:
 //   warp 0   TMA loads of operand chunks: k = 32 of all eight slices of A and
 //            B (96 KB, 64-byte swizzle), two stages;
 //   warp 1   72 MMAs per chunk (M 128, N 64, K 16) into eight accumulators of
 //            64 TMEM columns, one per order: all 512 columns;
-//   warps 2-9 epilogue: the eight orders of an entry into one 64-bit integer,
-//            TMEM released, then C -= integer * 2^e (one conversion and one
-//            multiply-add on the FP64 pipe) beside the next tile's MMAs.
+//   warps 2-9 epilogue: the eight orders of an entry into one 64-bit integer
+//            (shifted by its size: the low orders are kept whole where they
+//            reach its first 53 bits), TMEM released, then C -= integer * 2^e
+//            (one conversion and one multiply-add on the FP64 pipe) beside the
+//            next tile's MMAs, and the list of the entries to sum in FP64.
 // Bound: the MMAs' operand reads from shared memory (48 cycles per MMA of 32)
 // and the hand-over of the single set of accumulators.  128 x 64 tiles and not
 // 128 x 128: eight orders of 64 columns are all of TMEM, and one pass over the
 // operands serves all of them.
-// All updates of a factorisation, this kernel with its packing against the
-// library's FP64 GEMM: N = 8,000 19.7 against 319 ms (17 TFLOP/s of FP64
-// products), N = 12,331 64 against 1,173 ms; relative residuals of the solves
-// 1.2e-15 and 1.4e-15 with either.
+// All updates of a factorisation of the star's Jacobian, with packing and the
+// listed entries, against the library's FP64 GEMM: N = 7,819 24 (index notation)
+// and 30 against 301 ms, N = 12,331 97 against 1,172 ms; without the listed
+// entries 20 and 62 ms.
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -59,27 +77,38 @@ constexpr size_t S_SMEM = 1024 + static_cast<size_t>(S_NST) * S_STAGE;
 constexpr unsigned long long S_WAIT_NS = 2000000000ull;
 constexpr int EXP_NONFINITE = 1 << 20;                   // scale of a row or column that holds Inf or NaN
 constexpr int EXP_ZERO = -(1 << 20);                     // scale of a zero row or column
+constexpr int NEAR = 2;                                  // binades below the scale that count as large
+constexpr int NEAR_TERMS = 3;                            // large products that make a sum safe
+constexpr int SAFE_BITS = 4;                             // binades below R of a safe sum or result
+constexpr int MASK_WORDS = S_MAXK / 32;
+
+// Bit of k in a mask, so that a warp's ballots over two k a lane are its words:
+// word 2 (k / 64) + k % 2, bit (k % 64) / 2.  A row or column has two masks: of
+// its large entries, then of its nonzero ones.
+static_assert(S_MAXK == 128 && MASK_WORDS == 4, "two 64-wide halves, two words each");
 
 __device__ __forceinline__ uint32_t smem_addr(const void* p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
 
-// Smallest E with |v| < 2^E; EXP_ZERO for zero (and subnormals, which are
-// taken as zero), EXP_NONFINITE for Inf and NaN.
+// Smallest E with |v| < 2^E; EXP_ZERO for zero, EXP_NONFINITE for Inf and NaN.
 __device__ __forceinline__ int exponent_of(double v) {
-  const int e = static_cast<int>((static_cast<unsigned long long>(__double_as_longlong(v)) >> 52) & 0x7ff);
-  if (e == 0) return EXP_ZERO;
+  const unsigned long long b = static_cast<unsigned long long>(__double_as_longlong(v)) & 0x7fffffffffffffffull;
+  const int e = static_cast<int>(b >> 52);
   if (e == 0x7ff) return EXP_NONFINITE;
-  return e - 1022;
+  if (e != 0) return e - 1022;
+  return b ? -1010 - __clzll(static_cast<long long>(b)) : EXP_ZERO;  // subnormal: b 2^-1074
 }
 
 // v * 2^(62 - scale) rounded to an integer, for |v| < 2^scale.
 __device__ __forceinline__ long long fixed_point(double v, int scale) {
   const unsigned long long b = static_cast<unsigned long long>(__double_as_longlong(v));
-  const int e = static_cast<int>((b >> 52) & 0x7ff);
-  if (e == 0 || e == 0x7ff) return 0;
-  const unsigned long long m = ((b & 0xfffffffffffffull) | 0x10000000000000ull) << 9;
-  const int shift = scale - (e - 1022);
+  const int e = exponent_of(v);
+  if (e == EXP_ZERO || e == EXP_NONFINITE) return 0;
+  unsigned long long m = b & 0xfffffffffffffull;
+  if (e > -1022) m |= 0x10000000000000ull;
+  m <<= __clzll(static_cast<long long>(m)) - 2;  // first bit to place 61
+  const int shift = scale - e;
   long long f;
   if (shift <= 0) f = static_cast<long long>(m);  // shift is never negative
   else if (shift > 62) f = 0;
@@ -113,17 +142,20 @@ __global__ void slice_row_exponents(const double* __restrict__ B, long long ldb,
   if (m != EXP_ZERO) atomicMax(xk + kk, m);
 }
 
+// The exponents' start, and a zero behind them (the length of the list).
 __global__ void slice_fill(int* __restrict__ v, int n, int x) {
   if (static_cast<int>(threadIdx.x) < n) v[threadIdx.x] = x;
+  if (threadIdx.x == 0) v[n] = 0;
 }
 
 // Slices of B: out[s][column][kk] and the columns' scales; one warp a column.
 __global__ void slice_pack_b(const double* __restrict__ B, long long ldb, int k, int n, int kpad, int npad,
-                             const int* __restrict__ xk, __nv_bfloat16* __restrict__ out, int* __restrict__ scale) {
+                             const int* __restrict__ xk, __nv_bfloat16* __restrict__ out, int* __restrict__ scale,
+                             uint4* __restrict__ masks) {
   const int col = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (col >= npad) return;
   double v[4];  // kk = 2 lane, 2 lane + 1, then + 64
-  int x[4], mx = EXP_ZERO;
+  int x[4], ex[4], mx = EXP_ZERO;
   bool bad = false;
 #pragma unroll
   for (int q = 0; q < 4; q++) {
@@ -131,13 +163,23 @@ __global__ void slice_pack_b(const double* __restrict__ B, long long ldb, int k,
     v[q] = (col < n && kk < k) ? B[static_cast<long long>(col) * ldb + kk] : 0.0;
     x[q] = kk < k ? xk[kk] : 0;
     if (x[q] == EXP_ZERO) x[q] = 0;
-    const int e = exponent_of(v[q]);
-    if (e == EXP_NONFINITE) bad = true;
-    else if (e != EXP_ZERO) mx = max(mx, e - x[q]);
+    ex[q] = exponent_of(v[q]);
+    if (ex[q] == EXP_NONFINITE) bad = true;
+    else if (ex[q] != EXP_ZERO) mx = max(mx, ex[q] - x[q]);
   }
   for (int o = 16; o > 0; o >>= 1) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
   bad = __any_sync(0xffffffffu, bad);
-  if (lane == 0) scale[col] = bad ? EXP_NONFINITE : mx;
+  unsigned large[MASK_WORDS], some[MASK_WORDS];
+#pragma unroll
+  for (int q = 0; q < 4; q++) {
+    some[q] = __ballot_sync(0xffffffffu, ex[q] != EXP_ZERO);
+    large[q] = __ballot_sync(0xffffffffu, ex[q] != EXP_ZERO && ex[q] - x[q] >= mx - NEAR);
+  }
+  if (lane == 0) {
+    scale[col] = bad ? EXP_NONFINITE : mx;
+    masks[2 * col] = make_uint4(large[0], large[1], large[2], large[3]);
+    masks[2 * col + 1] = make_uint4(some[0], some[1], some[2], some[3]);
+  }
 #pragma unroll
   for (int p = 0; p < 2; p++) {
     const int kk = 2 * lane + 64 * p;
@@ -157,7 +199,8 @@ __global__ void slice_pack_b(const double* __restrict__ B, long long ldb, int k,
 constexpr int SA_ROWS = 32;
 __global__ void __launch_bounds__(256) slice_pack_a(const double* __restrict__ A, long long lda, int m, int k,
                                                     int kpad, int mpad, const int* __restrict__ xk,
-                                                    __nv_bfloat16* __restrict__ out, int* __restrict__ scale) {
+                                                    __nv_bfloat16* __restrict__ out, int* __restrict__ scale,
+                                                    unsigned* __restrict__ masks) {
   __shared__ double t[S_MAXK][SA_ROWS + 1];
   __shared__ int x[S_MAXK], part[8][SA_ROWS], sc[SA_ROWS];
   const int r0 = blockIdx.x * SA_ROWS, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -182,6 +225,17 @@ __global__ void __launch_bounds__(256) slice_pack_a(const double* __restrict__ A
     scale[r0 + lane] = mx;
   }
   __syncthreads();
+  {  // warp w: word w % 4 of the large entries (w < 4) or of the nonzero ones
+    const int s0 = sc[lane], word = w & (MASK_WORDS - 1);
+    unsigned bits = 0;
+    for (int i = 0; i < 32; i++) {
+      const int kk = 64 * (word >> 1) + 2 * i + (word & 1);
+      if (kk >= k) break;
+      const int e = exponent_of(t[kk][lane]);
+      if (e != EXP_ZERO && (w >= MASK_WORDS || e + x[kk] >= s0 - NEAR)) bits |= 1u << i;
+    }
+    masks[(2 * static_cast<size_t>(r0 + lane) + (w >= MASK_WORDS ? 1 : 0)) * MASK_WORDS + word] = bits;
+  }
   const int pairs = kpad / 2;
   for (int e = threadIdx.x; e < SA_ROWS * pairs; e += blockDim.x) {
     const int r = e / pairs, kk = 2 * (e - r * pairs), s0 = sc[r];
@@ -254,8 +308,10 @@ __device__ __forceinline__ void tmem_load8(uint32_t addr, uint32_t (&r)[8]) {
 
 __global__ void __launch_bounds__(S_THREADS, 1)
     f64_update_sliced(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB,
-                      const int* __restrict__ ea, const int* __restrict__ fb, double* __restrict__ C, long long ldc,
-                      int m, int n, int nkc, int ntm, int ntiles, int* __restrict__ err) {
+                      const int* __restrict__ ea, const int* __restrict__ fb, const uint4* __restrict__ ma,
+                      const uint4* __restrict__ mb, uint2* __restrict__ list, unsigned* __restrict__ listed,
+                      double* __restrict__ C, long long ldc, int m, int n, int nkc, int ntm, int ntiles,
+                      int* __restrict__ err) {
   extern __shared__ __align__(1024) unsigned char s_raw[];
   char* base = reinterpret_cast<char*>((reinterpret_cast<uintptr_t>(s_raw) + 1023) & ~uintptr_t(1023));
   __shared__ uint64_t op_full[S_NST], op_empty[S_NST], acc_full, acc_empty, drained;
@@ -376,6 +432,7 @@ __global__ void __launch_bounds__(S_THREADS, 1)
       }
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       long long v[32];
+      unsigned whole = 0, most = 0;  // entries shifted up by 16 and by 8, the others by 4
       const uint32_t t0 = tmem + (static_cast<uint32_t>(quarter * 32) << 16) + static_cast<uint32_t>(half * 32);
 #pragma unroll
       for (int c8 = 0; c8 < 32; c8 += 8) {
@@ -391,41 +448,82 @@ __global__ void __launch_bounds__(S_THREADS, 1)
           for (int o = 0; o < 6; o++) hi = (hi << 8) + __float2int_rn(__uint_as_float(r[o][q]));
           const long long lo = (static_cast<long long>(__float2int_rn(__uint_as_float(r[6][q]))) << 8) +
                                __float2int_rn(__uint_as_float(r[7][q]));
-          v[c8 + q] = hi + ((lo + 32768) >> 16);
+          // |hi| < 2^59 and |lo| < 2^33: the bits of lo that a double of the
+          // sum can hold
+          const long long size = hi < 0 ? -hi : hi;
+          if (size < 1ll << 46) {
+            v[c8 + q] = (hi << 16) + lo;
+            whole |= 1u << (c8 + q);
+          } else if (size < 1ll << 54) {
+            v[c8 + q] = (hi << 8) + ((lo + 128) >> 8);
+            most |= 1u << (c8 + q);
+          } else {
+            v[c8 + q] = (hi << 4) + ((lo + 2048) >> 12);
+          }
         }
       }
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       __syncwarp();
       if (lane == 0)
         asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_addr(&acc_empty)) : "memory");
-      // C -= v 2^(ea + fb - 52)
+      // C -= v 2^(ea + fb - 52 - shift)
       const int row = tm * S_M + quarter * 32 + lane;
       const int col0 = tn * S_N + half * 32;
       const int er = ea[row];
-      if (row < m) {
-        double* cp = C + static_cast<long long>(col0) * ldc + row;
+      const uint4 near_a = ma[2 * row];  // rows and columns up to a whole tile are packed
+      double* cp = C + static_cast<long long>(col0) * ldc + row;
 #pragma unroll
-        for (int c8 = 0; c8 < 32; c8 += 8) {
-          double c[8];
+      for (int c8 = 0; c8 < 32; c8 += 8) {
+        double c[8];
+        unsigned exact = 0;  // entries to sum in FP64: left as they are
 #pragma unroll
-          for (int q = 0; q < 8; q++) c[q] = col0 + c8 + q < n ? cp[static_cast<long long>(c8 + q) * ldc] : 0.0;
+        for (int q = 0; q < 8; q++)
+          c[q] = row < m && col0 + c8 + q < n ? cp[static_cast<long long>(c8 + q) * ldc] : 0.0;
+#pragma unroll
+        for (int q = 0; q < 8; q++) {
+          const int ec = fb[col0 + c8 + q];
+          if (er == EXP_NONFINITE || ec == EXP_NONFINITE) {
+            exact |= 1u << q;
+            continue;
+          }
+          if (er == EXP_ZERO || ec == EXP_ZERO) continue;
+          const unsigned bit = 1u << (c8 + q);
+          const int shift = (whole & bit) ? 16 : (most & bit) ? 8 : 4;
+          const long long s = v[c8 + q];
+          if (s != 0) {
+            const int e = er + ec - 52 - shift + 1023;
+            const double x = static_cast<double>(s);
+            if (e > 0 && e < 2047)
+              c[q] = fma(-x, __longlong_as_double(static_cast<long long>(e) << 52), c[q]);
+            else
+              c[q] -= scalbn(x, e - 1023);
+          }
+          const uint4 near_b = mb[2 * (col0 + c8 + q)];
+          const int near = __popc(near_a.x & near_b.x) + __popc(near_a.y & near_b.y) + __popc(near_a.z & near_b.z) +
+                           __popc(near_a.w & near_b.w);
+          const long long size = s < 0 ? -s : s;
+          const int ex = static_cast<int>((__double2hiint(c[q]) >> 20) & 0x7ff) - 1022;
+          if (near < NEAR_TERMS && (size >> (52 - SAFE_BITS + shift)) == 0 && ex <= er + ec - SAFE_BITS) exact |= 1u << q;
+        }
+        if (row >= m) exact = 0;
+        if (__any_sync(0xffffffffu, exact != 0u)) {
+          unsigned rows = 0;  // lane q: the rows listed of column q
 #pragma unroll
           for (int q = 0; q < 8; q++) {
-            const int ec = fb[col0 + c8 + q];
-            const int e = er + ec - 52 + 1023;
-            if (er == EXP_NONFINITE || ec == EXP_NONFINITE) {
-              c[q] = nan("");
-            } else if (v[c8 + q] != 0) {  // never with a zero row or column
-              const double x = static_cast<double>(v[c8 + q]);
-              if (e > 0 && e < 2047)
-                c[q] = fma(-x, __longlong_as_double(static_cast<long long>(e) << 52), c[q]);
-              else
-                c[q] -= scalbn(x, e - 1023);
-            }
+            const unsigned w = __ballot_sync(0xffffffffu, (exact >> q) & 1u);
+            if (lane == q && col0 + c8 + q < n) rows = w;
           }
+          const unsigned have = __ballot_sync(0xffffffffu, rows != 0u);
+          unsigned at = 0;
+          if (lane == 0) at = atomicAdd(listed, static_cast<unsigned>(__popc(have)));
+          at = __shfl_sync(0xffffffffu, at, 0) + __popc(have & ((1u << lane) - 1u));
+          // a place is 32 rows of a column: fewer than 2^32 of them
+          if (rows) list[at] = make_uint2(rows, static_cast<unsigned>(tm * (S_M / 32) + quarter) * n + col0 + c8 + lane);
+        }
+        if (row < m) {
 #pragma unroll
           for (int q = 0; q < 8; q++)
-            if (col0 + c8 + q < n) cp[static_cast<long long>(c8 + q) * ldc] = c[q];
+            if (col0 + c8 + q < n && !((exact >> q) & 1u)) cp[static_cast<long long>(c8 + q) * ldc] = c[q];
         }
       }
     }
@@ -436,6 +534,60 @@ __global__ void __launch_bounds__(S_THREADS, 1)
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512));
+}
+
+// C -= A B in FP64 for the listed entries, a warp a place of the list: the rows of
+// a 32-row block (bits) in one column.  Bound: the FP64 pipe where much is listed,
+// else latency; every SM full of warps, so that the loads of some (eight k at a
+// time) hide behind others.  (The epilogue did this first, and then warps by
+// column of the matrix: what is listed comes in clusters, so a few warps had most
+// of it, and the updates of the N = 7,819 factorisation took 49 ms, now 24.)
+constexpr int SUM_THREADS = 256;
+__global__ void __launch_bounds__(SUM_THREADS) sum_listed(const uint2* __restrict__ list,
+                                                         const unsigned* __restrict__ listed, const int* __restrict__ ea,
+                                                         const int* __restrict__ fb, const uint4* __restrict__ ma,
+                                                         const uint4* __restrict__ mb, const double* __restrict__ A,
+                                                         long long lda, const double* __restrict__ B, long long ldb,
+                                                         int k, double* __restrict__ C, long long ldc, int m, int n) {
+  constexpr unsigned ALL = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  const unsigned count = *listed, step = gridDim.x * (SUM_THREADS / 32);
+  for (unsigned at = blockIdx.x * (SUM_THREADS / 32) + (threadIdx.x >> 5); at < count; at += step) {
+    const uint2 e = list[at];
+    const int col = static_cast<int>(e.y % static_cast<unsigned>(n));
+    const int row = static_cast<int>(e.y / static_cast<unsigned>(n)) * 32 + lane;
+    const bool mine = row < m && ((e.x >> lane) & 1u);
+    const uint4 a = ma[2 * row + 1], b = mb[2 * col + 1];  // (rows up to a whole tile are packed)
+    const bool whole = __any_sync(ALL, mine && ea[row] == EXP_NONFINITE) || fb[col] == EXP_NONFINITE;
+    // the k that any of the rows needs: of half h, word 2 h holds the even ones, word 2 h + 1 the odd ones
+    const unsigned any[MASK_WORDS] = {
+        __reduce_or_sync(ALL, mine ? a.x & b.x : 0u), __reduce_or_sync(ALL, mine ? a.y & b.y : 0u),
+        __reduce_or_sync(ALL, mine ? a.z & b.z : 0u), __reduce_or_sync(ALL, mine ? a.w & b.w : 0u)};
+    const double* pa = A + min(row, m - 1);
+    const double* pb = B + static_cast<long long>(col) * ldb;
+    double sum = 0.0;
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+      const unsigned even = whole ? ALL : any[2 * h], odd = whole ? ALL : any[2 * h + 1];
+      if (!(even | odd)) continue;
+      for (int i = 0; i < 32; i += 4) {
+        const int k0 = 64 * h + 2 * i;
+        const unsigned ev = (even >> i) & 15u, od = (odd >> i) & 15u;
+        if (!(ev | od) || k0 >= k) continue;
+        double u[8], v[8];
+#pragma unroll
+        for (int q = 0; q < 8; q++) {
+          const bool in = k0 + q < k;
+          u[q] = in ? pa[static_cast<long long>(k0 + q) * lda] : 0.0;
+          v[q] = in ? pb[k0 + q] : 0.0;
+        }
+#pragma unroll
+        for (int q = 0; q < 8; q++)
+          if (((q & 1 ? od : ev) >> (q >> 1)) & 1u) sum = fma(u[q], v[q], sum);
+      }
+    }
+    if (mine) C[static_cast<long long>(col) * ldc + row] -= sum;
+  }
 }
 
 // 3-D bf16 map of out[slice][row][kk]: boxes of 32 x rows x all slices.
@@ -455,7 +607,8 @@ void make_slice_map(CUtensorMap* map, const void* ptr, int kpad, int rows, int b
 
 }  // namespace
 
-bool f64_sliced_update_possible(int k) { return k > 0 && k <= S_MAXK && tensor_map_encoder() != nullptr; }
+// (k = S_MAXK could fill the 64-bit sum's last bit)
+bool f64_sliced_update_possible(int k) { return k > 0 && k < S_MAXK && tensor_map_encoder() != nullptr; }
 
 void f64_sliced_update(Context* ctx, int m, int n, int k, const double* A, long long lda, const double* B,
                        long long ldb, double* C, long long ldc) {
@@ -463,15 +616,24 @@ void f64_sliced_update(Context* ctx, int m, int n, int k, const double* A, long 
   cudaStream_t s = ctx->stream();
   const int kpad = (k + S_KC - 1) / S_KC * S_KC;
   const int mpad = (m + S_M - 1) / S_M * S_M, npad = (n + S_N - 1) / S_N * S_N;
-  // slices, then the scales (rows of A, columns of B), then the row scaling of B
+  // slices, then the masks and scales (rows of A, columns of B), then the row scaling of B and the list
   const size_t abytes = static_cast<size_t>(S_SLICES) * mpad * kpad * 2, bbytes = static_cast<size_t>(S_SLICES) * npad * kpad * 2;
-  char* wa = static_cast<char*>(ctx->workspace(Context::WS_TC_A, abytes + sizeof(int) * mpad));
-  char* wb = static_cast<char*>(ctx->workspace(Context::WS_TC_B, bbytes + sizeof(int) * (static_cast<size_t>(npad) + S_MAXK)));
+  char* wa = static_cast<char*>(ctx->workspace(Context::WS_TC_A, abytes + (2 * sizeof(uint4) + sizeof(int)) * mpad));
+  // a place of the list for every 32 rows of every column
+  const size_t places = static_cast<size_t>((m + 31) / 32) * n;
+  if (places >> 32) throw KdError(KD_ERR_ARG, "sliced FP64 update: matrix too large");
+  char* wb = static_cast<char*>(ctx->workspace(
+      Context::WS_TC_B,
+      bbytes + (2 * sizeof(uint4) + sizeof(int)) * npad + sizeof(int) * (S_MAXK + 4) + sizeof(uint2) * places));
   auto* as = reinterpret_cast<__nv_bfloat16*>(wa);
   auto* bs = reinterpret_cast<__nv_bfloat16*>(wb);
-  int* ea = reinterpret_cast<int*>(wa + abytes);
-  int* fb = reinterpret_cast<int*>(wb + bbytes);
+  auto* ma = reinterpret_cast<uint4*>(wa + abytes);  // abytes and bbytes are multiples of 4,096
+  auto* mb = reinterpret_cast<uint4*>(wb + bbytes);
+  int* ea = reinterpret_cast<int*>(ma + 2 * mpad);
+  int* fb = reinterpret_cast<int*>(mb + 2 * npad);
   int* xk = fb + npad;
+  auto* listed = reinterpret_cast<unsigned*>(xk + S_MAXK);
+  auto* list = reinterpret_cast<uint2*>(xk + S_MAXK + 4);  // 16-byte aligned: npad is a multiple of 64
   bool fresh = false;
   int* err = static_cast<int*>(ctx->workspace(Context::WS_TC_FLAG, sizeof(int), &fresh));
   if (fresh) cuda_check(cudaMemsetAsync(err, 0, sizeof(int), s), "memset err");
@@ -484,15 +646,17 @@ void f64_sliced_update(Context* ctx, int m, int n, int k, const double* A, long 
   slice_fill<<<1, S_MAXK, 0, s>>>(xk, S_MAXK, EXP_ZERO);
   const int cols = 32;
   slice_row_exponents<<<(n + cols - 1) / cols, S_MAXK, 0, s>>>(B, ldb, k, n, cols, xk);
-  slice_pack_b<<<(npad + 7) / 8, 256, 0, s>>>(B, ldb, k, n, kpad, npad, xk, bs, fb);
-  slice_pack_a<<<mpad / SA_ROWS, 256, 0, s>>>(A, lda, m, k, kpad, mpad, xk, as, ea);
+  slice_pack_b<<<(npad + 7) / 8, 256, 0, s>>>(B, ldb, k, n, kpad, npad, xk, bs, fb, mb);
+  slice_pack_a<<<mpad / SA_ROWS, 256, 0, s>>>(A, lda, m, k, kpad, mpad, xk, as, ea, reinterpret_cast<unsigned*>(ma));
   CUtensorMap mA, mB;
   make_slice_map(&mA, as, kpad, mpad, S_M);
   make_slice_map(&mB, bs, kpad, npad, S_N);
   const int ntm = mpad / S_M, ntiles = ntm * (npad / S_N);
   const int grid = ntiles < ctx->sms() ? ntiles : ctx->sms();
-  f64_update_sliced<<<grid, S_THREADS, S_SMEM, s>>>(mA, mB, ea, fb, C, ldc, m, n, kpad / S_KC, ntm, ntiles, err);
-  ctx->launches += 5;
+  f64_update_sliced<<<grid, S_THREADS, S_SMEM, s>>>(mA, mB, ea, fb, ma, mb, list, listed, C, ldc, m, n, kpad / S_KC, ntm,
+                                                   ntiles, err);
+  sum_listed<<<8 * ctx->sms(), SUM_THREADS, 0, s>>>(list, listed, ea, fb, ma, mb, A, lda, B, ldb, k, C, ldc, m, n);
+  ctx->launches += 6;
   cuda_check(cudaGetLastError(), "sliced FP64 trailing update");
 }
 

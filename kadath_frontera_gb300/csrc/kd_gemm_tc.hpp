@@ -37,9 +37,9 @@ bool tf32x3_gemm_possible(int k, const float* C, long long ldc, int m, int c_row
 // results ran out of polls.
 int tf32_gemm_error_flag(Context* ctx);
 
-// C -= A * B in FP64 (column-major, k <= 128) by exact products of 8-bit
-// slices on the tensor cores (kd_gemm_f64.cu); a wait that ran out sets the
-// flag that tf32_gemm_error_flag reads.
+// C -= A * B in FP64 (column-major, k < 128) by exact products of 8-bit slices
+// on the tensor cores, and in FP64 where an entry needs it (kd_gemm_f64.cu); a
+// wait that ran out sets the flag that tf32_gemm_error_flag reads.
 bool f64_sliced_update_possible(int k);
 void f64_sliced_update(Context* ctx, int m, int n, int k, const double* A, long long lda, const double* B,
                        long long ldb, double* C, long long ldc);
