@@ -2129,9 +2129,10 @@ __global__ void __launch_bounds__(GP_THREADS) panel_grid_kernel(T* __restrict__ 
     } else if (tid >= 128 && tid < 128 + jb) {
       if (gi != j && gi >= r0 && gi < r1) tile[(tid - 128) * per + gi - r0] = __ldcg(ps.jrow + slot * jb + tid - 128);
     } else if (tid == 256) {  // the reciprocal, from the key, beside the row's load
-      T v = T(0);
+      T v = T(1);  // (not used below a zero pivot)
       if (best.key > KEY_OF_ZERO) modulus_of(best.key, v);
-      s_inv = v != T(0) ? T(1) / v : T(0);
+      else if (best.key == 0) v = static_cast<T>(nan(""));  // every candidate is
+      s_inv = T(1) / v;  // zero for an infinite pivot: so are its multipliers
       s_piv[jj] = gi;
       if (b == 0) {
         ipiv[j] = gi;
@@ -2142,7 +2143,7 @@ __global__ void __launch_bounds__(GP_THREADS) panel_grid_kernel(T* __restrict__ 
     // 5. scale the column below the pivot, rank-1 update of the rest
     const T inv = prow[jj] < T(0) ? -s_inv : s_inv;
     const int rs = (r0 > j + 1) ? r0 : j + 1;
-    if (inv != T(0) && rs < r1) {
+    if (prow[jj] != T(0) && rs < r1) {
       for (int i = rs + tid; i < r1; i += GP_THREADS) tile[jj * per + i - r0] *= inv;
       __syncthreads();
       // warps over (64-row group, column phase): rows along the lanes
