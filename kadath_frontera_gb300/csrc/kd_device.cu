@@ -5,6 +5,7 @@
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <utility>
 
 #include "kd_device.hpp"
@@ -381,16 +382,34 @@ __global__ void __launch_bounds__(256) op_list_kernel(const __grid_constant__ Kd
   }
 }
 
+// Lets a kernel use all the shared memory an SM gives a CTA, once per device
+// (`devices`: a bit each, the kernel's own).  The limit belongs to the kernel and
+// not to a context: setting it to each launch's size would let one thread lower it
+// between another's call and launch.
+cudaError_t allow_shared(const void* kernel, std::atomic<unsigned long long>& devices, size_t smem) {
+  if (smem <= 48 * 1024) return cudaSuccess;
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  const unsigned long long bit = 1ull << (dev & 63);
+  if (dev < 64 && (devices.load(std::memory_order_acquire) & bit)) return cudaSuccess;
+  cudaFuncAttributes a;
+  e = cudaFuncGetAttributes(&a, kernel);
+  if (e != cudaSuccess) return e;
+  e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           227 * 1024 - static_cast<int>(a.sharedSizeBytes));
+  if (e == cudaSuccess) devices.fetch_or(bit, std::memory_order_release);
+  return e;
+}
+
 template <int N>
 cudaError_t launch_op_list(const KdOpRec* ops, int n, size_t smem, const double* d_pool, cudaStream_t s) {
   KdOpList<N> list;
   list.n = n;
   for (int i = 0; i < n; i++) list.ops[i] = ops[i];
-  if (smem > 48 * 1024) {
-    const cudaError_t e =
-        cudaFuncSetAttribute(op_list_kernel<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-    if (e != cudaSuccess) return e;
-  }
+  static std::atomic<unsigned long long> devices{0};
+  const cudaError_t e = allow_shared(reinterpret_cast<const void*>(op_list_kernel<N>), devices, smem);
+  if (e != cudaSuccess) return e;
   op_list_kernel<N><<<n, 256, smem, s>>>(list, d_pool);
   return cudaGetLastError();
 }
@@ -398,11 +417,9 @@ cudaError_t launch_op_list(const KdOpRec* ops, int n, size_t smem, const double*
 template <int CL, class List>
 cudaError_t launch_lp_cluster(const List& list, int total_fields, size_t smem, const double* d_pool,
                               cudaStream_t s) {
-  if (smem > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(line_passes_cluster_kernel<CL, List>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-    if (e != cudaSuccess) return e;
-  }
+  static std::atomic<unsigned long long> devices{0};
+  cudaError_t e = allow_shared(reinterpret_cast<const void*>(line_passes_cluster_kernel<CL, List>), devices, smem);
+  if (e != cudaSuccess) return e;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(total_fields * CL, 1, 1);
   cfg.blockDim = dim3(128, 1, 1);
@@ -415,7 +432,7 @@ cudaError_t launch_lp_cluster(const List& list, int total_fields, size_t smem, c
   at[0].val.clusterDim.z = 1;
   cfg.attrs = at;
   cfg.numAttrs = 1;
-  cudaError_t e = cudaLaunchKernelEx(&cfg, line_passes_cluster_kernel<CL, List>, list, d_pool);
+  e = cudaLaunchKernelEx(&cfg, line_passes_cluster_kernel<CL, List>, list, d_pool);
   if (e != cudaSuccess) return e;
   return cudaGetLastError();
 }
@@ -429,11 +446,9 @@ cudaError_t launch_list(const List& list, size_t smem, const double* d_pool, cud
     case 8: return launch_lp_cluster<8>(list, total_fields, smem, d_pool, s);
     default: break;
   }
-  if (smem > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(line_passes_kernel<List>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         static_cast<int>(smem));
-    if (e != cudaSuccess) return e;
-  }
+  static std::atomic<unsigned long long> devices{0};
+  const cudaError_t e = allow_shared(reinterpret_cast<const void*>(line_passes_kernel<List>), devices, smem);
+  if (e != cudaSuccess) return e;
   const int threads = (shape.threads == 64 || shape.threads == 256) ? shape.threads : 128;
   int grid = total_fields < 152 * 8 ? total_fields : 152 * 8;
   line_passes_kernel<List><<<grid, threads, smem, s>>>(list, d_pool);
