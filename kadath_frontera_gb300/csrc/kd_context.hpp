@@ -285,8 +285,8 @@ struct ProfScope {
 };
 
 // A batch for its lifetime (none where a stream is forked or profiled).  When
-// an exception leaves it, what was collected is dropped: its outputs are
-// garbage to nobody, since the pass that collected it has failed.
+// an exception leaves it, what was collected is dropped: the pass that collected
+// it has failed, and must not have marked any of its outputs as computed.
 struct BatchScope {
   Context* c;
   bool mine;

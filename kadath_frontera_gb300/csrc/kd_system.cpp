@@ -1063,9 +1063,16 @@ void System::residual(double* d_F, bool record) {
   graphs_.push_back(std::move(g));
 }
 
+// The node values count as recorded once the whole pass has been launched: a pass
+// that throws while it exports leaves operations that were collected and dropped.
 void System::residual_pass(double* d_F, bool record) {
-  ctx->scratch().reset();
   vcache_.clear();
+  value_pass(d_F, record);
+  vcache_.valid = record;
+}
+
+void System::value_pass(double* d_F, bool record) {
+  ctx->scratch().reset();
   std::unique_ptr<ScratchRedirect> redirect;
   if (record) redirect = std::make_unique<ScratchRedirect>(ctx, &vcache_.arena);
   EvalState st;
@@ -1109,7 +1116,6 @@ void System::residual_pass(double* d_F, bool record) {
     lhs[i] = eqs_[i].lhs->eval(st);
     if (eqs_[i].kind == Equation::MATCHING) rhs[i] = eqs_[i].rhs->eval(st);
   }
-  vcache_.valid = record;
   if (nbr_conditions_ < 0) {
     int row = 0;
     for (auto& ie : ieqs_) ie.row = row++;

@@ -373,6 +373,7 @@ class System {
   long long graph_clock_ = 0;
   std::vector<long long> state_signature() const;
   void residual_pass(double* d_F, bool record);
+  void value_pass(double* d_F, bool record);
   // The Jacobian's seed passes as a CUDA graph: captured the second time a
   // signature is met, with the tangent cache as the pass left it (its host
   // side; the replay refills the device side at the same addresses).
