@@ -36,6 +36,7 @@ struct PtDom {
   int type;
   double alpha, beta, rin, rout;
   int nc0, nc1, nc2;
+  int ncheb;  // Chebyshev values its fields need: nc0, twice that with even or odd radial bases
 };
 
 struct PtArgs {
@@ -401,7 +402,7 @@ __global__ void __launch_bounds__(PT_THREADS) val_points_sorted_kernel(
       double x, y, z, r;
       pt_locate(a, xyz, p, x, y, z, r);
       const PtPos q = pt_position(D, x, y, z, r);
-      pt_chebyshev(q.xi, D.type == 1 ? 2 * D.nc0 : D.nc0, T, PT_THREADS);
+      pt_chebyshev(q.xi, D.ncheb, T, PT_THREADS);
       const int row = D.nc1 * PT_THREADS;
 #pragma unroll
       for (int odd = 0; odd < 2; odd++) {
@@ -439,7 +440,7 @@ __global__ void __launch_bounds__(PT_THREADS) val_points_few_kernel(const __grid
   if (dd >= 0) {
     const PtPos q = pt_position(D, x, y, z, r);
     const int row = nt_max * PPB;
-    if (sub == 0) pt_chebyshev(q.xi, D.type == 1 ? 2 * D.nc0 : D.nc0, T, PPB);
+    if (sub == 0) pt_chebyshev(q.xi, D.ncheb, T, PPB);
     if (sub == 1) pt_theta(q, 0, D.nc1, TH, TH + 2 * row, PPB);
     if (sub == 2) pt_theta(q, 1, D.nc1, TH + row, TH + 3 * row, PPB);
     if (sub == 3) {
@@ -507,6 +508,7 @@ void fields_val_points(Context* ctx, const std::vector<const Field*>& fields, lo
     a.d[d].nc0 = dm.nc[0];
     a.d[d].nc1 = dm.nc[1];
     a.d[d].nc2 = dm.nc[2];
+    a.d[d].ncheb = dm.nc[0];
   }
   // basis tables, and fields grouped by them
   std::vector<int> tab;
@@ -519,9 +521,12 @@ void fields_val_points(Context* ctx, const std::vector<const Field*>& fields, lo
       a.tab_off[f][d] = static_cast<int>(tab.size());
       const Base b = (pd.zero || !pd.base.def) ? dm.std_base() : pd.base;
       if (b.p != KD_COSSIN) throw KdError(KD_ERR_UNSUPPORTED, "val_points: phi basis other than COSSIN");
-      for (int code : b.r)
+      for (int code : b.r) {
         if (code != KD_CHEB && code != KD_CHEB_EVEN && code != KD_CHEB_ODD)
           throw KdError(KD_ERR_UNSUPPORTED, "val_points: radial basis not handled");
+        // (a file may hold any of them in any domain)
+        if (code != KD_CHEB) a.d[d].ncheb = 2 * dm.nc[0];
+      }
       for (int code : b.t)
         if (code != KD_COS_EVEN && code != KD_COS_ODD && code != KD_SIN_EVEN && code != KD_SIN_ODD)
           throw KdError(KD_ERR_UNSUPPORTED, "val_points: theta basis not handled");
