@@ -801,8 +801,8 @@ __global__ void scatter_perm(const double* __restrict__ z, const int* __restrict
 }
 
 // Inverse of the unit-lower (blockIdx.y 0) or upper part (1) of one TB x TB
-// diagonal block, row-major, zero padded to TB x TB; with FP32 factors as
-// (hi, lo) float pairs.  Eight lanes a column, rows l + 8 q each; a finished
+// diagonal block, row-major, zero padded to TB x TB: in FP64, or as (hi, lo) float
+// pairs (the one or the other is null).  Eight lanes a column, rows l + 8 q each; a finished
 // entry is broadcast by a shuffle and a warp starts at the first row of its four
 // columns.  Bound: the FP64 pipe.  (One thread a column took 140 us, a chain of
 // 2,000 dependent multiply-adds.)
@@ -853,8 +853,9 @@ __global__ void __launch_bounds__(ID_THREADS) invert_diag_blocks(const T* __rest
   for (int e = threadIdx.x; e < TB * TB; e += ID_THREADS) {
     const int i = e / TB, k = e % TB;  // row, column of the block
     const double v = (i < n && k < n) ? (upper ? X[(n - 1 - k) * (TB + 1) + n - 1 - i] : X[k * (TB + 1) + i]) : 0.0;
-    if constexpr (std::is_same<T, double>::value) out[e] = v;
-    if constexpr (std::is_same<T, float>::value) {
+    if (Linv) {
+      out[e] = v;
+    } else {
       const float h = static_cast<float>(v);
       out2[static_cast<size_t>(blk) * TB * TB + e] = make_float2(h, static_cast<float>(v - static_cast<double>(h)));
     }
@@ -1484,10 +1485,10 @@ __global__ void __launch_bounds__(256) invert_groups(const float* __restrict__ A
 // more way to L2; only the CTA whose turn is next polls without a pause.  Sums
 // are double-float (G and the right-hand side as float pairs, about 48 bits) of
 // FP32 products with x in sums of 8 terms: FP64 adds and conversions would run
-// at the FP64 rate.  TRANS: the transposed factor.  Inside the group the rows
-// run in sweep order (reversed when descending): G is lower triangular in all
-// four sweeps.  b enters times bscale, y leaves times yscale (null: 1).  Every CTA
-// is resident and a group waits for earlier ones only.
+// at the FP64 rate.  Inside the group the rows run in sweep order (reversed when
+// descending): G is lower triangular in both sweeps.  b enters times bscale, y
+// leaves times yscale (null: 1).  Every CTA is resident and a group waits for
+// earlier ones only.
 // N = 12,331: 0.177 ms a sweep (97 groups, about 3,700 cycles a link: 2,000 in
 // the order of the arithmetic, 1,250 of them G's product, and the way through
 // L2); 192-row groups chained block by block with a released counter 0.351 ms.
@@ -1512,7 +1513,6 @@ struct TgShared {
   float2 v[TG_ROWS];          // in sweep order
   int abort;
 };
-template <bool TRANS>
 __global__ void __launch_bounds__(256, 1) trsv_group(const float* __restrict__ A, long long ld, int N,
                                                      const double* __restrict__ b,
                                                      const double* __restrict__ bscale, double* __restrict__ y,
@@ -1527,8 +1527,8 @@ __global__ void __launch_bounds__(256, 1) trsv_group(const float* __restrict__ A
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   // This thread's 16 entries of a 64 x 64 tile: four columns from 4 slot on and
   // four rows; four 16-byte loads, 256 contiguous bytes a half-warp.
-  const int slot = TRANS ? lane & 15 : 2 * warp + (lane >> 4), c0 = 4 * slot;
-  auto tile_row = [&](int a) { return TRANS ? 8 * warp + 2 * a + (lane >> 4) : 4 * (lane & 15) + a; };
+  const int slot = 2 * warp + (lane >> 4), c0 = 4 * slot;
+  auto tile_row = [&](int a) { return 4 * (lane & 15) + a; };
   const int i0 = lane, i1 = TB - 1 - lane;  // G: two rows of each block, columns warp + 8 i
   const int rown = tid >> 1, half = tid & 1;
   auto group = [&](int pos) { return ascending ? pos : ng - 1 - pos; };
@@ -1552,21 +1552,18 @@ __global__ void __launch_bounds__(256, 1) trsv_group(const float* __restrict__ A
         const int k0 = p0 + cb * TB + c0;
         // the working copy's columns are 128-byte aligned, k0 and the first row multiples of 4
         if (inside && k0 + 4 <= N) {
-          const float* src = TRANS ? A + static_cast<long long>(R0 + tile_row(0)) * ld + k0
-                                   : A + static_cast<long long>(k0) * ld + R0 + tile_row(0);
-          const long long next = TRANS ? 2 * ld : ld;  // to the thread's next row, or its next column
+          const float* src = A + static_cast<long long>(k0) * ld + R0 + tile_row(0);
 #pragma unroll
           for (int rb = 0; rb < TG; rb++) {
-            const float* q = src + (TRANS ? static_cast<long long>(rb) * TB * ld : rb * TB);
+            const float* q = src + rb * TB;
 #pragma unroll
-            for (int u = 0; u < 4; u++) {
+            for (int u = 0; u < 4; u++) {  // the thread's columns
               const float4 v = __ldg(reinterpret_cast<const float4*>(q));
-              constexpr int s1 = TRANS ? 1 : 4, su = TRANS ? 4 : 1;
-              t[cb][rb][su * u] = v.x;
-              t[cb][rb][su * u + s1] = v.y;
-              t[cb][rb][su * u + 2 * s1] = v.z;
-              t[cb][rb][su * u + 3 * s1] = v.w;
-              q += next;
+              t[cb][rb][u] = v.x;
+              t[cb][rb][4 + u] = v.y;
+              t[cb][rb][8 + u] = v.z;
+              t[cb][rb][12 + u] = v.w;
+              q += ld;
             }
           }
         } else {
@@ -1577,9 +1574,7 @@ __global__ void __launch_bounds__(256, 1) trsv_group(const float* __restrict__ A
 #pragma unroll
               for (int j = 0; j < 4; j++) {
                 const int row = R0 + rb * TB + tile_row(a), k = k0 + j;
-                t[cb][rb][4 * a + j] =
-                    (row < N && k < N) ? A[TRANS ? static_cast<long long>(row) * ld + k : static_cast<long long>(k) * ld + row]
-                                       : 0.f;
+                t[cb][rb][4 * a + j] = (row < N && k < N) ? A[static_cast<long long>(k) * ld + row] : 0.f;
               }
         }
       }
@@ -1590,14 +1585,14 @@ __global__ void __launch_bounds__(256, 1) trsv_group(const float* __restrict__ A
 #pragma unroll 8
       for (int e = tid; e < TB * TB; e += 256) {
         const float2 d = blk < nblk ? Dinv2[static_cast<size_t>(blk) * TB * TB + e] : make_float2(0.f, 0.f);
-        int r = TRANS ? e % TB : e / TB, c = TRANS ? e / TB : e % TB;
+        int r = e / TB, c = e % TB;
         if (!ascending) r = TB - 1 - r, c = TB - 1 - c;
         sh.D[ob][r * TG_LD + c] = d;
       }
     }
 #pragma unroll 8
     for (int e = tid; e < TB * TB; e += 256) {
-      int r = TRANS ? e % TB : e / TB, c = TRANS ? e / TB : e % TB;
+      int r = e / TB, c = e % TB;
       if (!ascending) r = TB - 1 - r, c = TB - 1 - c;
       sh.X[r * TG_LD + c] = Xinv[static_cast<size_t>(group(pos)) * TB * TB + e];
     }
@@ -1738,9 +1733,17 @@ __global__ void __launch_bounds__(256, 1) trsv_group(const float* __restrict__ A
   }
 }
 
-// ---- sweeps over FP64 factors ----
-// A whole sweep in one cooperative launch, CH_R consecutive blocks per group
-// and one group at a time per CTA: CTA c owns the groups c, c + grid, ..., group g the sweep
+// ---- sweeps over FP64 factors, and transposed ones over FP32 factors ----
+// The latter in FP64 too: b enters times the column scales, which may span any
+// range, and x rounded to FP32 costs the refinement two or three steps (3 against
+// 5 or 6 on well-conditioned matrices; no convergence at all with column scales
+// of 2^-140 to 2^140).  Bound: the FP64 pipe of one SM, 2,048 cycles a tile of 64
+// x 64, so a group is one block, conversions are made on the bits, and x is its own
+// signal (y enters as all ones, a NaN that no x is stored as): 6,200 cycles a link.
+// N = 7,819: 0.39 ms a sweep; blocks by threes with the counter 1.1, by ones 0.49;
+// a launch a block, as before sweeps were chained, 2.5.
+// A whole sweep in one cooperative launch, R consecutive blocks per group and one
+// group at a time per CTA: CTA c owns the groups c, c + grid, ..., group g the sweep
 // positions g R .. g R + R - 1.  While earlier groups are worked on it
 // accumulates, for all the group's blocks at once, the products with every
 // finished x (phase A, one progress wait per finished block).  The group's
@@ -1757,23 +1760,43 @@ __global__ void __launch_bounds__(256, 1) trsv_group(const float* __restrict__ A
 // TRANS sweeps solve with the transposed factor: the tile of output block p
 // and finished block pi is the stored block (pi, p), whose columns are the
 // output rows, so a thread reads 16 consecutive entries of one column.
-constexpr int CH_R = 3;
+constexpr int CH_R = 3;   // FP64 factors
+constexpr int CH_RF = 1;  // FP32 factors: no more rows than the FP64 pipe of an SM keeps up with
 constexpr int CH_DST = TB + 1;  // row stride of the staged Dinv blocks (conflict-free row reads)
 constexpr int CH_LST = TB + 1;  // column stride of the staged internal blocks (transposed staging without conflicts)
 // dynamic shared memory: the internal L blocks, then Dinv of the own blocks
-constexpr size_t CH_SMEM = (static_cast<size_t>(CH_R * (CH_R - 1) / 2) * TB * CH_LST +
-                            static_cast<size_t>(CH_R) * TB * CH_DST) * sizeof(double);
+template <int R>
+constexpr size_t CH_SMEM = (static_cast<size_t>(R * (R - 1) / 2) * TB * CH_LST + static_cast<size_t>(R) * TB * CH_DST) *
+                           sizeof(double);
+// A factor's entry in FP64; of an FP32 one on its bits, since the conversion costs
+// as much as a multiply-add.  Subnormals count as zero: the working copy is scaled
+// to entries of size 1, so they lie 2^-73 below the rounding of an FP64 sum.
+__device__ __forceinline__ double ch_entry(double v) { return v; }
+__device__ __forceinline__ double ch_entry(float v) {
+  const unsigned u = __float_as_uint(v), m = u & 0x7fffffffu;
+  const bool normal = m >= 0x00800000u;
+  const unsigned rebias = m >= 0x7f800000u ? 1792u << 20 : 896u << 20;  // Inf and NaN stay so
+  const unsigned hi = (u & 0x80000000u) | (normal ? (m >> 3) + rebias : 0u);
+  return __hiloint2double(static_cast<int>(hi), normal ? static_cast<int>(u << 29) : 0);
+}
 
-template <bool TRANS>
-__global__ void __launch_bounds__(256) trsv_chain(const double* __restrict__ A, long long ld, int N,
-                                                  const double* __restrict__ b, double* __restrict__ y,
-                                                  const double* __restrict__ Dinv, int lower, unsigned* progress,
+constexpr unsigned long long CH_EMPTY = ~0ull;
+__device__ __forceinline__ ulonglong2 ld_relaxed_v2(const double* p) {
+  ulonglong2 v;
+  asm volatile("ld.relaxed.gpu.global.v2.u64 {%0, %1}, [%2];" : "=l"(v.x), "=l"(v.y) : "l"(p) : "memory");
+  return v;
+}
+// b enters times bscale (null: 1).
+template <class T, bool TRANS, int R>
+__global__ void __launch_bounds__(256) trsv_chain(const T* __restrict__ A, long long ld, int N,
+                                                  const double* __restrict__ b, const double* __restrict__ bscale,
+                                                  double* y, const double* __restrict__ Dinv, int lower, unsigned* progress,
                                                   int* err, unsigned long long wait_ns, unsigned stall) {
   extern __shared__ __align__(16) unsigned char ch_raw[];
   double* Lin = reinterpret_cast<double*>(ch_raw);  // internal blocks (r2, r1), r1 < r2: column-major, stride CH_LST
   // Dinv of the own blocks, row-major 64 x 64 each with row stride CH_DST
-  double* Dds = Lin + static_cast<size_t>(CH_R * (CH_R - 1) / 2) * TB * CH_LST;
-  __shared__ double bsm[CH_R][TB];
+  double* Dds = Lin + static_cast<size_t>(R * (R - 1) / 2) * TB * CH_LST;
+  __shared__ double bsm[R][TB];
   __shared__ double part[4][TB];
   __shared__ double vd[TB];
   __shared__ double xs[TB];
@@ -1790,8 +1813,8 @@ __global__ void __launch_bounds__(256) trsv_chain(const double* __restrict__ A, 
   // 16-byte vector loads of x only from an aligned y (callers pass offset
   // vectors, e.g. a work vector at an odd offset N)
   const bool y_aligned = (reinterpret_cast<unsigned long long>(y) & 15ull) == 0;
-  for (int p0 = blockIdx.x * CH_R; p0 < nblk; p0 += gridDim.x * CH_R) {
-  const int np = (nblk - p0 < CH_R) ? nblk - p0 : CH_R;
+  for (int p0 = blockIdx.x * R; p0 < nblk; p0 += gridDim.x * R) {
+  const int np = (nblk - p0 < R) ? nblk - p0 : R;
   // Stage what the own blocks need besides the x of earlier blocks: the
   // internal L blocks (rows of position p0 + r2, columns of p0 + r1), the
   // Dinv blocks and the right-hand side, 16 independent loads in flight
@@ -1806,7 +1829,7 @@ __global__ void __launch_bounds__(256) trsv_chain(const double* __restrict__ A, 
         for (int u = 0; u < 16; u++) {
           const int e = e0 + u * 256 + tid;
           const int row = (TRANS ? kc : kr) * TB + e % TB, col = (TRANS ? kr : kc) * TB + e / TB;
-          v[u] = (row < N && col < N) ? A[static_cast<long long>(col) * ld + row] : 0.0;
+          v[u] = (row < N && col < N) ? static_cast<double>(A[static_cast<long long>(col) * ld + row]) : 0.0;
         }
 #pragma unroll
         for (int u = 0; u < 16; u++) {  // entry (i, j) of the block at dst[j * CH_LST + i]
@@ -1832,95 +1855,147 @@ __global__ void __launch_bounds__(256) trsv_chain(const double* __restrict__ A, 
     }
     if (tid < TB) {
       const int row = blk(p0 + r) * TB + tid;
-      bsm[r][tid] = (row < N) ? b[row] : 0.0;
+      double v = (row < N) ? b[row] : 0.0;
+      if (bscale && row < N) v *= bscale[row];
+      bsm[r][tid] = v;
     }
   }
   __syncthreads();
-  double acc[CH_R];
+  double acc[R];
 #pragma unroll
-  for (int r = 0; r < CH_R; r++) acc[r] = 0.0;
+  for (int r = 0; r < R; r++) acc[r] = 0.0;
   // phase A: the finished blocks of earlier CTAs
   bool ok = true;
-  double a[CH_R][16];
+  // FP32 tiles are loaded a block ahead (FP64 ones would not fit twice in registers)
+  constexpr bool kAhead = std::is_same<T, float>::value;
+  T a[R][16], next[kAhead ? R : 1][16];
   // rows of this thread in its CTA's blocks (N when past the matrix)
-  int rowof[CH_R];
+  int rowof[R];
 #pragma unroll
-  for (int r = 0; r < CH_R; r++) {
+  for (int r = 0; r < R; r++) {
     const int row = blk(p0 + r) * TB + rr;
     rowof[r] = (r < np && row < N) ? row : N;
   }
-  auto load_tile = [&](int pi) {
+  auto load_tile = [&](int pi, T(&to)[R][16]) {
     const int cb = blk(pi) * TB + c0;
     if constexpr (TRANS) {
       // entries cb .. cb + 15 of column rowof[r]
 #pragma unroll
-      for (int r = 0; r < CH_R; r++) {
-        const double* src = A + static_cast<long long>(rowof[r] < N ? rowof[r] : 0) * ld + cb;
+      for (int r = 0; r < R; r++) {
+        const T* src = A + static_cast<long long>(rowof[r] < N ? rowof[r] : 0) * ld + cb;
+        if (std::is_same<T, float>::value && rowof[r] < N && cb + 16 <= N) {
+          // the working copy's columns are 128-byte aligned, cb a multiple of 16
 #pragma unroll
-        for (int j = 0; j < 16; j++) a[r][j] = (rowof[r] < N && cb + j < N) ? src[j] : 0.0;
+          for (int j = 0; j < 16; j += 4) {
+            const float4 v = *reinterpret_cast<const float4*>(src + j);
+            to[r][j] = static_cast<T>(v.x);
+            to[r][j + 1] = static_cast<T>(v.y);
+            to[r][j + 2] = static_cast<T>(v.z);
+            to[r][j + 3] = static_cast<T>(v.w);
+          }
+          continue;
+        }
+#pragma unroll
+        for (int j = 0; j < 16; j++) to[r][j] = (rowof[r] < N && cb + j < N) ? src[j] : T(0);
       }
       return;
     }
-    const double* colp = A + static_cast<long long>(cb) * ld;
+    const T* colp = A + static_cast<long long>(cb) * ld;
     if (cb + 16 <= N) {  // whole column quarter inside the matrix: no column predicates
 #pragma unroll
-      for (int r = 0; r < CH_R; r++) {
+      for (int r = 0; r < R; r++) {
         if (rowof[r] < N) {
-          const double* src = colp + rowof[r];
+          const T* src = colp + rowof[r];
 #pragma unroll
           for (int j = 0; j < 16; j++) {
-            a[r][j] = *src;
+            to[r][j] = *src;
             src += ld;
           }
         } else {
 #pragma unroll
-          for (int j = 0; j < 16; j++) a[r][j] = 0.0;
+          for (int j = 0; j < 16; j++) to[r][j] = T(0);
         }
       }
     } else {
 #pragma unroll
-      for (int r = 0; r < CH_R; r++)
+      for (int r = 0; r < R; r++)
 #pragma unroll
         for (int j = 0; j < 16; j++)
-          a[r][j] = (rowof[r] < N && cb + j < N) ? colp[static_cast<long long>(j) * ld + rowof[r]] : 0.0;
+          to[r][j] = (rowof[r] < N && cb + j < N) ? colp[static_cast<long long>(j) * ld + rowof[r]] : T(0);
     }
   };
+  if constexpr (kAhead)
+    if (p0 > 0) load_tile(0, next);
   for (int pi = 0; pi < p0; pi++) {
     const int cb = blk(pi) * TB + c0;
-    load_tile(pi);
-    if (static_cast<unsigned>(pi) >= avail) {
-      const unsigned v = wait_progress(progress, static_cast<unsigned>(pi) + 1 + stall, wait_ns);
-      if (v == 0) {
-        ok = false;
-        break;
-      }
-      avail = v - stall;  // positions known finished
+    if constexpr (kAhead) {
+#pragma unroll
+      for (int r = 0; r < R; r++)
+#pragma unroll
+        for (int j = 0; j < 16; j++) a[r][j] = next[r][j];
+      if (pi + 1 < p0) load_tile(pi + 1, next);
+    } else {
+      load_tile(pi, a);
     }
     double xq[16];
-    if (y_aligned && cb + 16 <= N) {  // y + cb is then 16-byte aligned (cb is a multiple of 16)
-      const double2* y2 = reinterpret_cast<const double2*>(y + cb);
+    if constexpr (kAhead) {
+      // x is its own signal: y enters as all ones, and is 16-byte aligned and as
+      // long as N rounded up to 32
+      unsigned long long t_first = 0;
+      for (unsigned it = 0; ok; it++) {
+        bool here = stall == 0;
 #pragma unroll
-      for (int j = 0; j < 8; j++) {
-        const double2 v = __ldcg(y2 + j);
-        xq[2 * j] = v.x;
-        xq[2 * j + 1] = v.y;
+        for (int j = 0; j < 16; j += 2) {
+          ulonglong2 v = make_ulonglong2(0ull, 0ull);
+          if (cb + j < N) v = ld_relaxed_v2(y + cb + j);
+          if (cb + j + 1 >= N) v.y = 0ull;
+          here = here && v.x != CH_EMPTY && v.y != CH_EMPTY;
+          xq[j] = __longlong_as_double(static_cast<long long>(v.x));
+          xq[j + 1] = __longlong_as_double(static_cast<long long>(v.y));
+        }
+        if (__all_sync(0xffffffffu, here)) break;
+        if (pi + 1 < p0) __nanosleep(400);
+        if ((it & 15) == 15) {
+          const unsigned long long now = globaltimer_ns();
+          if (t_first == 0) t_first = now;
+          if (__any_sync(0xffffffffu, now - t_first > wait_ns)) ok = false;
+        }
       }
+      if (!ok) break;
     } else {
+      if (static_cast<unsigned>(pi) >= avail) {
+        const unsigned v = wait_progress(progress, static_cast<unsigned>(pi) + 1 + stall, wait_ns);
+        if (v == 0) {
+          ok = false;
+          break;
+        }
+        avail = v - stall;  // positions known finished
+      }
+      if (y_aligned && cb + 16 <= N) {  // y + cb is then 16-byte aligned (cb is a multiple of 16)
+        const double2* y2 = reinterpret_cast<const double2*>(y + cb);
 #pragma unroll
-      for (int j = 0; j < 16; j++) xq[j] = (cb + j < N) ? __ldcg(y + cb + j) : 0.0;
+        for (int j = 0; j < 8; j++) {
+          const double2 v = __ldcg(y2 + j);
+          xq[2 * j] = v.x;
+          xq[2 * j + 1] = v.y;
+        }
+      } else {
+#pragma unroll
+        for (int j = 0; j < 16; j++) xq[j] = (cb + j < N) ? __ldcg(y + cb + j) : 0.0;
+      }
     }
 #pragma unroll
-    for (int r = 0; r < CH_R; r++) {
+    for (int r = 0; r < R; r++) {
       double sum = 0.0;
 #pragma unroll
-      for (int j = 0; j < 16; j++) sum = fma(a[r][j], xq[j], sum);
+      for (int j = 0; j < 16; j++) sum = fma(ch_entry(a[r][j]), xq[j], sum);
       acc[r] += sum;
     }
   }
   if (!ok) s_abort = 1;
   // phase B: this CTA's own blocks, chained in shared memory
 #pragma unroll
-  for (int r = 0; r < CH_R; r++) {
+  for (int r = 0; r < R; r++) {
     if (r >= np) break;
     const int k = blk(p0 + r);
     const int r0 = k * TB;
@@ -1952,17 +2027,25 @@ __global__ void __launch_bounds__(256) trsv_chain(const double* __restrict__ A, 
       double x = (part[0][tid] + part[1][tid]) + (part[2][tid] + part[3][tid]);
       if (tid >= n) x = 0.0;
       xs[tid] = x;
-      if (tid < n) y[r0 + tid] = x;
+      if constexpr (kAhead) {
+        unsigned long long bits = static_cast<unsigned long long>(__double_as_longlong(x));
+        if (bits == CH_EMPTY) bits >>= 1;  // still a NaN
+        if (tid < n)
+          asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(y + r0 + tid), "l"(bits) : "memory");
+      } else {
+        if (tid < n) y[r0 + tid] = x;
+      }
     }
+    if (kAhead && R == 1) break;  // no later own block
     __syncthreads();
     // release after the block barrier: the barrier orders every thread's
     // store of x before thread 0's release (no separate fence)
-    if (tid == 0)
+    if (!kAhead && tid == 0)
       asm volatile("red.release.gpu.global.max.u32 [%0], %1;" ::"l"(progress), "r"(static_cast<unsigned>(p0 + r) + 1)
                    : "memory");
     // products of the later own blocks with x_p
 #pragma unroll
-    for (int r2 = r + 1; r2 < CH_R; r2++) {
+    for (int r2 = r + 1; r2 < R; r2++) {
       if (r2 >= np) break;
       const double* L = Lin + static_cast<size_t>(tri(r2, r)) * TB * CH_LST;
       double sum = 0.0;
@@ -3273,29 +3356,27 @@ void DenseLU::tri_solve(const T* LU, long long ld, int N, const double* b, doubl
   double* w1 = tri_work_;
   double* w2 = tri_work_ + rnd;  // 256-byte aligned second vector
   constexpr bool kF = std::is_same<T, float>::value;
+  constexpr int RC = kF ? CH_RF : CH_R;
   static std::once_flag ch_attr;
   std::call_once(ch_attr, [] {
     auto smem = [](auto* kernel, size_t bytes) {
       cuda_check(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes)),
                  "cudaFuncSetAttribute(chain sweep)");
     };
-    if constexpr (kF) {
-      smem(trsv_group<false>, sizeof(TgShared));
-      smem(trsv_group<true>, sizeof(TgShared));
-    } else {
-      smem(trsv_chain<false>, CH_SMEM);
-      smem(trsv_chain<true>, CH_SMEM);
-    }
+    if constexpr (kF) smem(trsv_group, sizeof(TgShared));
+    else smem(trsv_chain<T, false, RC>, CH_SMEM<RC>);
+    smem(trsv_chain<T, true, RC>, CH_SMEM<RC>);
   });
   // one group of blocks per CTA while the device holds that many CTAs;
   // more groups go round the context's SMs.  The sums' order does not depend
   // on the grid, so concurrent and serial solves agree bit for bit.
-  constexpr int R = kF ? TG : CH_R;
+  const bool groups = kF && !trans;
+  const int R = groups ? TG : RC;
   const int gch = (nblk + R - 1) / R;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(gch <= nsm_ ? gch : ctx_->sms(), 1, 1);
   cfg.blockDim = dim3(256, 1, 1);
-  cfg.dynamicSmemBytes = kF ? sizeof(TgShared) : CH_SMEM;
+  cfg.dynamicSmemBytes = groups ? sizeof(TgShared) : CH_SMEM<RC>;
   cfg.stream = s;
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeCooperative;
@@ -3303,28 +3384,35 @@ void DenseLU::tri_solve(const T* LU, long long ld, int N, const double* b, doubl
   cfg.attrs = at;
   cfg.numAttrs = 1;
   const unsigned stall = ctx_->stall_waits ? 1u : 0u;
-  // FP32 copies of the two sweeps' outputs (FP32 factors only)
+  // FP32 copies of the two sweeps' outputs (group sweeps only)
   float* yf = reinterpret_cast<float*>(tri_work_ + 2 * rnd);
-  if constexpr (kF)
+  if (groups)
     cuda_check(cudaMemsetAsync(yf, 0xff, 2 * rnd * sizeof(float), s), "memset sweep outputs");
+  else if (kF)
+    cuda_check(cudaMemsetAsync(w1, 0xff, 2 * rnd * sizeof(double), s), "memset sweep outputs");
   else
     cuda_check(cudaMemsetAsync(tri_bar_, 0, 2 * sizeof(unsigned), s), "memset sweep progress");
-  // sweep number k over L (or its transpose) or U
+  if (kF && trans) prepare_transposed();
+  // sweep number k over L (or its transpose) or U; scales on entry, and on exit
+  // where x is not read back by the sweep itself
   auto sweep = [&](int k, bool over_l, const double* in, const double* iscale, double* out, const double* oscale,
                    const char* what) {
     ProfScope ps(ctx_, Context::PROF_LU_SOLVE, sweep_bytes);
     const int ascending = k == 0 ? 1 : 0;
-    if constexpr (kF) {
-      cuda_check(cudaLaunchKernelEx(&cfg, trans ? trsv_group<true> : trsv_group<false>, LU, ld, N, in, iscale, out,
-                                    oscale, yf + k * rnd, over_l ? dinv2_l_ : dinv2_u_,
-                                    over_l ? group_x_l_ : group_x_u_, ascending, panel_err_, ctx_->grid_wait_ns, stall),
-                 what);
-    } else {
-      cuda_check(cudaLaunchKernelEx(&cfg, trans ? trsv_chain<true> : trsv_chain<false>, LU, ld, N, in, out,
-                                    over_l ? dinv_l_ : dinv_u_, ascending, tri_bar_ + k, panel_err_,
-                                    ctx_->grid_wait_ns, stall),
-                 what);
-    }
+    if constexpr (kF)
+      if (groups) {
+        cuda_check(cudaLaunchKernelEx(&cfg, trsv_group, LU, ld, N, in, iscale, out, oscale, yf + k * rnd,
+                                      over_l ? dinv2_l_ : dinv2_u_, over_l ? group_x_l_ : group_x_u_, ascending,
+                                      panel_err_, ctx_->grid_wait_ns, stall),
+                   what);
+        return;
+      }
+    auto* kernel = trsv_chain<T, true, RC>;
+    if constexpr (!kF)
+      if (!trans) kernel = trsv_chain<T, false, RC>;
+    cuda_check(cudaLaunchKernelEx(&cfg, kernel, LU, ld, N, in, iscale, out, over_l ? dinv_l_ : dinv_u_, ascending,
+                                  tri_bar_ + k, panel_err_, ctx_->grid_wait_ns, stall),
+               what);
   };
   if (!trans) {
     // L y = P b, then U x = y
@@ -3377,33 +3465,64 @@ void DenseLU::ensure_bsave() {
   }
 }
 
-// After factorisation: pivots as one permutation, inverses of the 64 x 64
-// diagonal blocks of L (unit lower) and U.
+void DenseLU::ensure_dinv(size_t need) {
+  if (need <= dinv_cap_) return;
+  cudaFree(dinv_l_);
+  cudaFree(dinv_u_);
+  dinv_l_ = dinv_u_ = nullptr;
+  dinv_cap_ = 0;
+  cuda_check(cudaMalloc(&dinv_l_, need * sizeof(double)), "cudaMalloc(Linv)");
+  cuda_check(cudaMalloc(&dinv_u_, need * sizeof(double)), "cudaMalloc(Uinv)");
+  dinv_cap_ = need;
+}
+
 template <class T>
-void DenseLU::prepare_solves(const T* LU, long long ld, int N) {
-  cudaStream_t s = ctx_->stream();
-  const int nblk = (N + TB - 1) / TB;
-  size_t need = static_cast<size_t>(nblk) * TB * TB;
-  if (need > dinv_cap_) {
-    cudaFree(dinv_l_);
-    cudaFree(dinv_u_);
-    cuda_check(cudaMalloc(&dinv_l_, need * sizeof(double)), "cudaMalloc(Linv)");
-    cuda_check(cudaMalloc(&dinv_u_, need * sizeof(double)), "cudaMalloc(Uinv)");
-    cudaFree(dinv2_l_);
-    cudaFree(dinv2_u_);
-    dinv2_l_ = dinv2_u_ = nullptr;
-    cuda_check(cudaMalloc(&dinv2_l_, need * sizeof(float2)), "cudaMalloc(Linv pairs)");
-    cuda_check(cudaMalloc(&dinv2_u_, need * sizeof(float2)), "cudaMalloc(Uinv pairs)");
-    dinv_cap_ = need;
-  }
+void DenseLU::invert_blocks(const T* LU, long long ld, int N, double* linv, double* uinv, float2* linv2,
+                            float2* uinv2) {
   constexpr size_t smem = sizeof(double) * (TB * TB + TB * (TB + 1));
   static std::once_flag attr_set;
   std::call_once(attr_set, [] {
-    cudaFuncSetAttribute(invert_diag_blocks<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-    cudaFuncSetAttribute(invert_diag_blocks<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+    cuda_check(cudaFuncSetAttribute(invert_diag_blocks<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    static_cast<int>(smem)),
+               "cudaFuncSetAttribute(diagonal inverses)");
   });
-  invert_diag_blocks<T><<<dim3(nblk, 2), ID_THREADS, smem, s>>>(LU, ld, N, dinv_l_, dinv_u_, dinv2_l_, dinv2_u_);
+  invert_diag_blocks<T><<<dim3((N + TB - 1) / TB, 2), ID_THREADS, smem, ctx_->stream()>>>(LU, ld, N, linv, uinv, linv2,
+                                                                                         uinv2);
   ctx_->launches++;
+}
+
+// The FP64 inverses of the diagonal blocks of FP32 factors, which only their
+// transposed sweeps read: made when the first of them needs them.
+void DenseLU::prepare_transposed() {
+  if (transposed_ready_) return;
+  ensure_dinv(static_cast<size_t>((N_ + TB - 1) / TB) * TB * TB);
+  invert_blocks<float>(A32_, ld32_, N_, dinv_l_, dinv_u_, nullptr, nullptr);
+  transposed_ready_ = true;
+}
+
+// After factorisation: inverses of the 64 x 64 diagonal blocks of L (unit lower)
+// and U, and with FP32 factors of the groups.
+template <class T>
+void DenseLU::prepare_solves(const T* LU, long long ld, int N) {
+  const int nblk = (N + TB - 1) / TB;
+  const size_t need = static_cast<size_t>(nblk) * TB * TB;
+  constexpr bool kF = std::is_same<T, float>::value;
+  transposed_ready_ = false;
+  if constexpr (kF) {
+    if (need > dinv2_cap_) {
+      cudaFree(dinv2_l_);
+      cudaFree(dinv2_u_);
+      dinv2_l_ = dinv2_u_ = nullptr;
+      dinv2_cap_ = 0;
+      cuda_check(cudaMalloc(&dinv2_l_, need * sizeof(float2)), "cudaMalloc(Linv pairs)");
+      cuda_check(cudaMalloc(&dinv2_u_, need * sizeof(float2)), "cudaMalloc(Uinv pairs)");
+      dinv2_cap_ = need;
+    }
+    invert_blocks<float>(LU, ld, N, nullptr, nullptr, dinv2_l_, dinv2_u_);
+  } else {
+    ensure_dinv(need);
+    invert_blocks<double>(LU, ld, N, dinv_l_, dinv_u_, nullptr, nullptr);
+  }
   if constexpr (std::is_same<T, float>::value) {
     const int ng = (nblk + TG - 1) / TG;
     const size_t gx = static_cast<size_t>(ng) * TB * TB;
@@ -3422,7 +3541,7 @@ void DenseLU::prepare_solves(const T* LU, long long ld, int N) {
                                       static_cast<int>(GI_SMEM)),
                  "cudaFuncSetAttribute(group inverses)");
     });
-    invert_groups<<<dim3(ng, 2), 256, GI_SMEM, s>>>(LU, ld, N, dinv2_l_, dinv2_u_, group_x_l_, group_x_u_);
+    invert_groups<<<dim3(ng, 2), 256, GI_SMEM, ctx_->stream()>>>(LU, ld, N, dinv2_l_, dinv2_u_, group_x_l_, group_x_u_);
     ctx_->launches++;
   }
   cuda_check(cudaGetLastError(), "solve preparation");

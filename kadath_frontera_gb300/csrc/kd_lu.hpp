@@ -105,6 +105,10 @@ class DenseLU {
                  const double* xscale);
   template <class T>
   void prepare_solves(const T* LU, long long ld, int N);
+  void prepare_transposed();
+  void ensure_dinv(size_t need);
+  template <class T>
+  void invert_blocks(const T* LU, long long ld, int N, double* linv, double* uinv, float2* linv2, float2* uinv2);
   void factor_f32_nopiv(float* A, long long ld, int N, bool tf32);
   void factor_mixed(double* A, long long ld, int N, int mode, const int* perm);
   int read_info();
@@ -115,12 +119,14 @@ class DenseLU {
   int pivoted_iters_ = 1000;  // refinement iterations with the last pivoted factors
   double* bsave_ = nullptr;   // right-hand side kept for a re-solve
   size_t bsave_cap_ = 0;
-  double* dinv_l_ = nullptr;  // inverses of the 64 x 64 diagonal blocks (FP64 factors)
+  double* dinv_l_ = nullptr;  // inverses of the 64 x 64 diagonal blocks (FP64 factors, transposed FP32 factors)
   double* dinv_u_ = nullptr;
+  size_t dinv_cap_ = 0;
+  bool transposed_ready_ = false;  // they are those of the present FP32 factors
   float2* dinv2_l_ = nullptr;  // the same as (hi, lo) FP32 pairs (FP32 factors)
   float2* dinv2_u_ = nullptr;
-  size_t dinv_cap_ = 0;
-  float2* group_x_l_ = nullptr;  // off-diagonal blocks of the inverses of the 192-row groups (FP32 factors)
+  size_t dinv2_cap_ = 0;
+  float2* group_x_l_ = nullptr;  // off-diagonal blocks of the inverses of the 128-row groups (FP32 factors)
   float2* group_x_u_ = nullptr;
   size_t group_x_cap_ = 0;
   int* perm_ = nullptr;       // pivots as one permutation
