@@ -132,6 +132,66 @@ __device__ __forceinline__ void run_item(const KdItem& it, const double* mats, d
   for (int e = threadIdx.x; e < n_out_elems; e += blockDim.x) dst[e] = X[e];
 }
 
+// The passes of one field from the lines' matrices in the pool, every entry of
+// them, for items without lists: nothing has to be compiled for a field that is
+// transformed once.  LP_CL CTAs of a cluster share a pass's outputs, stored into
+// all their buffers.  (Not inlined: the listed passes keep their registers.)
+template <int LP_CL>
+__device__ __noinline__ void run_plain(const KdItem& it, const double* __restrict__ pool, double* __restrict__ dst,
+                                       double* X, double* Y, int rank) {
+  namespace cg = cooperative_groups;
+  int d0 = it.n0, d1 = it.n1, d2 = it.n2, px = it.pitch;
+  for (int q = 0; q < it.npass; q++) {
+    const KdPass& p = it.pass[q];
+    const bool last = (q == it.npass - 1);
+    const int o0 = p.dim == 0 ? p.n_out : d0, o1 = p.dim == 1 ? p.n_out : d1, o2 = p.dim == 2 ? p.n_out : d2;
+    const int total = o0 * o1 * o2, nin = p.n_in;
+    for (int e = rank * blockDim.x + threadIdx.x; e < total; e += LP_CL * blockDim.x) {
+      const int c2 = e % o2, t = e / o2, c1 = t % o1, c0 = t / o1;
+      int row, off, base, stride;
+      if (p.dim == 0) {
+        row = c0;
+        off = p.mat[c1 * p.mat_ld + c2];
+        base = c1 * px + c2;
+        stride = d1 * px;
+      } else if (p.dim == 1) {
+        row = c1;
+        off = p.mat[c2];
+        base = c0 * d1 * px + c2;
+        stride = px;
+      } else {
+        row = c2;
+        off = p.mat[0];
+        base = (c0 * d1 + c1) * px;
+        stride = 1;
+      }
+      double acc = 0.0;
+      if (off >= 0) {
+        const double* M = pool + off + static_cast<long long>(row) * nin;
+#pragma unroll 4
+        for (int k = 0; k < nin; k++) acc = fma(__ldg(M + k), X[base + k * stride], acc);
+      }
+      if (last) {
+        dst[e] = acc * it.scale;
+      } else if (LP_CL == 1) {
+        Y[e] = acc;
+      } else {
+#pragma unroll
+        for (int r = 0; r < LP_CL; r++) cg::this_cluster().map_shared_rank(Y, r)[e] = acc;
+      }
+    }
+    if (last) return;
+    if (LP_CL == 1) __syncthreads();
+    else cg::this_cluster().sync();  // every CTA's Y is complete and nobody reads X any more
+    d0 = o0;
+    d1 = o1;
+    d2 = px = o2;
+    double* tmp = X;
+    X = Y;
+    Y = tmp;
+  }
+}
+
 // The item of field f of a launch.
 __device__ __forceinline__ int item_of(const KdItemList1&, int) { return 0; }
 __device__ __forceinline__ int item_of(const KdItemList& list, int f) {
@@ -158,7 +218,11 @@ __global__ void line_passes_kernel(const __grid_constant__ List list, const doub
     }
     copy_async_wait();
     __syncthreads();
-    run_item(it, it.nmats ? at : pool, it.out + field_in_item * it.out_stride, smem, smem + it.stage);
+    double* dst = it.out + field_in_item * it.out_stride;
+    if (it.pass[0].out)
+      run_item(it, it.nmats ? at : pool, dst, smem, smem + it.stage);
+    else
+      run_plain<1>(it, pool, dst, smem, smem + it.stage, 0);
     __syncthreads();
   }
 }
@@ -195,6 +259,10 @@ __global__ void line_passes_cluster_kernel(const __grid_constant__ List list, co
   copy_async_wait();
   __syncthreads();
   cluster.barrier_wait(std::move(started));
+  if (!it.pass[0].out) {
+    run_plain<LP_CL>(it, pool, dst, X, Y, rank);
+    return;
+  }
   const double* mats = it.nmats ? at : pool;
 #pragma unroll
   for (int q = 0; q < 3; q++) {

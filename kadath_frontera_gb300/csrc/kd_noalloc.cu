@@ -9,7 +9,7 @@
 // code running between the steps of such an application, where a cudaFree
 // would also synchronise the whole device.  Every GPU that loads the library
 // holds these arrays until the process exits (2 x 8 MiB of doubles plus
-// 681 KiB of table space).  The call allocates nothing: the per-line matrices
+// 64 KiB of table space).  The call allocates nothing: the per-line matrices
 // go into the context's matrix pool, which is allocated once when the context
 // is created.
 //
@@ -35,10 +35,7 @@ namespace kd {
 
 static __device__ __align__(256) double g_noalloc_in[KD_NOALLOC_MAX_DOUBLES];
 static __device__ __align__(256) double g_noalloc_out[KD_NOALLOC_MAX_DOUBLES];
-// The pass tables list four ints per output of each pass, and a stage of a
-// field that fits in shared memory holds at most 14,528 outputs.
-constexpr int kTabInts = 12 * 14528;
-static __device__ __align__(256) int g_noalloc_tab[kTabInts];
+static __device__ __align__(256) int g_noalloc_tab[KD_NOALLOC_MAX_TABLE];
 
 namespace {
 
@@ -105,23 +102,18 @@ void coef_host_noalloc(Context& ctx, const Base& base, const int np[3], const in
   const long long n_out = static_cast<long long>(nc[0]) * nc[1] * nc[2];
   if (n_in * batch > KD_NOALLOC_MAX_DOUBLES || n_out * batch > KD_NOALLOC_MAX_DOUBLES)
     throw KdError(KD_ERR_ARG, "kd_coef_host_noalloc: batch * field size exceeds KD_NOALLOC_MAX_DOUBLES");
-  if (1LL + nc[2] + static_cast<long long>(nc[1]) * nc[2] > KD_NOALLOC_MAX_TABLE)
-    throw KdError(KD_ERR_ARG, "kd_coef_host_noalloc: basis table exceeds KD_NOALLOC_MAX_TABLE");
-  // Tables of the three passes, laid out back to back.
-  std::vector<LinePassSpec> specs = coef_specs(ctx, base, np, nc);
-  LinePlan plan;
-  PassLists lists[3];
-  std::vector<double> mats;
+  // Per-line matrix offsets of the three passes, laid out back to back (no
+  // output lists: they would be compiled and uploaded again on every call).
+  const std::vector<LinePassSpec> specs = coef_specs(ctx, base, np, nc);
   std::vector<int> tab;
   size_t start[3];
-  compile_passes(ctx, specs, np, false, false, plan, lists, mats);  // matrices read from the pool
   for (int q = 0; q < 3; q++) {
     start[q] = tab.size();
-    const std::vector<int> t = pass_table(lists[q]);
-    tab.insert(tab.end(), t.begin(), t.end());
+    tab.insert(tab.end(), specs[q].offsets.begin(), specs[q].offsets.end());
   }
-  if (static_cast<long long>(tab.size()) > kTabInts)
-    throw KdError(KD_ERR_ARG, "kd_coef_host_noalloc: field too large");
+  if (static_cast<long long>(tab.size()) > KD_NOALLOC_MAX_TABLE)
+    throw KdError(KD_ERR_ARG, "kd_coef_host_noalloc: basis table exceeds KD_NOALLOC_MAX_TABLE");
+  LinePlan plan = plain_plan(specs, np);
   const DevicePtrs& p = device_ptrs(ctx.device());
   cudaStream_t s = ctx.stream();
   const double* pool = ctx.pool();  // uploads new matrices into the existing pool (no allocation)
@@ -131,9 +123,12 @@ void coef_host_noalloc(Context& ctx, const Base& base, const int np[3], const in
   list.nitems = 1;
   list.prefix[0] = 0;
   list.prefix[1] = batch;
-  for (int q = 0; q < 3; q++) set_pass_table(plan.pass[q], p.tab + start[q]);
+  for (int q = 0; q < 3; q++) plan.pass[q].mat = p.tab + start[q];
   list.items[0] = make_item(plan, p.in, p.out, np, n_in, n_out, 1.0);
-  cuda_check(launch_line_passes(list, pool, s), "line_passes kernel (no-alloc)");
+  // few fields share 8 CTAs each, else a CTA a field
+  LpShape shape;
+  shape.cluster = batch <= 32 ? 8 : 1;
+  cuda_check(launch_line_passes(list, pool, s, shape), "line_passes kernel (no-alloc)");
   ctx.launches++;
   cuda_check(cudaMemcpyAsync(h_out, p.out, sizeof(double) * n_out * batch, cudaMemcpyDeviceToHost, s), "D2H");
   cuda_check(cudaStreamSynchronize(s), "sync");

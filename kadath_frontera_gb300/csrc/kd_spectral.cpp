@@ -163,6 +163,12 @@ struct Line {
   int x, y;  // first input and output element
 };
 
+// What a pass's table holds: its outputs, then its mirrored pairs.
+struct PassLists {
+  std::vector<KdOut> outs;
+  std::vector<int> before, after;
+};
+
 // Outputs and mirrored pairs of one pass over a block of dims d with row (phi)
 // pitches px (input) and py (output).  place(matrix, folded) says where a
 // matrix lies among the ones the kernel reads.
@@ -245,9 +251,9 @@ void list_pass(Context& ctx, const LinePassSpec& s, const int d[3], int px, int 
   out.outs.insert(out.outs.end(), zeros.begin(), zeros.end());
 }
 
-}  // namespace
-
-void compile_passes(Context& ctx, const std::vector<LinePassSpec>& specs, const int dims_in[3], bool fold, bool stage,
+// The passes of a plan over a field of dims_in, their lists and the matrices to
+// stage (none when they do not fit).
+void compile_passes(Context& ctx, const std::vector<LinePassSpec>& specs, const int dims_in[3], bool fold,
                     LinePlan& plan, PassLists lists[3], std::vector<double>& mats) {
   if (specs.empty() || specs.size() > 3) throw KdError(KD_ERR_ARG, "one to three passes per item");
   plan.npass = static_cast<int>(specs.size());
@@ -271,14 +277,12 @@ void compile_passes(Context& ctx, const std::vector<LinePassSpec>& specs, const 
   // the matrices beside the stages when they fit; otherwise the kernel reads
   // the (unfolded) ones of the pool
   std::map<std::pair<size_t, bool>, int> at;
-  if (stage) {
-    long long room = MAX_SMEM_DOUBLES - 2 * stage_doubles;
-    std::set<int> seen;
-    for (const LinePassSpec& s : specs)
-      for (int off : s.offsets)
-        if (off >= 0 && seen.insert(off).second) room -= (static_cast<long long>(s.n_in) * s.n_out + 1) & ~1LL;
-    stage = room >= 0;
-  }
+  long long room = MAX_SMEM_DOUBLES - 2 * stage_doubles;
+  std::set<int> seen;
+  for (const LinePassSpec& s : specs)
+    for (int off : s.offsets)
+      if (off >= 0 && seen.insert(off).second) room -= (static_cast<long long>(s.n_in) * s.n_out + 1) & ~1LL;
+  const bool stage = room >= 0;
   auto place = [&](const Mat1d& m, bool folded) -> int {
     if (!stage) return static_cast<int>(m.pool_offset);
     auto key = std::make_pair(m.pool_offset, folded);
@@ -324,13 +328,11 @@ void set_pass_table(KdPass& p, const int* table) {
   p.pairs = table + 4 * static_cast<size_t>(p.nout);
 }
 
-namespace {
-
 void compile_plan(Context& ctx, const std::vector<LinePassSpec>& specs, const int dims_in[3], bool fold,
                   LinePlan& plan) {
   PassLists lists[3];
   std::vector<double> mats;
-  compile_passes(ctx, specs, dims_in, fold, true, plan, lists, mats);
+  compile_passes(ctx, specs, dims_in, fold, plan, lists, mats);
   for (int q = 0; q < plan.npass; q++) set_pass_table(plan.pass[q], ctx.table(pass_table(lists[q])));
   plan.mats = mats.empty() ? nullptr : ctx.dtable(mats);
 }
@@ -346,6 +348,30 @@ std::vector<int> plan_key(int op, int dim, const Base& b, const int n_in[3], con
 }
 
 }  // namespace
+
+LinePlan plain_plan(const std::vector<LinePassSpec>& specs, const int dims_in[3]) {
+  LinePlan plan;
+  plan.npass = static_cast<int>(specs.size());
+  int d[3] = {dims_in[0], dims_in[1], dims_in[2]};
+  long long m = static_cast<long long>(d[0]) * d[1] * d[2];
+  for (int q = 0; q < plan.npass; q++) {
+    const LinePassSpec& s = specs[q];
+    KdPass& p = plan.pass[q];
+    p.dim = s.dim;
+    p.n_in = s.n_in;
+    p.n_out = s.n_out;
+    p.mat_ld = s.mat_ld;
+    d[s.dim] = s.n_out;
+    m = std::max(m, static_cast<long long>(d[0]) * d[1] * d[2]);
+  }
+  m = (m + 1) & ~1LL;
+  if (2 * m > MAX_SMEM_DOUBLES)
+    throw KdError(KD_ERR_CUDA, "line_passes kernel: a field of this size does not fit in an SM's shared memory");
+  plan.stage = static_cast<int>(m);
+  plan.pitch = dims_in[2];
+  for (int i = 0; i < 3; i++) plan.dims_in[i] = dims_in[i];
+  return plan;
+}
 
 const LinePlan& coef_plan(Context& ctx, const Base& base, const int np[3], const int nc[3], bool inverse,
                           long long fields) {

@@ -50,18 +50,9 @@ std::vector<LinePassSpec> coef_i_specs(Context& ctx, const Base& base, const int
 // same domain: r, theta, then phi, each line through OP_RESAMPLE.
 std::vector<LinePassSpec> resample_specs(Context& ctx, const Base& base, const int nc_old[3], const int np_new[3]);
 
-// What a pass's table holds: its outputs, then its mirrored pairs.
-struct PassLists {
-  std::vector<KdOut> outs;
-  std::vector<int> before, after;
-};
-// The passes of a plan over a field of dims_in, their lists and the matrices
-// to stage (none when `stage` is off or they do not fit).  The caller puts the
-// lists and matrices into device memory and sets the plan's pointers.
-void compile_passes(Context& ctx, const std::vector<LinePassSpec>& specs, const int dims_in[3], bool fold, bool stage,
-                    LinePlan& plan, PassLists lists[3], std::vector<double>& mats);
-std::vector<int> pass_table(const PassLists& l);
-void set_pass_table(KdPass& p, const int* table);
+// The passes of a field of dims_in without output lists, rows unpadded; the caller
+// sets the lines' matrices (KdPass::mat).
+LinePlan plain_plan(const std::vector<LinePassSpec>& specs, const int dims_in[3]);
 
 // Compiled pass lists, kept by the context by what they depend on (operator,
 // dims, every line's basis).  A transform of more than FOLD_MIN_FIELDS fields
