@@ -304,7 +304,8 @@ struct BatchScope {
 // that dim.  Used by transforms and by coefficient-space operators.
 struct LinePassSpec {
   int dim, n_in, n_out, mat_ld;
-  std::vector<int> offsets;  // per line, -1 for zero lines
+  std::vector<int> offsets;  // per line: its matrix in the pool, -1 for a zero line
+  std::vector<char> dead;    // phi columns whose lines may be left out where all values are finite (or empty)
 };
 
 }  // namespace kd

@@ -27,7 +27,8 @@ struct KdPass {
   const KdOut* out;    // null in every pass of an item: no lists, see mat
   const int* pairs;    // first element | second << 16: before, then after
   // The lines' matrices (row-major n_out x n_in) as offsets in doubles into the
-  // pool, -1 for a line whose output is zero, for passes without lists:
+  // pool, -1 for a line whose output is zero, for passes without lists and for
+  // fields with non-finite values:
   //   dim 0 (r):     mat[j * mat_ld + k]   (basis depends on theta/phi indices)
   //   dim 1 (theta): mat[k]                (basis depends on the phi index)
   //   dim 2 (phi):   mat[0]

@@ -72,21 +72,17 @@ std::vector<LinePassSpec> coef_specs(Context& ctx, const Base& base, const int n
   const Mat1d& phi = ctx.bank().at(ctx.bank().get(OP_COEF, base.p, np[2], nc[2]));
   std::vector<char> dead(nc[2]);
   for (int k = 0; k < nc[2]; k++) dead[k] = phi.row_zero(k);
+  v[1].dead = v[2].dead = dead;
   v[1].offsets.resize(nc[2]);
-  for (int k = 0; k < nc[2]; k++) {
-    const int off = mat_offset(ctx, OP_COEF, base.t[k], np[1], nc[1], nullptr);
-    v[1].offsets[k] = dead[k] ? -1 : off;
-  }
+  for (int k = 0; k < nc[2]; k++) v[1].offsets[k] = mat_offset(ctx, OP_COEF, base.t[k], np[1], nc[1], nullptr);
   v[2].dim = 0;
   v[2].n_in = np[0];
   v[2].n_out = nc[0];
   v[2].mat_ld = nc[2];
   v[2].offsets.resize(static_cast<size_t>(nc[1]) * nc[2]);
   for (int j = 0; j < nc[1]; j++)
-    for (int k = 0; k < nc[2]; k++) {
-      const int off = mat_offset(ctx, OP_COEF, base.rb(j, k), np[0], nc[0], nullptr);
-      v[2].offsets[j * nc[2] + k] = dead[k] ? -1 : off;
-    }
+    for (int k = 0; k < nc[2]; k++)
+      v[2].offsets[j * nc[2] + k] = mat_offset(ctx, OP_COEF, base.rb(j, k), np[0], nc[0], nullptr);
   return v;
 }
 
@@ -105,19 +101,15 @@ std::vector<LinePassSpec> coef_i_specs(Context& ctx, const Base& base, const int
   v[0].mat_ld = nc[2];
   v[0].offsets.resize(static_cast<size_t>(nc[1]) * nc[2]);
   for (int j = 0; j < nc[1]; j++)
-    for (int k = 0; k < nc[2]; k++) {
-      const int off = mat_offset(ctx, OP_COEF_I, base.rb(j, k), nc[0], np[0], nullptr);
-      v[0].offsets[j * nc[2] + k] = dead[k] ? -1 : off;
-    }
+    for (int k = 0; k < nc[2]; k++)
+      v[0].offsets[j * nc[2] + k] = mat_offset(ctx, OP_COEF_I, base.rb(j, k), nc[0], np[0], nullptr);
+  v[0].dead = v[1].dead = dead;
   v[1].dim = 1;
   v[1].n_in = nc[1];
   v[1].n_out = np[1];
   v[1].mat_ld = 0;
   v[1].offsets.resize(nc[2]);
-  for (int k = 0; k < nc[2]; k++) {
-    const int off = mat_offset(ctx, OP_COEF_I, base.t[k], nc[1], np[1], nullptr);
-    v[1].offsets[k] = dead[k] ? -1 : off;
-  }
+  for (int k = 0; k < nc[2]; k++) v[1].offsets[k] = mat_offset(ctx, OP_COEF_I, base.t[k], nc[1], np[1], nullptr);
   v[2].dim = 2;
   v[2].n_in = nc[2];
   v[2].n_out = np[2];
@@ -195,6 +187,7 @@ void list_pass(Context& ctx, const LinePassSpec& s, const int d[3], int px, int 
         off = s.offsets[0];
         l = {(a * d[1] + b) * px, (a * d[1] + b) * py};
       }
+      if (s.dim != 2 && !s.dead.empty() && s.dead[b]) off = -1;
       if (off < 0) {
         for (int r = 0; r < s.n_out; r++) zeros.push_back({0, 0, l.y + r * ys, 0});
         continue;
@@ -333,7 +326,11 @@ void compile_plan(Context& ctx, const std::vector<LinePassSpec>& specs, const in
   PassLists lists[3];
   std::vector<double> mats;
   compile_passes(ctx, specs, dims_in, fold, plan, lists, mats);
-  for (int q = 0; q < plan.npass; q++) set_pass_table(plan.pass[q], ctx.table(pass_table(lists[q])));
+  for (int q = 0; q < plan.npass; q++) {
+    set_pass_table(plan.pass[q], ctx.table(pass_table(lists[q])));
+    plan.pass[q].mat = ctx.table(specs[q].offsets);
+    plan.pass[q].mat_ld = specs[q].mat_ld;
+  }
   plan.mats = mats.empty() ? nullptr : ctx.dtable(mats);
 }
 
