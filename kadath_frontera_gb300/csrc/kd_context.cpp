@@ -184,7 +184,9 @@ void Context::mark(std::initializer_list<const void*> reads, const void* write, 
 bool Context::defer_item(const LinePlan& plan, const double* in, double* out) {
   // larger fields keep their launches of a cluster per field: one CTA would
   // take longer than the launch it saves (60 us for a (25,13,14) transform)
-  if (!batch_.on || plan.stage > 3000) return false;
+  // (nor do the kernel's own 256 bytes of shared memory fit beside what a field's
+  // own launch may take)
+  if (!batch_.on || plan.stage > 3000 || 2 * plan.stage + plan.nmats > 227 * 1024 / 8 - 128) return false;
   if (!plan.dev) {
     if (capturing) return false;
     const KdItem it = make_item(plan, nullptr, nullptr, plan.dims_in, 0, 0, 1.0);
