@@ -422,11 +422,4 @@ KdItem make_item(const LinePlan& plan, const double* in, double* out, const int 
   return it;
 }
 
-KdItem make_item(Context& ctx, const std::vector<LinePassSpec>& specs, const double* in, double* out,
-                 const int dims_in[3], long long in_stride, long long out_stride, double scale) {
-  LinePlan plan;
-  compile_plan(ctx, specs, dims_in, false, plan);
-  return make_item(plan, in, out, dims_in, in_stride, out_stride, scale);
-}
-
 }  // namespace kd

@@ -68,8 +68,4 @@ const LinePlan& ope_1d_plan(Context& ctx, int op, int dim, const Base& base, con
 KdItem make_item(const LinePlan& plan, const double* in, double* out, const int dims_in[3], long long in_stride,
                  long long out_stride, double scale);
 
-// Turns pass specs into a kernel item (device tables resolved through ctx).
-KdItem make_item(Context& ctx, const std::vector<LinePassSpec>& specs, const double* in, double* out,
-                 const int dims_in[3], long long in_stride, long long out_stride, double scale);
-
 }  // namespace kd

@@ -77,7 +77,10 @@ void regrid(Field& dst, Field& src) {
     list.nitems = 1;
     list.prefix[0] = 0;
     list.prefix[1] = 1;
-    list.items[0] = make_item(ctx, specs, v.cf, pn.c, nco, dmo.ncoefs(), dmn.npts(), 1.0);
+    // (one field: compiling lists would take longer than the passes save)
+    LinePlan plan = plain_plan(specs, nco);
+    for (int q = 0; q < plan.npass; q++) plan.pass[q].mat = ctx.table(specs[q].offsets);
+    list.items[0] = make_item(plan, v.cf, pn.c, nco, dmo.ncoefs(), dmn.npts(), 1.0);
     cuda_check(launch_line_passes(list, ctx.pool(), ctx.stream()), "regrid line passes");
     ctx.launches++;
     cuda_check(cudaStreamSynchronize(ctx.stream()), "sync regrid");
