@@ -10,10 +10,13 @@
 // product of slices i and j has integer entries, summed exactly in FP32: an
 // order o = i + j adds at most 8 pairs of k <= 128 products below 2^14, at
 // most 2^24 in all.  Orders 2..9 (36 of the 64 pairs) are kept.  Before
-// splitting, row k of B is scaled by a power of two to a largest entry in
-// [1/2, 1) and column k of A by its inverse, so that rows of B of very different
-// sizes (a Jacobian's second derivatives beside its boundary rows) do not cost
-// each other digits.
+// splitting, row k of B is scaled by a power of two and column k of A by its
+// inverse so that the mean exponents of their nonzero entries agree: then the k
+// that are large in A's rows are those that are large in B's columns, and rows of
+// B of very different sizes (a Jacobian's second derivatives beside its boundary
+// rows) do not cost each other digits.  (With the largest entry of row k of B at 1
+// instead, one outlier moved the whole row: of a matrix of 8,000 rows over six
+// decades 54 million entries had to be listed below, 0.7 million now.)
 //
 // Error.  With R the bound 2^(row's scale + column's scale) of the products of
 // an entry, the orders left out and the rounding of the digits come to about
@@ -25,32 +28,32 @@
 //   column's scale (bit masks made while packing), or
 //   the sum itself, or the updated entry, is at least 2^-4 R in size.
 // Every other entry, and every entry of a row or column with Inf or NaN, is left
-// as it is and listed, and sum_listed forms it in FP64, term by term in the order
-// of k over the k that are nonzero in both operands, as a plain product would.
+// as it is and listed, and sum_listed forms it in FP64, as a plain product would.
 // Unknowns in different units need that: where one row of B is small in every
 // column but those of its own group, the sums in that group's columns are far
 // below R (groups 40 binades apart: componentwise backward errors of 1e-8 to 1e-2
 // with the slices alone, 7e-16 now and with LAPACK).  Sparse Jacobians too: of the
-// star's entries 0.4 % (index notation) to 2.4 % are listed.
+// star's entries 0.5 % (index notation) to 2.9 % are listed.
 //
 // One persistent CTA per SM, 128 x 64 tiles:
 //   warp 0   TMA loads of operand chunks: k = 32 of all eight slices of A and
 //            B (96 KB, 64-byte swizzle), two stages;
 //   warp 1   72 MMAs per chunk (M 128, N 64, K 16) into eight accumulators of
 //            64 TMEM columns, one per order: all 512 columns;
-//   warps 2-9 epilogue: the eight orders of an entry into one 64-bit integer
-//            (shifted by its size: the low orders are kept whole where they
-//            reach its first 53 bits), TMEM released, then C -= integer * 2^e
-//            (one conversion and one multiply-add on the FP64 pipe) beside the
-//            next tile's MMAs, and the list of the entries to sum in FP64.
+//   warps 2-17 epilogue: the eight orders of an entry into one integer of 80
+//            bits, TMEM released, then C -= its first 62 bits * 2^e (one
+//            conversion and one multiply-add on the FP64 pipe) beside the next
+//            tile's MMAs, and the list of the entries to sum in FP64.
 // Bound: the MMAs' operand reads from shared memory (48 cycles per MMA of 32)
 // and the hand-over of the single set of accumulators.  128 x 64 tiles and not
 // 128 x 128: eight orders of 64 columns are all of TMEM, and one pass over the
 // operands serves all of them.
-// All updates of a factorisation of the star's Jacobian, with packing and the
-// listed entries, against the library's FP64 GEMM: N = 7,819 24 (index notation)
-// and 30 against 301 ms, N = 12,331 97 against 1,172 ms; without the listed
-// entries 20 and 62 ms.
+// Sixteen epilogue warps: with eight, of 32 columns each, their integer work was
+// longer than a tile's MMAs (all updates at N = 8,000: 32 against 23 ms).
+// All updates of a factorisation, with packing and the listed entries, against the
+// library's FP64 GEMM: a dense matrix of N = 8,000 with rows over six decades 23
+// against 319 ms, the star's Jacobian at N = 7,819 22 (index notation) and 28
+// against 301, at N = 12,331 91 against 1,172.
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -72,7 +75,9 @@ constexpr int S_A_SLICE = S_M * S_KC * 2;                // bytes of one slice o
 constexpr int S_B_SLICE = S_N * S_KC * 2;
 constexpr int S_STAGE = S_SLICES * (S_A_SLICE + S_B_SLICE);
 constexpr int S_NST = 2;
-constexpr int S_THREADS = 320;
+constexpr int S_EPI = 16;                                // epilogue warps
+constexpr int S_THREADS = 64 + 32 * S_EPI;
+constexpr int S_COLS = S_N / (S_EPI / 4);                // columns of an epilogue thread
 constexpr size_t S_SMEM = 1024 + static_cast<size_t>(S_NST) * S_STAGE;
 constexpr unsigned long long S_WAIT_NS = 2000000000ull;
 constexpr int EXP_NONFINITE = 1 << 20;                   // scale of a row or column that holds Inf or NaN
@@ -126,31 +131,61 @@ __device__ __forceinline__ void digits_of(long long f, __nv_bfloat16 (&d)[S_SLIC
     d[s] = __float2bfloat16_rn(static_cast<float>(static_cast<int>((g >> (8 * (7 - s))) & 255) - 128));
 }
 
-// xk[kk] = max over the columns of the exponents of row kk of B (k x n,
-// column-major); xk starts at EXP_ZERO.
-__global__ void slice_row_exponents(const double* __restrict__ B, long long ldb, int k, int n, int cols,
-                                    int* __restrict__ xk) {
-  const int kk = threadIdx.x;
-  if (kk >= k) return;
-  const int c0 = blockIdx.x * cols, c1 = min(n, c0 + cols);
-  int m = EXP_ZERO;
+// Sums and numbers of the exponents of the nonzero finite entries of B's rows and
+// A's columns, stat[quantity][kk]: 0 and 1 of B (k x n, column-major), 2 and 3 of A
+// (m x k); stat starts at zero.  The first `nb` CTAs take STAT_COLS columns of B
+// each, the others STAT_ROWS rows of one column of A.
+constexpr int STAT_THREADS = 128, STAT_COLS = 32, STAT_ROWS = 2048;
+__global__ void __launch_bounds__(STAT_THREADS) slice_exponents(const double* __restrict__ A, long long lda, int m,
+                                                                const double* __restrict__ B, long long ldb, int k,
+                                                                int n, int nb, int* __restrict__ stat) {
+  static_assert(STAT_THREADS >= S_MAXK, "a thread a row of B");
+  int sum = 0, count = 0;
+  auto take = [&](double v) {
+    const int e = exponent_of(v);
+    if (e == EXP_NONFINITE || e == EXP_ZERO) return;
+    sum += e;
+    count++;
+  };
+  if (static_cast<int>(blockIdx.x) < nb) {
+    const int kk = threadIdx.x, c0 = blockIdx.x * STAT_COLS, c1 = min(n, c0 + STAT_COLS);
+    if (kk >= k) return;
 #pragma unroll 8
-  for (int c = c0; c < c1; c++) {
-    const int e = exponent_of(B[static_cast<long long>(c) * ldb + kk]);
-    if (e != EXP_NONFINITE) m = max(m, e);
+    for (int c = c0; c < c1; c++) take(B[static_cast<long long>(c) * ldb + kk]);
+    if (count) {
+      atomicAdd(stat + kk, sum);
+      atomicAdd(stat + S_MAXK + kk, count);
+    }
+    return;
   }
-  if (m != EXP_ZERO) atomicMax(xk + kk, m);
+  const int t = blockIdx.x - nb, kk = t % k, r0 = t / k * STAT_ROWS, r1 = min(m, r0 + STAT_ROWS);
+  const double* a = A + static_cast<long long>(kk) * lda;
+#pragma unroll 8
+  for (int r = r0 + threadIdx.x; r < r1; r += STAT_THREADS) take(a[r]);
+  sum = __reduce_add_sync(0xffffffffu, sum);
+  count = __reduce_add_sync(0xffffffffu, count);
+  if ((threadIdx.x & 31) == 0 && count) {
+    atomicAdd(stat + 2 * S_MAXK + kk, sum);
+    atomicAdd(stat + 3 * S_MAXK + kk, count);
+  }
 }
 
-// The exponents' start, and a zero behind them (the length of the list).
-__global__ void slice_fill(int* __restrict__ v, int n, int x) {
-  if (static_cast<int>(threadIdx.x) < n) v[threadIdx.x] = x;
-  if (threadIdx.x == 0) v[n] = 0;
+// The exponent that row kk of B is divided by and column kk of A multiplied by.
+__device__ __forceinline__ int balance(const int* __restrict__ stat, int kk) {
+  const int nb = stat[S_MAXK + kk], na = stat[3 * S_MAXK + kk];
+  if (nb == 0 || na == 0) return 0;
+  return __float2int_rn(0.5f * (static_cast<float>(stat[kk]) / nb - static_cast<float>(stat[2 * S_MAXK + kk]) / na));
+}
+
+// Zeros: the statistics and, behind them, the length of the list.
+constexpr int STAT_INTS = 4 * S_MAXK + 4;
+__global__ void slice_clear(int* __restrict__ v) {
+  for (int i = threadIdx.x; i < STAT_INTS; i += blockDim.x) v[i] = 0;
 }
 
 // Slices of B: out[s][column][kk] and the columns' scales; one warp a column.
 __global__ void slice_pack_b(const double* __restrict__ B, long long ldb, int k, int n, int kpad, int npad,
-                             const int* __restrict__ xk, __nv_bfloat16* __restrict__ out, int* __restrict__ scale,
+                             const int* __restrict__ stat, __nv_bfloat16* __restrict__ out, int* __restrict__ scale,
                              uint4* __restrict__ masks) {
   const int col = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (col >= npad) return;
@@ -161,8 +196,7 @@ __global__ void slice_pack_b(const double* __restrict__ B, long long ldb, int k,
   for (int q = 0; q < 4; q++) {
     const int kk = 2 * lane + (q & 1) + 64 * (q >> 1);
     v[q] = (col < n && kk < k) ? B[static_cast<long long>(col) * ldb + kk] : 0.0;
-    x[q] = kk < k ? xk[kk] : 0;
-    if (x[q] == EXP_ZERO) x[q] = 0;
+    x[q] = kk < k ? balance(stat, kk) : 0;
     ex[q] = exponent_of(v[q]);
     if (ex[q] == EXP_NONFINITE) bad = true;
     else if (ex[q] != EXP_ZERO) mx = max(mx, ex[q] - x[q]);
@@ -198,16 +232,13 @@ __global__ void slice_pack_b(const double* __restrict__ B, long long ldb, int k,
 // rows a CTA, staged so that reads run along rows and writes along kk.
 constexpr int SA_ROWS = 32;
 __global__ void __launch_bounds__(256) slice_pack_a(const double* __restrict__ A, long long lda, int m, int k,
-                                                    int kpad, int mpad, const int* __restrict__ xk,
+                                                    int kpad, int mpad, const int* __restrict__ stat,
                                                     __nv_bfloat16* __restrict__ out, int* __restrict__ scale,
                                                     unsigned* __restrict__ masks) {
   __shared__ double t[S_MAXK][SA_ROWS + 1];
   __shared__ int x[S_MAXK], part[8][SA_ROWS], sc[SA_ROWS];
   const int r0 = blockIdx.x * SA_ROWS, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  for (int e = threadIdx.x; e < S_MAXK; e += blockDim.x) {
-    const int v = e < k ? xk[e] : 0;
-    x[e] = v == EXP_ZERO ? 0 : v;
-  }
+  for (int e = threadIdx.x; e < S_MAXK; e += blockDim.x) x[e] = e < k ? balance(stat, e) : 0;
   __syncthreads();
   int mx = EXP_ZERO;
   for (int kk = w; kk < kpad; kk += 8) {
@@ -300,9 +331,9 @@ __device__ constexpr uint32_t bf16_idesc(int M, int N) {
          (static_cast<uint32_t>(M >> 4) << 24);
 }
 
-__device__ __forceinline__ void tmem_load8(uint32_t addr, uint32_t (&r)[8]) {
-  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+__device__ __forceinline__ void tmem_load4(uint32_t addr, uint32_t (&r)[4]) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
                : "r"(addr));
 }
 
@@ -327,7 +358,7 @@ __global__ void __launch_bounds__(S_THREADS, 1)
     }
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(&acc_full)));
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(&drained)));
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 8;" ::"r"(smem_addr(&acc_empty)));  // the epilogue's warps
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(&acc_empty)), "n"(S_EPI));
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&mapA)) : "memory");
     asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&mapB)) : "memory");
@@ -421,8 +452,8 @@ __global__ void __launch_bounds__(S_THREADS, 1)
                    : "memory");
       if (!s_wait(&drained, 0)) *abort_v = 1;
     }
-  } else {  // ---------------------------------------------- epilogue (2-9)
-    const int quarter = warp & 3, half = (warp - 2) >> 2;
+  } else {  // --------------------------------------------- epilogue (2-17)
+    const int quarter = warp & 3, part = (warp - 2) >> 2;
     int it = 0;
     for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x, it++) {
       const int tm = tile % ntm, tn = tile / ntm;
@@ -431,65 +462,59 @@ __global__ void __launch_bounds__(S_THREADS, 1)
         break;
       }
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      long long v[32];
-      unsigned whole = 0, most = 0;  // entries shifted up by 16 and by 8, the others by 4
-      const uint32_t t0 = tmem + (static_cast<uint32_t>(quarter * 32) << 16) + static_cast<uint32_t>(half * 32);
+      // a sum in units of 2^-68 R: v 2^16 + low
+      long long v[S_COLS];
+      unsigned low[S_COLS / 2];
+      const uint32_t t0 = tmem + (static_cast<uint32_t>(quarter * 32) << 16) + static_cast<uint32_t>(part * S_COLS);
 #pragma unroll
-      for (int c8 = 0; c8 < 32; c8 += 8) {
-        uint32_t r[S_SLICES][8];
+      for (int c4 = 0; c4 < S_COLS; c4 += 4) {
+        uint32_t r[S_SLICES][4];
 #pragma unroll
-        for (int o = 0; o < S_SLICES; o++) tmem_load8(t0 + static_cast<uint32_t>(o * S_N + c8), r[o]);
+        for (int o = 0; o < S_SLICES; o++) tmem_load4(t0 + static_cast<uint32_t>(o * S_N + c4), r[o]);
         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-        for (int q = 0; q < 8; q++) {
+        for (int q = 0; q < 4; q++) {
           // orders 2..7 weigh 2^40 .. 1, orders 8 and 9 2^-8 and 2^-16
           long long hi = 0;
 #pragma unroll
           for (int o = 0; o < 6; o++) hi = (hi << 8) + __float2int_rn(__uint_as_float(r[o][q]));
           const long long lo = (static_cast<long long>(__float2int_rn(__uint_as_float(r[6][q]))) << 8) +
                                __float2int_rn(__uint_as_float(r[7][q]));
-          // |hi| < 2^59 and |lo| < 2^33: the bits of lo that a double of the
-          // sum can hold
-          const long long size = hi < 0 ? -hi : hi;
-          if (size < 1ll << 46) {
-            v[c8 + q] = (hi << 16) + lo;
-            whole |= 1u << (c8 + q);
-          } else if (size < 1ll << 54) {
-            v[c8 + q] = (hi << 8) + ((lo + 128) >> 8);
-            most |= 1u << (c8 + q);
-          } else {
-            v[c8 + q] = (hi << 4) + ((lo + 2048) >> 12);
-          }
+          v[c4 + q] = hi + (lo >> 16);
+          const unsigned l = static_cast<unsigned>(lo) & 0xffffu;
+          if (q & 1) low[(c4 + q) / 2] |= l << 16;
+          else low[(c4 + q) / 2] = l;
         }
       }
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       __syncwarp();
       if (lane == 0)
         asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_addr(&acc_empty)) : "memory");
-      // C -= v 2^(ea + fb - 52 - shift)
+      // C -= s 2^(ea + fb - 52 - shift), s the first 62 bits of a sum
       const int row = tm * S_M + quarter * 32 + lane;
-      const int col0 = tn * S_N + half * 32;
+      const int col0 = tn * S_N + part * S_COLS;
       const int er = ea[row];
       const uint4 near_a = ma[2 * row];  // rows and columns up to a whole tile are packed
       double* cp = C + static_cast<long long>(col0) * ldc + row;
 #pragma unroll
-      for (int c8 = 0; c8 < 32; c8 += 8) {
-        double c[8];
+      for (int c4 = 0; c4 < S_COLS; c4 += 4) {
+        double c[4];
         unsigned exact = 0;  // entries to sum in FP64: left as they are
 #pragma unroll
-        for (int q = 0; q < 8; q++)
-          c[q] = row < m && col0 + c8 + q < n ? cp[static_cast<long long>(c8 + q) * ldc] : 0.0;
+        for (int q = 0; q < 4; q++)
+          c[q] = row < m && col0 + c4 + q < n ? cp[static_cast<long long>(c4 + q) * ldc] : 0.0;
 #pragma unroll
-        for (int q = 0; q < 8; q++) {
-          const int ec = fb[col0 + c8 + q];
+        for (int q = 0; q < 4; q++) {
+          const int ec = fb[col0 + c4 + q];
           if (er == EXP_NONFINITE || ec == EXP_NONFINITE) {
             exact |= 1u << q;
             continue;
           }
           if (er == EXP_ZERO || ec == EXP_ZERO) continue;
-          const unsigned bit = 1u << (c8 + q);
-          const int shift = (whole & bit) ? 16 : (most & bit) ? 8 : 4;
-          const long long s = v[c8 + q];
+          const long long hi = v[c4 + q];
+          const unsigned l = (low[(c4 + q) / 2] >> (16 * (q & 1))) & 0xffffu;
+          const int shift = min(16, __clzll(hi < 0 ? ~hi : hi) - 2);
+          const long long s = (hi << shift) + (l >> (16 - shift));
           if (s != 0) {
             const int e = er + ec - 52 - shift + 1023;
             const double x = static_cast<double>(s);
@@ -498,7 +523,7 @@ __global__ void __launch_bounds__(S_THREADS, 1)
             else
               c[q] -= scalbn(x, e - 1023);
           }
-          const uint4 near_b = mb[2 * (col0 + c8 + q)];
+          const uint4 near_b = mb[2 * (col0 + c4 + q)];
           const int near = __popc(near_a.x & near_b.x) + __popc(near_a.y & near_b.y) + __popc(near_a.z & near_b.z) +
                            __popc(near_a.w & near_b.w);
           const long long size = s < 0 ? -s : s;
@@ -509,21 +534,21 @@ __global__ void __launch_bounds__(S_THREADS, 1)
         if (__any_sync(0xffffffffu, exact != 0u)) {
           unsigned rows = 0;  // lane q: the rows listed of column q
 #pragma unroll
-          for (int q = 0; q < 8; q++) {
+          for (int q = 0; q < 4; q++) {
             const unsigned w = __ballot_sync(0xffffffffu, (exact >> q) & 1u);
-            if (lane == q && col0 + c8 + q < n) rows = w;
+            if (lane == q && col0 + c4 + q < n) rows = w;
           }
           const unsigned have = __ballot_sync(0xffffffffu, rows != 0u);
           unsigned at = 0;
           if (lane == 0) at = atomicAdd(listed, static_cast<unsigned>(__popc(have)));
           at = __shfl_sync(0xffffffffu, at, 0) + __popc(have & ((1u << lane) - 1u));
           // a place is 32 rows of a column: fewer than 2^32 of them
-          if (rows) list[at] = make_uint2(rows, static_cast<unsigned>(tm * (S_M / 32) + quarter) * n + col0 + c8 + lane);
+          if (rows) list[at] = make_uint2(rows, static_cast<unsigned>(tm * (S_M / 32) + quarter) * n + col0 + c4 + lane);
         }
         if (row < m) {
 #pragma unroll
-          for (int q = 0; q < 8; q++)
-            if (col0 + c8 + q < n && !((exact >> q) & 1u)) cp[static_cast<long long>(c8 + q) * ldc] = c[q];
+          for (int q = 0; q < 4; q++)
+            if (col0 + c4 + q < n && !((exact >> q) & 1u)) cp[static_cast<long long>(c4 + q) * ldc] = c[q];
         }
       }
     }
@@ -541,8 +566,12 @@ __global__ void __launch_bounds__(S_THREADS, 1)
 // else latency; every SM full of warps, so that the loads of some (eight k at a
 // time) hide behind others.  (The epilogue did this first, and then warps by
 // column of the matrix: what is listed comes in clusters, so a few warps had most
-// of it, and the updates of the N = 7,819 factorisation took 49 ms, now 24.)
+// of it, and the updates of the N = 7,819 factorisation took 49 ms, now 22.)
 constexpr int SUM_THREADS = 256;
+// Rows of a place up to which they go one after the other, 32 lanes a row (3 or 4
+// multiply-adds and 5 additions of a warp each), instead of side by side (k
+// multiply-adds for all).
+constexpr int SUM_FEW = 8;
 __global__ void __launch_bounds__(SUM_THREADS) sum_listed(const uint2* __restrict__ list,
                                                          const unsigned* __restrict__ listed, const int* __restrict__ ea,
                                                          const int* __restrict__ fb, const uint4* __restrict__ ma,
@@ -555,7 +584,25 @@ __global__ void __launch_bounds__(SUM_THREADS) sum_listed(const uint2* __restric
   for (unsigned at = blockIdx.x * (SUM_THREADS / 32) + (threadIdx.x >> 5); at < count; at += step) {
     const uint2 e = list[at];
     const int col = static_cast<int>(e.y % static_cast<unsigned>(n));
-    const int row = static_cast<int>(e.y / static_cast<unsigned>(n)) * 32 + lane;
+    const int row0 = static_cast<int>(e.y / static_cast<unsigned>(n)) * 32, row = row0 + lane;
+    const double* pb = B + static_cast<long long>(col) * ldb;
+    if (__popc(e.x) <= SUM_FEW) {  // the lanes share each row's terms
+      double v[MASK_WORDS];
+#pragma unroll
+      for (int q = 0; q < MASK_WORDS; q++) v[q] = lane + 32 * q < k ? pb[lane + 32 * q] : 0.0;
+      for (unsigned rows = e.x; rows; rows &= rows - 1) {
+        const int r = row0 + __ffs(rows) - 1;
+        double u[MASK_WORDS], sum = 0.0;
+#pragma unroll
+        for (int q = 0; q < MASK_WORDS; q++)
+          u[q] = lane + 32 * q < k ? A[static_cast<long long>(lane + 32 * q) * lda + r] : 0.0;
+#pragma unroll
+        for (int q = 0; q < MASK_WORDS; q++) sum = fma(u[q], v[q], sum);
+        for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(ALL, sum, o);
+        if (lane == 0) C[static_cast<long long>(col) * ldc + r] -= sum;
+      }
+      continue;
+    }
     const bool mine = row < m && ((e.x >> lane) & 1u);
     const uint4 a = ma[2 * row + 1], b = mb[2 * col + 1];  // (rows up to a whole tile are packed)
     const bool whole = __any_sync(ALL, mine && ea[row] == EXP_NONFINITE) || fb[col] == EXP_NONFINITE;
@@ -564,7 +611,6 @@ __global__ void __launch_bounds__(SUM_THREADS) sum_listed(const uint2* __restric
         __reduce_or_sync(ALL, mine ? a.x & b.x : 0u), __reduce_or_sync(ALL, mine ? a.y & b.y : 0u),
         __reduce_or_sync(ALL, mine ? a.z & b.z : 0u), __reduce_or_sync(ALL, mine ? a.w & b.w : 0u)};
     const double* pa = A + min(row, m - 1);
-    const double* pb = B + static_cast<long long>(col) * ldb;
     double sum = 0.0;
 #pragma unroll
     for (int h = 0; h < 2; h++) {
@@ -616,7 +662,7 @@ void f64_sliced_update(Context* ctx, int m, int n, int k, const double* A, long 
   cudaStream_t s = ctx->stream();
   const int kpad = (k + S_KC - 1) / S_KC * S_KC;
   const int mpad = (m + S_M - 1) / S_M * S_M, npad = (n + S_N - 1) / S_N * S_N;
-  // slices, then the masks and scales (rows of A, columns of B), then the row scaling of B and the list
+  // slices, then the masks and scales (rows of A, columns of B), then the statistics and the list
   const size_t abytes = static_cast<size_t>(S_SLICES) * mpad * kpad * 2, bbytes = static_cast<size_t>(S_SLICES) * npad * kpad * 2;
   char* wa = static_cast<char*>(ctx->workspace(Context::WS_TC_A, abytes + (2 * sizeof(uint4) + sizeof(int)) * mpad));
   // a place of the list for every 32 rows of every column
@@ -624,16 +670,16 @@ void f64_sliced_update(Context* ctx, int m, int n, int k, const double* A, long 
   if (places >> 32) throw KdError(KD_ERR_ARG, "sliced FP64 update: matrix too large");
   char* wb = static_cast<char*>(ctx->workspace(
       Context::WS_TC_B,
-      bbytes + (2 * sizeof(uint4) + sizeof(int)) * npad + sizeof(int) * (S_MAXK + 4) + sizeof(uint2) * places));
+      bbytes + (2 * sizeof(uint4) + sizeof(int)) * npad + sizeof(int) * STAT_INTS + sizeof(uint2) * places));
   auto* as = reinterpret_cast<__nv_bfloat16*>(wa);
   auto* bs = reinterpret_cast<__nv_bfloat16*>(wb);
   auto* ma = reinterpret_cast<uint4*>(wa + abytes);  // abytes and bbytes are multiples of 4,096
   auto* mb = reinterpret_cast<uint4*>(wb + bbytes);
   int* ea = reinterpret_cast<int*>(ma + 2 * mpad);
   int* fb = reinterpret_cast<int*>(mb + 2 * npad);
-  int* xk = fb + npad;
-  auto* listed = reinterpret_cast<unsigned*>(xk + S_MAXK);
-  auto* list = reinterpret_cast<uint2*>(xk + S_MAXK + 4);  // 16-byte aligned: npad is a multiple of 64
+  int* stat = fb + npad;
+  auto* listed = reinterpret_cast<unsigned*>(stat + 4 * S_MAXK);
+  auto* list = reinterpret_cast<uint2*>(stat + STAT_INTS);  // 16-byte aligned: npad is a multiple of 64
   bool fresh = false;
   int* err = static_cast<int*>(ctx->workspace(Context::WS_TC_FLAG, sizeof(int), &fresh));
   if (fresh) cuda_check(cudaMemsetAsync(err, 0, sizeof(int), s), "memset err");
@@ -643,11 +689,11 @@ void f64_sliced_update(Context* ctx, int m, int n, int k, const double* A, long 
                                     static_cast<int>(S_SMEM)),
                "cudaFuncSetAttribute(sliced update)");
   });
-  slice_fill<<<1, S_MAXK, 0, s>>>(xk, S_MAXK, EXP_ZERO);
-  const int cols = 32;
-  slice_row_exponents<<<(n + cols - 1) / cols, S_MAXK, 0, s>>>(B, ldb, k, n, cols, xk);
-  slice_pack_b<<<(npad + 7) / 8, 256, 0, s>>>(B, ldb, k, n, kpad, npad, xk, bs, fb, mb);
-  slice_pack_a<<<mpad / SA_ROWS, 256, 0, s>>>(A, lda, m, k, kpad, mpad, xk, as, ea, reinterpret_cast<unsigned*>(ma));
+  slice_clear<<<1, 256, 0, s>>>(stat);
+  const int nb = (n + STAT_COLS - 1) / STAT_COLS, na = (m + STAT_ROWS - 1) / STAT_ROWS * k;
+  slice_exponents<<<nb + na, STAT_THREADS, 0, s>>>(A, lda, m, B, ldb, k, n, nb, stat);
+  slice_pack_b<<<(npad + 7) / 8, 256, 0, s>>>(B, ldb, k, n, kpad, npad, stat, bs, fb, mb);
+  slice_pack_a<<<mpad / SA_ROWS, 256, 0, s>>>(A, lda, m, k, kpad, mpad, stat, as, ea, reinterpret_cast<unsigned*>(ma));
   CUtensorMap mA, mB;
   make_slice_map(&mA, as, kpad, mpad, S_M);
   make_slice_map(&mB, bs, kpad, npad, S_N);
