@@ -449,7 +449,8 @@ def run_exporter(args, ctx, wl, stream, local):
     points (radii up to 4x the outer shell, every domain including the
     compactified one) on the GPU: kd_fields_val_points_device, all unknown
     fields at once, points already resident in HBM.  Work per point and
-    field: 2 flops per coefficient of the domain holding the point."""
+    field: 2 flops per coefficient (the always-zero phi columns left out)
+    of the domain holding the point."""
     import numpy as np
     import torch
 
@@ -474,22 +475,23 @@ def run_exporter(args, ctx, wl, stream, local):
     ev1.record(stream)
     ev1.synchronize()
     ms = ev0.elapsed_time(ev1) / reps
-    # algorithmic flops: 2 per coefficient of the point's domain, per field
+    # algorithmic flops: 2 per coefficient of the point's domain, per field,
+    # without the phi columns of sin 0 and of the highest sine, which are zero
     space = wl.space
     radii = r.cpu().numpy()
     ncoef = []
     for d in range(space.get_nbr_domains()):
         info = space.domain_info(d)
         nc = info["nbr_coefs"]
-        ncoef.append(int(nc[0] * nc[1] * nc[2]))
+        ncoef.append(int(nc[0] * nc[1] * (nc[2] - 2)))
     edges = list(workloads_bounds(wl))
     dom_of = np.searchsorted(np.asarray(edges), radii, side="left")
     flops = 2.0 * len(fields) * float(np.sum(np.asarray(ncoef)[np.minimum(dom_of, len(ncoef) - 1)]))
     achieved = flops / (ms * 1e-3) / 1e12
     return {"points": n, "fields": len(fields), "ms": ms, "points_per_s": n / (ms * 1e-3),
-            "kernel": "pt_classify + pt_scatter + val_points_sorted_kernel", "achieved_tflops_fp64": achieved,
+            "kernel": "pt_count + pt_scatter + val_points_sorted_kernel", "achieved_tflops_fp64": achieved,
             "work": "2 flops per coefficient of the point's domain per field (spectral summation), "
-                    "the always-zero phi columns included, which the kernel skips"}
+                    "without the always-zero phi columns"}
 
 
 def workloads_bounds(wl):
@@ -560,7 +562,9 @@ def measure_fp64_peak(device):
 
 # The kernel behind each profile category of the mixed-precision step, and
 # the resource that bounds it.  `work` of every category but the transforms
-# is algorithmic bytes (include/kadath_gb300.h, kd_ctx_profile_read).
+# is algorithmic bytes (include/kadath_gb300.h, kd_ctx_profile_read).  Profile
+# mode times single launches: the value passes, which run collected into levels
+# otherwise, are launched operation by operation there.
 ROOF_KERNELS = {
     "lu_solve": ("trsv_group", "one triangular sweep over the FP32 factors (forward L or backward U)"),
     "lu_gemm": ("tf32_update_persistent", "3xTF32 tcgen05 trailing update"),
@@ -604,7 +608,8 @@ def roofline_for(cat, st, peaks, peak_kind, fp64_tflops=None):
         out.update({"bound": "fp64", "achieved": achieved, "peak": fp64_tflops, "unit": "TFLOP/s",
                     "frac": (achieved / fp64_tflops) if fp64_tflops else None, "traffic": None,
                     "work_per_launch": work_per_launch,
-                    "peak_note": "FP64 DGEMM throughput measured in this run; work = algorithmic FP64 flops"})
+                    "peak_note": "FP64 DGEMM throughput measured in this run; work = flops of the "
+                                 "dense products, the zeros that the kernels skip included"})
         return out
     achieved = work_per_launch / (per_launch_ms * 1e-3) / 1e9
     peak = peaks.get("hbm_gbs", PEAKS_FALLBACK["hbm_gbs"])

@@ -15,8 +15,9 @@ namespace kd {
 namespace {
 
 // Line passes.  Bound: the FP64 pipe (measured 1.10 TFLOP/s on the whole GPU:
-// an SM starts one FP64 warp instruction in 16 cycles, so index arithmetic and
-// shared-memory loads hide behind it).  Hence every pass runs as few FP64 warp
+// an SM starts one FP64 warp instruction in 16 cycles; it is busy 81 % of the time
+// on 2,580 fields of (13,9,4) and 88 % on 3,000 of (21,11,14), the rest is a
+// field's staging and its barriers).  Hence every pass runs as few FP64 warp
 // instructions as it can: zero entries of a matrix row are skipped (derivatives
 // are triangular with a parity, multiplications and divisions by sin and x are
 // banded or triangular, two phi rows are zero), lines whose output is zero are

@@ -44,10 +44,11 @@
 //            bits, TMEM released, then C -= its first 62 bits * 2^e (one
 //            conversion and one multiply-add on the FP64 pipe) beside the next
 //            tile's MMAs, and the list of the entries to sum in FP64.
-// Bound: the MMAs' operand reads from shared memory (48 cycles per MMA of 32)
-// and the hand-over of the single set of accumulators.  128 x 64 tiles and not
-// 128 x 128: eight orders of 64 columns are all of TMEM, and one pass over the
-// operands serves all of them.
+// Bound: the hand-over of the single set of accumulators and the latency of the
+// epilogue behind it, 25,000 cycles a tile of which the tensor pipe works 29 %, the
+// FP64 pipe 34 % and the issue slots 37 % (first update of N = 4,000).  128 x 64
+// tiles and not 128 x 128: eight orders of 64 columns are all of TMEM, and one pass
+// over the operands serves all of them.  (C prefetched into L2: 1 %.)
 // Sixteen epilogue warps: with eight, of 32 columns each, their integer work was
 // longer than a tile's MMAs (all updates at N = 8,000: 32 against 23 ms).
 // All updates of a factorisation, with packing and the listed entries, against the

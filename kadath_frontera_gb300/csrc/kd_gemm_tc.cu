@@ -348,13 +348,6 @@ __device__ __forceinline__ void p_tma_store_stream(const CUtensorMap* map, const
                : "memory");
 }
 
-__device__ __forceinline__ void p_tma_store(const CUtensorMap* map, const void* src, int x, int y) {
-  asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%2, %3}], [%1];" ::"l"(
-                   reinterpret_cast<uint64_t>(map)),
-               "r"(smem_u32(src)), "r"(x), "r"(y)
-               : "memory");
-}
-
 __device__ __forceinline__ void tf32_mma(uint32_t d, uint64_t ad, uint64_t bd, uint32_t idesc, uint32_t accum) {
   asm volatile(
       "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
@@ -644,8 +637,9 @@ int tf32_update_max_clusters16() {
   return maxc;
 }
 
-// When an update takes 256-column tiles: 3xTF32 with k above 128 and at least
-// two tiles an SM.  There the operands' way from L2 is the bound (85 KB a k-block
+// When an update takes 256-column tiles: 3xTF32 with k above 128, at least two
+// tiles an SM, and at least four tiles across, so that the padding of the last one
+// is at most a quarter of the work.  There the operands' way from L2 is the bound (85 KB a k-block
 // and 128 x 128 tile, C included, against 826 cycles of MMA), and the wider tile
 // needs a quarter less of them: all updates of 40,081 rows 294 -> 234 ms, the
 // factorisation of 12,331 rows in a reused order, whose updates run as clusters
@@ -655,6 +649,7 @@ int tf32_update_max_clusters16() {
 // stream is the bound and wants the longer ring.
 constexpr int WIDE_MIN_K = 128;
 constexpr int WIDE_MIN_WAVES = 2;
+constexpr int WIDE_MIN_N = 1024;
 
 void tf32_gemm_update(Context* ctx, int m, int n, int k, const float* A, long long lda, const float* B, long long ldb,
                       float* C, long long ldc, int c_rows_writable, int terms, int clusters, int max_ctas) {
@@ -698,7 +693,6 @@ void tf32_gemm_update(Context* ctx, int m, int n, int k, const float* A, long lo
     make_map(&mB, bt, kpad, npad, static_cast<long long>(kpad) * 4, TC_KBLK, TC_N, true);
     make_map(&mAl, at_lo, kpad, mpad, static_cast<long long>(kpad) * 4, TC_KBLK, TC_M, true);
     make_map(&mBl, bt_lo, kpad, npad, static_cast<long long>(kpad) * 4, TC_KBLK, TC_N, true);
-    
     static int nsm = 0;
     static std::once_flag pattr;
     std::call_once(pattr, [] {
@@ -712,7 +706,7 @@ void tf32_gemm_update(Context* ctx, int m, int n, int k, const float* A, long lo
     });
     const int ntm = mpad / TC_M;
     const int cap_sms = ctx->sms() < nsm ? ctx->sms() : nsm;
-    const bool wide = split3 && kpad > WIDE_MIN_K && n >= 1024 &&
+    const bool wide = split3 && kpad > WIDE_MIN_K && n >= WIDE_MIN_N &&
                       static_cast<long long>(ntm) * ((n + 255) / 256) >= WIDE_MIN_WAVES * cap_sms;
     const int tn = wide ? 256 : TC_N;
     const int ccols = p_ccols(tn), chunk_bytes = TC_M * ccols * 4;

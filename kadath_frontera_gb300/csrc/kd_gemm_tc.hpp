@@ -13,7 +13,7 @@ namespace kd {
 // scratch that the update may overwrite (the padding of a matrix whose
 // leading dimension is rounded up); pass m when there is none.
 // terms: 1 = plain TF32 products; 3 = 3xTF32 (hi*hi + hi*lo + lo*hi, about
-// FP32 accuracy), used where possible (k <= 96, TMA-aligned C).
+// FP32 accuracy), used where possible (k <= 192, TMA-aligned C).
 // clusters: 0 runs the persistent tensor-core update on the whole GPU;
 // 1 runs it as 16-CTA clusters, one cluster fewer than the GPU can hold, so
 // that a 16-CTA cluster kernel launched beside it (the next panel) always

@@ -1,13 +1,16 @@
 // Dense LU with partial pivoting (column-major) and triangular solves.
-// Blocked right-looking factorisation, per panel of jb <= 96 columns:
-//   panel    one cooperative kernel over the whole GPU, rows of the panel
-//            held in shared memory, one grid barrier per column;
+// Blocked right-looking factorisation, per panel of jb <= 96 columns (192 as two
+// halves where the update is better off with k = 192):
+//   panel    the rows of the panel held in shared memory, by one 16-CTA cluster
+//            (FP32), by a cooperative kernel over the whole GPU with one exchange
+//            a column, or, in a kept pivot order, without any search;
 //   swaps    the panel's row exchanges as one list of row moves, applied
 //            to the other columns by one warp per column;
 //   TRSM     U12 = L11^{-1} A12 with L11 staged in shared memory;
-//   update   A22 -= L21 U12 as a GEMM (FP64 library GEMM, or the TF32
-//            tensor-core kernel of kd_gemm_tc.cu for the mixed modes).
-// Solves use inverses of the 64 x 64 diagonal blocks (one launch per block).
+//   update   A22 -= L21 U12 on the tensor cores: 3xTF32 (kd_gemm_tc.cu) for the
+//            mixed modes, exact slices (kd_gemm_f64.cu) for FP64; the library's
+//            GEMM for small FP64 updates and the FP32 mode.
+// Solves are one launch a sweep, with inverses of the 64 x 64 diagonal blocks.
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
@@ -1290,11 +1293,6 @@ __device__ __forceinline__ unsigned long long globaltimer_ns() {
   return t;
 }
 
-template <class V>
-__device__ __forceinline__ bool better(V v, int i, V bv, int bi) {
-  return v > bv || (v == bv && i < bi);
-}
-
 // The modulus of v as an integer that orders the same way: 0 for NaN (never a
 // pivot), else its bits + 1.  Integer compares, because an FP64 compare costs
 // an FP64 instruction.
@@ -1332,18 +1330,10 @@ __device__ __forceinline__ void modulus_of(unsigned long long key, float& v) {
 }
 
 // Double-float arithmetic (a value is an unevaluated sum hi + lo of two
-// floats): Dekker's product with a fused multiply-add and Knuth's two-sum,
-// about 48 significant bits on the FP32 pipe.
+// floats): Knuth's two-sum, about 48 significant bits on the FP32 pipe.
 struct DF {
   float h, l;
 };
-__device__ __forceinline__ DF df_mul(float ah, float al, float bh, float bl) {
-  const float p = ah * bh;
-  float e = fmaf(ah, bh, -p);
-  e = fmaf(ah, bl, fmaf(al, bh, e));
-  const float s = p + e;
-  return {s, e - (s - p)};
-}
 __device__ __forceinline__ DF df_add(DF a, DF b) {
   const float s = a.h + b.h;
   const float v = s - a.h;
