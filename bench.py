@@ -449,8 +449,8 @@ def run_exporter(args, ctx, wl, stream, local):
     points (radii up to 4x the outer shell, every domain including the
     compactified one) on the GPU: kd_fields_val_points_device, all unknown
     fields at once, points already resident in HBM.  Work per point and
-    field: 2 flops per coefficient (the always-zero phi columns left out)
-    of the domain holding the point."""
+    field: 2 flops per coefficient (phi columns that are zero left out) of
+    the domain holding the point."""
     import numpy as np
     import torch
 
@@ -476,22 +476,23 @@ def run_exporter(args, ctx, wl, stream, local):
     ev1.synchronize()
     ms = ev0.elapsed_time(ev1) / reps
     # algorithmic flops: 2 per coefficient of the point's domain, per field,
-    # without the phi columns of sin 0 and of the highest sine, which are zero
+    # without the phi columns that hold nothing
     space = wl.space
     radii = r.cpu().numpy()
     ncoef = []
     for d in range(space.get_nbr_domains()):
         info = space.domain_info(d)
         nc = info["nbr_coefs"]
-        ncoef.append(int(nc[0] * nc[1] * (nc[2] - 2)))
+        live = sum(int(np.any(f.get_coef(d), axis=(0, 1)).sum()) for f in fields)
+        ncoef.append(int(nc[0] * nc[1]) * live)
     edges = list(workloads_bounds(wl))
     dom_of = np.searchsorted(np.asarray(edges), radii, side="left")
-    flops = 2.0 * len(fields) * float(np.sum(np.asarray(ncoef)[np.minimum(dom_of, len(ncoef) - 1)]))
+    flops = 2.0 * float(np.sum(np.asarray(ncoef)[np.minimum(dom_of, len(ncoef) - 1)]))
     achieved = flops / (ms * 1e-3) / 1e12
     return {"points": n, "fields": len(fields), "ms": ms, "points_per_s": n / (ms * 1e-3),
             "kernel": "pt_count + pt_scatter + val_points_sorted_kernel", "achieved_tflops_fp64": achieved,
             "work": "2 flops per coefficient of the point's domain per field (spectral summation), "
-                    "without the always-zero phi columns"}
+                    "without the phi columns that are zero"}
 
 
 def workloads_bounds(wl):
