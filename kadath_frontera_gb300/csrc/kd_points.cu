@@ -200,7 +200,7 @@ __device__ __forceinline__ PtPos pt_position(const PtDom& D, double x, double y,
     q.st = 0.0;
     q.cp = 1.0;
     q.sp = 0.0;
-  } else if (isinf(r)) {  // the angles of a point at infinity
+  } else if (isinf(r) || rho < 1e-140) {  // a point at infinity, or squares among the subnormals: angles first
     double th = (z != 0.0) ? atan(rho / z) : M_PI / 2;
     if (th < 0) th += M_PI;
     sincos(th, &q.st, &q.ct);
