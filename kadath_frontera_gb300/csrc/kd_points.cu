@@ -178,6 +178,11 @@ struct PtPos {
   double xi, ct, st, cp, sp;
 };
 
+// Whether every sine of phi is left out: at phi = 0, where all are exactly zero.
+// (Elsewhere Inf and NaN among the coefficients of a column reach the point even
+// where its factor happens to be zero.)
+__device__ __forceinline__ bool pt_no_sines(const PtPos& q) { return q.sp == 0.0 && q.cp > 0.0; }
+
 __device__ __forceinline__ int pt_locate(const PtArgs& a, const double* __restrict__ xyz, long long p, double& x,
                                          double& y, double& z, double& r) {
   x = xyz[3 * p] - a.cx;
@@ -331,6 +336,7 @@ __device__ __forceinline__ void pt_group(const PtArgs& a, int g, int dd, const P
   double val[NF];
 #pragma unroll
   for (int f = 0; f < NF; f++) val[f] = 0.0;
+  const bool no_sines = pt_no_sines(q);
   double cm = 1.0, sm = 0.0;  // cos(m phi), sin(m phi), m = k / 2 (COSSIN)
   for (int k = 0; k < D.nc2; k++) {
     const double phik = (k & 1) ? sm : cm;
@@ -339,7 +345,7 @@ __device__ __forceinline__ void pt_group(const PtArgs& a, int g, int dd, const P
       sm = sm * q.cp + cm * q.sp;
       cm = cn;
     }
-    if (k == 1 || !live[k]) continue;  // sin(0), or no coefficient
+    if (k == 1 || !live[k] || (no_sines && (k & 1))) continue;  // sin(0), or no coefficient
     const double* th = TH + a.slot[pt_theta_kind(__ldg(tb + k))] * D.nc1 * PT_THREADS;
     double acc[NF];
 #pragma unroll
@@ -437,8 +443,10 @@ __global__ void __launch_bounds__(PT_THREADS) val_points_few_kernel(const __grid
   double x, y, z, r;
   const int dd = p < npts ? pt_locate(a, xyz, p, x, y, z, r) : -1;
   const PtDom& D = a.d[dd < 0 ? 0 : dd];
+  bool no_sines = false;
   if (dd >= 0) {
     const PtPos q = pt_position(D, x, y, z, r);
+    no_sines = pt_no_sines(q);
     const int row = nt_max * PPB;
     if (sub == 0) pt_chebyshev(q.xi, D.ncheb, T, PPB);
     if (sub == 1) pt_theta(q, 0, D.nc1, TH, TH + 2 * row, PPB);
@@ -465,8 +473,8 @@ __global__ void __launch_bounds__(PT_THREADS) val_points_few_kernel(const __grid
       const int* tb = rb + lines;
       for (int l = sub; l < lines; l += PT_SUB) {
         const int k = l % D.nc2, j = l / D.nc2;
+        if (k == 1 || (no_sines && (k & 1))) continue;
         const double phik = PH[k * PPB];
-        if (phik == 0.0) continue;
         const int br = __ldg(rb + l);
         const double* t = T + (br == B_CHEB_ODD ? PPB : 0);
         const int ts = (br == B_CHEB ? 1 : 2) * PPB;
