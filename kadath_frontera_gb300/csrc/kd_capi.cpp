@@ -217,8 +217,10 @@ int kd_ope_1d(kd_ctx* ctx, int op, int dim, const kd_transform_desc* desc, int* 
     kd::Context& c = *ctx->c;
     kd::Base b = base_from_desc(*desc);
     kd::Base bo = b;
-    const kd::LinePlan& plan = kd::ope_1d_plan(c, op, dim, b, desc->nbr_coefs, bo);
-    if (desc->batch > 0) {
+    if (desc->batch == 0) {  // the bases alone, of fields of any size
+      kd::ope_1d_spec(c, op, dim, b, desc->nbr_coefs, bo);
+    } else {
+      const kd::LinePlan& plan = kd::ope_1d_plan(c, op, dim, b, desc->nbr_coefs, bo);
       auto it = kd::make_item(plan, desc->in, desc->out, desc->nbr_coefs, prod3(desc->nbr_coefs),
                               prod3(desc->nbr_coefs), 1.0);
       c.run_items({it}, {desc->batch});
