@@ -569,7 +569,7 @@ LpShape lp_default_shape(int total_fields, int stage) {
   LpShape sh;
   sh.threads = 256;
   if (total_fields <= 32)
-    sh.cluster = (total_fields > 8 || stage < 1024) ? 4 : 8;
+    sh.cluster = (total_fields > 12 || stage < 1024) ? 4 : 8;
   else if (total_fields <= 76 && stage >= 2048)
     sh.cluster = 4;
   return sh;

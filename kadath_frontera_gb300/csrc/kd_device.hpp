@@ -96,12 +96,13 @@ struct LpShape {
 };
 // The rule without a tuning table, from the fields of the launch and the
 // doubles of the largest item's stage.  Up to 32 fields are bound by latency:
-// clusters of 8 CTAs, or of 4 where the field is small or the clusters no
-// longer all get SMs of their own (us per launch with 8 / 4 CTAs: one (9,5,4)
-// field 6.2 / 6.2, 30 of them 10.2 / 6.2; one (21,11,14) field 18.4 / 24.6, 30
-// of them 26.6 / 24.6).  Beyond that one 256-thread CTA per field (150 fields
-// of (15,11,12): 26.6 against 42.4 with 128 threads and 39.5 with clusters of
-// 4), except that large fields that leave half of the SMs idle keep clusters
+// clusters of 8 CTAs, or of 4 where the field is small or there are too many
+// clusters for each of their CTAs to have an SM of its own (us per launch with
+// 8 / 4 CTAs: one (9,5,4) field 6.2 / 6.2, 30 of them 10.2 / 6.2; (21,11,14)
+// fields 20.7 / 26.9 up to 12 of them, 28.9 / 26.9 for 32; (33,17,16) 49.5 / 75.7
+// for 12, 94.5 / 76.0 for 16).  Beyond that one 256-thread CTA per field (150
+// fields of (15,11,12): 26.6 against 42.4 with 128 threads and 39.5 with clusters
+// of 4), except that large fields that leave half of the SMs idle keep clusters
 // of 4 (60 fields of (21,11,14): 34.0 against 43.0).
 LpShape lp_default_shape(int total_fields, int stage);
 
