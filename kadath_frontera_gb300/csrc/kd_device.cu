@@ -567,7 +567,7 @@ cudaError_t launch_ops(const KdOpRec* ops, int n, const double* d_pool, cudaStre
 
 LpShape lp_default_shape(int total_fields, int stage) {
   LpShape sh;
-  sh.threads = 256;
+  sh.threads = (total_fields > 4 * 152 && stage < 640) ? 128 : 256;
   if (total_fields <= 32)
     sh.cluster = (total_fields > 12 || stage < 1024) ? 4 : 8;
   else if (total_fields <= 76 && stage >= 2048)

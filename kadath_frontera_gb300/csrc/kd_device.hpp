@@ -103,7 +103,11 @@ struct LpShape {
 // for 12, 94.5 / 76.0 for 16).  Beyond that one 256-thread CTA per field (150
 // fields of (15,11,12): 26.6 against 42.4 with 128 threads and 39.5 with clusters
 // of 4), except that large fields that leave half of the SMs idle keep clusters
-// of 4 (60 fields of (21,11,14): 34.0 against 43.0).
+// of 4 (60 fields of (21,11,14): 34.0 against 43.0), and that small fields, whose
+// passes have fewer outputs than 256 threads, take 128 threads once there are more
+// than four of them an SM (3,600 fields: (5,5,4) 23.5 against 29.0, (9,5,4) 35.1
+// against 39.9, (11,7,4) 59.8 against 61.9, (13,9,4) 90.2 against 90.3; 300 of
+// (9,5,4) 10.5 against 9.7).
 LpShape lp_default_shape(int total_fields, int stage);
 
 // Runs the pass lists of all items with the given shape (default rule: the

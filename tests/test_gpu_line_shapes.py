@@ -42,7 +42,8 @@ def _time(fn, ctx):
 
 
 @pytest.mark.parametrize("shape,batch", [((33, 17, 16), 8), ((33, 17, 16), 9), ((33, 17, 16), 12), ((21, 11, 14), 12),
-                                         ((33, 17, 16), 16), ((13, 9, 4), 32), ((5, 5, 4), 300), ((13, 9, 4), 300)])
+                                         ((33, 17, 16), 16), ((13, 9, 4), 32), ((5, 5, 4), 300), ((5, 5, 4), 1200),
+                                         ((5, 5, 4), 3600), ((9, 5, 4), 3600), ((13, 9, 4), 300)])
 def test_rule(ctx, tmp_path, shape, batch):
     d, keep = _desc(shape, batch)
     table = tmp_path / "table.json"
