@@ -81,7 +81,9 @@ void regrid(Field& dst, Field& src) {
     LinePlan plan = plain_plan(specs, nco);
     for (int q = 0; q < plan.npass; q++) plan.pass[q].mat = ctx.table(specs[q].offsets);
     list.items[0] = make_item(plan, v.cf, pn.c, nco, dmo.ncoefs(), dmn.npts(), 1.0);
-    cuda_check(launch_line_passes(list, ctx.pool(), ctx.stream()), "regrid line passes");
+    LpShape shape;
+    shape.cluster = 8;
+    cuda_check(launch_line_passes(list, ctx.pool(), ctx.stream(), shape), "regrid line passes");
     ctx.launches++;
     cuda_check(cudaStreamSynchronize(ctx.stream()), "sync regrid");
     ctx.scratch().release_to(mark);
