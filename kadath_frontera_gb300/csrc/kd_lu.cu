@@ -3531,8 +3531,13 @@ void DenseLU::prepare_solves(const T* LU, long long ld, int N) {
                                       static_cast<int>(GI_SMEM)),
                  "cudaFuncSetAttribute(group inverses)");
     });
-    invert_groups<<<dim3(ng, 2), 256, GI_SMEM, ctx_->stream()>>>(LU, ld, N, dinv2_l_, dinv2_u_, group_x_l_, group_x_u_);
-    ctx_->launches++;
+    if (nblk > 1) {
+      invert_groups<<<dim3(ng, 2), 256, GI_SMEM, ctx_->stream()>>>(LU, ld, N, dinv2_l_, dinv2_u_, group_x_l_, group_x_u_);
+      ctx_->launches++;
+    } else {  // one block: nothing beside it
+      cuda_check(cudaMemsetAsync(group_x_l_, 0, gx * sizeof(float2), ctx_->stream()), "memset group inverses");
+      cuda_check(cudaMemsetAsync(group_x_u_, 0, gx * sizeof(float2), ctx_->stream()), "memset group inverses");
+    }
   }
   cuda_check(cudaGetLastError(), "solve preparation");
 }
